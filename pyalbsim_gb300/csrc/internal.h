@@ -22,15 +22,6 @@ constexpr int kJacParams = ALB_ADJ_PARAMS - 1;
 long long launches_total();
 void note_launch();
 
-// Uniform key grid over a bounding box; axes with no extent carry no key bits.
-struct KeyGrid {
-    double lo[3];
-    double scale[3];
-    double maxq[3];
-    int ax[3];
-    int naxes;
-};
-
 // Unsorted records of one channel as appended by the forward tracer.
 // The two halves of a record are interleaved in one allocation owned by `a`: record r is
 // a[2 r] = (x, y, z, energy) and b[2 r] = a[2 r + 1] = (dx, dy, dz, time), so a record is one
@@ -132,7 +123,6 @@ class Workspace {
 };
 
 // ---- map build (mapbuild.cu)
-KeyGrid make_key_grid(const float lo[3], const float hi[3], int bits3, int bits2);
 int compute_bbox(Workspace& ws, const float4* a, uint64_t n, float lo[3], float hi[3], cudaStream_t st,
                  uint64_t stride = 1);
 int build_map_index(Workspace& ws, const RecordStore& rec, uint64_t n, MapIndex& m, cudaStream_t st);
