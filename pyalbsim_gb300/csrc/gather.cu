@@ -16,6 +16,7 @@
 // query's k neighbours (k points lie within it, so it bounds the k-th distance; never looser
 // than the triangle bound r_k(prev) + |q - prev|), inflated by 2^-14 so that every point of
 // the float32 boundary band is still admitted.
+#include <algorithm>
 #include <cfloat>
 
 #include "device_common.cuh"
@@ -25,11 +26,13 @@ namespace alb {
 
 constexpr int kGatherWarps = 8;   // 8-warp CTAs, 4 per SM: 32 warps hide the gather's latency
 constexpr int kGatherBlocksPerSM = 4;
-// consecutive sorted queries handled by one warp: each chunk's first search runs without a
-// bound, longer chunks balance worse (scatter map at 1e7 photons: 32 -> 546 ms, 64 -> 529 ms,
-// 128 -> 524 ms; the planar maps' gathers lose 2-3% at 128)
+// At most this many consecutive sorted queries are handled by one warp: each chunk's first
+// search runs without a bound, longer chunks balance worse (scatter map at 1e7 photons: 32 ->
+// 546 ms, 64 -> 529 ms, 128 -> 524 ms; the planar maps' gathers lose 2-3% at 128). Fewer
+// queries than fill the resident warps with such chunks take shorter ones (query_chunk).
 constexpr int kQueryChunk = 64;
 constexpr int kQueryChunkScatter = 128;
+constexpr int kQueryChunkMin = 2;
 constexpr int kStack = 32 * kMaxLevels;
 constexpr int kCap = 288;         // candidate buffer (k <= kCap - 32)
 constexpr int kSelectAt = 192;    // shrink the buffer once it holds more than this
@@ -970,7 +973,7 @@ constexpr int kModeKnn = 0, kModeKnnAdjoint = 1, kModeRadius = 2, kModeKnnHeat =
 
 template <int CHANNEL, int MODE>
 __global__ void __launch_bounds__(kGatherWarps * 32, kGatherBlocksPerSM) k_gather(SceneDev sc, MapDev m, QueryDev q, Accum acc, int k,
-                                                              int* err) {
+                                                              int* err, uint32_t kChunk) {
     __shared__ WarpSmem smem[kGatherWarps];
     __shared__ BinCache bc;
     for (int i = threadIdx.x; i < kBinCache; i += blockDim.x) {
@@ -982,7 +985,6 @@ __global__ void __launch_bounds__(kGatherWarps * 32, kGatherBlocksPerSM) k_gathe
     const int w = threadIdx.x >> 5, l = lane_id();
     WarpSmem& s = smem[w];
     const uint64_t warps = (uint64_t)gridDim.x * kGatherWarps;
-    constexpr int kChunk = CHANNEL == ALB_SCATTER ? kQueryChunkScatter : kQueryChunk;
     const uint64_t chunks = (q.n + kChunk - 1) / kChunk;
     bool failed = false;
     // search counters accumulate in the warp's shared memory, not in registers held through
@@ -1222,30 +1224,51 @@ __global__ void __launch_bounds__(kGatherWarps * 32) k_knn(MapDev m, const doubl
     }
 }
 
-static unsigned gather_blocks(uint64_t nq) {
+static int sm_count() {
     int dev = 0, sms = 148;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    return sms;
+}
+
+static unsigned gather_blocks(uint64_t nq) {
     uint64_t want = (nq + kGatherWarps - 1) / kGatherWarps;
-    uint64_t cap = (uint64_t)sms * 16;
+    uint64_t cap = (uint64_t)sm_count() * 16;
     return (unsigned)(want < cap ? (want ? want : 1) : cap);
+}
+
+// Consecutive queries per warp: as many as the resident warps need to take every query in one
+// wave, within [kQueryChunkMin, kQueryChunk or kQueryChunkScatter]. With 64 whatever the count,
+// 25 000 queries ran on 391 of the 4864 resident warps and took as long as 250 000 (bottom
+// gather 1.67 ms; with chunks of 6, 0.24 ms); 5000 queries take 0.07 ms at a floor of 2, 0.12
+// at 4, 0.21 at 8. The fixed-radius gather carries nothing from query to query and its visits
+// differ by four orders of magnitude between neighbouring queries: one query at a time (surface
+// gather of 25 000 queries at 0.5 m: 22.3 -> 13.1 ms).
+static uint32_t query_chunk(int channel, uint64_t nq, bool radius) {
+    if (radius) return 1;
+    const uint64_t most = channel == ALB_SCATTER ? kQueryChunkScatter : kQueryChunk;
+    const uint64_t warps = (uint64_t)sm_count() * kGatherBlocksPerSM * kGatherWarps;
+    const uint64_t fit = (nq + warps - 1) / warps;
+    return (uint32_t)std::min<uint64_t>(most, std::max<uint64_t>(fit, kQueryChunkMin));
 }
 
 template <int MODE>
 static void launch_gather_mode(const MapDev& map, const QueryDev& q, int channel, const SceneDev& sc, const Accum& acc,
-                               int* err, unsigned blocks, int k, cudaStream_t st) {
+                               int* err, uint64_t nq, int k, cudaStream_t st) {
+    const uint32_t chunk = query_chunk(channel, nq, MODE == kModeRadius);
+    const unsigned blocks = gather_blocks((nq + chunk - 1) / chunk);
     switch (channel) {
         case ALB_BOTTOM_REFLECTION:
-            k_gather<ALB_BOTTOM_REFLECTION, MODE><<<blocks, kGatherWarps * 32, 0, st>>>(sc, map, q, acc, k, err);
+            k_gather<ALB_BOTTOM_REFLECTION, MODE><<<blocks, kGatherWarps * 32, 0, st>>>(sc, map, q, acc, k, err, chunk);
             break;
         case ALB_SCATTER:
-            k_gather<ALB_SCATTER, MODE><<<blocks, kGatherWarps * 32, 0, st>>>(sc, map, q, acc, k, err);
+            k_gather<ALB_SCATTER, MODE><<<blocks, kGatherWarps * 32, 0, st>>>(sc, map, q, acc, k, err, chunk);
             break;
         case ALB_SURFACE_REFLECTION:
-            k_gather<ALB_SURFACE_REFLECTION, MODE><<<blocks, kGatherWarps * 32, 0, st>>>(sc, map, q, acc, k, err);
+            k_gather<ALB_SURFACE_REFLECTION, MODE><<<blocks, kGatherWarps * 32, 0, st>>>(sc, map, q, acc, k, err, chunk);
             break;
         default:
-            k_gather<ALB_SURFACE_TRANSMISSION_UP, MODE><<<blocks, kGatherWarps * 32, 0, st>>>(sc, map, q, acc, k, err);
+            k_gather<ALB_SURFACE_TRANSMISSION_UP, MODE><<<blocks, kGatherWarps * 32, 0, st>>>(sc, map, q, acc, k, err, chunk);
             break;
     }
     note_launch();
@@ -1254,12 +1277,11 @@ static void launch_gather_mode(const MapDev& map, const QueryDev& q, int channel
 void launch_gather(const SceneDev& sc, const MapDev& map, const QueryDev& q, int channel, const Accum& acc,
                    int* err, int* launches, cudaStream_t st) {
     if (q.n == 0) return;
-    unsigned blocks = gather_blocks(q.n);
     int k = sc.k;
-    if (sc.radius > 0.0) launch_gather_mode<kModeRadius>(map, q, channel, sc, acc, err, blocks, k, st);
-    else if (acc.jac_lo) launch_gather_mode<kModeKnnAdjoint>(map, q, channel, sc, acc, err, blocks, k, st);
-    else if (acc.hw_lo && map.fwi) launch_gather_mode<kModeKnnHeat>(map, q, channel, sc, acc, err, blocks, k, st);
-    else launch_gather_mode<kModeKnn>(map, q, channel, sc, acc, err, blocks, k, st);
+    if (sc.radius > 0.0) launch_gather_mode<kModeRadius>(map, q, channel, sc, acc, err, q.n, k, st);
+    else if (acc.jac_lo) launch_gather_mode<kModeKnnAdjoint>(map, q, channel, sc, acc, err, q.n, k, st);
+    else if (acc.hw_lo && map.fwi) launch_gather_mode<kModeKnnHeat>(map, q, channel, sc, acc, err, q.n, k, st);
+    else launch_gather_mode<kModeKnn>(map, q, channel, sc, acc, err, q.n, k, st);
     if (launches) ++*launches;
 }
 

@@ -1,0 +1,37 @@
+"""The gather's result does not depend on how its queries are ordered or cut into chunks: the
+waveform is a sum in fixed point over exact neighbour sets. Query counts around the edges of the
+chunk rule (one query, a few, one per resident warp) and of the key width (2^18), each against the
+unsorted order, bit for bit."""
+
+import dataclasses
+
+import numpy as np
+import pytest
+
+from pyalbsim_gb300 import workloads
+from pyalbsim_gb300.config.gpu import GpuRunOptions
+from pyalbsim_gb300.engine import GpuEngine
+
+pytestmark = pytest.mark.gpu
+
+
+def _waveform(cfg, n_backward, sort):
+    with GpuEngine(cfg, GpuRunOptions(sort_queries=sort)) as eng:
+        eng.forward(20_000, 5)
+        eng.build_maps()
+        eng.backward(n_backward, 5)
+        return eng.waveform_array(f64=True)
+
+
+@pytest.mark.parametrize("n_backward", [1, 3, 2_433, 70_001])
+@pytest.mark.parametrize("k", [1, 100])
+def test_waveform_does_not_depend_on_the_query_order(gpu_available, n_backward, k):
+    cfg = dataclasses.replace(workloads.small(), photon_mapping_k=k)
+    a, b = _waveform(cfg, n_backward, True), _waveform(cfg, n_backward, False)
+    assert np.abs(a).sum() > 0
+    np.testing.assert_array_equal(a, b)
+
+
+def test_radius_waveform_does_not_depend_on_the_query_order(gpu_available):
+    cfg = workloads.small(0.9, radius=0.2)
+    np.testing.assert_array_equal(_waveform(cfg, 2_000, True), _waveform(cfg, 2_000, False))
