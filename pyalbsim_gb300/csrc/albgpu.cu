@@ -281,6 +281,8 @@ static std::string set_scene(AlbCtx* ctx, const AlbSceneParams* p) {
     s.floor_albedo = p->seafloor_albedo;
     s.floor_albedo32 = (float)p->seafloor_albedo;
     s.surface_albedo = p->surface_albedo;
+    s.floor_lambert = (float)(p->seafloor_albedo / kPi);
+    s.surface_lambert = (float)(p->surface_albedo / kPi);
     s.roughness = p->roughness;
     double ga = p->roughness * p->roughness;
     s.ggx_a2 = (float)(ga * ga);
@@ -849,6 +851,7 @@ extern "C" int alb_trace(AlbCtx* ctx, int pass, uint64_t n, uint64_t seed, uint6
             q.a = ctx->qa[k];
             q.b = ctx->qb[k];
             q.c = ctx->qc[k];
+            q.lo_zero = !ctx->precise && !rp;
             q.s = ctx->sc.adjoint ? ctx->qs[k] : nullptr;
             q.n = nq;
             q.rk_out = ctx->keep_ids ? ctx->qrk[k][g == 3 ? 1 : 0] : nullptr;

@@ -34,6 +34,7 @@ struct SceneDev {
     double radius;            // extension: fixed gather radius (m), 0 = k nearest
     double slope_sigma;       // extension: Gaussian surface-slope std (0 = flat surface)
     float floor_albedo32;
+    float floor_lambert, surface_lambert;  // albedo / pi
     float ggx_a2;             // (roughness^2)^2 as used by the GGX distribution
     double rot_d[9];          // float32 laser rotation, widened
     double div, fov, cos_fov, aperture, pulse_sigma32, eff_rate32;

@@ -11,12 +11,14 @@
 // survives, and the boundary band is resolved with float64 distances exactly as the
 // reference's KDTree (float64 on float32-cast map positions) orders them.
 //
-// Each warp takes contiguous chunks of the spatially sorted queries; from the second query
-// of a chunk on, the search starts with the largest distance from the query to the previous
+// Planar maps: each warp takes contiguous chunks of the spatially sorted queries; from the second
+// query of a chunk on, the search starts with the largest distance from the query to the previous
 // query's k neighbours (k points lie within it, so it bounds the k-th distance; never looser
 // than the triangle bound r_k(prev) + |q - prev|), inflated by 2^-14 so that every point of
-// the float32 boundary band is still admitted.
+// the float32 boundary band is still admitted. The scatter map's queries go in runs that share
+// one walk of the tree (gather_group.cuh).
 #include <algorithm>
+#include <atomic>
 #include <cfloat>
 
 #include "device_common.cuh"
@@ -37,12 +39,6 @@ constexpr int kStack = 32 * kMaxLevels;
 constexpr int kCap = 288;         // candidate buffer (k <= kCap - 32)
 constexpr int kSelectAt = 192;    // shrink the buffer once it holds more than this
 constexpr int kBand = 32;         // near-tie entries resolved in float64
-constexpr int kLeafList = 2 * kBand;  // leaf list of a search under a guess (aliases the band)
-// Squared widening of the previous query's k-th distance that the scatter-map search first
-// admits within (1.1^2): consecutive sorted queries' k-th distances differ by less than 10%
-// for 97% of them; a guess that does not hold is detected and the search redone (measured
-// at 1e7 photons: 1.1^2 gave the fastest scatter gather of 1.1^2, 1.15^2 and 1.2^2).
-constexpr float kGuessWiden2 = 1.21f;
 // Admission margin of the float32 screening distance (its error is below 2^-22 relative).
 constexpr float kRelMargin = 9.5367431640625e-07f;  // 2^-20
 
@@ -51,20 +47,19 @@ constexpr float kRelMargin = 9.5367431640625e-07f;  // 2^-20
 // them to ~2^-40 relative); only entries within one key unit of the k-th are resolved in
 // float64.
 struct WarpSmem {
+    static constexpr int kCap = alb::kCap, kSelectAt = alb::kSelectAt, kTmp = 2 * kStack;
     uint32_t stk[kStack];
     float stk_d[kStack];
     float cd[kCap];
     uint32_t ci[kCap];
     int16_t cl[kCap];
     uint32_t hist[128];  // 256 radix bins, two 16-bit counters per word
-    union {
-        double bd[kBand];               // near-tie band: float64 distances (after the search)
-        uint32_t leafl[kLeafList];      // leaves to screen (during a search under a guess)
-    };
+    double bd[kBand];    // near-tie band: float64 distances
     uint32_t bi[kBand];  // map positions
     uint64_t bt[kBand];  // tie keys from the record's content (or 0)
-    float prev_rk2;      // squared k-th distance of the warp's previous query (kept out of registers)
     unsigned long long st[5];  // the warp's search counters: leaves, nodes, selects, queries, inexact
+    // scratch words of the boundary band (the stack is free after the search)
+    ALB_DEVICE uint32_t& tmp(int i) { return i < kStack ? stk[i] : reinterpret_cast<uint32_t*>(stk_d)[i - kStack]; }
 };
 
 // Lower bound of the squared distance from the float64 query (qx + lx, ...) to a box:
@@ -136,7 +131,8 @@ ALB_DEVICE int16_t frac16(float hi, float lo) {
     return (int16_t)q;
 }
 
-ALB_DEVICE uint64_t cand_key(const WarpSmem& s, int i) {
+template <class S>
+ALB_DEVICE uint64_t cand_key(const S& s, int i) {
     return ((uint64_t)__float_as_uint(s.cd[i]) << 16) | (uint32_t)((int)s.cl[i] + 32768);
 }
 
@@ -196,7 +192,8 @@ ALB_DEVICE void warp_sort32(float& key, uint32_t& val) {
 
 // Shared radix-select step: from the 256-bin histogram in s.hist (two 16-bit counters per
 // word) pick the digit holding the need-th (1-based) entry; need becomes its rank inside.
-ALB_DEVICE uint32_t radix_pick(const WarpSmem& s, int& need) {
+template <class S>
+ALB_DEVICE uint32_t radix_pick(const S& s, int& need) {
     const int l = lane_id();
     uint32_t h[8], run = 0;
 #pragma unroll
@@ -231,7 +228,8 @@ ALB_DEVICE uint32_t radix_pick(const WarpSmem& s, int& need) {
 }
 
 // k-th smallest (1-based) float32 part cd[off .. off + cnt) (all >= 0): warp radix select.
-ALB_DEVICE float warp_kth32(WarpSmem& s, int off, int cnt, int k) {
+template <class S>
+ALB_DEVICE float warp_kth32(S& s, int off, int cnt, int k) {
     const int l = lane_id();
     uint32_t prefix = 0u, pmask = 0u;
     int need = k;
@@ -261,7 +259,8 @@ ALB_DEVICE float warp_kth32(WarpSmem& s, int off, int cnt, int k) {
 // clamped, which is monotone in d, so the bins keep the order), then an exact rank among the
 // entries of the bin that holds the k-th (usually one to three). Falls back to the four-pass
 // radix select when hi gives no spread or that bin holds more than 32 entries.
-ALB_DEVICE float warp_kth32_lin(WarpSmem& s, int cnt, int k, float hi) {
+template <class S>
+ALB_DEVICE float warp_kth32_lin(S& s, int cnt, int k, float hi) {
     const float scale = 256.f / hi;
     if (!(hi > 0.f) || !(scale < 1.0e30f)) return warp_kth32(s, 0, cnt, k);
     const int l = lane_id();
@@ -307,8 +306,8 @@ ALB_DEVICE float warp_kth32_lin(WarpSmem& s, int cnt, int k, float hi) {
 
 // k-th smallest (1-based) 48-bit candidate key by warp radix select over its top
 // 8 * PASSES bits (PASSES = 4: the float32 part only; the lower bits return as 0).
-template <int PASSES>
-ALB_DEVICE uint64_t warp_kth_key(WarpSmem& s, int off, int cnt, int k) {
+template <int PASSES, class S>
+ALB_DEVICE uint64_t warp_kth_key(S& s, int off, int cnt, int k) {
     const int l = lane_id();
     uint64_t prefix = 0ull, pmask = 0ull;
     int need = k;
@@ -333,7 +332,8 @@ ALB_DEVICE uint64_t warp_kth_key(WarpSmem& s, int off, int cnt, int k) {
 }
 
 // Keep the candidates whose float32 part is <= thr (order not preserved).
-ALB_DEVICE int warp_compact(WarpSmem& s, int cnt, float thr) {
+template <class S>
+ALB_DEVICE int warp_compact(S& s, int cnt, float thr) {
     const int l = lane_id();
     int out = 0;
 #pragma unroll 1
@@ -365,7 +365,6 @@ struct KnnResult {
     int nodes;     // internal nodes expanded
     int selects;   // candidate-buffer reductions
     int clipped;   // 1 if a buffer bound forced an inexact answer (mass ties)
-    int retried;   // 1 if an optimistic first threshold did not hold and the search was redone
     int fail;      // 0, or why the search has no answer (s.ci is then not valid):
                    // ALB_ERR_ITER_CAP (traversal guard) or ALB_ERR_INVALID (fewer than k
                    // finite points admitted: a NaN or infinite query or map coordinates)
@@ -374,7 +373,8 @@ struct KnnResult {
 // float64 ranking of the band entries bi[0..nb) by (distance, tie key, map position); the
 // `take` smallest go to ci[dst ..] in rank order. Returns the float64 squared distance of
 // the take-th (0 if the band holds fewer).
-ALB_DEVICE double rank_band(const MapDev& m, WarpSmem& s, int dst, int nb, int take, double qx, double qy,
+template <class S>
+ALB_DEVICE double rank_band(const MapDev& m, S& s, int dst, int nb, int take, double qx, double qy,
                             double qz, const float4* tie_rec) {
     const int l = lane_id();
     double di = 0.0;
@@ -409,7 +409,8 @@ ALB_DEVICE double rank_band(const MapDev& m, WarpSmem& s, int dst, int nb, int t
 // The k_sub nearest among the entries [off, off + n) whose cd/cl hold refined keys: keys more
 // than one unit below the k_sub-th are in, keys within one unit of it are ranked in float64.
 // The chosen map positions end up in ci[off .. off + k_sub).
-ALB_DEVICE double select_refined(const MapDev& m, WarpSmem& s, int off, int n, int k_sub, double qx, double qy,
+template <class S>
+ALB_DEVICE double select_refined(const MapDev& m, S& s, int off, int n, int k_sub, double qx, double qy,
                                  double qz, const float4* tie_rec, int& clipped) {
     const int l = lane_id();
     const uint64_t K = warp_kth_key<6>(s, off, n, k_sub);
@@ -443,14 +444,9 @@ ALB_DEVICE double select_refined(const MapDev& m, WarpSmem& s, int off, int n, i
 
 // Full k-NN search for one query. Returns false when the map has fewer than k records; the
 // k nearest map positions are then in s.ci[0 .. k).
-// thr_safe: an upper bound of the squared k-th distance that already includes the band margin
-// (FLT_MAX when none is known). thr0 <= thr_safe: the first search's threshold, which may be
-// an optimistic guess. A search under a guess is accepted only when its own answer proves it
-// complete: at least k candidates, and the k-th with its band margin within the guess (every
-// point that can rank among the k nearest then had a distance below the admission
-// threshold, and every box holding one was opened). Otherwise the search is repeated under
-// thr_safe, and under no bound at all if that fails too. Either way the answer is the one a
-// search from no bound gives.
+// bound: an upper bound of the squared k-th distance that already includes the band margin
+// (FLT_MAX when none is known). A search that admits fewer than k points under it is repeated
+// without one, so the answer is always the one a search from no bound gives.
 // The query is (fx + lx, fy + ly, fz + lz) = (qx, qy, qz) exactly, |l*| <= half an ulp of f*.
 // Points at exactly the same float64 distance rank by a key taken from their record content
 // (time, then a hash of direction, time and energy; when tie_rec is given) and then by map
@@ -460,26 +456,20 @@ ALB_DEVICE double select_refined(const MapDev& m, WarpSmem& s, int off, int n, i
 // holds entries within one float32 ulp of the k-th: needed where many points sit at nearly
 // the same distance (queries far from a dense planar map). Without it candidates carry the
 // float32 screening distance and only a crowded final band is refined.
-template <bool REFINE, bool QSPLIT = false>
-ALB_DEVICE bool warp_knn(const MapDev& m, WarpSmem& s, int k, double qx, double qy, double qz, float fx,
-                         float fy, float fz, float lx, float ly, float lz, float thr0, float thr_safe,
-                         const float4* tie_rec, KnnResult& res) {
+template <bool REFINE, bool QSPLIT = false, class S>
+ALB_DEVICE bool warp_knn(const MapDev& m, S& s, int k, double qx, double qy, double qz, float fx,
+                         float fy, float fz, float lx, float ly, float lz, float bound, const float4* tie_rec,
+                         KnnResult& res) {
     const int l = lane_id();
     if (m.n_real < (uint64_t)k) return false;
-    float thr = thr0;  // admission threshold (float32 squared distance, with margin)
+    float thr = bound;  // admission threshold (float32 squared distance, with margin)
     int cnt = 0;
-    float kth_known = -1.f;  // the float32 k-th of the accepted search (!REFINE), when computed
-    res.leaves = res.nodes = res.selects = res.clipped = res.retried = res.fail = 0;
-    // Thresholds in turn: the first guess, the safe bound, no bound. A carried safe bound can
-    // only fail through a degenerate previous result (a clipped boundary band).
-    float start = thr0;
-    for (int attempt = 0; attempt < 3; ++attempt) {
+    res.leaves = res.nodes = res.selects = res.clipped = res.fail = 0;
+    // The carried bound first, then none: a bound can only fail through a degenerate previous
+    // result (a clipped boundary band).
+    float start = bound;
+    for (int attempt = 0; attempt < 2; ++attempt) {
         if (attempt == 1) {
-            if (!(thr_safe > thr0)) continue;  // the guess was the safe bound itself
-            start = thr_safe;
-            res.retried = 1;
-        }
-        if (attempt == 2) {
             if (start == FLT_MAX) break;
             start = FLT_MAX;
         }
@@ -507,14 +497,6 @@ ALB_DEVICE bool warp_knn(const MapDev& m, WarpSmem& s, int k, double qx, double 
             __syncwarp();
         }
         int guard = 0;
-        // Under a guessed threshold the threshold rarely shrinks, so the order of the boxes
-        // does not change which leaves are opened: the leaves of expanded leaf parents are
-        // collected in s.leafl and screened in batches, with the next leaf's records loaded
-        // while the current leaf is screened, so the leaf visits do not form one chain of
-        // dependent loads. The ordered search (a safe bound, or none) takes its leaves from
-        // the stack, nearest first.
-        const bool listed = !REFINE && start < thr_safe;
-        int nlist = 0;
         // screen the 32 records of leaf `leaf` (p = this lane's record) against the threshold
         auto admit = [&](uint32_t leaf, float4 p) {
             ++res.leaves;
@@ -537,7 +519,7 @@ ALB_DEVICE bool warp_knn(const MapDev& m, WarpSmem& s, int k, double qx, double 
             }
             cnt += __popc(b);
             __syncwarp();
-            if (cnt >= k && (thr == FLT_MAX || cnt > kSelectAt)) {
+            if (cnt >= k && (thr == FLT_MAX || cnt > S::kSelectAt)) {
                 ++res.selects;
                 // planar maps (REFINE) crowd their candidates into one linear bin: radix select
                 const float kth = REFINE ? warp_kth32(s, 0, cnt, k) : warp_kth32_lin(s, cnt, k, thr);
@@ -546,21 +528,16 @@ ALB_DEVICE bool warp_knn(const MapDev& m, WarpSmem& s, int k, double qx, double 
                 // rank among the k nearest, nothing beyond can; otherwise the float32
                 // screening margin decides
                 cnt = warp_compact(s, cnt, REFINE ? __uint_as_float(__float_as_uint(kth) + 1u) : thr);
-                if (cnt > kCap - 32) {  // mass ties
+                if (cnt > S::kCap - 32) {  // mass ties
                     cnt = warp_compact(s, cnt, kth);
                     res.clipped = 1;
                 }
-                if (cnt > kCap - 32) cnt = kCap - 32;  // keeps the buffer in bounds
+                if (cnt > S::kCap - 32) cnt = S::kCap - 32;  // keeps the buffer in bounds
             }
         };
         auto load_leaf = [&](uint32_t leaf) {
             const uint64_t r = (uint64_t)leaf * 32 + l;
             return r < m.n ? m.a[r] : make_float4(0.f, 0.f, 0.f, 0.f);
-        };
-        auto flush = [&]() {
-#pragma unroll 1
-            for (int i = 0; i < nlist; ++i) admit(s.leafl[i], load_leaf(s.leafl[i]));
-            nlist = 0;
         };
         while (sp > 0) {
             if (++guard > (1 << 22)) {  // reported, never a silent partial answer
@@ -589,7 +566,7 @@ ALB_DEVICE bool warp_knn(const MapDev& m, WarpSmem& s, int k, double qx, double 
                 __syncwarp();
             }
             if ((etop >> 29) == 0) {
-                // a leaf of the ordered search: admit its points within the threshold
+                // a leaf: admit its points within the threshold
                 admit(etop, load_leaf(etop));
             } else {
                 ++res.nodes;
@@ -605,23 +582,7 @@ ALB_DEVICE bool warp_knn(const MapDev& m, WarpSmem& s, int k, double qx, double 
                 uint32_t cc = (uint32_t)c;
                 const unsigned vm = __ballot_sync(0xffffffffu, d < FLT_MAX);
                 int nv = __popc(vm);
-                if (listed) {
-                    // children are taken as they come, without ordering them; leaves go to
-                    // the list
-                    if (d < FLT_MAX) {
-                        const int pos = __popc(vm & lanemask_lt());
-                        if (cl == 0) {
-                            s.leafl[nlist + pos] = cc;
-                        } else {
-                            s.stk[sp + pos] = ((uint32_t)cl << 29) | cc;
-                            s.stk_d[sp + pos] = d;
-                        }
-                    }
-                    if (cl == 0) {
-                        nlist += nv;
-                        nv = 0;
-                    }
-                } else if (nv <= 16) {
+                if (nv <= 16) {
                     // few children within the threshold: extract them nearest first
                     // (non-negative floats order like their bit patterns)
                     unsigned key = __float_as_uint(d);
@@ -643,20 +604,9 @@ ALB_DEVICE bool warp_knn(const MapDev& m, WarpSmem& s, int k, double qx, double 
                 }
                 sp += nv;
                 __syncwarp();
-                if (nlist > kLeafList - 32) flush();  // room for the next parent's 32 leaves
             }
         }
-        if (!res.fail) flush();
-        if (res.fail || start == FLT_MAX) break;
-        if (cnt < k) continue;
-        if (REFINE || start >= thr_safe) break;
-        // a guess: accepted when the k-th with its band margin lies within it
-        ++res.selects;
-        const float kth = warp_kth32_lin(s, cnt, k, start);
-        if (kth * (1.0f + 2.0f * kRelMargin) <= start) {
-            kth_known = kth;
-            break;
-        }
+        if (res.fail || start == FLT_MAX || cnt >= k) break;
     }
     if (!res.fail && cnt < k) res.fail = ALB_ERR_INVALID;
     if (res.fail) return true;
@@ -673,7 +623,7 @@ ALB_DEVICE bool warp_knn(const MapDev& m, WarpSmem& s, int k, double qx, double 
     } else {
         // float32 k-th; entries clearly below it are in, the band within the screening
         // margin around it is resolved exactly (refined keys when it is crowded)
-        const float kth = kth_known >= 0.f ? kth_known : warp_kth32(s, 0, cnt, k);
+        const float kth = warp_kth32(s, 0, cnt, k);
         const float blo = kth * (1.0f - 2.0f * kRelMargin), bhi = kth * (1.0f + 2.0f * kRelMargin);
         int n_in = 0, n_band = 0;
 #pragma unroll 1
@@ -690,25 +640,22 @@ ALB_DEVICE bool warp_knn(const MapDev& m, WarpSmem& s, int k, double qx, double 
             if (in) s.ci[n_in + __popc(bin & lanemask_lt())] = id;
             if (band) {
                 const int pos = n_band + __popc(bb & lanemask_lt());
-                if (pos < kStack) s.stk[pos] = id;  // the stack is free after the search
+                if (pos < S::kTmp) s.tmp(pos) = id;
             }
             n_in += __popc(bin);
             n_band += __popc(bb);
             __syncwarp();
         }
-        if (n_band > kStack) {
-            n_band = kStack;
-            res.clipped = 1;
-        }
+        static_assert(S::kCap <= S::kTmp, "the band is a subset of the candidates");
         const int take = k - n_in;
         if (n_band <= kBand) {
-            if (l < n_band) s.bi[l] = s.stk[l];
+            if (l < n_band) s.bi[l] = s.tmp(l);
             __syncwarp();
             rk2 = rank_band(m, s, n_in, n_band, take, qx, qy, qz, tie_rec);
         } else {
 #pragma unroll 1
             for (int j = l; j < n_band; j += 32) {
-                const uint32_t id = s.stk[j];
+                const uint32_t id = s.tmp(j);
                 float hi, lo;
                 point_dist2_df(fx, fy, fz, lx, ly, lz, m.a[id], hi, lo);
                 s.cd[n_in + j] = hi;
@@ -723,6 +670,10 @@ ALB_DEVICE bool warp_knn(const MapDev& m, WarpSmem& s, int k, double qx, double 
     res.rkf = sqrt_to_f32(rk2);
     return true;
 }
+
+}  // namespace alb
+#include "gather_group.cuh"
+namespace alb {
 
 // ----------------------------------------------------------------------------------------
 // per-neighbour weights (float32 restatement of the reference's energy multipliers)
@@ -855,6 +806,19 @@ ALB_DEVICE void bin_add(BinCache& bc, const Accum& acc, int channel, int bin, co
     }
 }
 
+// The CTA's cached bins into the global waveform (after a block barrier).
+template <int CHANNEL>
+ALB_DEVICE void bin_flush(const BinCache& bc, const Accum& acc) {
+    for (int i = threadIdx.x; i < kBinCache; i += blockDim.x) {
+        int t = bc.tag[i];
+        if (t >= 0) {
+            uint64_t o = (uint64_t)CHANNEL * acc.nbins + t;
+            Fix128 f{bc.lo[i], (long long)bc.hi[i]};
+            fix_atomic_add(acc.wf_lo + o, acc.wf_hi + o, f);
+        }
+    }
+}
+
 // Extension (no counterpart in the reference): every record within the fixed radius R of
 // the query, visited in any order. Screening as in the k-NN search; points within the
 // float32 error band of R are decided on their float64 distance. visit(record) runs on the
@@ -971,6 +935,80 @@ ALB_DEVICE void heat_add(const SceneDev& sc, const MapDev& m, const Accum& acc, 
 // and fetch.
 constexpr int kModeKnn = 0, kModeKnnAdjoint = 1, kModeRadius = 2, kModeKnnHeat = 3;
 
+// The energy of candidate j, where the search kept it.
+template <class S>
+ALB_DEVICE auto neighbour_energy(const S& s, int j) -> decltype(s.ce[0] + 0.f) { return s.ce[j]; }
+ALB_DEVICE float neighbour_energy(const WarpSmem&, int) { return 0.f; }
+
+// One query's k neighbours s.ci[0 .. k) into the waveform (and Jacobian, heatmaps): Es, qb, qy the
+// query's energy, direction and time, and float64 depth; rk the k-th distance. CE: the search
+// left the neighbours' energies in s.ce.
+template <int CHANNEL, int MODE, bool CE, class S>
+ALB_DEVICE void accumulate(const SceneDev& sc, const MapDev& m, const QueryDev& q, const Accum& acc, BinCache& bc, int* err,
+                           S& s, int k, uint64_t src, float Es, float4 qb, double qy, float rk) {
+    const int l = lane_id();
+    const float ts = qb.w;
+    float norm;
+    if (CHANNEL == ALB_SCATTER) norm = 1.0f / ((4.0f / 3.0f) * 3.14159265358979f * rk * rk * rk);
+    else norm = 1.0f / (3.14159265358979f * rk * rk);
+    // query-constant pieces
+    float vinv = rsqrtf(fmaf(qb.x, qb.x, fmaf(qb.y, qb.y, qb.z * qb.z)));
+    float vx = -qb.x * vinv, vy = -qb.y * vinv, vz = -qb.z * vinv;  // normalize(-d_query)
+    float wconst = 0.f;
+    if (CHANNEL == ALB_BOTTOM_REFLECTION) wconst = sc.floor_lambert * fmaxf(0.f, -qb.y);
+    if (CHANNEL == ALB_SURFACE_TRANSMISSION_UP) wconst = sc.surface_lambert;
+    // WaterModel.scatter_energy picks the layer of the query depth (water.py:418-447)
+    const int layer = (CHANNEL == ALB_SCATTER && sc.n_layers > 1) ? layer_of(sc, qy) : 0;
+    float4 sq = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (MODE == kModeKnnAdjoint && q.s) sq = q.s[src];
+    // the next neighbour's record is loaded while this one is weighted
+    uint32_t idx_n = l < k ? s.ci[l] : 0u;
+    float4 pb_n = make_float4(0.f, 0.f, 0.f, 0.f);
+    float e_n = 0.f;
+    if (l < k) {
+        pb_n = m.b[idx_n];
+        e_n = CE ? neighbour_energy(s, l) : m.a[idx_n].w;
+    }
+#pragma unroll 1
+    for (int j = l; j < k; j += 32) {
+        const uint32_t idx = idx_n;
+        const float4 pb = pb_n;
+        const float Ep = e_n;
+        if (j + 32 < k) {
+            idx_n = s.ci[j + 32];
+            pb_n = m.b[idx_n];
+            e_n = CE ? neighbour_energy(s, j + 32) : m.a[idx_n].w;
+        }
+        float w;
+        if (CHANNEL == ALB_BOTTOM_REFLECTION || CHANNEL == ALB_SURFACE_TRANSMISSION_UP) w = wconst;
+        else if (CHANNEL == ALB_SCATTER) w = scatter_weight(sc, layer, pb.x, pb.y, pb.z, vx, vy, vz);
+        else w = ggx_weight(sc.ggx_a2, (float)sc.f0, -pb.x, -pb.y, -pb.z, vx, vy, vz);
+        const float c = ((Es * Ep) * norm) * w;
+        const int bin = (int)((ts + pb.w) / (float)sc.mult) - (int)sc.gate_lo;
+        if (bin >= 0 && bin < acc.nbins) {
+            bin_add(bc, acc, CHANNEL, bin, f32_to_fix(c));
+            if (MODE == kModeKnnAdjoint && acc.jac_lo)
+                jac_add<CHANNEL>(sc, m, acc, layer, bin, idx, c, sq, pb, vx, vy, vz);
+        } else if (!sc.gated) {
+            atomicCAS(err, 0, ALB_ERR_CAPACITY);
+        }
+    }
+    if (MODE != kModeKnn && acc.hw_lo && m.fwi) {
+        // accumulate_to_heatmap, alb_sim/math/accumulate_heatmap.py:6-61 (a separate,
+        // non-unrolled pass: heatmaps are off in production runs)
+#pragma unroll 1
+        for (int j = l; j < k; j += 32) {
+            const uint32_t idx = s.ci[j];
+            const float4 pb = m.b[idx];
+            float w;
+            if (CHANNEL == ALB_BOTTOM_REFLECTION || CHANNEL == ALB_SURFACE_TRANSMISSION_UP) w = wconst;
+            else if (CHANNEL == ALB_SCATTER) w = scatter_weight(sc, layer, pb.x, pb.y, pb.z, vx, vy, vz);
+            else w = ggx_weight(sc.ggx_a2, (float)sc.f0, -pb.x, -pb.y, -pb.z, vx, vy, vz);
+            heat_add(sc, m, acc, idx, ((Es * m.a[idx].w) * norm) * w);
+        }
+    }
+}
+
 template <int CHANNEL, int MODE>
 __global__ void __launch_bounds__(kGatherWarps * 32, kGatherBlocksPerSM) k_gather(SceneDev sc, MapDev m, QueryDev q, Accum acc, int k,
                                                               int* err, uint32_t kChunk) {
@@ -1010,8 +1048,8 @@ __global__ void __launch_bounds__(kGatherWarps * 32, kGatherBlocksPerSM) k_gathe
                 const float vinv = rsqrtf(fmaf(qb.x, qb.x, fmaf(qb.y, qb.y, qb.z * qb.z)));
                 const float vx = -qb.x * vinv, vy = -qb.y * vinv, vz = -qb.z * vinv;
                 float wconst = 0.f;
-                if (CHANNEL == ALB_BOTTOM_REFLECTION) wconst = (float)(sc.floor_albedo / kPi) * fmaxf(0.f, -qb.y);
-                if (CHANNEL == ALB_SURFACE_TRANSMISSION_UP) wconst = (float)(sc.surface_albedo / kPi);
+                if (CHANNEL == ALB_BOTTOM_REFLECTION) wconst = sc.floor_lambert * fmaxf(0.f, -qb.y);
+                if (CHANNEL == ALB_SURFACE_TRANSMISSION_UP) wconst = sc.surface_lambert;
                 const int layer = (CHANNEL == ALB_SCATTER) ? layer_of(sc, qy) : 0;
                 const float4 sq = q.s ? q.s[src] : make_float4(0.f, 0.f, 0.f, 0.f);
                 warp_radius_visit(m, s, qx, qy, qz, qa.x, qa.y, qa.z, qc.x, qc.y, qc.z, sc.radius,
@@ -1047,7 +1085,8 @@ __global__ void __launch_bounds__(kGatherWarps * 32, kGatherBlocksPerSM) k_gathe
                 __syncwarp();
                 continue;
             }
-            float thr_safe = FLT_MAX, thr0 = FLT_MAX;
+            // k points lie within the farthest of the previous query's neighbours
+            float bound = FLT_MAX;
             if (have_prev) {
                 // the float32 screening error (below 2^-21) is far inside the 2^-14 inflation
                 unsigned mx = 0u;
@@ -1060,18 +1099,10 @@ __global__ void __launch_bounds__(kGatherWarps * 32, kGatherBlocksPerSM) k_gathe
                     mx = max(mx, __float_as_uint(d));  // non-negative floats order like their bits
                 }
                 const float t = __uint_as_float(__reduce_max_sync(0xffffffffu, mx)) * (1.f + 1.f / 16384.f);
-                if (t < 1.0e37f) thr_safe = t;
-                // The safe bound is the farthest of the previous query's neighbours, about
-                // twice the k-th distance here (the sorted queries are about one k-th
-                // distance apart): eight times the ball. Consecutive k-th distances differ by
-                // less than 20% for 99.7% of the scatter map's sorted queries, so the first
-                // search uses (1.2 r_prev)^2 and is redone under the safe bound when that
-                // does not hold. Planar maps keep the safe bound.
-                thr0 = (CHANNEL == ALB_SCATTER) ? fminf(thr_safe, s.prev_rk2 * kGuessWiden2) : thr_safe;
+                if (t < 1.0e37f) bound = t;
             }
             KnnResult r;
-            if (!warp_knn<CHANNEL != ALB_SCATTER, true>(m, s, k, 0.0, 0.0, 0.0, qa.x, qa.y, qa.z, qc.x, qc.y, qc.z,
-                                                         thr0, thr_safe, m.b, r)) {
+            if (!warp_knn<true, true>(m, s, k, 0.0, 0.0, 0.0, qa.x, qa.y, qa.z, qc.x, qc.y, qc.z, bound, m.b, r)) {
                 if (l == 0) atomicCAS(err, 0, ALB_ERR_TOO_FEW);
                 failed = true;
                 break;
@@ -1085,7 +1116,6 @@ __global__ void __launch_bounds__(kGatherWarps * 32, kGatherBlocksPerSM) k_gathe
             const float4 qb = q.b[src];
             const double qy = (double)qa.y + (double)qc.y;
             have_prev = true;
-            if (l == 0) s.prev_rk2 = (float)r.rk2;  // read after the next query's __syncwarp
             if (q.rk_out && l == 0) q.rk_out[src] = sqrt(r.rk2);
             if (l == 0) {
                 s.st[0] += r.leaves;
@@ -1094,68 +1124,7 @@ __global__ void __launch_bounds__(kGatherWarps * 32, kGatherBlocksPerSM) k_gathe
                 s.st[3] += 1;
                 s.st[4] += r.clipped;
             }
-            if (r.retried && l == 0 && q.retries) atomicAdd(q.retries, 1ull);  // rare: no register kept
-            const float Es = qa.w, ts = qb.w;
-            const float rk = r.rkf;
-            float norm;
-            if (CHANNEL == ALB_SCATTER) norm = 1.0f / ((4.0f / 3.0f) * 3.14159265358979f * rk * rk * rk);
-            else norm = 1.0f / (3.14159265358979f * rk * rk);
-            // query-constant pieces
-            float vinv = rsqrtf(fmaf(qb.x, qb.x, fmaf(qb.y, qb.y, qb.z * qb.z)));
-            float vx = -qb.x * vinv, vy = -qb.y * vinv, vz = -qb.z * vinv;  // normalize(-d_query)
-            float wconst = 0.f;
-            if (CHANNEL == ALB_BOTTOM_REFLECTION) wconst = (float)(sc.floor_albedo / kPi) * fmaxf(0.f, -qb.y);
-            if (CHANNEL == ALB_SURFACE_TRANSMISSION_UP) wconst = (float)(sc.surface_albedo / kPi);
-            // WaterModel.scatter_energy picks the layer of the query depth (water.py:418-447)
-            const int layer = (CHANNEL == ALB_SCATTER) ? layer_of(sc, qy) : 0;
-            float4 sq = make_float4(0.f, 0.f, 0.f, 0.f);
-            if (MODE == kModeKnnAdjoint && q.s) sq = q.s[src];
-            // the next neighbour's record is loaded while this one is weighted
-            uint32_t idx_n = l < k ? s.ci[l] : 0u;
-            float4 pb_n = make_float4(0.f, 0.f, 0.f, 0.f);
-            float e_n = 0.f;
-            if (l < k) {
-                pb_n = m.b[idx_n];
-                e_n = m.a[idx_n].w;
-            }
-#pragma unroll 1
-            for (int j = l; j < k; j += 32) {
-                const uint32_t idx = idx_n;
-                const float4 pb = pb_n;
-                const float Ep = e_n;
-                if (j + 32 < k) {
-                    idx_n = s.ci[j + 32];
-                    pb_n = m.b[idx_n];
-                    e_n = m.a[idx_n].w;
-                }
-                float w;
-                if (CHANNEL == ALB_BOTTOM_REFLECTION || CHANNEL == ALB_SURFACE_TRANSMISSION_UP) w = wconst;
-                else if (CHANNEL == ALB_SCATTER) w = scatter_weight(sc, layer, pb.x, pb.y, pb.z, vx, vy, vz);
-                else w = ggx_weight(sc.ggx_a2, (float)sc.f0, -pb.x, -pb.y, -pb.z, vx, vy, vz);
-                const float c = ((Es * Ep) * norm) * w;
-                const int bin = (int)((ts + pb.w) / (float)sc.mult) - (int)sc.gate_lo;
-                if (bin >= 0 && bin < acc.nbins) {
-                    bin_add(bc, acc, CHANNEL, bin, f32_to_fix(c));
-                    if (MODE == kModeKnnAdjoint && acc.jac_lo)
-                        jac_add<CHANNEL>(sc, m, acc, layer, bin, idx, c, sq, pb, vx, vy, vz);
-                } else if (!sc.gated) {
-                    atomicCAS(err, 0, ALB_ERR_CAPACITY);
-                }
-            }
-            if (MODE != kModeKnn && acc.hw_lo && m.fwi) {
-                // accumulate_to_heatmap, alb_sim/math/accumulate_heatmap.py:6-61 (a separate,
-                // non-unrolled pass: heatmaps are off in production runs)
-#pragma unroll 1
-                for (int j = l; j < k; j += 32) {
-                    const uint32_t idx = s.ci[j];
-                    const float4 pb = m.b[idx];
-                    float w;
-                    if (CHANNEL == ALB_BOTTOM_REFLECTION || CHANNEL == ALB_SURFACE_TRANSMISSION_UP) w = wconst;
-                    else if (CHANNEL == ALB_SCATTER) w = scatter_weight(sc, layer, pb.x, pb.y, pb.z, vx, vy, vz);
-                    else w = ggx_weight(sc.ggx_a2, (float)sc.f0, -pb.x, -pb.y, -pb.z, vx, vy, vz);
-                    heat_add(sc, m, acc, idx, ((Es * m.a[idx].w) * norm) * w);
-                }
-            }
+            accumulate<CHANNEL, MODE, false>(sc, m, q, acc, bc, err, s, k, src, qa.w, qb, qy, r.rkf);
             __syncwarp();
         }
     }
@@ -1169,14 +1138,145 @@ __global__ void __launch_bounds__(kGatherWarps * 32, kGatherBlocksPerSM) k_gathe
         if (q.inexact && s.st[4]) atomicAdd(q.inexact, s.st[4]);
     }
     __syncthreads();
+    bin_flush<CHANNEL>(bc, acc);
+}
+
+// The search of one query alone, out of line: the grouped kernel takes it for the first query of
+// a chunk, runs whose list does not fit, guesses that fail and near ties, 1-3% of the queries,
+// and its code and registers stay out of the hot loop.
+template <class S>
+__device__ __noinline__ bool cold_knn(const MapDev& m, S& s, int k, float fx, float fy, float fz, float lx, float ly,
+                                      float lz, float bound, KnnResult& res) {
+    if (!warp_knn<false, true>(m, s, k, 0.0, 0.0, 0.0, fx, fy, fz, lx, ly, lz, bound, m.b, res)) return false;
+    if (!res.fail) {
+        for (int j = lane_id(); j < k; j += 32) s.ce[j] = m.a[s.ci[j]].w;
+        __syncwarp();
+    }
+    return true;
+}
+
+// Scatter-map gather, k nearest, by runs of neighbouring queries (gather_group.cuh).
+template <int MODE, int CAP, int BLOCKS>
+__global__ void __launch_bounds__(kGatherWarps * 32, BLOCKS)
+    k_gather_scatter(const __grid_constant__ SceneDev sc, const __grid_constant__ MapDev m,
+                     const __grid_constant__ QueryDev q, const __grid_constant__ Accum acc, int k, int* err, uint32_t chunk) {
+    extern __shared__ __align__(16) unsigned char group_raw[];
+    using S = GroupSmem<CAP>;
+    S* smem = reinterpret_cast<S*>(group_raw);
+    BinCache& bc = *reinterpret_cast<BinCache*>(group_raw + kGatherWarps * sizeof(S));
     for (int i = threadIdx.x; i < kBinCache; i += blockDim.x) {
-        int t = bc.tag[i];
-        if (t >= 0) {
-            uint64_t o = (uint64_t)CHANNEL * acc.nbins + t;
-            Fix128 f{bc.lo[i], (long long)bc.hi[i]};
-            fix_atomic_add(acc.wf_lo + o, acc.wf_hi + o, f);
+        bc.tag[i] = -1;
+        bc.lo[i] = 0ull;
+        bc.hi[i] = 0ull;
+    }
+    __syncthreads();
+    const int w = threadIdx.x >> 5, l = lane_id();
+    S& s = smem[w];
+    const uint64_t warps = (uint64_t)gridDim.x * kGatherWarps;
+    const uint64_t chunks = (q.n + chunk - 1) / chunk;
+    // edge of a cubic leaf over the k-th distance: 32 records against k in the ball
+    const float side_rk = cbrtf(134.04f / (float)k);
+    bool failed = false;
+    if (l < 5) s.st[l] = 0ull;
+    __syncwarp();
+    for (uint64_t ch = (uint64_t)blockIdx.x * kGatherWarps + w; ch < chunks && !failed; ch += warps) {
+        const uint64_t q_end = min((ch + 1) * chunk, q.n);
+        QueryRun run{0, 0, 0.f};
+        uint64_t r_base = 0;  // first query of the run the lanes hold
+        uint32_t gsrc = 0u;   // this lane's query of the run: index and position
+        float gx = 0.f, gy = 0.f, gz = 0.f;
+        float prev2 = -1.f;   // squared k-th distance of the previous query
+        for (uint64_t qi = ch * chunk; qi < q_end; ++qi) {
+            const float guess = prev2 * kGroupGuess2;
+            bool listed = prev2 > 0.f;
+            if (qi >= r_base + run.take || !(guess <= run.T2)) {
+                // a new run starts here
+                const int avail = (int)min(q_end - qi, (uint64_t)32);
+                r_base = qi;
+                float la = 0.f;
+                if (l < avail) {
+                    gsrc = q.perm ? q.perm[qi + l] : (uint32_t)(qi + l);
+                    const float4 a = q.a[gsrc];
+                    gx = a.x; gy = a.y; gz = a.z;
+                    if (!q.lo_zero) {
+                        const float4 c = q.c[gsrc];
+                        la = fmaxf(fabsf(c.x), fmaxf(fabsf(c.y), fabsf(c.z)));
+                    }
+                }
+                run.take = 1;
+                run.n = 0;
+                if (listed) listed = build_run(m, s, avail, gx, gy, gz, la, prev2, side_rk * sqrtf(prev2), run);
+                if (!listed) run.take = 1;
+            }
+            const int at = (int)(qi - r_base);
+            const uint32_t src = __shfl_sync(0xffffffffu, gsrc, at);
+            const float fx = __shfl_sync(0xffffffffu, gx, at), fy = __shfl_sync(0xffffffffu, gy, at),
+                        fz = __shfl_sync(0xffffffffu, gz, at);
+            float lx = 0.f, ly = 0.f, lz = 0.f;
+            if (!q.lo_zero) {
+                const float4 c = q.c[src];
+                lx = c.x; ly = c.y; lz = c.z;
+            }
+            float rk, d2;
+            int got = 0, leaves = 0;
+            float kth = 0.f;
+            uint32_t kid = 0u;
+            if (listed) {
+                got = run_search(m, s, k, run.n, fx, fy, fz, lx, ly, lz, guess, kth, kid, leaves);
+                if (got == 0) {
+                    if (l == 0 && q.retries) atomicAdd(q.retries, 1ull);
+                    got = run_search(m, s, k, run.n, fx, fy, fz, lx, ly, lz, run.T2, kth, kid, leaves);
+                }
+            }
+            if (got == 1) {
+                rk = dist_f32(fx, fy, fz, lx, ly, lz, m.a[kid], d2);
+                if (q.rk_out && l == 0)
+                    q.rk_out[src] = sqrt(point_dist2_f64((double)fx + (double)lx, (double)fy + (double)ly,
+                                                         (double)fz + (double)lz, m.a[kid]));
+                if (l == 0) {
+                    s.st[0] += leaves;
+                    s.st[2] += 1;
+                    s.st[3] += 1;
+                }
+            } else {
+                // a proven k-th distance bounds the search; the run's boxes share its scratch
+                const float bound = got < 0 && kth > 0.f ? kth * (1.f + 1.f / 16384.f) : FLT_MAX;
+                run.take = 0;
+                KnnResult r;
+                const bool enough = cold_knn(m, s, k, fx, fy, fz, lx, ly, lz, bound, r);
+                if (!enough || r.fail) {  // no valid neighbour set: report it and stop this warp's work
+                    if (l == 0) atomicCAS(err, 0, enough ? r.fail : ALB_ERR_TOO_FEW);
+                    failed = true;
+                    break;
+                }
+                rk = r.rkf;
+                d2 = (float)r.rk2;
+                if (q.rk_out && l == 0) q.rk_out[src] = sqrt(r.rk2);
+                if (l == 0) {
+                    s.st[0] += r.leaves;
+                    s.st[1] += r.nodes;
+                    s.st[2] += r.selects;
+                    s.st[3] += 1;
+                    s.st[4] += r.clipped;
+                }
+            }
+            prev2 = d2;
+            const float4 qb = q.b[src];
+            accumulate<ALB_SCATTER, MODE, true>(sc, m, q, acc, bc, err, s, k, src, q.a[src].w, qb, (double)fy + (double)ly, rk);
+            __syncwarp();
         }
     }
+    if (l == 0) {
+        if (q.stats && s.st[3]) {
+            atomicAdd(q.stats + 0, s.st[0]);
+            atomicAdd(q.stats + 1, s.st[1]);
+            atomicAdd(q.stats + 2, s.st[2]);
+            atomicAdd(q.stats + 3, s.st[3]);
+        }
+        if (q.inexact && s.st[4]) atomicAdd(q.inexact, s.st[4]);
+    }
+    __syncthreads();
+    bin_flush<ALB_SCATTER>(bc, acc);
 }
 
 // Standalone KDTree.query(x, k): sorted indices and float64 distances.
@@ -1192,7 +1292,7 @@ __global__ void __launch_bounds__(kGatherWarps * 32) k_knn(MapDev m, const doubl
         const float fx = (float)qx, fy = (float)qy, fz = (float)qz;
         int why = 0;
         if (!warp_knn<true>(m, s, k, qx, qy, qz, fx, fy, fz, (float)(qx - (double)fx), (float)(qy - (double)fy),
-                            (float)(qz - (double)fz), FLT_MAX, FLT_MAX, nullptr, r))
+                            (float)(qz - (double)fz), FLT_MAX, nullptr, r))
             why = ALB_ERR_TOO_FEW;
         else if (r.fail)
             why = r.fail;
@@ -1252,6 +1352,21 @@ static uint32_t query_chunk(int channel, uint64_t nq, bool radius) {
     return (uint32_t)std::min<uint64_t>(most, std::max<uint64_t>(fit, kQueryChunkMin));
 }
 
+template <int MODE, int CAP, int BLOCKS>
+static void launch_scatter(const SceneDev& sc, const MapDev& map, const QueryDev& q, const Accum& acc, int k, int* err,
+                           unsigned blocks, uint32_t chunk, cudaStream_t st) {
+    constexpr int bytes = kGatherWarps * (int)sizeof(GroupSmem<CAP>) + (int)sizeof(BinCache);
+    auto kernel = k_gather_scatter<MODE, CAP, BLOCKS>;
+    static std::atomic<bool> attr_set[64];  // per device; batched runs launch from several host threads
+    int dev = 0;
+    cudaGetDevice(&dev);
+    if (dev < 0 || dev >= 64 || !attr_set[dev].load(std::memory_order_acquire)) {
+        cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+        if (dev >= 0 && dev < 64) attr_set[dev].store(true, std::memory_order_release);
+    }
+    kernel<<<blocks, kGatherWarps * 32, bytes, st>>>(sc, map, q, acc, k, err, chunk);
+}
+
 template <int MODE>
 static void launch_gather_mode(const MapDev& map, const QueryDev& q, int channel, const SceneDev& sc, const Accum& acc,
                                int* err, uint64_t nq, int k, cudaStream_t st) {
@@ -1262,7 +1377,13 @@ static void launch_gather_mode(const MapDev& map, const QueryDev& q, int channel
             k_gather<ALB_BOTTOM_REFLECTION, MODE><<<blocks, kGatherWarps * 32, 0, st>>>(sc, map, q, acc, k, err, chunk);
             break;
         case ALB_SCATTER:
-            k_gather<ALB_SCATTER, MODE><<<blocks, kGatherWarps * 32, 0, st>>>(sc, map, q, acc, k, err, chunk);
+            if constexpr (MODE == kModeRadius) {
+                k_gather<ALB_SCATTER, MODE><<<blocks, kGatherWarps * 32, 0, st>>>(sc, map, q, acc, k, err, chunk);
+            } else if (k <= 128) {
+                launch_scatter<MODE, 224, 4>(sc, map, q, acc, k, err, blocks, chunk, st);
+            } else {
+                launch_scatter<MODE, 448, 3>(sc, map, q, acc, k, err, blocks, chunk, st);
+            }
             break;
         case ALB_SURFACE_REFLECTION:
             k_gather<ALB_SURFACE_REFLECTION, MODE><<<blocks, kGatherWarps * 32, 0, st>>>(sc, map, q, acc, k, err, chunk);

@@ -76,6 +76,7 @@ struct QueryDev {
     const float4* a;   // x_hi, y_hi, z_hi, energy
     const float4* b;   // dx, dy, dz, time
     const float4* c;   // x_lo, y_lo, z_lo
+    bool lo_zero;      // every low part is zero (the float32 tracer's queries)
     const float4* s;   // adjoint path scores (a, b, g, albedo), nullable
     const uint32_t* perm;  // optional processing order
     uint64_t n;

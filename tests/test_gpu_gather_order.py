@@ -35,3 +35,26 @@ def test_waveform_does_not_depend_on_the_query_order(gpu_available, n_backward, 
 def test_radius_waveform_does_not_depend_on_the_query_order(gpu_available):
     cfg = workloads.small(0.9, radius=0.2)
     np.testing.assert_array_equal(_waveform(cfg, 2_000, True), _waveform(cfg, 2_000, False))
+
+
+@pytest.mark.parametrize("precise", [False, True])
+@pytest.mark.parametrize("k", [1, 31, 100, 128, 129, 256])
+def test_scatter_search_finds_the_kth_distance(gpu_available, k, precise):
+    """The scatter search on both sides of its candidate-buffer sizes (k = 128 / 129) and with
+    queries of one and two floats per coordinate: the k-th distances against scipy's KDTree. Both
+    are float64 distances between the same points; they differ by the rounding of three
+    products and two sums, under 4 eps."""
+    from scipy.spatial import cKDTree
+
+    cfg = dataclasses.replace(workloads.small(), photon_mapping_k=k)
+    for n_backward in (2, 700):
+        with GpuEngine(cfg, GpuRunOptions(precise=precise)) as eng:
+            eng.keep_record_ids()
+            eng.forward(20_000, 7)
+            eng.build_maps()
+            eng.backward(n_backward, 7)
+            q = eng.ctx.export_queries(1)
+            pts = eng.ctx.export_map(1)[0]
+        d = cKDTree(pts.astype(np.float64)).query(q["pos"], k=[k])[0][:, 0]
+        assert len(d) > 0
+        np.testing.assert_allclose(q["rk"], d, rtol=4 * np.finfo(np.float64).eps, atol=0)
