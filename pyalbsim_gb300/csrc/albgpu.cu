@@ -123,6 +123,9 @@ struct AlbCtx {
     unsigned* hm_radius = nullptr;
     // adjoint Jacobian: lo words then hi words, [2][kJacParams][channels][nbins]
     unsigned long long* jac = nullptr;
+    // sums of one gather by exponent class (every gather leaves them zero)
+    unsigned long long *cls = nullptr, *jac_cls = nullptr, *heat_cls = nullptr;
+    int64_t cls_bins = 0, jac_cls_bins = 0, heat_cls_cells = 0;
     int64_t wf_bins = 0, jac_bins = 0, hm_cells = 0, hm_radius_cells = 0;  // accumulator capacities
     // per-layer scene tables (device), reused when the context takes a new scene
     struct LayerTables {
@@ -271,6 +274,8 @@ static std::string set_scene(AlbCtx* ctx, const AlbSceneParams* p) {
         }
     }
     s.mult = p->sample_multiplier;
+    s.mult32 = (float)p->sample_multiplier;
+    s.mult32_inv = 1.0f / s.mult32;
     s.k = p->k;
     s.ys = p->surface_y;
     s.yf = p->floor_y;
@@ -310,6 +315,16 @@ static std::string set_scene(AlbCtx* ctx, const AlbSceneParams* p) {
         s.wc[i] = p->water_center[i];
         s.fc[i] = p->floor_center[i];
     }
+    for (int i = 0; i < 2; ++i) {
+        const float w = (float)s.wc[2 * i], f = (float)s.fc[2 * i];
+        s.hm_wc32[i] = make_float2(w, (float)(s.wc[2 * i] - (double)w));
+        s.hm_fc32[i] = make_float2(f, (float)(s.fc[2 * i] - (double)f));
+    }
+    s.hm_wext32 = (float)s.hm_wext;
+    s.hm_fext32 = (float)s.hm_fext;
+    const bool small_map = s.hm_bins > 0 && s.hm_bins <= 512;
+    s.hm_winv = small_map && s.hm_wbin > 0.0 ? (float)(1.0 / s.hm_wbin) : 0.f;
+    s.hm_finv = small_map && s.hm_fbin > 0.0 ? (float)(1.0 / s.hm_fbin) : 0.f;
     s.adjoint = adjoint;
     s.inv_albedo = p->seafloor_albedo > 0.0 ? (float)(1.0 / p->seafloor_albedo) : 0.f;
     s.dla2_drough = (float)(4.0 * p->roughness * p->roughness * p->roughness);
@@ -347,6 +362,7 @@ static std::string set_scene(AlbCtx* ctx, const AlbSceneParams* p) {
         s.layer_alpha[l] = L.alpha;
         s.layer_ssa[l] = L.ssa;
         s.layer_binw[l] = (float)L.bin_width;
+        s.layer_binw_inv[l] = 1.0f / s.layer_binw[l];
         s.layer_h[l] = L.height;
         s.layer_top32[l] = L.top32;
         s.layer_prof[l] = L.profiled ? 1 : 0;
@@ -441,12 +457,17 @@ static std::string ensure_accumulators(AlbCtx* ctx) {
         have = need;
         return true;
     };
-    if (!regrow(ctx->wf, ctx->wf_bins, s.nbins, (size_t)2 * ALB_CHANNELS)) return "waveform allocation failed";
-    if (s.adjoint && !regrow(ctx->jac, ctx->jac_bins, s.nbins, (size_t)2 * kJacParams * ALB_CHANNELS))
+    if (!regrow(ctx->wf, ctx->wf_bins, s.nbins, (size_t)2 * ALB_CHANNELS) ||
+        !regrow(ctx->cls, ctx->cls_bins, s.nbins, 16))
+        return "waveform allocation failed";
+    if (s.adjoint && (!regrow(ctx->jac, ctx->jac_bins, s.nbins, (size_t)2 * kJacParams * ALB_CHANNELS) ||
+                      !regrow(ctx->jac_cls, ctx->jac_cls_bins, s.nbins, (size_t)16 * kJacParams)))
         return "jacobian allocation failed";
     if (s.heatmap) {
         const int64_t hb = (int64_t)s.hm_bins * s.hm_bins;
         if (!regrow(ctx->hm, ctx->hm_cells, hb, 4)) return "heatmap allocation failed";
+        // two maps of class words: 10 MB at the default 200 bins; larger maps add directly
+        if (s.hm_bins <= 512 && !regrow(ctx->heat_cls, ctx->heat_cls_cells, hb, 32)) return "heatmap allocation failed";
         if (!ctx->hm_radius || ctx->hm_radius_cells < hb) {
             if (ctx->hm_radius) {
                 cudaStreamSynchronize(ctx->st);
@@ -510,7 +531,7 @@ extern "C" void alb_destroy(AlbCtx* ctx) {
         cudaFree(ctx->qa[k]); cudaFree(ctx->qb[k]); cudaFree(ctx->qc[k]); cudaFree(ctx->qid[k]); cudaFree(ctx->qperm[k]);
         cudaFree(ctx->qrk[k][0]); cudaFree(ctx->qrk[k][1]); cudaFree(ctx->qs[k]);
     }
-    cudaFree(ctx->wf); cudaFree(ctx->hm); cudaFree(ctx->hm_radius); cudaFree(ctx->jac);
+    cudaFree(ctx->wf); cudaFree(ctx->cls); cudaFree(ctx->jac_cls); cudaFree(ctx->heat_cls); cudaFree(ctx->hm); cudaFree(ctx->hm_radius); cudaFree(ctx->jac);
     for (auto& t : ctx->lt) {
         cudaFree(t.th); cudaFree(t.cdf); cudaFree(t.sl); cudaFree(t.w); cudaFree(t.dlw); cudaFree(t.dsg); cudaFree(t.inv);
     }
@@ -795,10 +816,12 @@ extern "C" int alb_trace(AlbCtx* ctx, int pass, uint64_t n, uint64_t seed, uint6
     Accum acc{};
     acc.wf_lo = ctx->wf;
     acc.wf_hi = ctx->wf + (size_t)ALB_CHANNELS * ctx->sc.nbins;
+    acc.cls = ctx->cls;
     acc.nbins = ctx->sc.nbins;
     if (ctx->sc.adjoint) {
         acc.jac_lo = ctx->jac;
         acc.jac_hi = ctx->jac + (size_t)kJacParams * ALB_CHANNELS * ctx->sc.nbins;
+        acc.jac_cls = ctx->jac_cls;
     }
     if (ctx->sc.heatmap) {
         size_t hb = (size_t)ctx->sc.hm_bins * ctx->sc.hm_bins;
@@ -806,6 +829,7 @@ extern "C" int alb_trace(AlbCtx* ctx, int pass, uint64_t n, uint64_t seed, uint6
         acc.hw_hi = ctx->hm + hb;
         acc.hf_lo = ctx->hm + 2 * hb;
         acc.hf_hi = ctx->hm + 3 * hb;
+        acc.heat_cls = ctx->sc.hm_bins <= 512 ? ctx->heat_cls : nullptr;
     }
     const bool chunked = !ctx->keep_exit && !ctx->keep_ids && !rp;
     const uint64_t chunk = chunked ? kBackwardChunk : std::max<uint64_t>(n, 1);

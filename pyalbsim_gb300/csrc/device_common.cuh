@@ -27,6 +27,7 @@ struct SceneDev {
     int32_t gated;            // 1: bins outside the window are dropped, not an error
     int32_t pad_gate;
     int32_t mult;
+    float mult32, mult32_inv;  // mult and 1 / mult, rounded to nearest
     int32_t k;
     double ys, yf, v_air;
     double n_water, eta, f0;
@@ -45,11 +46,15 @@ struct SceneDev {
     int32_t pad0;
     double hm_wext, hm_fext, hm_wbin, hm_fbin;
     double wc[3], fc[3];
+    // float32 forms for the heatmap cells: centre x and z as high and low parts, 1 / bin (0: always float64)
+    float2 hm_wc32[2], hm_fc32[2];
+    float hm_wext32, hm_fext32, hm_winv, hm_finv;
     double layer_bottom[ALB_MAX_LAYERS];
     double layer_speed[ALB_MAX_LAYERS];
     float layer_alpha[ALB_MAX_LAYERS];
     float layer_ssa[ALB_MAX_LAYERS];
     float layer_binw[ALB_MAX_LAYERS];
+    float layer_binw_inv[ALB_MAX_LAYERS];  // 1 / layer_binw, rounded to nearest
     const double* layer_theta[ALB_MAX_LAYERS];
     const double* layer_cdf[ALB_MAX_LAYERS];
     const double* layer_slope[ALB_MAX_LAYERS];

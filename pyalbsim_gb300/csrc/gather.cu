@@ -33,7 +33,9 @@ constexpr int kGatherBlocksPerSM = 4;
 // 546 ms, 64 -> 529 ms, 128 -> 524 ms; the planar maps' gathers lose 2-3% at 128). Fewer
 // queries than fill the resident warps with such chunks take shorter ones (query_chunk).
 constexpr int kQueryChunk = 64;
-constexpr int kQueryChunkScatter = 128;
+// scatter queries a warp fetches at a time (large scene, 1e7 photons: 16 -> 296 ms, 32 -> 297, 64 -> 305;
+// 1e6: 30.5, 29.7, 30.1)
+constexpr int kScatterChunk = 32;
 constexpr int kQueryChunkMin = 2;
 constexpr int kStack = 32 * kMaxLevels;
 constexpr int kCap = 288;         // candidate buffer (k <= kCap - 32)
@@ -780,6 +782,68 @@ ALB_DEVICE Fix128 f32_to_fix(float v) {
     return r;
 }
 
+// One contribution to cell `i` of a 128-bit accumulator: one 64-bit add whose result nobody waits
+// for. A float32 is 24 bits at a shift sh (value 2^64 = mant 2^sh); its class is sh / 4, and the
+// class's word of the cell takes +- mant << (sh % 4), below 2^27, so 2^36 contributions fit
+// (kClassMost, kept by the launches). k_merge_classes sums the words exactly into the
+// accumulator and leaves them zero. A direct 128-bit add takes two atomics, the second on the
+// first one's carry, and the warp waits for both: scatter gather of the large scene, 1e6 photons,
+// 29.7 -> 24.8 ms. Bins in shared memory caught less than half of the scatter contributions
+// (multiple scattering spreads a range of queries over ten thousand bins).
+// 2^23 and more, and what is not finite, goes the direct way.
+constexpr int kClasses = 16;
+constexpr uint64_t kClassMost = 1ull << 36;
+ALB_DEVICE void class_add(unsigned long long* cls, uint32_t n, uint32_t i, float c, unsigned long long* lo,
+                          unsigned long long* hi) {
+    const uint32_t b = __float_as_uint(c) & 0x7fffffffu;
+    if (b < 0x4b000000u) {
+        if (b < 0x00800000u) return;  // zero or subnormal
+        uint32_t mant = (b & 0x7fffffu) | 0x800000u;
+        int sh = (int)(b >> 23) - 86;
+        if (sh < 0) {
+            mant >>= min(-sh, 31);
+            sh = 0;
+        }
+        const long long v = (long long)(mant << (sh & 3));
+        atomicAdd(cls + ((uint64_t)(uint32_t)(sh >> 2) * n + i), (unsigned long long)(c < 0.f ? -v : v));
+        return;
+    }
+    fix_atomic_add(lo + i, hi + i, f32_to_fix(c));
+}
+
+// The same where the accumulator may have no class words (cls null: direct).
+ALB_DEVICE void cell_add(unsigned long long* cls, uint32_t n, uint32_t i, float c, unsigned long long* lo,
+                         unsigned long long* hi) {
+    if (cls) class_add(cls, n, i, c, lo, hi);
+    else fix_atomic_add(lo + i, hi + i, f32_to_fix(c));
+}
+
+// The class words of n cells (blockIdx.y: one of several accumulators, cls_step and out_step words
+// apart) into their 128-bit words; the class words are left zero.
+__global__ void k_merge_classes(unsigned long long* cls, uint32_t n, unsigned long long* lo, unsigned long long* hi,
+                                uint64_t cls_step, uint64_t out_step) {
+    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    cls += blockIdx.y * cls_step;
+    unsigned long long w[kClasses];
+    unsigned long long any = 0ull;
+#pragma unroll
+    for (int c = 0; c < kClasses; ++c) {
+        w[c] = cls[(uint64_t)c * n + i];
+        any |= w[c];
+    }
+    if (!any) return;
+    Fix128 sum{0ull, 0ll};
+#pragma unroll
+    for (int c = 0; c < kClasses; ++c) {
+        if (!w[c]) continue;
+        cls[(uint64_t)c * n + i] = 0ull;
+        fix_add(sum, Fix128{w[c] << (4 * c), (long long)w[c] >> (c ? 64 - 4 * c : 63)});
+    }
+    const uint64_t o = blockIdx.y * out_step + i;
+    fix_atomic_add(lo + o, hi + o, sum);
+}
+
 // Per-CTA shared-memory cache of waveform bins: direct-mapped on the bin index, a slot is
 // claimed once by CAS on its tag; hits are exact 128-bit integer adds in shared memory,
 // misses go to global memory. Flushed once when the CTA finishes. The sum is integer, so
@@ -884,7 +948,7 @@ ALB_DEVICE void warp_radius_visit(const MapDev& m, WarpSmem& s, double qx, doubl
 }
 
 // Adjoint (extension): one neighbour's c (s_query + s_record + d ln w / d theta) into the
-// Jacobian for theta = a, b, g, albedo, roughness (128-bit fixed point, global atomics).
+// Jacobian for theta = a, b, g, albedo, roughness (128-bit fixed point by class words).
 template <int CHANNEL>
 ALB_DEVICE void jac_add(const SceneDev& sc, const MapDev& m, const Accum& acc, int layer, int bin, uint32_t idx,
                         float c, float4 sq, float4 pb, float vx, float vy, float vz) {
@@ -901,29 +965,41 @@ ALB_DEVICE void jac_add(const SceneDev& sc, const MapDev& m, const Accum& acc, i
     if (CHANNEL == ALB_SURFACE_REFLECTION) d[4] = sc.dla2_drough * ggx_dlog_da2(sc.ggx_a2, -pb.x, -pb.y, -pb.z, vx, vy, vz);
 #pragma unroll
     for (int p = 0; p < kJacParams; ++p) {
-        const float v = c * d[p];
-        if (v != 0.f) {
-            const uint64_t o = ((uint64_t)p * ALB_CHANNELS + CHANNEL) * acc.nbins + bin;
-            fix_atomic_add(acc.jac_lo + o, acc.jac_hi + o, f32_to_fix(v));
-        }
+        const uint64_t o = ((uint64_t)p * ALB_CHANNELS + CHANNEL) * acc.nbins;
+        cell_add(acc.jac_cls ? acc.jac_cls + (uint64_t)p * kClasses * acc.nbins : nullptr, (uint32_t)acc.nbins,
+                 (uint32_t)bin, c * d[p], acc.jac_lo + o, acc.jac_hi + o);
     }
+}
+
+// (long long)((x - c + ext) / bin) in float64, as numpy forms the heatmap cell, or -1 outside
+// [0, bins). The float32 value v decides wherever it is farther from an integer than its own
+// error: five roundings of terms up to |v| + 2 ext / bin <= 1024 cells, under 3.1e-4 (the host
+// sets inv = 0 for more than 512 bins, which always takes the float64 path). A neighbour's four
+// float64 divisions cost more issue time than the rest of its contribution: two FP64 lanes per SM.
+ALB_DEVICE int heat_cell(float x, double c, double ext, double bin, float2 cf, float extf, float inv, int bins) {
+    const float v = ((x - cf.x) - cf.y + extf) * inv;
+    if (inv != 0.f && (v < -1.5f || v > (float)bins + 0.5f)) return -1;
+    long long i;
+    if (fabsf(v - rintf(v)) > 4.8828125e-04f) i = (long long)(int)v;
+    else i = (long long)(((double)x - c + ext) / bin);
+    return i >= 0 && i < bins ? (int)i : -1;
 }
 
 // accumulate_to_heatmap (alb_sim/math/accumulate_heatmap.py:6-61) for one neighbour
 ALB_DEVICE void heat_add(const SceneDev& sc, const MapDev& m, const Accum& acc, uint32_t idx, float c) {
     const float4 fw = m.fwi[idx], sf = m.sfi[idx];
-    const Fix128 f = f32_to_fix(c);
+    const uint32_t cells = (uint32_t)(sc.hm_bins * sc.hm_bins);
     if (fw.x == fw.x) {
-        long long xi = (long long)(((double)fw.x - sc.wc[0] + sc.hm_wext) / sc.hm_wbin);
-        long long zi = (long long)(((double)fw.z - sc.wc[2] + sc.hm_wext) / sc.hm_wbin);
-        if (xi >= 0 && xi < sc.hm_bins && zi >= 0 && zi < sc.hm_bins)
-            fix_atomic_add(acc.hw_lo + xi * sc.hm_bins + zi, acc.hw_hi + xi * sc.hm_bins + zi, f);
+        const int xi = heat_cell(fw.x, sc.wc[0], sc.hm_wext, sc.hm_wbin, sc.hm_wc32[0], sc.hm_wext32, sc.hm_winv, sc.hm_bins);
+        const int zi = heat_cell(fw.z, sc.wc[2], sc.hm_wext, sc.hm_wbin, sc.hm_wc32[1], sc.hm_wext32, sc.hm_winv, sc.hm_bins);
+        if (xi >= 0 && zi >= 0) cell_add(acc.heat_cls, cells, (uint32_t)(xi * sc.hm_bins + zi), c, acc.hw_lo, acc.hw_hi);
     }
     if (sf.x == sf.x) {
-        long long xi = (long long)(((double)sf.x - sc.fc[0] + sc.hm_fext) / sc.hm_fbin);
-        long long zi = (long long)(((double)sf.z - sc.fc[2] + sc.hm_fext) / sc.hm_fbin);
-        if (xi >= 0 && xi < sc.hm_bins && zi >= 0 && zi < sc.hm_bins)
-            fix_atomic_add(acc.hf_lo + xi * sc.hm_bins + zi, acc.hf_hi + xi * sc.hm_bins + zi, f);
+        const int xi = heat_cell(sf.x, sc.fc[0], sc.hm_fext, sc.hm_fbin, sc.hm_fc32[0], sc.hm_fext32, sc.hm_finv, sc.hm_bins);
+        const int zi = heat_cell(sf.z, sc.fc[2], sc.hm_fext, sc.hm_fbin, sc.hm_fc32[1], sc.hm_fext32, sc.hm_finv, sc.hm_bins);
+        if (xi >= 0 && zi >= 0)
+            cell_add(acc.heat_cls ? acc.heat_cls + (uint64_t)kClasses * cells : nullptr, cells,
+                          (uint32_t)(xi * sc.hm_bins + zi), c, acc.hf_lo, acc.hf_hi);
     }
 }
 
@@ -935,30 +1011,20 @@ ALB_DEVICE void heat_add(const SceneDev& sc, const MapDev& m, const Accum& acc, 
 // and fetch.
 constexpr int kModeKnn = 0, kModeKnnAdjoint = 1, kModeRadius = 2, kModeKnnHeat = 3;
 
-// The energy of candidate j, where the search kept it.
-template <class S>
-ALB_DEVICE auto neighbour_energy(const S& s, int j) -> decltype(s.ce[0] + 0.f) { return s.ce[j]; }
-ALB_DEVICE float neighbour_energy(const WarpSmem&, int) { return 0.f; }
-
-// One query's k neighbours s.ci[0 .. k) into the waveform (and Jacobian, heatmaps): Es, qb, qy the
-// query's energy, direction and time, and float64 depth; rk the k-th distance. CE: the search
-// left the neighbours' energies in s.ce.
-template <int CHANNEL, int MODE, bool CE, class S>
+// One query's k neighbours s.ci[0 .. k) of a planar map into the waveform (and Jacobian,
+// heatmaps): Es, qb the query's energy, direction and time; rk the k-th distance.
+template <int CHANNEL, int MODE>
 ALB_DEVICE void accumulate(const SceneDev& sc, const MapDev& m, const QueryDev& q, const Accum& acc, BinCache& bc, int* err,
-                           S& s, int k, uint64_t src, float Es, float4 qb, double qy, float rk) {
+                           const WarpSmem& s, int k, uint64_t src, float Es, float4 qb, float rk) {
     const int l = lane_id();
     const float ts = qb.w;
-    float norm;
-    if (CHANNEL == ALB_SCATTER) norm = 1.0f / ((4.0f / 3.0f) * 3.14159265358979f * rk * rk * rk);
-    else norm = 1.0f / (3.14159265358979f * rk * rk);
+    const float norm = 1.0f / (3.14159265358979f * rk * rk);
     // query-constant pieces
     float vinv = rsqrtf(fmaf(qb.x, qb.x, fmaf(qb.y, qb.y, qb.z * qb.z)));
     float vx = -qb.x * vinv, vy = -qb.y * vinv, vz = -qb.z * vinv;  // normalize(-d_query)
     float wconst = 0.f;
     if (CHANNEL == ALB_BOTTOM_REFLECTION) wconst = sc.floor_lambert * fmaxf(0.f, -qb.y);
     if (CHANNEL == ALB_SURFACE_TRANSMISSION_UP) wconst = sc.surface_lambert;
-    // WaterModel.scatter_energy picks the layer of the query depth (water.py:418-447)
-    const int layer = (CHANNEL == ALB_SCATTER && sc.n_layers > 1) ? layer_of(sc, qy) : 0;
     float4 sq = make_float4(0.f, 0.f, 0.f, 0.f);
     if (MODE == kModeKnnAdjoint && q.s) sq = q.s[src];
     // the next neighbour's record is loaded while this one is weighted
@@ -967,7 +1033,7 @@ ALB_DEVICE void accumulate(const SceneDev& sc, const MapDev& m, const QueryDev& 
     float e_n = 0.f;
     if (l < k) {
         pb_n = m.b[idx_n];
-        e_n = CE ? neighbour_energy(s, l) : m.a[idx_n].w;
+        e_n = m.a[idx_n].w;
     }
 #pragma unroll 1
     for (int j = l; j < k; j += 32) {
@@ -977,18 +1043,17 @@ ALB_DEVICE void accumulate(const SceneDev& sc, const MapDev& m, const QueryDev& 
         if (j + 32 < k) {
             idx_n = s.ci[j + 32];
             pb_n = m.b[idx_n];
-            e_n = CE ? neighbour_energy(s, j + 32) : m.a[idx_n].w;
+            e_n = m.a[idx_n].w;
         }
         float w;
         if (CHANNEL == ALB_BOTTOM_REFLECTION || CHANNEL == ALB_SURFACE_TRANSMISSION_UP) w = wconst;
-        else if (CHANNEL == ALB_SCATTER) w = scatter_weight(sc, layer, pb.x, pb.y, pb.z, vx, vy, vz);
-        else w = ggx_weight(sc.ggx_a2, (float)sc.f0, -pb.x, -pb.y, -pb.z, vx, vy, vz);
+                else w = ggx_weight(sc.ggx_a2, (float)sc.f0, -pb.x, -pb.y, -pb.z, vx, vy, vz);
         const float c = ((Es * Ep) * norm) * w;
         const int bin = (int)((ts + pb.w) / (float)sc.mult) - (int)sc.gate_lo;
         if (bin >= 0 && bin < acc.nbins) {
             bin_add(bc, acc, CHANNEL, bin, f32_to_fix(c));
             if (MODE == kModeKnnAdjoint && acc.jac_lo)
-                jac_add<CHANNEL>(sc, m, acc, layer, bin, idx, c, sq, pb, vx, vy, vz);
+                jac_add<CHANNEL>(sc, m, acc, 0, bin, idx, c, sq, pb, vx, vy, vz);
         } else if (!sc.gated) {
             atomicCAS(err, 0, ALB_ERR_CAPACITY);
         }
@@ -1002,8 +1067,7 @@ ALB_DEVICE void accumulate(const SceneDev& sc, const MapDev& m, const QueryDev& 
             const float4 pb = m.b[idx];
             float w;
             if (CHANNEL == ALB_BOTTOM_REFLECTION || CHANNEL == ALB_SURFACE_TRANSMISSION_UP) w = wconst;
-            else if (CHANNEL == ALB_SCATTER) w = scatter_weight(sc, layer, pb.x, pb.y, pb.z, vx, vy, vz);
-            else w = ggx_weight(sc.ggx_a2, (float)sc.f0, -pb.x, -pb.y, -pb.z, vx, vy, vz);
+                        else w = ggx_weight(sc.ggx_a2, (float)sc.f0, -pb.x, -pb.y, -pb.z, vx, vy, vz);
             heat_add(sc, m, acc, idx, ((Es * m.a[idx].w) * norm) * w);
         }
     }
@@ -1112,9 +1176,8 @@ __global__ void __launch_bounds__(kGatherWarps * 32, kGatherBlocksPerSM) k_gathe
                 failed = true;
                 break;
             }
-            // the query's direction and time, and its float64 depth, are needed from here on
+            // the query's direction and time are needed from here on
             const float4 qb = q.b[src];
-            const double qy = (double)qa.y + (double)qc.y;
             have_prev = true;
             if (q.rk_out && l == 0) q.rk_out[src] = sqrt(r.rk2);
             if (l == 0) {
@@ -1124,7 +1187,7 @@ __global__ void __launch_bounds__(kGatherWarps * 32, kGatherBlocksPerSM) k_gathe
                 s.st[3] += 1;
                 s.st[4] += r.clipped;
             }
-            accumulate<CHANNEL, MODE, false>(sc, m, q, acc, bc, err, s, k, src, qa.w, qb, qy, r.rkf);
+            accumulate<CHANNEL, MODE>(sc, m, q, acc, bc, err, s, k, src, qa.w, qb, r.rkf);
             __syncwarp();
         }
     }
@@ -1141,8 +1204,60 @@ __global__ void __launch_bounds__(kGatherWarps * 32, kGatherBlocksPerSM) k_gathe
     bin_flush<CHANNEL>(bc, acc);
 }
 
+// x / b from r = the float32 nearest 1 / b: the quotient estimate corrected by its exact residual
+// (Markstein, "Computation of elementary functions on the IBM RISC System/6000 processor", IBM J.
+// Res. Dev. 34, 1990), the correctly rounded quotient the division operator gives.
+ALB_DEVICE float div_by(float x, float b, float r) {
+    const float q = x * r;
+    return fmaf(fmaf(-q, b, x), r, q);
+}
+
+// One query's k neighbours s.ci / s.ce [0 .. k) of the scatter map into the waveform (and Jacobian,
+// heatmaps); qy the query's float64 depth, rk the k-th distance.
+template <int MODE, class S>
+ALB_DEVICE void accumulate_scatter(const SceneDev& sc, const MapDev& m, const QueryDev& q, const Accum& acc,
+                                   int* err, const S& s, int k, uint32_t src, float Es, float4 qb,
+                                   double qy, float rk) {
+    const int l = lane_id();
+    const float norm = 1.0f / ((4.0f / 3.0f) * 3.14159265358979f * rk * rk * rk);
+    const float vinv = rsqrtf(fmaf(qb.x, qb.x, fmaf(qb.y, qb.y, qb.z * qb.z)));
+    const float vx = -qb.x * vinv, vy = -qb.y * vinv, vz = -qb.z * vinv;  // normalize(-d_query)
+    // WaterModel.scatter_energy picks the layer of the query depth (water.py:418-447)
+    const int layer = sc.n_layers > 1 ? layer_of(sc, qy) : 0;
+    const float* wtab = sc.layer_weight[layer];
+    const float binw = sc.layer_binw[layer], binw_inv = sc.layer_binw_inv[layer];
+    const int gate = (int)sc.gate_lo;
+    const uint32_t nbins = (uint32_t)acc.nbins;
+    unsigned long long* wf_lo = acc.wf_lo + (uint64_t)ALB_SCATTER * acc.nbins;
+    unsigned long long* wf_hi = acc.wf_hi + (uint64_t)ALB_SCATTER * acc.nbins;
+    float4 sq = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (MODE == kModeKnnAdjoint && q.s) sq = q.s[src];
+    // the next neighbour's record is loaded while this one is weighted
+    float4 pb_n = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (l < k) pb_n = m.b[s.ci[l]];
+#pragma unroll 1
+    for (int j = l; j < k; j += 32) {
+        const float4 pb = pb_n;
+        if (j + 32 < k) pb_n = m.b[s.ci[j + 32]];
+        // scatter_bin with its division by a constant
+        const float n = rsqrtf(fmaf(pb.x, pb.x, fmaf(pb.y, pb.y, pb.z * pb.z)));
+        const float ca = fminf(fmaxf(fmaf(pb.x, vx, fmaf(pb.y, vy, pb.z * vz)) * n, -1.f), 1.f);
+        const int a = min(max((int)div_by(acosf(ca) - kEps32, binw, binw_inv), 0), ALB_PHASE_DIVISIONS - 1);
+        const float c = ((Es * s.ce[j]) * norm) * __ldg(wtab + a);
+        const int bin = (int)div_by(qb.w + pb.w, sc.mult32, sc.mult32_inv) - gate;
+        if ((uint32_t)bin < nbins) {
+            class_add(acc.cls, nbins, (uint32_t)bin, c, wf_lo, wf_hi);
+            if (MODE == kModeKnnAdjoint && acc.jac_lo)
+                jac_add<ALB_SCATTER>(sc, m, acc, layer, bin, s.ci[j], c, sq, pb, vx, vy, vz);
+        } else if (!sc.gated) {
+            atomicCAS(err, 0, ALB_ERR_CAPACITY);
+        }
+        if (MODE != kModeKnn && acc.hw_lo && m.fwi) heat_add(sc, m, acc, s.ci[j], c);
+    }
+}
+
 // The search of one query alone, out of line: the grouped kernel takes it for the first query of
-// a chunk, runs whose list does not fit, guesses that fail and near ties, 1-3% of the queries,
+// a CTA, runs whose list does not fit, guesses that fail and near ties, 1-3% of the queries,
 // and its code and registers stay out of the hot loop.
 template <class S>
 __device__ __noinline__ bool cold_knn(const MapDev& m, S& s, int k, float fx, float fy, float fz, float lx, float ly,
@@ -1155,78 +1270,87 @@ __device__ __noinline__ bool cold_knn(const MapDev& m, S& s, int k, float fx, fl
     return true;
 }
 
-// Scatter-map gather, k nearest, by runs of neighbouring queries (gather_group.cuh).
-template <int MODE, int CAP, int BLOCKS>
-__global__ void __launch_bounds__(kGatherWarps * 32, BLOCKS)
+// Scatter-map gather, k nearest, by runs of neighbouring queries (gather_group.cuh). One CTA per SM
+// takes one contiguous range of the sorted queries, so that its leaves stay local; its warps fetch
+// chunks of the range in turn.
+template <int MODE, int CAP, int WARPS>
+__global__ void __launch_bounds__(WARPS * 32, 1)
     k_gather_scatter(const __grid_constant__ SceneDev sc, const __grid_constant__ MapDev m,
-                     const __grid_constant__ QueryDev q, const __grid_constant__ Accum acc, int k, int* err, uint32_t chunk) {
+                     const __grid_constant__ QueryDev q, const __grid_constant__ Accum acc, int k, int* err, uint32_t chunk,
+                     uint64_t first, uint64_t n) {
     extern __shared__ __align__(16) unsigned char group_raw[];
     using S = GroupSmem<CAP>;
     S* smem = reinterpret_cast<S*>(group_raw);
-    BinCache& bc = *reinterpret_cast<BinCache*>(group_raw + kGatherWarps * sizeof(S));
-    for (int i = threadIdx.x; i < kBinCache; i += blockDim.x) {
-        bc.tag[i] = -1;
-        bc.lo[i] = 0ull;
-        bc.hi[i] = 0ull;
+    __shared__ uint32_t next;  // the CTA's next chunk
+    __shared__ float last2;    // squared k-th distance of some query just answered (a chunk's first guess)
+    if (threadIdx.x == 0) {
+        next = 0u;
+        last2 = -1.f;
     }
     __syncthreads();
     const int w = threadIdx.x >> 5, l = lane_id();
     S& s = smem[w];
-    const uint64_t warps = (uint64_t)gridDim.x * kGatherWarps;
-    const uint64_t chunks = (q.n + chunk - 1) / chunk;
+    const uint64_t seg0 = first + n * blockIdx.x / gridDim.x, seg1 = first + n * (blockIdx.x + 1) / gridDim.x;
     // edge of a cubic leaf over the k-th distance: 32 records against k in the ball
     const float side_rk = cbrtf(134.04f / (float)k);
     bool failed = false;
     if (l < 5) s.st[l] = 0ull;
     __syncwarp();
-    for (uint64_t ch = (uint64_t)blockIdx.x * kGatherWarps + w; ch < chunks && !failed; ch += warps) {
-        const uint64_t q_end = min((ch + 1) * chunk, q.n);
+    while (!failed) {
+        uint32_t ch = 0u;
+        if (l == 0) ch = atomicAdd(&next, 1u);
+        ch = __shfl_sync(0xffffffffu, ch, 0);
+        const uint64_t c0 = seg0 + (uint64_t)ch * chunk;
+        if (c0 >= seg1) break;
+        const uint64_t q_end = min(c0 + chunk, seg1);
         QueryRun run{0, 0, 0.f};
         uint64_t r_base = 0;  // first query of the run the lanes hold
         uint32_t gsrc = 0u;   // this lane's query of the run: index and position
         float gx = 0.f, gy = 0.f, gz = 0.f;
-        float prev2 = -1.f;   // squared k-th distance of the previous query
-        for (uint64_t qi = ch * chunk; qi < q_end; ++qi) {
-            const float guess = prev2 * kGroupGuess2;
-            bool listed = prev2 > 0.f;
-            if (qi >= r_base + run.take || !(guess <= run.T2)) {
-                // a new run starts here
-                const int avail = (int)min(q_end - qi, (uint64_t)32);
-                r_base = qi;
-                float la = 0.f;
-                if (l < avail) {
-                    gsrc = q.perm ? q.perm[qi + l] : (uint32_t)(qi + l);
-                    const float4 a = q.a[gsrc];
-                    gx = a.x; gy = a.y; gz = a.z;
-                    if (!q.lo_zero) {
-                        const float4 c = q.c[gsrc];
-                        la = fmaxf(fabsf(c.x), fmaxf(fabsf(c.y), fabsf(c.z)));
-                    }
-                }
-                run.take = 1;
-                run.n = 0;
-                if (listed) listed = build_run(m, s, avail, gx, gy, gz, la, prev2, side_rk * sqrtf(prev2), run);
-                if (!listed) run.take = 1;
-            }
-            const int at = (int)(qi - r_base);
-            const uint32_t src = __shfl_sync(0xffffffffu, gsrc, at);
-            const float fx = __shfl_sync(0xffffffffu, gx, at), fy = __shfl_sync(0xffffffffu, gy, at),
-                        fz = __shfl_sync(0xffffffffu, gz, at);
-            float lx = 0.f, ly = 0.f, lz = 0.f;
-            if (!q.lo_zero) {
-                const float4 c = q.c[src];
-                lx = c.x; ly = c.y; lz = c.z;
-            }
-            float rk, d2;
+        // squared k-th distance of the previous query; a chunk starts from the CTA's latest
+        float prev2 = *reinterpret_cast<volatile float*>(&last2);
+        for (uint64_t qi = c0; qi < q_end; ++qi) {
+            // the guess, the whole list, then lists of 1.25 times the radius for this query
+            float thr = prev2 * kGroupGuess2;
+            bool fresh = qi >= r_base + run.take || !(thr <= run.T2);
+            float fx, fy, fz, lx = 0.f, ly = 0.f, lz = 0.f, kth = 0.f, rk, d2;
+            uint32_t src, kid = 0u;
             int got = 0, leaves = 0;
-            float kth = 0.f;
-            uint32_t kid = 0u;
-            if (listed) {
-                got = run_search(m, s, k, run.n, fx, fy, fz, lx, ly, lz, guess, kth, kid, leaves);
-                if (got == 0) {
-                    if (l == 0 && q.retries) atomicAdd(q.retries, 1ull);
-                    got = run_search(m, s, k, run.n, fx, fy, fz, lx, ly, lz, run.T2, kth, kid, leaves);
+#pragma unroll 1
+            for (int tries = 0;; ++tries) {
+                bool listed = prev2 > 0.f;
+                if (fresh) {
+                    const int avail = (int)min(q_end - qi, (uint64_t)32);
+                    r_base = qi;
+                    float la = 0.f;
+                    if (l < avail) {
+                        gsrc = q.perm ? q.perm[qi + l] : (uint32_t)(qi + l);
+                        const float4 a = q.a[gsrc];
+                        gx = a.x; gy = a.y; gz = a.z;
+                        if (!q.lo_zero) {
+                            const float4 c = q.c[gsrc];
+                            la = fmaxf(fabsf(c.x), fmaxf(fabsf(c.y), fabsf(c.z)));
+                        }
+                    }
+                    run.take = 1;
+                    if (listed) listed = build_run(m, s, avail, gx, gy, gz, la, prev2, side_rk * sqrtf(prev2), run);
                 }
+                const int at = (int)(qi - r_base);
+                src = __shfl_sync(0xffffffffu, gsrc, at);
+                fx = __shfl_sync(0xffffffffu, gx, at);
+                fy = __shfl_sync(0xffffffffu, gy, at);
+                fz = __shfl_sync(0xffffffffu, gz, at);
+                if (!q.lo_zero) {
+                    const float4 c = q.c[src];
+                    lx = c.x; ly = c.y; lz = c.z;
+                }
+                if (!listed) break;
+                got = run_search(m, s, k, run.n, fx, fy, fz, lx, ly, lz, thr, kth, kid, leaves);
+                if (got != 0 || tries == 6) break;
+                if (l == 0 && q.retries) atomicAdd(q.retries, 1ull);
+                fresh = !(thr < run.T2);
+                if (fresh) prev2 = run.T2;
+                thr = fresh ? prev2 * kGroupList2 : run.T2;
             }
             if (got == 1) {
                 rk = dist_f32(fx, fy, fz, lx, ly, lz, m.a[kid], d2);
@@ -1262,9 +1386,10 @@ __global__ void __launch_bounds__(kGatherWarps * 32, BLOCKS)
             }
             prev2 = d2;
             const float4 qb = q.b[src];
-            accumulate<ALB_SCATTER, MODE, true>(sc, m, q, acc, bc, err, s, k, src, q.a[src].w, qb, (double)fy + (double)ly, rk);
+            accumulate_scatter<MODE>(sc, m, q, acc, err, s, k, src, q.a[src].w, qb, (double)fy + (double)ly, rk);
             __syncwarp();
         }
+        if (l == 0) last2 = prev2;
     }
     if (l == 0) {
         if (q.stats && s.st[3]) {
@@ -1275,8 +1400,6 @@ __global__ void __launch_bounds__(kGatherWarps * 32, BLOCKS)
         }
         if (q.inexact && s.st[4]) atomicAdd(q.inexact, s.st[4]);
     }
-    __syncthreads();
-    bin_flush<ALB_SCATTER>(bc, acc);
 }
 
 // Standalone KDTree.query(x, k): sorted indices and float64 distances.
@@ -1338,25 +1461,49 @@ static unsigned gather_blocks(uint64_t nq) {
 }
 
 // Consecutive queries per warp: as many as the resident warps need to take every query in one
-// wave, within [kQueryChunkMin, kQueryChunk or kQueryChunkScatter]. With 64 whatever the count,
+// wave, within [kQueryChunkMin, kQueryChunk]. With 64 whatever the count,
 // 25 000 queries ran on 391 of the 4864 resident warps and took as long as 250 000 (bottom
 // gather 1.67 ms; with chunks of 6, 0.24 ms); 5000 queries take 0.07 ms at a floor of 2, 0.12
 // at 4, 0.21 at 8. The fixed-radius gather carries nothing from query to query and its visits
 // differ by four orders of magnitude between neighbouring queries: one query at a time (surface
 // gather of 25 000 queries at 0.5 m: 22.3 -> 13.1 ms).
-static uint32_t query_chunk(int channel, uint64_t nq, bool radius) {
+static uint32_t query_chunk(uint64_t nq, bool radius) {
     if (radius) return 1;
-    const uint64_t most = channel == ALB_SCATTER ? kQueryChunkScatter : kQueryChunk;
     const uint64_t warps = (uint64_t)sm_count() * kGatherBlocksPerSM * kGatherWarps;
     const uint64_t fit = (nq + warps - 1) / warps;
-    return (uint32_t)std::min<uint64_t>(most, std::max<uint64_t>(fit, kQueryChunkMin));
+    return (uint32_t)std::min<uint64_t>(kQueryChunk, std::max<uint64_t>(fit, kQueryChunkMin));
 }
 
-template <int MODE, int CAP, int BLOCKS>
+// The class words that a gather of `channel` filled (waveform: the scatter gather only).
+static void merge_classes(const SceneDev& sc, const Accum& acc, int channel, bool waveform, cudaStream_t st) {
+    const uint32_t nb = (uint32_t)acc.nbins;
+    const unsigned blocks = (nb + 255u) / 256u;
+    if (waveform) {
+        k_merge_classes<<<blocks, 256, 0, st>>>(acc.cls, nb, acc.wf_lo + (uint64_t)channel * nb,
+                                                acc.wf_hi + (uint64_t)channel * nb, 0, 0);
+        note_launch();
+    }
+    if (acc.jac_lo && acc.jac_cls) {
+        k_merge_classes<<<dim3(blocks, kJacParams), 256, 0, st>>>(acc.jac_cls, nb, acc.jac_lo + (uint64_t)channel * nb,
+                                                                  acc.jac_hi + (uint64_t)channel * nb,
+                                                                  (uint64_t)kClasses * nb, (uint64_t)ALB_CHANNELS * nb);
+        note_launch();
+    }
+    if (acc.hw_lo && acc.heat_cls) {
+        // the two maps' words lie 2 cells apart: hw_lo, hw_hi, hf_lo, hf_hi
+        const uint32_t cells = (uint32_t)(sc.hm_bins * sc.hm_bins);
+        k_merge_classes<<<dim3((cells + 255u) / 256u, 2), 256, 0, st>>>(acc.heat_cls, cells, acc.hw_lo, acc.hw_hi,
+                                                                        (uint64_t)kClasses * cells, (uint64_t)2 * cells);
+        note_launch();
+    }
+}
+
+template <int MODE, int CAP, int WARPS>
 static void launch_scatter(const SceneDev& sc, const MapDev& map, const QueryDev& q, const Accum& acc, int k, int* err,
-                           unsigned blocks, uint32_t chunk, cudaStream_t st) {
-    constexpr int bytes = kGatherWarps * (int)sizeof(GroupSmem<CAP>) + (int)sizeof(BinCache);
-    auto kernel = k_gather_scatter<MODE, CAP, BLOCKS>;
+                           cudaStream_t st) {
+    constexpr int bytes = WARPS * (int)sizeof(GroupSmem<CAP>);
+    static_assert(bytes <= 232448, "one CTA's shared memory");
+    auto kernel = k_gather_scatter<MODE, CAP, WARPS>;
     static std::atomic<bool> attr_set[64];  // per device; batched runs launch from several host threads
     int dev = 0;
     cudaGetDevice(&dev);
@@ -1364,13 +1511,23 @@ static void launch_scatter(const SceneDev& sc, const MapDev& map, const QueryDev
         cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
         if (dev >= 0 && dev < 64) attr_set[dev].store(true, std::memory_order_release);
     }
-    kernel<<<blocks, kGatherWarps * 32, bytes, st>>>(sc, map, q, acc, k, err, chunk);
+    // a class word holds kClassMost contributions: more queries go in slices
+    const uint64_t most = kClassMost / (uint64_t)k;
+    for (uint64_t first = 0; first < q.n; first += most) {
+        const uint64_t n = std::min<uint64_t>(most, q.n - first);
+        const uint64_t blocks = std::min<uint64_t>(sm_count(), n);
+        const uint64_t fit = (n + blocks * WARPS - 1) / (blocks * WARPS);
+        const uint32_t chunk = (uint32_t)std::min<uint64_t>(kScatterChunk, fit);
+        kernel<<<(unsigned)blocks, WARPS * 32, bytes, st>>>(sc, map, q, acc, k, err, chunk, first, n);
+        note_launch();
+        merge_classes(sc, acc, ALB_SCATTER, true, st);
+    }
 }
 
 template <int MODE>
 static void launch_gather_mode(const MapDev& map, const QueryDev& q, int channel, const SceneDev& sc, const Accum& acc,
                                int* err, uint64_t nq, int k, cudaStream_t st) {
-    const uint32_t chunk = query_chunk(channel, nq, MODE == kModeRadius);
+    const uint32_t chunk = query_chunk(nq, MODE == kModeRadius);
     const unsigned blocks = gather_blocks((nq + chunk - 1) / chunk);
     switch (channel) {
         case ALB_BOTTOM_REFLECTION:
@@ -1379,10 +1536,11 @@ static void launch_gather_mode(const MapDev& map, const QueryDev& q, int channel
         case ALB_SCATTER:
             if constexpr (MODE == kModeRadius) {
                 k_gather<ALB_SCATTER, MODE><<<blocks, kGatherWarps * 32, 0, st>>>(sc, map, q, acc, k, err, chunk);
-            } else if (k <= 128) {
-                launch_scatter<MODE, 224, 4>(sc, map, q, acc, k, err, blocks, chunk, st);
             } else {
-                launch_scatter<MODE, 448, 3>(sc, map, q, acc, k, err, blocks, chunk, st);
+                // candidates of a first guess: 1.33 k, twice that where the map thickens
+                if (k <= 128) launch_scatter<MODE, 224, 32>(sc, map, q, acc, k, err, st);
+                else launch_scatter<MODE, 448, 22>(sc, map, q, acc, k, err, st);
+                return;
             }
             break;
         case ALB_SURFACE_REFLECTION:
@@ -1393,12 +1551,18 @@ static void launch_gather_mode(const MapDev& map, const QueryDev& q, int channel
             break;
     }
     note_launch();
+    if (MODE != kModeKnn) merge_classes(sc, acc, channel, false, st);
 }
 
-void launch_gather(const SceneDev& sc, const MapDev& map, const QueryDev& q, int channel, const Accum& acc,
+void launch_gather(const SceneDev& sc, const MapDev& map, const QueryDev& q, int channel, const Accum& accum,
                    int* err, int* launches, cudaStream_t st) {
     if (q.n == 0) return;
     int k = sc.k;
+    Accum acc = accum;
+    // contributions of the launch at most (a fixed radius admits any number of the map's records);
+    // the k-NN scatter gather keeps below kClassMost by slices
+    const uint64_t per = sc.radius > 0.0 ? std::max<uint64_t>(map.n, 1) : (uint64_t)k;
+    if (q.n > kClassMost / per && (sc.radius > 0.0 || channel != ALB_SCATTER)) acc.jac_cls = acc.heat_cls = nullptr;
     if (sc.radius > 0.0) launch_gather_mode<kModeRadius>(map, q, channel, sc, acc, err, q.n, k, st);
     else if (acc.jac_lo) launch_gather_mode<kModeKnnAdjoint>(map, q, channel, sc, acc, err, q.n, k, st);
     else if (acc.hw_lo && map.fwi) launch_gather_mode<kModeKnnHeat>(map, q, channel, sc, acc, err, q.n, k, st);

@@ -95,6 +95,10 @@ struct Accum {
     unsigned long long* hf_lo;  // sampled seafloor heatmap
     unsigned long long* hf_hi;
     int64_t nbins;
+    // sums of one gather by exponent class, [16][cells], all zero between gathers (gather.cu, class_add)
+    unsigned long long* cls;       // waveform
+    unsigned long long* jac_cls;   // Jacobian, one set per parameter (nullable)
+    unsigned long long* heat_cls;  // water, then seafloor heatmap (nullable)
     unsigned long long* jac_lo;  // adjoint [5 params][channels][nbins] (nullable)
     unsigned long long* jac_hi;
 };

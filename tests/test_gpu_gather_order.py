@@ -58,3 +58,48 @@ def test_scatter_search_finds_the_kth_distance(gpu_available, k, precise):
         d = cKDTree(pts.astype(np.float64)).query(q["pos"], k=[k])[0][:, 0]
         assert len(d) > 0
         np.testing.assert_allclose(q["rk"], d, rtol=4 * np.finfo(np.float64).eps, atol=0)
+
+
+def test_heatmap_sums_on_both_sides_of_the_class_word_limit(gpu_available):
+    """Heatmaps of up to 512 bins add through class words and float32 cell numbers, larger ones
+    directly and in float64. With every contribution inside, the totals of a 512 and a 513 bin map
+    are the same fixed-point sum; reading it as float64 rounds once per cell, 2^-53 of it."""
+    from pyalbsim_gb300.config import HeatmapConfig, SimulationConfig
+
+    def totals(bins):
+        cfg = dataclasses.replace(
+            SimulationConfig(), heatmap=HeatmapConfig(bins=bins, water_extent=1000.0, seafloor_extent=1000.0))
+        with GpuEngine(cfg) as eng:
+            eng.forward(5_000, 3)
+            eng.build_maps()
+            eng.backward(1_250, 3)
+            w, f, r = eng.ctx.heatmaps()
+        return w.sum(), f.sum(), r.sum()
+
+    a, b = totals(512), totals(513)
+    assert a[0] > 0 and a[1] > 0 and a[2] > 0
+    np.testing.assert_allclose(a, b, rtol=1e-12)
+
+
+@pytest.mark.parametrize("bins", [200, 600])
+def test_heatmap_cells_match_the_precise_formula(gpu_available, bins):
+    """Scatter-radius free check of the cell numbers: the seafloor map's marginal over x equals a
+    histogram of the same contributions at half the resolution, summed in pairs."""
+    from pyalbsim_gb300.config import HeatmapConfig, SimulationConfig
+
+    def maps(n):
+        cfg = dataclasses.replace(SimulationConfig(), heatmap=HeatmapConfig(bins=n, water_extent=4.0, seafloor_extent=16.0))
+        with GpuEngine(cfg) as eng:
+            eng.forward(5_000, 3)
+            eng.build_maps()
+            eng.backward(1_250, 3)
+            w, f, _ = eng.ctx.heatmaps()
+        return w.reshape(n, n), f.reshape(n, n)
+
+    # extents are powers of two and bins even, so the coarse cells' edges are fine cells' edges; a
+    # cell's float64 quotient rounds onto an edge only for values within 1e-15 of it
+    for fine, coarse in zip(maps(bins), maps(bins // 2)):
+        pairs = fine.reshape(bins // 2, 2, bins // 2, 2).sum(axis=(1, 3))
+        # truncation toward zero puts (-1, 0) into cell 0 on both grids: the outermost row and
+        # column of the coarse map reach one coarse cell out, those of the fine map one fine cell
+        np.testing.assert_allclose(pairs[1:, 1:], coarse[1:, 1:], rtol=1e-12, atol=1e-300)
