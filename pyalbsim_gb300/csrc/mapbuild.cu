@@ -178,192 +178,249 @@ ALB_DEVICE uint32_t query_key(const QueryGrid& g, float x, float y, float z) {
     return (hi << (3 * g.m)) | hilbert_key<3>(q, g.m);
 }
 
-__global__ void k_keys(const float4* __restrict__ a, uint64_t n, const unsigned* __restrict__ box, int total,
-                       uint32_t* keys, uint32_t* vals) {
-    const QueryGrid g = make_query_grid(box, total);
-    for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n;
-         i += (uint64_t)gridDim.x * blockDim.x) {
-        const float4 p = a[i];
-        keys[i] = query_key(g, p.x, p.y, p.z);
-        vals[i] = (uint32_t)i;
-    }
-}
-
 // ------------------------------------------------------------------------------------------
-// LSD radix sort of (u32 key, u32 value), 8-bit digits, stable.
-// Tile = 8 warps x 16 rounds x 32 lanes; key t of warp w, round j, lane l is
-// tile_base + w*512 + j*32 + l, so ranking warps in order, rounds in order and lanes in
-// order preserves the input order of equal digits.
+// LSD radix sort of (u32 key, u32 value), 8-bit digits, stable. Blocks own contiguous ranges of
+// whole tiles. A pass is three launches and waits for nothing else: per block a histogram of the
+// digit (the first one comes with the keys), per digit a scan over the blocks, and a scatter in
+// which a block keeps one running offset per digit. A tile is ranked by warps in order, rounds in
+// order and lanes in order, put in digit order in shared memory and written out from there, so
+// that a digit's records leave in runs (16 on average) instead of one by one.
+// Bound by the ranking's latency (a warp match and a shared counter per round) beside its DRAM
+// traffic, 20 B per record and pass (key read for the histogram; key and value read and written):
+// 9.5e7 queries of the large scene at 1e7 photons sort in 5.3 ms with their box and keys (12.3 ms
+// with one tile per block, 32-record ranges scattered straight from registers and
+// a device-wide scan); 8 rounds and 3 blocks per SM against 16 and 2: 5.8 ms, 12 and 2: 5.5 ms.
 // ------------------------------------------------------------------------------------------
-constexpr int kRsWarps = 8, kRsItems = 16, kRsThreads = kRsWarps * 32;
+constexpr int kRsBlocksPerSM = 3;
+constexpr int kRsWarps = 16, kRsItems = 8, kRsThreads = kRsWarps * 32;
 constexpr int kRsTile = kRsThreads * kRsItems;
 
-template <class K>
-__global__ void __launch_bounds__(kRsThreads) k_rs_hist(const K* __restrict__ keys, uint64_t n,
-                                                         int shift, uint32_t* hist, uint32_t ntiles) {
+struct SortPlan {
+    uint32_t blocks;
+    uint64_t per;  // records per block, a multiple of the tile
+};
+
+static SortPlan sort_plan(uint64_t n) {
+    int dev = 0, sms = 148;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    const uint64_t tiles = (n + kRsTile - 1) / kRsTile;
+    const uint64_t each = (tiles + kRsBlocksPerSM * sms - 1) / (kRsBlocksPerSM * sms);  // resident blocks
+    return SortPlan{(uint32_t)((tiles + each - 1) / each), each * kRsTile};
+}
+
+__global__ void __launch_bounds__(kRsThreads) k_rs_hist(const uint32_t* __restrict__ keys, uint64_t n, int shift,
+                                                         uint64_t per, uint32_t* hist) {
     __shared__ uint32_t h[256];
-    for (int i = threadIdx.x; i < 256; i += blockDim.x) h[i] = 0;
+    if (threadIdx.x < 256) h[threadIdx.x] = 0;
     __syncthreads();
-    uint64_t base = (uint64_t)blockIdx.x * kRsTile;
-    for (int j = threadIdx.x; j < kRsTile; j += kRsThreads) {
-        uint64_t i = base + j;
-        if (i < n) atomicAdd(&h[(uint32_t)(keys[i] >> shift) & 255u], 1u);
+    const uint64_t r0 = blockIdx.x * per, r1 = min(r0 + per, n);
+    for (uint64_t i = r0 + 4 * threadIdx.x; i < r1; i += 4 * kRsThreads) {
+        if (i + 4 <= r1) {  // r0 is a multiple of the tile: 16-byte aligned
+            const uint4 v = *reinterpret_cast<const uint4*>(keys + i);
+            atomicAdd(&h[(v.x >> shift) & 255u], 1u);
+            atomicAdd(&h[(v.y >> shift) & 255u], 1u);
+            atomicAdd(&h[(v.z >> shift) & 255u], 1u);
+            atomicAdd(&h[(v.w >> shift) & 255u], 1u);
+        } else {
+            for (uint64_t j = i; j < r1; ++j) atomicAdd(&h[(keys[j] >> shift) & 255u], 1u);
+        }
     }
     __syncthreads();
-    for (int d = threadIdx.x; d < 256; d += kRsThreads) hist[(uint64_t)d * ntiles + blockIdx.x] = h[d];
+    if (threadIdx.x < 256) hist[(uint64_t)threadIdx.x * gridDim.x + blockIdx.x] = h[threadIdx.x];
 }
 
-template <class K>
-__global__ void __launch_bounds__(kRsThreads) k_rs_scatter(const K* __restrict__ kin,
-                                                            const uint32_t* __restrict__ vin,
-                                                            K* __restrict__ kout,
-                                                            uint32_t* __restrict__ vout, uint64_t n,
-                                                            int shift, const uint32_t* __restrict__ offs,
-                                                            uint32_t ntiles) {
-    __shared__ uint32_t wcnt[kRsWarps][256];
-    __shared__ uint32_t goff[256];
-    const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
-    for (int i = threadIdx.x; i < kRsWarps * 256; i += kRsThreads) (&wcnt[0][0])[i] = 0;
-    for (int d = threadIdx.x; d < 256; d += kRsThreads) goff[d] = offs[(uint64_t)d * ntiles + blockIdx.x];
-    __syncthreads();
-    const uint64_t base = (uint64_t)blockIdx.x * kRsTile + (uint64_t)w * (kRsItems * 32);
-    K key[kRsItems];
-    uint32_t val[kRsItems], rank[kRsItems];
-    const unsigned lt = lanemask_lt();
-#pragma unroll
-    for (int j = 0; j < kRsItems; ++j) {
-        uint64_t i = base + (uint64_t)j * 32 + l;
-        bool valid = i < n;
-        key[j] = valid ? kin[i] : (K)0;
-        val[j] = valid ? vin[i] : 0u;
-        unsigned act = __ballot_sync(0xffffffffu, valid);
-        rank[j] = 0;
-        if (valid) {
-            uint32_t d = (uint32_t)(key[j] >> shift) & 255u;
-            unsigned peers = __match_any_sync(act, d);
-            uint32_t cur = wcnt[w][d];
-            __syncwarp(act);
-            rank[j] = cur + __popc(peers & lt);
-            if (l == __ffs(peers) - 1) wcnt[w][d] = cur + __popc(peers);
-            __syncwarp(act);
-        }
-    }
-    __syncthreads();
-    if (threadIdx.x < 256) {
-        uint32_t run = 0;
-#pragma unroll
-        for (int ww = 0; ww < kRsWarps; ++ww) {
-            uint32_t c = wcnt[ww][threadIdx.x];
-            wcnt[ww][threadIdx.x] = run;
-            run += c;
-        }
-    }
-    __syncthreads();
-#pragma unroll
-    for (int j = 0; j < kRsItems; ++j) {
-        uint64_t i = base + (uint64_t)j * 32 + l;
-        if (i < n) {
-            uint32_t d = (uint32_t)(key[j] >> shift) & 255u;
-            uint32_t dst = goff[d] + wcnt[w][d] + rank[j];
-            kout[dst] = key[j];
-            vout[dst] = val[j];
-        }
-    }
-}
-
-// Exclusive scan of u32 (device-wide, recursive over block sums).
-constexpr int kScanThreads = 256, kScanItems = 8, kScanTile = kScanThreads * kScanItems;
-
-__global__ void __launch_bounds__(kScanThreads) k_scan_tile(uint32_t* data, uint64_t n, uint32_t* sums) {
-    __shared__ uint32_t warp_tot[kScanThreads / 32];
-    const uint64_t base = (uint64_t)blockIdx.x * kScanTile + (uint64_t)threadIdx.x * kScanItems;
-    uint32_t v[kScanItems];
-    uint32_t acc = 0;
-#pragma unroll
-    for (int j = 0; j < kScanItems; ++j) {
-        uint64_t i = base + j;
-        v[j] = i < n ? data[i] : 0u;
-        acc += v[j];
-    }
-    // exclusive scan of per-thread totals across the block
+// One block per digit: exclusive scan of its counts over the sorting blocks; total[digit].
+__global__ void __launch_bounds__(256) k_rs_scan(uint32_t* hist, uint32_t blocks, uint32_t* total) {
+    __shared__ uint32_t wsum[8];
     const int l = threadIdx.x & 31, w = threadIdx.x >> 5;
-    uint32_t incl = acc;
-    for (int o = 1; o < 32; o <<= 1) {
-        uint32_t t = __shfl_up_sync(0xffffffffu, incl, o);
-        if (l >= o) incl += t;
-    }
-    if (l == 31) warp_tot[w] = incl;
-    __syncthreads();
-    if (w == 0) {
-        uint32_t t = l < kScanThreads / 32 ? warp_tot[l] : 0u;
-        uint32_t ti = t;
+    uint32_t* h = hist + (uint64_t)blockIdx.x * blocks;
+    uint32_t carry = 0;
+    for (uint32_t b0 = 0; b0 < blocks; b0 += 256) {
+        const uint32_t i = b0 + threadIdx.x;
+        const uint32_t v = i < blocks ? h[i] : 0u;
+        uint32_t inc = v;
         for (int o = 1; o < 32; o <<= 1) {
-            uint32_t u = __shfl_up_sync(0xffffffffu, ti, o);
-            if (l >= o) ti += u;
+            const uint32_t t = __shfl_up_sync(0xffffffffu, inc, o);
+            if (l >= o) inc += t;
         }
-        if (l < kScanThreads / 32) warp_tot[l] = ti - t;
-        if (l == kScanThreads / 32 - 1 && sums) sums[blockIdx.x] = ti;
+        if (l == 31) wsum[w] = inc;
+        __syncthreads();
+        uint32_t before = carry, all = 0;
+        for (int j = 0; j < 8; ++j) {
+            before += j < w ? wsum[j] : 0u;
+            all += wsum[j];
+        }
+        if (i < blocks) h[i] = before + inc - v;
+        carry += all;
+        __syncthreads();
+    }
+    if (threadIdx.x == 0) total[blockIdx.x] = carry;
+}
+
+struct SortSmem {
+    uint32_t key[kRsTile], val[kRsTile];
+    uint32_t wcnt[kRsWarps][256];
+    uint32_t goff[256];   // next global position of the digit
+    uint32_t shift[256];  // goff of the tile less the digit's place in it
+    uint32_t wsum[8];
+};
+
+// FIRST: the values are the records' own numbers.
+template <bool FIRST>
+__global__ void __launch_bounds__(kRsThreads, kRsBlocksPerSM) k_rs_scatter(const uint32_t* __restrict__ kin,
+                                                               const uint32_t* __restrict__ vin,
+                                                               uint32_t* __restrict__ kout, uint32_t* __restrict__ vout,
+                                                               uint64_t n, int shift, uint64_t per,
+                                                               const uint32_t* __restrict__ offs,
+                                                               const uint32_t* __restrict__ total) {
+    extern __shared__ __align__(16) unsigned char smraw[];
+    SortSmem& s = *reinterpret_cast<SortSmem*>(smraw);
+    const int t = threadIdx.x, w = t >> 5, l = t & 31;
+    const unsigned lt = lanemask_lt();
+    // exclusive scan of one value per thread of the first 256 threads
+    auto scan256 = [&](uint32_t v) {
+        uint32_t inc = v;
+        if (t < 256) {
+            for (int o = 1; o < 32; o <<= 1) {
+                const uint32_t u = __shfl_up_sync(0xffffffffu, inc, o);
+                if (l >= o) inc += u;
+            }
+            if (l == 31) s.wsum[w] = inc;
+        }
+        __syncthreads();
+        uint32_t before = 0;
+        if (t < 256)
+            for (int j = 0; j < w; ++j) before += s.wsum[j];
+        __syncthreads();
+        return before + inc - v;
+    };
+    {
+        const uint32_t base = scan256(t < 256 ? total[t] : 0u);
+        if (t < 256) s.goff[t] = base + offs[(uint64_t)t * gridDim.x + blockIdx.x];
+    }
+    const uint64_t r0 = blockIdx.x * per, r1 = min(r0 + per, n);
+    for (uint64_t t0 = r0; t0 < r1; t0 += kRsTile) {
+        const uint32_t have = (uint32_t)min((uint64_t)kRsTile, r1 - t0);
+        for (int i = t; i < kRsWarps * 256; i += kRsThreads) (&s.wcnt[0][0])[i] = 0u;
+        uint32_t key[kRsItems], val[kRsItems], rank[kRsItems];
+        const uint32_t w0 = w * (kRsItems * 32) + l;
+#pragma unroll
+        for (int j = 0; j < kRsItems; ++j) {
+            const uint32_t i = w0 + j * 32;
+            key[j] = i < have ? kin[t0 + i] : 0xffffffffu;
+            if (!FIRST) val[j] = i < have ? vin[t0 + i] : 0u;
+        }
+        __syncthreads();
+#pragma unroll
+        for (int j = 0; j < kRsItems; ++j) {
+            const uint32_t i = w0 + j * 32;
+            const bool valid = i < have;
+            const uint32_t d = valid ? (key[j] >> shift) & 255u : 256u;  // lanes past the end match one another
+            const unsigned peers = __match_any_sync(0xffffffffu, d);
+            const uint32_t cur = valid ? s.wcnt[w][d] : 0u;
+            __syncwarp();
+            rank[j] = cur + __popc(peers & lt);
+            if (valid && l == __ffs(peers) - 1) s.wcnt[w][d] = cur + __popc(peers);
+            __syncwarp();
+        }
+        __syncthreads();
+        uint32_t cnt = 0;
+        if (t < 256) {
+#pragma unroll
+            for (int ww = 0; ww < kRsWarps; ++ww) {
+                const uint32_t c = s.wcnt[ww][t];
+                s.wcnt[ww][t] = cnt;
+                cnt += c;
+            }
+        }
+        const uint32_t place = scan256(cnt);
+        if (t < 256) {
+#pragma unroll
+            for (int ww = 0; ww < kRsWarps; ++ww) s.wcnt[ww][t] += place;
+            s.shift[t] = s.goff[t] - place;
+            s.goff[t] += cnt;
+        }
+        __syncthreads();
+#pragma unroll
+        for (int j = 0; j < kRsItems; ++j) {
+            const uint32_t i = w0 + j * 32;
+            if (i < have) {
+                const uint32_t at = s.wcnt[w][(key[j] >> shift) & 255u] + rank[j];
+                s.key[at] = key[j];
+                s.val[at] = FIRST ? (uint32_t)(t0 + i) : val[j];
+            }
+        }
+        __syncthreads();
+#pragma unroll 4
+        for (uint32_t i = t; i < have; i += kRsThreads) {
+            const uint32_t k = s.key[i];
+            const uint32_t dst = s.shift[(k >> shift) & 255u] + i;
+            kout[dst] = k;
+            vout[dst] = s.val[i];
+        }
+        __syncthreads();
+    }
+}
+
+// Keys of query positions and their first digit's histogram, by sorting block.
+__global__ void __launch_bounds__(kRsThreads) k_keys(const float4* __restrict__ a, uint64_t stride, uint64_t n,
+                                                      uint64_t per, const unsigned* __restrict__ box, int total,
+                                                      uint32_t* keys, uint32_t* hist) {
+    __shared__ uint32_t h[256];
+    if (threadIdx.x < 256) h[threadIdx.x] = 0;
+    __syncthreads();
+    const QueryGrid g = make_query_grid(box, total);
+    const uint64_t r0 = blockIdx.x * per, r1 = min(r0 + per, n);
+    for (uint64_t i = r0 + threadIdx.x; i < r1; i += kRsThreads) {
+        const float4 p = a[i * stride];
+        const uint32_t key = query_key(g, p.x, p.y, p.z);
+        keys[i] = key;
+        atomicAdd(&h[key & 255u], 1u);
     }
     __syncthreads();
-    uint32_t run = warp_tot[w] + incl - acc;
-#pragma unroll
-    for (int j = 0; j < kScanItems; ++j) {
-        uint64_t i = base + j;
-        if (i < n) data[i] = run;
-        run += v[j];
-    }
+    if (threadIdx.x < 256) hist[(uint64_t)threadIdx.x * gridDim.x + blockIdx.x] = h[threadIdx.x];
 }
 
-__global__ void k_scan_add(uint32_t* data, uint64_t n, const uint32_t* sums) {
-    uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
-    if (i < n) data[i] += sums[i / kScanTile];
-}
-
-// Returns -1 when a temporary could not be allocated (nothing is launched on it).
-static int exclusive_scan(Workspace& ws, uint32_t* data, uint64_t n, cudaStream_t st) {
-    uint64_t tiles = (n + kScanTile - 1) / kScanTile;
-    if (tiles <= 1) {
-        k_scan_tile<<<1, kScanThreads, 0, st>>>(data, n, nullptr);
-        note_launch();
-        return 0;
+// Record numbers of the positions a[0], a[stride], ... in Hilbert order of `bits`-bit keys into
+// order[n]; keys_out (nullable) receives the buffer of sorted keys, owned by ws. Returns -1
+// when a temporary could not be allocated (nothing is launched on it).
+static int hilbert_sort(Workspace& ws, const float4* a, uint64_t stride, uint64_t n, const unsigned* box, int bits,
+                        uint32_t* order, uint32_t** keys_out, cudaStream_t st) {
+    const SortPlan p = sort_plan(n);
+    uint32_t* hist = ws.take_u32((uint64_t)p.blocks * 256 + 256);
+    uint32_t* k0 = ws.take_u32(n);
+    uint32_t* k1 = ws.take_u32(n);
+    uint32_t* other = ws.take_u32(n);
+    if (!hist || !k0 || !k1 || !other) return -1;
+    uint32_t* total = hist + (uint64_t)p.blocks * 256;
+    static std::atomic<bool> attr_set[64];  // batched runs sort from several host threads
+    int dev = 0;
+    cudaGetDevice(&dev);
+    if (dev < 0 || dev >= 64 || !attr_set[dev].load(std::memory_order_acquire)) {
+        cudaFuncSetAttribute(k_rs_scatter<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(SortSmem));
+        cudaFuncSetAttribute(k_rs_scatter<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(SortSmem));
+        if (dev >= 0 && dev < 64) attr_set[dev].store(true, std::memory_order_release);
     }
-    uint32_t* sums = ws.take_u32(tiles);
-    if (!sums) return -1;
-    k_scan_tile<<<(unsigned)tiles, kScanThreads, 0, st>>>(data, n, sums);
-    note_launch();
-    if (exclusive_scan(ws, sums, tiles, st) != 0) return -1;
-    k_scan_add<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(data, n, sums);
-    note_launch();
+    const int passes = bits / 8;
+    // the passes alternate between the value buffers: the last one writes `order`
+    uint32_t* vin = nullptr;
+    uint32_t* vout = passes % 2 ? order : other;
+    for (int i = 0; i < passes; ++i) {
+        if (i == 0) k_keys<<<p.blocks, kRsThreads, 0, st>>>(a, stride, n, p.per, box, bits, k0, hist);
+        else k_rs_hist<<<p.blocks, kRsThreads, 0, st>>>(k0, n, 8 * i, p.per, hist);
+        k_rs_scan<<<256, 256, 0, st>>>(hist, p.blocks, total);
+        if (i == 0)
+            k_rs_scatter<true><<<p.blocks, kRsThreads, sizeof(SortSmem), st>>>(k0, vin, k1, vout, n, 0, p.per, hist, total);
+        else
+            k_rs_scatter<false><<<p.blocks, kRsThreads, sizeof(SortSmem), st>>>(k0, vin, k1, vout, n, 8 * i, p.per, hist, total);
+        for (int j = 0; j < 3; ++j) note_launch();
+        std::swap(k0, k1);
+        vin = vout;
+        vout = vin == order ? other : order;
+    }
+    if (keys_out) *keys_out = k0;
     return 0;
-}
-
-template <class K>
-static int radix_sort_pairs(Workspace& ws, K*& keys, uint32_t*& vals, K*& keys_alt, uint32_t*& vals_alt, uint64_t n,
-                            int bits, cudaStream_t st) {
-    if (n <= 1) return 0;
-    const uint32_t ntiles = (uint32_t)((n + kRsTile - 1) / kRsTile);
-    size_t mark = ws.mark();
-    uint32_t* hist = ws.take_u32((uint64_t)ntiles * 256);
-    if (!hist) {
-        ws.release(mark);
-        return -1;
-    }
-    int passes = 0;
-    for (int shift = 0; shift < bits; shift += 8) {
-        k_rs_hist<<<ntiles, kRsThreads, 0, st>>>(keys, n, shift, hist, ntiles);
-        note_launch();
-        if (exclusive_scan(ws, hist, (uint64_t)ntiles * 256, st) != 0) {
-            ws.release(mark);
-            return -1;
-        }
-        k_rs_scatter<<<ntiles, kRsThreads, 0, st>>>(keys, vals, keys_alt, vals_alt, n, shift, hist, ntiles);
-        note_launch();
-        std::swap(keys, keys_alt);
-        std::swap(vals, vals_alt);
-        ++passes;
-    }
-    ws.release(mark);
-    return passes;
 }
 
 // ------------------------------------------------------------------------------------------
@@ -1831,26 +1888,11 @@ void launch_single_cell_index(const float4* pts, uint32_t n, const uint32_t* per
 int sort_queries(Workspace& ws, const float4* qa, uint64_t n, uint32_t* perm, cudaStream_t st) {
     if (n == 0) return 0;
     const unsigned* box = bbox_device(ws, qa, n, st, 1);
+    if (!box) return -1;
     size_t mark = ws.mark();
-    uint32_t* keys = ws.take_u32(n);
-    uint32_t* vals2 = ws.take_u32(n);
-    uint32_t* keys2 = ws.take_u32(n);
-    if (!box || !keys || !keys2 || !vals2) {  // nothing launched on a failed allocation
-        ws.release(mark);
-        return -1;
-    }
-    const int bits = n <= (1ull << 18) ? 24 : 32;
-    // the passes swap the buffers: start so that the last one writes perm
-    uint32_t* k0 = keys;
-    uint32_t* v0 = (bits / 8) % 2 ? vals2 : perm;
-    uint32_t* v1 = (bits / 8) % 2 ? perm : vals2;
-    if (n == 1) v0 = perm;
-    unsigned blocks = (unsigned)std::min<uint64_t>((n + 255) / 256, 8192);
-    k_keys<<<blocks, 256, 0, st>>>(qa, n, box, bits, k0, v0);
-    note_launch();
-    const int rc = radix_sort_pairs<uint32_t>(ws, k0, v0, keys2, v1, n, bits, st);
+    const int rc = hilbert_sort(ws, qa, 1, n, box, n <= (1ull << 18) ? 24 : 32, perm, nullptr, st);
     ws.release(mark);
-    return rc < 0 ? -1 : 0;
+    return rc;
 }
 
 }  // namespace alb
