@@ -139,7 +139,7 @@ struct AlbCtx {
     uint64_t ex_cap = 0, ex_n = 0;
     // misc
     int* d_err = nullptr;
-    unsigned long long* d_stats = nullptr;
+    unsigned long long* d_stats = nullptr;  // 32 counters, then the scatter gather's work counter
     int keep_exit = 0, keep_ids = 0, precise = 1, sort_q = 1;
     int64_t map_cap_hint = 0;
     int launches = 0;
@@ -504,7 +504,7 @@ extern "C" int alb_create(const AlbSceneParams* p, int device, AlbCtx** out) {
     if (e.empty()) e = ensure_accumulators(ctx);
     if (!e.empty()) return bad(e);
     if (cudaMalloc(&ctx->d_rec_count, ALB_CHANNELS * 8) != cudaSuccess || cudaMalloc(&ctx->d_q_count, 3 * 8) != cudaSuccess ||
-        cudaMalloc(&ctx->d_err, sizeof(int)) != cudaSuccess || cudaMalloc(&ctx->d_stats, 32 * 8) != cudaSuccess)
+        cudaMalloc(&ctx->d_err, sizeof(int)) != cudaSuccess || cudaMalloc(&ctx->d_stats, 33 * 8) != cudaSuccess)
         return bad("counter allocation failed");
     cudaMemset(ctx->d_rec_count, 0, ALB_CHANNELS * 8);
     cudaMemset(ctx->d_q_count, 0, 3 * 8);
@@ -882,6 +882,7 @@ extern "C" int alb_trace(AlbCtx* ctx, int pass, uint64_t n, uint64_t seed, uint6
             q.stats = ctx->d_stats + 4 + 4 * c;  // per channel: leaves, nodes, selects, queries
             q.inexact = ctx->d_stats + 24 + c;
             q.retries = ctx->d_stats + 30;
+            q.ticket = (uint32_t*)(ctx->d_stats + 32);
             if (ctx->sort_q) {
                 PhaseTimer ps(ctx, 3);
                 const int src = sort_queries(ctx->ws, ctx->qa[k], nq, ctx->qperm[k], ctx->st);
@@ -1181,47 +1182,40 @@ extern "C" int alb_knn(AlbCtx* ctx, const float* pts, uint64_t m, const double* 
     if (m < (uint64_t)k) return fail(ctx, ALB_ERR_TOO_FEW, "fewer points than k");
     CK(cudaSetDevice(ctx->device));
     // the record's w lane carries its original index (bit pattern) through the sort
-    std::vector<float4> ha(m);
-    for (uint64_t i = 0; i < m; ++i) {
-        uint32_t tag = (uint32_t)i;
-        float w;
-        std::memcpy(&w, &tag, 4);
-        ha[i] = make_float4(pts[3 * i], pts[3 * i + 1], pts[3 * i + 2], w);
-    }
     RecordStore r{};
-    size_t mark = ctx->ws.mark();
+    const size_t mark = ctx->ws.mark();
     r.a = (float4*)ctx->ws.take_bytes(m * 32);  // interleaved store (RecordStore)
     r.b = r.a ? r.a + 1 : nullptr;
+    float* dp = (float*)ctx->ws.take_bytes(m * 12);
     double* dq = (double*)ctx->ws.take_bytes(nq * 24);
+    float4* qa = (float4*)ctx->ws.take_bytes(nq * 16);
+    uint32_t* perm = ctx->ws.take_u32(nq);
     int32_t* di = (int32_t*)ctx->ws.take_bytes(nq * k * 4);
     double* dd = (double*)ctx->ws.take_bytes(nq * k * 8);
-    if (!r.a || !dq || !di || !dd) return fail(ctx, ALB_ERR_CUDA, "knn allocation failed");
-    CK(cudaMemsetAsync(r.a, 0, m * 32, ctx->st));
-    CK(cudaMemcpy2DAsync(r.a, 32, ha.data(), 16, 16, m, cudaMemcpyHostToDevice, ctx->st));
-    CK(cudaMemcpyAsync(dq, qs, nq * 24, cudaMemcpyHostToDevice, ctx->st));
     MapIndex mi;
-    if (build_map_index(ctx->ws, r, m, mi, ctx->st) != 0) return fail(ctx, ALB_ERR_CAPACITY, "knn index build failed");
-    // indices returned by the search refer to the sorted order: map them back
-    launch_knn(map_dev(mi), dq, nq, k, di, dd, ctx->d_err, ctx->st);
-    std::vector<int32_t> sorted_idx(nq * k);
-    int rc = check_device(ctx, "knn");
-    if (rc) {
+    auto done = [&](int rc) {
         cudaFree(mi.a); cudaFree(mi.b); cudaFree(mi.box_lo); cudaFree(mi.box_hi);
         ctx->ws.release(mark);
         return rc;
-    }
-    CK(cudaMemcpy(sorted_idx.data(), di, nq * k * 4, cudaMemcpyDeviceToHost));
-    CK(cudaMemcpy(dist, dd, nq * k * 8, cudaMemcpyDeviceToHost));
-    std::vector<float4> sa(mi.n);  // the index may hold more slots than points
-    CK(cudaMemcpy(sa.data(), mi.a, mi.n * 16, cudaMemcpyDeviceToHost));
-    cudaFree(mi.a); cudaFree(mi.b); cudaFree(mi.box_lo); cudaFree(mi.box_hi);
-    ctx->ws.release(mark);
-    for (uint64_t i = 0; i < nq * (uint64_t)k; ++i) {
-        uint32_t tag;
-        std::memcpy(&tag, &sa[sorted_idx[i]].w, 4);
-        idx[i] = (int32_t)tag;
-    }
-    return ALB_OK;
+    };
+    if (!r.a || !dp || !dq || !qa || !perm || !di || !dd) return done(fail(ctx, ALB_ERR_CUDA, "knn allocation failed"));
+    auto ok = [&](cudaError_t e) { return e == cudaSuccess; };
+    if (!ok(cudaMemcpyAsync(dp, pts, m * 12, cudaMemcpyHostToDevice, ctx->st)) ||
+        !ok(cudaMemcpyAsync(dq, qs, nq * 24, cudaMemcpyHostToDevice, ctx->st)))
+        return done(fail(ctx, ALB_ERR_CUDA, "knn upload failed"));
+    pack_knn_points(dp, m, r.a, ctx->st);
+    if (build_map_index(ctx->ws, r, m, mi, ctx->st) != 0)
+        return done(fail(ctx, ALB_ERR_CAPACITY, "knn index build failed"));
+    if (nq) pack_knn_queries(dq, nq, qa, ctx->st);
+    if (sort_queries(ctx->ws, qa, nq, perm, ctx->st) != 0) return done(fail(ctx, ALB_ERR_CUDA, "knn query sort failed"));
+    launch_knn(map_dev(mi), dq, perm, nq, k, di, dd, ctx->d_err, ctx->st);
+    const int rc = check_device(ctx, "knn");
+    if (rc) return done(rc);
+    if (!ok(cudaMemcpyAsync(idx, di, nq * k * 4, cudaMemcpyDeviceToHost, ctx->st)) ||
+        !ok(cudaMemcpyAsync(dist, dd, nq * k * 8, cudaMemcpyDeviceToHost, ctx->st)) ||
+        !ok(cudaStreamSynchronize(ctx->st)))
+        return done(fail(ctx, ALB_ERR_CUDA, "knn download failed"));
+    return done(ALB_OK);
 }
 
 extern "C" int alb_stats(AlbCtx* ctx, int64_t* out, int n) {

@@ -33,9 +33,6 @@ constexpr int kGatherBlocksPerSM = 4;
 // 546 ms, 64 -> 529 ms, 128 -> 524 ms; the planar maps' gathers lose 2-3% at 128). Fewer
 // queries than fill the resident warps with such chunks take shorter ones (query_chunk).
 constexpr int kQueryChunk = 64;
-// scatter queries a warp fetches at a time (large scene, 1e7 photons: 16 -> 296 ms, 32 -> 297, 64 -> 305;
-// 1e6: 30.5, 29.7, 30.1)
-constexpr int kScatterChunk = 32;
 constexpr int kQueryChunkMin = 2;
 constexpr int kStack = 32 * kMaxLevels;
 constexpr int kCap = 288;         // candidate buffer (k <= kCap - 32)
@@ -372,11 +369,16 @@ struct KnnResult {
                    // finite points admitted: a NaN or infinite query or map coordinates)
 };
 
+// Position of a point: a map record's, or one of a packed array.
+ALB_DEVICE float4 point_at(const MapDev& m, uint32_t i) { return m.a[i]; }
+template <class P>
+ALB_DEVICE float4 point_at(const P& p, uint32_t i) { return p.at(i); }
+
 // float64 ranking of the band entries bi[0..nb) by (distance, tie key, map position); the
 // `take` smallest go to ci[dst ..] in rank order. Returns the float64 squared distance of
 // the take-th (0 if the band holds fewer).
-template <class S>
-ALB_DEVICE double rank_band(const MapDev& m, S& s, int dst, int nb, int take, double qx, double qy,
+template <class M, class S>
+ALB_DEVICE double rank_band(const M& m, S& s, int dst, int nb, int take, double qx, double qy,
                             double qz, const float4* tie_rec) {
     const int l = lane_id();
     double di = 0.0;
@@ -385,7 +387,7 @@ ALB_DEVICE double rank_band(const MapDev& m, S& s, int dst, int nb, int take, do
     int rank = 0;
     if (l < nb) {
         ii = s.bi[l];
-        const float4 a = m.a[ii];
+        const float4 a = point_at(m, ii);
         di = point_dist2_f64(qx, qy, qz, a);
         ti = tie_rec ? record_tie_key(a, tie_rec[ii]) : 0ull;
         s.bd[l] = di;
@@ -411,8 +413,8 @@ ALB_DEVICE double rank_band(const MapDev& m, S& s, int dst, int nb, int take, do
 // The k_sub nearest among the entries [off, off + n) whose cd/cl hold refined keys: keys more
 // than one unit below the k_sub-th are in, keys within one unit of it are ranked in float64.
 // The chosen map positions end up in ci[off .. off + k_sub).
-template <class S>
-ALB_DEVICE double select_refined(const MapDev& m, S& s, int off, int n, int k_sub, double qx, double qy,
+template <class M, class S>
+ALB_DEVICE double select_refined(const M& m, S& s, int off, int n, int k_sub, double qx, double qy,
                                  double qz, const float4* tie_rec, int& clipped) {
     const int l = lane_id();
     const uint64_t K = warp_kth_key<6>(s, off, n, k_sub);
@@ -1270,40 +1272,81 @@ __device__ __noinline__ bool cold_knn(const MapDev& m, S& s, int k, float fx, fl
     return true;
 }
 
-// Scatter-map gather, k nearest, by runs of neighbouring queries (gather_group.cuh). One CTA per SM
-// takes one contiguous range of the sorted queries, so that its leaves stay local; its warps fetch
-// chunks of the range in turn.
+// Scatter-map gather, k nearest, by runs of neighbouring queries (gather_group.cuh). One CTA per SM.
+// The sorted queries are cut into segments that CTAs take in turn: the first half of them in
+// four per CTA, half of the rest in four per CTA, and so on (ScatterPlan), since the work of a
+// range varies with the density of the map around it: with one range per SM the slowest of 152 SMs
+// issued 19% more than the mean, 27.5 against 22.9 ms at 1e6 photons of the large scene. (Two
+// segments per CTA and level: 22.9 ms, 237 at 1e7 photons; four: 23.1, 234; eight: 23.5, 230.)
+// A segment is 64 chunks; the CTA's warps fetch chunks in turn.
+struct ScatterPlan {
+    uint64_t first, n;  // the launch's range of the sorted queries
+    uint32_t pieces;    // segments per level
+    int levels;         // level L holds half of what the levels before it left, the last one the rest
+    uint32_t* ticket;   // segments taken, zero at the launch
+};
+constexpr int kSegChunks = 64;
+constexpr int kSegRing = 64;  // segments of a CTA whose numbers are kept
+
+ALB_DEVICE void segment_range(const ScatterPlan& p, uint32_t g, uint64_t& s0, uint64_t& s1) {
+    const uint32_t lev = g / p.pieces, j = g % p.pieces;
+    const uint64_t left = p.n >> lev;
+    const uint64_t m = (int)lev == p.levels - 1 ? left : left - (p.n >> (lev + 1));
+    const uint64_t base = p.first + (p.n - left);
+    s0 = base + m * j / p.pieces;
+    s1 = base + m * (j + 1) / p.pieces;
+}
+
 template <int MODE, int CAP, int WARPS>
 __global__ void __launch_bounds__(WARPS * 32, 1)
     k_gather_scatter(const __grid_constant__ SceneDev sc, const __grid_constant__ MapDev m,
-                     const __grid_constant__ QueryDev q, const __grid_constant__ Accum acc, int k, int* err, uint32_t chunk,
-                     uint64_t first, uint64_t n) {
+                     const __grid_constant__ QueryDev q, const __grid_constant__ Accum acc, int k, int* err,
+                     const __grid_constant__ ScatterPlan plan) {
     extern __shared__ __align__(16) unsigned char group_raw[];
     using S = GroupSmem<CAP>;
     S* smem = reinterpret_cast<S*>(group_raw);
     __shared__ uint32_t next;  // the CTA's next chunk
     __shared__ float last2;    // squared k-th distance of some query just answered (a chunk's first guess)
+    // (the CTA's segment number << 32) | its global number; a segment's number is fetched by the
+    // warp that takes the first chunk of the one before it
+    __shared__ unsigned long long ring[kSegRing];
+    if (threadIdx.x < kSegRing) ring[threadIdx.x] = ~0ull;
+    __syncthreads();
     if (threadIdx.x == 0) {
         next = 0u;
         last2 = -1.f;
+        ring[0] = atomicAdd(plan.ticket, 1u);
     }
     __syncthreads();
     const int w = threadIdx.x >> 5, l = lane_id();
     S& s = smem[w];
-    const uint64_t seg0 = first + n * blockIdx.x / gridDim.x, seg1 = first + n * (blockIdx.x + 1) / gridDim.x;
+    const uint32_t segments = plan.pieces * (uint32_t)plan.levels;
     // edge of a cubic leaf over the k-th distance: 32 records against k in the ball
     const float side_rk = cbrtf(134.04f / (float)k);
     bool failed = false;
     if (l < 5) s.st[l] = 0ull;
     __syncwarp();
     while (!failed) {
-        uint32_t ch = 0u;
-        if (l == 0) ch = atomicAdd(&next, 1u);
-        ch = __shfl_sync(0xffffffffu, ch, 0);
-        const uint64_t c0 = seg0 + (uint64_t)ch * chunk;
-        if (c0 >= seg1) break;
-        const uint64_t q_end = min(c0 + chunk, seg1);
-        QueryRun run{0, 0, 0.f};
+        uint32_t t = 0u, g = 0u;
+        if (l == 0) {
+            t = atomicAdd(&next, 1u);
+            const uint32_t seg = t / kSegChunks;
+            volatile unsigned long long* v = ring;
+            if (t % kSegChunks == 0) v[(seg + 1) % kSegRing] = (unsigned long long)(seg + 1) << 32 | atomicAdd(plan.ticket, 1u);
+            // published 64 chunks ago; the bound only guards against a lost slot
+            unsigned long long e = v[seg % kSegRing];
+            for (int wait = 0; (uint32_t)(e >> 32) != seg && wait < (1 << 20); ++wait) e = v[seg % kSegRing];
+            if ((uint32_t)(e >> 32) != seg) atomicCAS(err, 0, ALB_ERR_ITER_CAP);
+            g = (uint32_t)(e >> 32) == seg ? (uint32_t)e : 0xffffffffu;
+        }
+        t = __shfl_sync(0xffffffffu, t, 0) % kSegChunks;
+        g = __shfl_sync(0xffffffffu, g, 0);
+        if (g >= segments) break;
+        uint64_t s0, s1;
+        segment_range(plan, g, s0, s1);
+        const uint64_t c0 = s0 + (s1 - s0) * t / kSegChunks, q_end = s0 + (s1 - s0) * (t + 1) / kSegChunks;
+        if (c0 == q_end) continue;
+        QueryRun run{0, 0, 0, 0.f};
         uint64_t r_base = 0;  // first query of the run the lanes hold
         uint32_t gsrc = 0u;   // this lane's query of the run: index and position
         float gx = 0.f, gy = 0.f, gz = 0.f;
@@ -1333,7 +1376,9 @@ __global__ void __launch_bounds__(WARPS * 32, 1)
                         }
                     }
                     run.take = 1;
+                    run.nodes = 0;
                     if (listed) listed = build_run(m, s, avail, gx, gy, gz, la, prev2, side_rk * sqrtf(prev2), run);
+                    if (l == 0) s.st[1] += run.nodes;
                 }
                 const int at = (int)(qi - r_base);
                 src = __shfl_sync(0xffffffffu, gsrc, at);
@@ -1402,48 +1447,182 @@ __global__ void __launch_bounds__(WARPS * 32, 1)
     }
 }
 
-// Standalone KDTree.query(x, k): sorted indices and float64 distances.
-__global__ void __launch_bounds__(kGatherWarps * 32) k_knn(MapDev m, const double* __restrict__ qs, uint64_t nq,
-                                                           int k, int32_t* out_idx, double* out_dist, int* err) {
+// The float64 squared distance from (qx, qy, qz) to point r, for the answers of a search.
+struct MapPoints {
+    const float4* a;
+    ALB_DEVICE float4 at(uint32_t r) const { return a[r]; }
+};
+struct PackedPoints {
+    const float* p;
+    ALB_DEVICE float4 at(uint32_t r) const { return make_float4(p[3 * r], p[3 * r + 1], p[3 * r + 2], 0.f); }
+};
+
+// One query's k neighbours s.ci[0 .. k) in order of (float64 distance, index), as out_idx / out_dist
+// rows of k. Every distance is formed once and ranked as its bit pattern against the others in
+// shared memory (non-negative doubles order like integers): comparing k x k freshly formed
+// distances took 4400 FP64 instructions per query at k = 100, at two FP64 lanes per SM and cycle.
+// tag: the index to report for a position (nullptr: the position itself).
+template <class P>
+ALB_DEVICE void write_sorted(const P& pts, WarpSmem& s, int k, double qx, double qy, double qz, const float4* tag,
+                             int32_t* out_idx, double* out_dist) {
+    const int l = lane_id();
+    static_assert(sizeof(s.stk) + sizeof(s.stk_d) >= 256 * sizeof(uint64_t), "the bit patterns lie in the stack");
+    uint64_t* bits = reinterpret_cast<uint64_t*>(s.stk);
+    for (int j = l; j < k; j += 32)
+        bits[j] = (uint64_t)__double_as_longlong(point_dist2_f64(qx, qy, qz, pts.at(s.ci[j])));
+    __syncwarp();
+    int sum = 0;
+    for (int j0 = 0; j0 < k; j0 += 128) {
+        uint64_t own[4];
+        int rank[4] = {0, 0, 0, 0};
+#pragma unroll
+        for (int i = 0; i < 4; ++i) own[i] = j0 + i * 32 + l < k ? bits[j0 + i * 32 + l] : 0ull;
+#pragma unroll 2
+        for (int t = 0; t < k; ++t) {
+            const uint64_t o = bits[t];
+#pragma unroll
+            for (int i = 0; i < 4; ++i) rank[i] += o < own[i] ? 1 : 0;
+        }
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const int j = j0 + i * 32 + l;
+            if (j < k) {
+                sum += rank[i];
+                s.cd[j] = __int_as_float(rank[i]);
+            }
+        }
+    }
+    __syncwarp();
+    // equal distances leave the ranks short of 0 .. k - 1: rank those by index too
+    if (__reduce_add_sync(0xffffffffu, sum) != k * (k - 1) / 2) {
+        for (int j = l; j < k; j += 32) {
+            int extra = 0;
+            for (int t = 0; t < k; ++t) extra += bits[t] == bits[j] && s.ci[t] < s.ci[j] ? 1 : 0;
+            s.cd[j] = __int_as_float(__float_as_int(s.cd[j]) + extra);
+        }
+    }
+    for (int j = l; j < k; j += 32) {
+        const uint32_t idx = s.ci[j];
+        const int rank = __float_as_int(s.cd[j]);
+        out_idx[rank] = tag ? (int32_t)__float_as_uint(tag[idx].w) : (int32_t)idx;
+        out_dist[rank] = sqrt(__longlong_as_double((long long)bits[j]));
+    }
+    __syncwarp();
+}
+
+// A query without an answer gets index -1 and distance NaN in all its k slots, so no slot is left
+// holding whatever the caller's buffer held before.
+ALB_DEVICE void write_failed(int k, int32_t* out_idx, double* out_dist) {
+    for (int j = lane_id(); j < k; j += 32) {
+        out_idx[j] = -1;
+        out_dist[j] = __longlong_as_double(0x7ff8000000000000ll);
+    }
+    __syncwarp();
+}
+
+// Standalone KDTree.query(x, k): sorted indices (the w lanes of the map's records) and float64
+// distances. Queries go in `perm` order, `chunk` consecutive ones per warp, each bounded by the
+// farthest of its predecessor's neighbours.
+__global__ void __launch_bounds__(kGatherWarps * 32, kGatherBlocksPerSM)
+    k_knn(MapDev m, const double* __restrict__ qs, const uint32_t* __restrict__ perm, uint64_t nq, uint32_t chunk, int k,
+          int32_t* out_idx, double* out_dist, int* err) {
     __shared__ WarpSmem smem[kGatherWarps];
     const int w = threadIdx.x >> 5, l = lane_id();
     WarpSmem& s = smem[w];
     const uint64_t warps = (uint64_t)gridDim.x * kGatherWarps;
-    for (uint64_t qi = (uint64_t)blockIdx.x * kGatherWarps + w; qi < nq; qi += warps) {
-        double qx = qs[3 * qi], qy = qs[3 * qi + 1], qz = qs[3 * qi + 2];
-        KnnResult r;
-        const float fx = (float)qx, fy = (float)qy, fz = (float)qz;
-        int why = 0;
-        if (!warp_knn<true>(m, s, k, qx, qy, qz, fx, fy, fz, (float)(qx - (double)fx), (float)(qy - (double)fy),
-                            (float)(qz - (double)fz), FLT_MAX, nullptr, r))
-            why = ALB_ERR_TOO_FEW;
-        else if (r.fail)
-            why = r.fail;
-        if (why) {
-            // a query without an answer gets index -1 and distance NaN in all its k slots,
-            // so no slot is left holding whatever the caller's buffer held before
-            if (l == 0) atomicCAS(err, 0, why);
-            for (int j = l; j < k; j += 32) {
-                out_idx[qi * k + j] = -1;
-                out_dist[qi * k + j] = __longlong_as_double(0x7ff8000000000000ll);
+    const uint64_t chunks = (nq + chunk - 1) / chunk;
+    for (uint64_t ch = (uint64_t)blockIdx.x * kGatherWarps + w; ch < chunks; ch += warps) {
+        const uint64_t q_end = min((ch + 1) * chunk, nq);
+        bool have_prev = false;
+        for (uint64_t i = ch * chunk; i < q_end; ++i) {
+            const uint64_t qi = perm[i];
+            const double qx = qs[3 * qi], qy = qs[3 * qi + 1], qz = qs[3 * qi + 2];
+            const float fx = (float)qx, fy = (float)qy, fz = (float)qz;
+            const float lx = (float)(qx - (double)fx), ly = (float)(qy - (double)fy), lz = (float)(qz - (double)fz);
+            float bound = FLT_MAX;
+            if (have_prev) {
+                unsigned mx = 0u;
+                for (int j = l; j < k; j += 32)
+                    mx = max(mx, __float_as_uint(point_dist2(fx, fy, fz, lx, ly, lz, m.a[s.ci[j]])));
+                const float t = __uint_as_float(__reduce_max_sync(0xffffffffu, mx)) * (1.f + 1.f / 16384.f);
+                if (t < 1.0e37f) bound = t;
             }
-            __syncwarp();
+            KnnResult r;
+            int why = 0;
+            if (!warp_knn<true>(m, s, k, qx, qy, qz, fx, fy, fz, lx, ly, lz, bound, nullptr, r)) why = ALB_ERR_TOO_FEW;
+            else if (r.fail) why = r.fail;
+            have_prev = !why;
+            if (why) {
+                if (l == 0) atomicCAS(err, 0, why);
+                write_failed(k, out_idx + qi * k, out_dist + qi * k);
+                continue;
+            }
+            write_sorted(MapPoints{m.a}, s, k, qx, qy, qz, m.a, out_idx + qi * k, out_dist + qi * k);
+        }
+    }
+}
+
+// The k nearest of at most a few thousand points float[3 m] by screening all of them, one warp per
+// query: no index, no scratch memory, one launch. At 4096 points the 128 screening steps cost what
+// a walk over a tree does, and the tree's one-CTA build cost 0.8 ms on top.
+constexpr int kBruteWarps = 4;
+__global__ void __launch_bounds__(kBruteWarps * 32) k_knn_brute(const float* __restrict__ pts, uint32_t m,
+                                                                const double* __restrict__ qs, uint64_t nq, int k,
+                                                                int32_t* out_idx, double* out_dist) {
+    __shared__ WarpSmem smem[kBruteWarps];
+    const int w = threadIdx.x >> 5, l = lane_id();
+    WarpSmem& s = smem[w];
+    const PackedPoints pp{pts};
+    for (uint64_t qi = (uint64_t)blockIdx.x * kBruteWarps + w; qi < nq; qi += (uint64_t)gridDim.x * kBruteWarps) {
+        const double qx = qs[3 * qi], qy = qs[3 * qi + 1], qz = qs[3 * qi + 2];
+        const float fx = (float)qx, fy = (float)qy, fz = (float)qz;
+        const float lx = (float)(qx - (double)fx), ly = (float)(qy - (double)fy), lz = (float)(qz - (double)fz);
+        float thr = FLT_MAX;
+        int cnt = 0, clipped = 0;
+        constexpr int kAhead = 4;  // steps whose points are loaded together
+        for (uint32_t r0 = 0; r0 < m; r0 += 32 * kAhead) {
+            float4 p[kAhead];
+#pragma unroll
+            for (int i = 0; i < kAhead; ++i) {
+                const uint32_t r = r0 + i * 32 + l;
+                p[i] = r < m ? pp.at(r) : make_float4(0.f, 0.f, 0.f, 0.f);
+            }
+#pragma unroll
+            for (int i = 0; i < kAhead; ++i) {
+                const uint32_t r = r0 + i * 32 + l;
+                const float d = point_dist2(fx, fy, fz, lx, ly, lz, p[i]);
+                const bool take = r < m && d <= thr;
+                const unsigned b = __ballot_sync(0xffffffffu, take);
+                if (take) {
+                    const int pos = cnt + __popc(b & lanemask_lt());
+                    float hi, lo;
+                    point_dist2_df(fx, fy, fz, lx, ly, lz, p[i], hi, lo);
+                    s.ci[pos] = r;
+                    s.cd[pos] = hi;
+                    s.cl[pos] = frac16(hi, lo);
+                }
+                cnt += __popc(b);
+                __syncwarp();
+                if (cnt >= k && (thr == FLT_MAX || cnt > kCap - 32)) {
+                    // refined distances within one float32 ulp of the k-th can still rank
+                    const float kth = warp_kth32(s, 0, cnt, k);
+                    thr = fminf(thr, kth * (1.0f + 2.0f * kRelMargin));
+                    cnt = warp_compact(s, cnt, __uint_as_float(__float_as_uint(kth) + 1u));
+                    if (cnt > kCap - 32) {  // mass ties
+                        cnt = warp_compact(s, cnt, kth);
+                        clipped = 1;
+                    }
+                    if (cnt > kCap - 32) cnt = kCap - 32;
+                }
+            }
+        }
+        if (cnt < k) {
+            write_failed(k, out_idx + qi * k, out_dist + qi * k);
             continue;
         }
-        // float64 distances of the k neighbours, then rank-sort them (k <= kMaxK)
-        for (int j = l; j < k; j += 32) {
-            uint32_t idx = s.ci[j];
-            double d = point_dist2_f64(qx, qy, qz, m.a[idx]);
-            int rank = 0;
-            for (int t = 0; t < k; ++t) {
-                uint32_t it = s.ci[t];
-                double dt = point_dist2_f64(qx, qy, qz, m.a[it]);
-                rank += (dt < d || (dt == d && it < idx)) ? 1 : 0;
-            }
-            out_idx[qi * k + rank] = (int32_t)idx;
-            out_dist[qi * k + rank] = sqrt(d);
-        }
-        __syncwarp();
+        // select_refined ranks the near ties on their float64 distances
+        select_refined(pp, s, 0, cnt, k, qx, qy, qz, nullptr, clipped);
+        write_sorted(pp, s, k, qx, qy, qz, nullptr, out_idx + qi * k, out_dist + qi * k);
     }
 }
 
@@ -1514,11 +1693,13 @@ static void launch_scatter(const SceneDev& sc, const MapDev& map, const QueryDev
     // a class word holds kClassMost contributions: more queries go in slices
     const uint64_t most = kClassMost / (uint64_t)k;
     for (uint64_t first = 0; first < q.n; first += most) {
-        const uint64_t n = std::min<uint64_t>(most, q.n - first);
-        const uint64_t blocks = std::min<uint64_t>(sm_count(), n);
-        const uint64_t fit = (n + blocks * WARPS - 1) / (blocks * WARPS);
-        const uint32_t chunk = (uint32_t)std::min<uint64_t>(kScatterChunk, fit);
-        kernel<<<(unsigned)blocks, WARPS * 32, bytes, st>>>(sc, map, q, acc, k, err, chunk, first, n);
+        ScatterPlan plan{first, std::min<uint64_t>(most, q.n - first), 0u, 1, q.ticket};
+        const uint64_t blocks = std::min<uint64_t>(sm_count(), plan.n);
+        plan.pieces = (uint32_t)(4 * blocks);
+        // levels until a segment's chunks hold eight queries
+        while (plan.levels < 16 && (plan.n >> plan.levels) >= (uint64_t)plan.pieces * kSegChunks * 8) ++plan.levels;
+        cudaMemsetAsync(q.ticket, 0, sizeof(uint32_t), st);
+        kernel<<<(unsigned)blocks, WARPS * 32, bytes, st>>>(sc, map, q, acc, k, err, plan);
         note_launch();
         merge_classes(sc, acc, ALB_SCATTER, true, st);
     }
@@ -1570,10 +1751,19 @@ void launch_gather(const SceneDev& sc, const MapDev& map, const QueryDev& q, int
     if (launches) ++*launches;
 }
 
-void launch_knn(const MapDev& map, const double* queries, uint64_t nq, int k, int32_t* out_idx, double* out_dist,
-                int* err, cudaStream_t st) {
+void launch_knn(const MapDev& map, const double* queries, const uint32_t* perm, uint64_t nq, int k, int32_t* out_idx,
+                double* out_dist, int* err, cudaStream_t st) {
     if (nq == 0) return;
-    k_knn<<<gather_blocks(nq), kGatherWarps * 32, 0, st>>>(map, queries, nq, k, out_idx, out_dist, err);
+    const uint32_t chunk = query_chunk(nq, false);
+    k_knn<<<gather_blocks((nq + chunk - 1) / chunk), kGatherWarps * 32, 0, st>>>(map, queries, perm, nq, chunk, k, out_idx,
+                                                                                  out_dist, err);
+    note_launch();
+}
+
+void launch_knn_brute(const float* pts, uint32_t m, const double* queries, uint64_t nq, int k, int32_t* out_idx,
+                      double* out_dist, cudaStream_t st) {
+    const unsigned blocks = (unsigned)std::min<uint64_t>((nq + kBruteWarps - 1) / kBruteWarps, (uint64_t)sm_count() * 16);
+    k_knn_brute<<<blocks, kBruteWarps * 32, 0, st>>>(pts, m, queries, nq, k, out_idx, out_dist);
     note_launch();
 }
 

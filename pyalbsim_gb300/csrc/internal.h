@@ -83,6 +83,7 @@ struct QueryDev {
     double* rk_out;    // optional per-query k-th neighbour distance
     unsigned long long* stats;    // optional [leaves, nodes, selects, queries] accumulators
     unsigned long long* inexact;  // optional count of answers a buffer bound made inexact (mass ties)
+    uint32_t* ticket;  // work counter of the scatter gather
     unsigned long long* retries;  // optional count of searches redone because a first guess did not hold
 };
 
@@ -128,11 +129,8 @@ class Workspace {
 };
 
 // ---- map build (mapbuild.cu)
-int compute_bbox(Workspace& ws, const float4* a, uint64_t n, float lo[3], float hi[3], cudaStream_t st,
-                 uint64_t stride = 1);
 int build_map_index(Workspace& ws, const RecordStore& rec, uint64_t n, MapIndex& m, cudaStream_t st);
 void release_map_index(MapIndex& m);
-int build_box_tree(Workspace& ws, MapIndex& m, cudaStream_t st);
 int sort_queries(Workspace& ws, const float4* qa, uint64_t n, uint32_t* perm, cudaStream_t st);
 
 // ---- tracer (tracer.cu)
@@ -144,8 +142,12 @@ void launch_trace(const SceneDev& sc, const TraceOut& out, int pass, uint64_t n,
 // ---- gather (gather.cu)
 void launch_gather(const SceneDev& sc, const MapDev& map, const QueryDev& q, int channel, const Accum& acc,
                    int* err, int* launches, cudaStream_t st);
-void launch_knn(const MapDev& map, const double* queries, uint64_t nq, int k, int32_t* out_idx,
+void launch_knn(const MapDev& map, const double* queries, const uint32_t* perm, uint64_t nq, int k, int32_t* out_idx,
                 double* out_dist, int* err, cudaStream_t st);
+void launch_knn_brute(const float* pts, uint32_t m, const double* queries, uint64_t nq, int k, int32_t* out_idx,
+                      double* out_dist, cudaStream_t st);
+void pack_knn_points(const float* pts, uint64_t m, float4* rec, cudaStream_t st);
+void pack_knn_queries(const double* qs, uint64_t n, float4* qa, cudaStream_t st);
 
 inline MapDev map_dev(const MapIndex& m) {
     MapDev d{};

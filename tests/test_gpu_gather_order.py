@@ -103,3 +103,39 @@ def test_heatmap_cells_match_the_precise_formula(gpu_available, bins):
         # truncation toward zero puts (-1, 0) into cell 0 on both grids: the outermost row and
         # column of the coarse map reach one coarse cell out, those of the fine map one fine cell
         np.testing.assert_allclose(pairs[1:, 1:], coarse[1:, 1:], rtol=1e-12, atol=1e-300)
+
+
+def _check_knn(pts, qs, k):
+    from scipy.spatial import cKDTree
+
+    with GpuEngine(workloads.small()) as eng:
+        dist, idx = eng.ctx.knn(pts, qs, k)
+    ref, _ = cKDTree(pts.astype(np.float64)).query(qs, k=range(1, k + 1))
+    # the same three products and two sums in float64, and a square root: under 4 eps
+    np.testing.assert_allclose(dist, ref, rtol=4 * np.finfo(np.float64).eps, atol=0)
+    d = np.sqrt(((pts[idx].astype(np.float64) - qs[:, None, :]) ** 2).sum(axis=2))
+    np.testing.assert_allclose(d, dist, rtol=4 * np.finfo(np.float64).eps, atol=0)
+
+
+@pytest.mark.parametrize("planar", [False, True])
+@pytest.mark.parametrize("m", [1, 31, 33, 255, 256, 257, 4_097, 65_536, 65_537])
+def test_index_of_every_size_answers_like_kdtree(gpu_available, m, planar):
+    """Records at the edges of a leaf, of a warp's 256, of a sort tile and of the 24-bit keys."""
+    rng = np.random.default_rng(m)
+    pts = rng.normal(scale=[0.3, 1.0, 0.3], size=(m, 3)).astype(np.float32)
+    qs = rng.uniform(-2.0, 2.0, size=(200, 3))
+    if planar:
+        pts[:, 1] = -400.0
+        qs[:, 1] = -400.0
+    _check_knn(pts, qs, min(m, 20))
+
+
+@pytest.mark.parametrize("m", [3_000, 70_001])
+def test_index_of_crowded_keys_answers_like_kdtree(gpu_available, m):
+    """One point a thousand kilometres away: the keys cannot tell the others apart, and the records
+    take the exact k-d order. Duplicates and a lattice beside it."""
+    rng = np.random.default_rng(m)
+    pts = rng.normal(scale=0.2, size=(m, 3))
+    pts[: m // 3] = np.round(pts[: m // 3] * 20.0) / 20.0
+    pts[0] = [1.0e6, 0.0, 0.0]
+    _check_knn(pts.astype(np.float32), rng.uniform(-0.5, 0.5, size=(100, 3)), 33)
