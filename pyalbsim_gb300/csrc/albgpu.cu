@@ -129,7 +129,8 @@ struct AlbCtx {
     int64_t wf_bins = 0, jac_bins = 0, hm_cells = 0, hm_radius_cells = 0;  // accumulator capacities
     // per-layer scene tables (device), reused when the context takes a new scene
     struct LayerTables {
-        void *th = nullptr, *cdf = nullptr, *sl = nullptr, *w = nullptr, *dlw = nullptr, *dsg = nullptr, *inv = nullptr;
+        void *th = nullptr, *cdf = nullptr, *sl = nullptr, *w = nullptr, *dlw = nullptr, *dsg = nullptr, *inv = nullptr,
+             *guide = nullptr;
     } lt[ALB_MAX_LAYERS];
     bool keep_records = false;  // keep the append stores after indexing (batched runs)
     // exit states
@@ -363,12 +364,17 @@ static std::string set_scene(AlbCtx* ctx, const AlbSceneParams* p) {
         s.layer_ssa[l] = L.ssa;
         s.layer_binw[l] = (float)L.bin_width;
         s.layer_binw_inv[l] = 1.0f / s.layer_binw[l];
+        s.layer_bottom32[l] = (float)L.bottom_depth;
+        s.layer_speed32[l] = (float)L.speed;
+        s.layer_floor32[l] = (float)(s.ys - L.bottom_depth);
         s.layer_h[l] = L.height;
+        s.layer_hinv[l] = 1.0 / L.height;
         s.layer_top32[l] = L.top32;
         s.layer_prof[l] = L.profiled ? 1 : 0;
         s.layer_lut_n[l] = 0;
         s.layer_lut_z[l] = nullptr;
-        s.layer_lut_a[l] = nullptr;
+        s.layer_lut_a[l] = s.layer_lut_s[l] = nullptr;
+        s.layer_lut_inv[l] = 0.f;
         s.layer_nkind[l] = s.layer_akind[l] = 0;
         s.layer_n0[l] = s.layer_n1[l] = s.layer_a0[l] = s.layer_a1[l] = 0.0;
         if (L.profiled) {
@@ -376,16 +382,24 @@ static std::string set_scene(AlbCtx* ctx, const AlbSceneParams* p) {
             if (!(L.height > 0.0)) return std::string("profiled layer needs a positive height");
             if (L.n_kind < 0 || L.n_kind > 2 || L.a_kind < 0 || L.a_kind > 2) return std::string("unknown profile kind");
             float* lz;
-            double* la;
-            if (cudaMalloc(&lz, L.lut_n * sizeof(float)) != cudaSuccess ||
-                cudaMalloc(&la, L.lut_n * sizeof(double)) != cudaSuccess)
-                return std::string("table allocation failed");
-            ctx->tables.insert(ctx->tables.end(), {lz, la});
+            double* la;  // values, then slopes
+            if (cudaMalloc(&lz, L.lut_n * sizeof(float)) != cudaSuccess) return std::string("table allocation failed");
+            ctx->tables.push_back(lz);
+            if (cudaMalloc(&la, 2 * L.lut_n * sizeof(double)) != cudaSuccess) return std::string("table allocation failed");
+            ctx->tables.push_back(la);
+            std::vector<double> slopes(L.lut_n, 0.0);
+            for (int i = 0; i + 1 < L.lut_n; ++i)
+                slopes[i] = (L.lut_alpha[i + 1] - L.lut_alpha[i]) / ((double)L.lut_z[i + 1] - (double)L.lut_z[i]);
             cudaMemcpyAsync(lz, L.lut_z, L.lut_n * sizeof(float), cudaMemcpyHostToDevice, ctx->st);
             cudaMemcpyAsync(la, L.lut_alpha, L.lut_n * sizeof(double), cudaMemcpyHostToDevice, ctx->st);
+            cudaMemcpyAsync(la + L.lut_n, slopes.data(), L.lut_n * sizeof(double), cudaMemcpyHostToDevice, ctx->st);
+            cudaStreamSynchronize(ctx->st);
             s.layer_lut_n[l] = L.lut_n;
             s.layer_lut_z[l] = lz;
             s.layer_lut_a[l] = la;
+            s.layer_lut_s[l] = la + L.lut_n;
+            const double span = (double)L.lut_z[L.lut_n - 1] - (double)L.lut_z[0];
+            s.layer_lut_inv[l] = span > 0.0 && L.lut_z[0] == 0.f ? (float)((L.lut_n - 1) / span) : 0.f;
             s.layer_nkind[l] = L.n_kind;
             s.layer_akind[l] = L.a_kind;
             s.layer_n0[l] = L.n_start;
@@ -410,28 +424,34 @@ static std::string set_scene(AlbCtx* ctx, const AlbSceneParams* p) {
         s.layer_cdf[l] = cdf;
         s.layer_slope[l] = sl;
         s.layer_weight[l] = w;
-        // inverse CDF theta(u) at u = j / kInvCdf for the fast tracer (numpy.interp restated)
-        std::vector<float> inv(kInvCdf + 1);
-        for (int j = 0; j <= kInvCdf; ++j) {
-            double u = (double)j / kInvCdf;
-            double t;
-            if (u < L.phase_cdf[0]) t = L.phase_theta[0];
-            else if (u >= L.phase_cdf[N - 1]) t = L.phase_theta[N - 1];
-            else {
-                int lo = 0, hi = N - 1;
-                while (hi - lo > 1) {
-                    int mid = (lo + hi) / 2;
-                    if (L.phase_cdf[mid] <= u) lo = mid; else hi = mid;
-                }
-                t = (u == L.phase_cdf[lo]) ? L.phase_theta[lo] : L.phase_slope[lo] * (u - L.phase_cdf[lo]) + L.phase_theta[lo];
-            }
-            inv[j] = (float)t;
-        }
         float* dinv = (float*)table_buf(ctx->lt[l].inv, (kInvCdf + 1) * sizeof(float));
-        if (!dinv) return std::string("table allocation failed");
-        cudaMemcpyAsync(dinv, inv.data(), (kInvCdf + 1) * sizeof(float), cudaMemcpyHostToDevice, ctx->st);
+        uint16_t* guide = (uint16_t*)table_buf(ctx->lt[l].guide, (kInvCdf + 1) * sizeof(uint16_t));
+        if (!dinv || !guide) return std::string("table allocation failed");
+        launch_phase_tables(cdf, th, sl, dinv, guide, ctx->st);
+        s.layer_guide[l] = guide;
         cudaStreamSynchronize(ctx->st);  // the host staging vectors die with this iteration
         ctx->fast.inv_theta[l] = dinv;
+    }
+    bool logs = false;
+    for (int l = 0; l < s.n_layers; ++l) {
+        s.layer_nl0[l] = s.layer_ndl[l] = s.layer_al0[l] = s.layer_adl[l] = 0.0;
+        logs = logs || s.layer_nkind[l] == 2 || s.layer_akind[l] == 2;
+    }
+    if (logs) {
+        double* d = nullptr;
+        double h[4 * ALB_MAX_LAYERS];
+        if (cudaMalloc(&d, sizeof h) != cudaSuccess) return std::string("table allocation failed");
+        launch_profile_logs(s, d, ctx->st);
+        const cudaError_t e = cudaMemcpyAsync(h, d, sizeof h, cudaMemcpyDeviceToHost, ctx->st);
+        cudaStreamSynchronize(ctx->st);
+        cudaFree(d);
+        if (e != cudaSuccess) return std::string("profile tables failed");
+        for (int l = 0; l < s.n_layers; ++l) {
+            s.layer_nl0[l] = h[4 * l];
+            s.layer_ndl[l] = h[4 * l + 1];
+            s.layer_al0[l] = h[4 * l + 2];
+            s.layer_adl[l] = h[4 * l + 3];
+        }
     }
     return std::string();
 }
@@ -533,7 +553,7 @@ extern "C" void alb_destroy(AlbCtx* ctx) {
     }
     cudaFree(ctx->wf); cudaFree(ctx->cls); cudaFree(ctx->jac_cls); cudaFree(ctx->heat_cls); cudaFree(ctx->hm); cudaFree(ctx->hm_radius); cudaFree(ctx->jac);
     for (auto& t : ctx->lt) {
-        cudaFree(t.th); cudaFree(t.cdf); cudaFree(t.sl); cudaFree(t.w); cudaFree(t.dlw); cudaFree(t.dsg); cudaFree(t.inv);
+        cudaFree(t.th); cudaFree(t.cdf); cudaFree(t.sl); cudaFree(t.w); cudaFree(t.dlw); cudaFree(t.dsg); cudaFree(t.inv); cudaFree(t.guide);
     }
     cudaFree(ctx->ex_pos); cudaFree(ctx->ex_dir); cudaFree(ctx->ex_f);
     cudaFree(ctx->d_rec_count); cudaFree(ctx->d_q_count); cudaFree(ctx->d_err); cudaFree(ctx->d_stats);

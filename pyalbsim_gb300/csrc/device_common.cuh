@@ -15,6 +15,7 @@ constexpr int kWarp = 32;
 constexpr double kTwoPi = 6.283185307179586;   // 2 * np.pi as the reference forms it
 constexpr double kPi = 3.141592653589793;
 constexpr float kEps32 = 1.1920928955078125e-07f;  // np.finfo(np.float32).eps
+constexpr int kInvCdf = 65536;  // the inverse-CDF and guide tables have kInvCdf + 1 entries per layer
 constexpr int kMaxEventsPerPhoton = 1 << 22;    // device loop cap -> ALB_ERR_ITER_CAP
 
 // Scene constants in __constant__ memory (one copy per loaded module).
@@ -58,17 +59,27 @@ struct SceneDev {
     const double* layer_theta[ALB_MAX_LAYERS];
     const double* layer_cdf[ALB_MAX_LAYERS];
     const double* layer_slope[ALB_MAX_LAYERS];
+    const uint16_t* layer_guide[ALB_MAX_LAYERS];  // CDF interval of j / kInvCdf
     const float* layer_weight[ALB_MAX_LAYERS];
     // depth-profiled layers (layer_prof != 0): per-step speed, attenuation and albedo
     int32_t layer_prof[ALB_MAX_LAYERS];
     int32_t layer_lut_n[ALB_MAX_LAYERS];
     const float* layer_lut_z[ALB_MAX_LAYERS];
     const double* layer_lut_a[ALB_MAX_LAYERS];
+    const double* layer_lut_s[ALB_MAX_LAYERS];  // slopes between the table's entries
+    float layer_lut_inv[ALB_MAX_LAYERS];        // entries per metre
     int32_t layer_nkind[ALB_MAX_LAYERS];
     int32_t layer_akind[ALB_MAX_LAYERS];
     double layer_n0[ALB_MAX_LAYERS], layer_n1[ALB_MAX_LAYERS];
     double layer_a0[ALB_MAX_LAYERS], layer_a1[ALB_MAX_LAYERS];
+    // of exponential profiles: the start's logarithm and the difference to the end's (device log)
+    double layer_nl0[ALB_MAX_LAYERS], layer_ndl[ALB_MAX_LAYERS];
+    double layer_al0[ALB_MAX_LAYERS], layer_adl[ALB_MAX_LAYERS];
     double layer_h[ALB_MAX_LAYERS], layer_top32[ALB_MAX_LAYERS];
+    double layer_hinv[ALB_MAX_LAYERS];  // 1 / layer_h, rounded to nearest
+    // float32 forms for the float32 tracer
+    float layer_bottom32[ALB_MAX_LAYERS], layer_speed32[ALB_MAX_LAYERS];
+    float layer_floor32[ALB_MAX_LAYERS];  // height of the layer's lower boundary
     // adjoint (extension): path scores for theta = (a, b, g) and the seafloor albedo
     int32_t adjoint;
     int32_t pad1;

@@ -139,6 +139,10 @@ void launch_trace(const SceneDev& sc, const TraceOut& out, int pass, uint64_t n,
                   uint64_t seed, const AlbReplay* replay_dev, int* launches, cudaStream_t st,
                   const FastScene* fast);
 
+void launch_phase_tables(const double* cdf, const double* theta, const double* slope, float* inv, uint16_t* guide,
+                         cudaStream_t st);
+void launch_profile_logs(const SceneDev& sc, double* out, cudaStream_t st);
+
 // ---- gather (gather.cu)
 void launch_gather(const SceneDev& sc, const MapDev& map, const QueryDev& q, int channel, const Accum& acc,
                    int* err, int* launches, cudaStream_t st);

@@ -216,38 +216,43 @@ ALB_DEVICE int layer_of(const SceneDev& sc, double y) {
 // below the layer top (depth - float32 layer offset, water.py:306-308).
 // ----------------------------------------------------------------------------------------
 
-// Profile value at local depth z of a layer of height h: kind 1 is LinearParameter
-// (float32: t = f32(z / h), f32(start) + t * f32(end - start)), kind 2 ExponentialParameter
-// (float64), kind 0 the constant `p0`.
-ALB_DEVICE double profile_value(int kind, double p0, double p1, double z, double h) {
+// x / b for float64 from r = the float64 nearest 1 / b: the quotient estimate corrected by its exact
+// residual (Markstein, IBM J. Res. Dev. 34, 1990), the correctly rounded quotient of the division
+// operator at a quarter of its FP64 instructions (two FP64 lanes per SM and cycle here).
+ALB_DEVICE double div64_by(double x, double b, double r) {
+    const double q = x * r;
+    return fma(fma(-q, b, x), r, q);
+}
+
+// Profile value at the fraction q = z / h of a layer: kind 1 is LinearParameter
+// (float32: t = f32(q), f32(start) + t * f32(end - start)), kind 2 ExponentialParameter
+// (float64, from the logarithm l0 of its start and the difference dl to its end's), kind 0 the
+// constant p0.
+ALB_DEVICE double profile_value(int kind, double p0, double p1, double l0, double dl, double q) {
     if (kind == 1) {
-        const float t = __double2float_rn(z / h);
+        const float t = __double2float_rn(q);
         return (double)__fadd_rn(__double2float_rn(p0), __fmul_rn(t, __double2float_rn(p1 - p0)));
     }
-    if (kind == 2) {
-        const double l0 = log(p0), l1 = log(p1);
-        return exp(l0 + (z / h) * (l1 - l0));
-    }
+    if (kind == 2) return exp(l0 + q * dl);
     return p0;
 }
 
-// numpy.interp(f32(z), lut_z, lut_alpha) (clamped at both ends), in float64
+// numpy.interp(f32(z), lut_z, lut_alpha) (clamped at both ends), in float64. The table's depths are
+// evenly spaced but for their rounding, so the interval is one off the product's at most (the
+// loops are right for any increasing table).
 ALB_DEVICE double profile_alpha64(const SceneDev& sc, int L, double z) {
     const float* xp = sc.layer_lut_z[L];
     const double* fp = sc.layer_lut_a[L];
     const int n = sc.layer_lut_n[L];
-    const double x = (double)__double2float_rn(z);
-    if (!(x >= (double)xp[0])) return fp[0];
-    if (x >= (double)xp[n - 1]) return fp[n - 1];
-    int lo = 0, hi = n - 1;
-    while (hi - lo > 1) {
-        const int mid = (lo + hi) >> 1;
-        if ((double)xp[mid] <= x) lo = mid;
-        else hi = mid;
-    }
-    if (x == (double)xp[lo]) return fp[lo];
-    const double slope = __ddiv_rn(__dsub_rn(fp[lo + 1], fp[lo]), __dsub_rn((double)xp[lo + 1], (double)xp[lo]));
-    return __dadd_rn(__dmul_rn(slope, __dsub_rn(x, (double)xp[lo])), fp[lo]);
+    const float x = __double2float_rn(z);
+    if (!(x >= __ldg(xp))) return __ldg(fp);
+    if (x >= __ldg(xp + n - 1)) return __ldg(fp + n - 1);
+    int lo = min((int)(x * sc.layer_lut_inv[L]), n - 2);
+    while (__ldg(xp + lo) > x) --lo;
+    while (__ldg(xp + lo + 1) <= x) ++lo;
+    const float x0 = __ldg(xp + lo);
+    if (x == x0) return __ldg(fp + lo);
+    return __dadd_rn(__dmul_rn(__ldg(sc.layer_lut_s[L] + lo), __dsub_rn((double)x, (double)x0)), __ldg(fp + lo));
 }
 
 ALB_DEVICE double local_depth(const SceneDev& sc, int L, double y) { return -(y - sc.ys) - sc.layer_top32[L]; }
@@ -257,7 +262,8 @@ ALB_DEVICE double water_speed(const SceneDev& sc, int L, double y) {
     if (!sc.layer_prof[L]) return sc.layer_speed[L];
     const double z = local_depth(sc, L, y);
     const int kind = sc.layer_nkind[L];
-    const double n = profile_value(kind, sc.layer_n0[L], sc.layer_n1[L], z, sc.layer_h[L]);
+    const double n = profile_value(kind, sc.layer_n0[L], sc.layer_n1[L], sc.layer_nl0[L], sc.layer_ndl[L],
+                                   div64_by(z, sc.layer_h[L], sc.layer_hinv[L]));
     if (kind == 1) return (double)__fdiv_rn(299800000.0f, (float)n);  // float32 profile
     return (double)__double2float_rn(299800000.0 / n);
 }
@@ -275,7 +281,8 @@ ALB_DEVICE float water_ssa(const SceneDev& sc, double y) {
     if (!sc.layer_prof[L]) return sc.layer_ssa[L];
     const double z = local_depth(sc, L, y);
     const double al = profile_alpha64(sc, L, z);
-    const double a = profile_value(sc.layer_akind[L], sc.layer_a0[L], sc.layer_a1[L], z, sc.layer_h[L]);
+    const double a = profile_value(sc.layer_akind[L], sc.layer_a0[L], sc.layer_a1[L], sc.layer_al0[L], sc.layer_adl[L],
+                                   div64_by(z, sc.layer_h[L], sc.layer_hinv[L]));
     return __double2float_rn(__ddiv_rn(__dsub_rn(al, a), al));
 }
 
@@ -283,12 +290,20 @@ ALB_DEVICE double norm3(double x, double y, double z) {
     return sqrt(__dadd_rn(__dadd_rn(__dmul_rn(x, x), __dmul_rn(y, y)), __dmul_rn(z, z)));
 }
 
+// Steps of size sy from y0 to lim, to a millionth (the callers correct the count with the exact
+// comparison): a float32 quotient costs two FP64 instructions where the float64 one costs a dozen.
+ALB_DEVICE double steps_to(double y0, double sy, double lim) {
+    const float d = (float)(lim - y0), s = (float)sy;
+    return fabsf(s) > 1.0e-30f && fabsf(d) > 1.0e-30f ? (double)__fdividef(d, s) : (lim - y0) / sy;
+}
+
 // Smallest n >= 1 (<= nmax + 1) with y0 + n * sy <= lim, for sy < 0 and y0 > lim.
 ALB_DEVICE int64_t first_at_or_below(double y0, double sy, double lim, int64_t nmax) {
-    double est = (lim - y0) / sy;
-    if (!(est < (double)nmax + 1.0)) return nmax + 1;
+    const double est = steps_to(y0, sy, lim);
+    if (!(est < (double)nmax + 8.0)) return nmax + 1;
     int64_t n = (int64_t)ceil(est);
     if (n < 1) n = 1;
+    if (n > nmax + 1) n = nmax + 1;
     while (n > 1 && fma((double)(n - 1), sy, y0) <= lim) --n;
     while (!(fma((double)n, sy, y0) <= lim)) {
         ++n;
@@ -299,10 +314,11 @@ ALB_DEVICE int64_t first_at_or_below(double y0, double sy, double lim, int64_t n
 
 // Smallest n >= 1 (<= nmax + 1) with y0 + n * sy > lim, for sy > 0 and y0 <= lim.
 ALB_DEVICE int64_t first_above(double y0, double sy, double lim, int64_t nmax) {
-    double est = (lim - y0) / sy;
-    if (!(est < (double)nmax + 1.0)) return nmax + 1;
+    const double est = steps_to(y0, sy, lim);
+    if (!(est < (double)nmax + 8.0)) return nmax + 1;
     int64_t n = (int64_t)floor(est) + 1;
     if (n < 1) n = 1;
+    if (n > nmax + 1) n = nmax + 1;
     while (n > 1 && fma((double)(n - 1), sy, y0) > lim) --n;
     while (!(fma((double)n, sy, y0) > lim)) {
         ++n;
@@ -341,59 +357,67 @@ ALB_DEVICE int64_t first_layer_change(const SceneDev& sc, int layer, double y0, 
 // then holds the value after nmax steps). Exact emulation of the reference's float32
 // accumulation (core/simulation.py:339-344): within the float32 binade [2^e, 2^e+1) every
 // step adds the same rounded increment D, so runs of steps are taken in integer units of
-// the binade's ulp and only binade crossings are stepped explicitly.
+// the binade's ulp and only binade crossings are stepped explicitly. A free path crosses a dozen
+// binades; each takes one float64 add and its rounding, the rest is 32-bit integer arithmetic
+// (GB300 issues two FP64 lanes per SM and cycle, and a 64-bit integer division is a subroutine).
 ALB_DEVICE int64_t tau_run(float& tau, double inc, float target, int64_t nmax) {
+    const uint64_t ib = (uint64_t)__double_as_longlong(inc);
+    const uint64_t im = (ib & 0xfffffffffffffull) | 0x10000000000000ull;  // inc = im 2^ie
+    const int ie = (int)((ib >> 52) & 0x7ff) - 1075;
+    const uint32_t tb = __float_as_uint(target);
+    const int tex = (int)((tb >> 23) & 0xffu);
+    const bool never = !(target == target) || tex == 255;
     int64_t m = 0;
     int guard = 0;
     while (m < nmax) {
         if (++guard > 4096) break;
-        float t1 = __double2float_rn(__dadd_rn((double)tau, inc));
-        uint32_t bits = __float_as_uint(tau);
-        int ex = (int)((bits >> 23) & 0xffu);
-        uint32_t b1 = __float_as_uint(t1);
-        int ex1 = (int)((b1 >> 23) & 0xffu);
-        if (ex == 0 || ex >= 254 || ex1 != ex) {
-            // zero / subnormal start, or the step leaves the binade: explicit step
-            tau = t1;
-            ++m;
-            if (tau >= target) return m;
-            continue;
-        }
-        int64_t T = (int64_t)((bits & 0x7fffffu) | 0x800000u);
-        int64_t Dk = (int64_t)((b1 & 0x7fffffu) | 0x800000u) - T;
-        if (Dk <= 0) {  // increment below half an ulp: tau never changes again
+        const float t1 = __double2float_rn(__dadd_rn((double)tau, inc));
+        const uint32_t bits = __float_as_uint(tau);
+        const int ex = (int)((bits >> 23) & 0xffu);
+        const uint32_t b1 = __float_as_uint(t1);
+        const int ex1 = (int)((b1 >> 23) & 0xffu);
+        // increment in units of this binade's ulp: im 2^sh, integer part I, fraction
+        const int sh = ie + 150 - ex;
+        bool step = ex == 0 || ex >= 254 || ex1 != ex;  // zero / subnormal start, or it leaves the binade
+        const int32_t T = (int32_t)((bits & 0x7fffffu) | 0x800000u);
+        const int32_t Dk = (int32_t)((b1 & 0x7fffffu) | 0x800000u) - T;
+        if (!step && Dk <= 0) {  // increment below half an ulp: tau never changes again
             tau = t1;
             return 0;
         }
-        double inc_u = ldexp(inc, 150 - ex);  // inc in units of this binade's ulp
-        double If = floor(inc_u);
-        if (inc_u - If == 0.5) {  // exact tie: rounding alternates with parity, step it
+        // (within the binade the increment is below 2^24 ulps, so sh < 0 here)
+        int32_t I = 0;
+        if (!step && sh > -64) {
+            I = (int32_t)(im >> -sh);
+            // exact tie: rounding alternates with parity, step it
+            step = (im << (64 + sh)) == 0x8000000000000000ull;
+        }
+        if (step) {
             tau = t1;
             ++m;
             if (tau >= target) return m;
             continue;
         }
-        int64_t I = (int64_t)If;
-        int64_t room = (int64_t)(1 << 24) - 1 - T - I;
-        int64_t J = (room >= 0) ? room / Dk + 1 : 1;  // steps keeping the sum in the binade
+        const int32_t room = (1 << 24) - 1 - T - I;
+        int32_t J = room >= 0 ? (int32_t)((uint32_t)room / (uint32_t)Dk) + 1 : 1;  // steps keeping the sum in the binade
         // first step reaching the target within the run
-        int64_t jt;
-        uint32_t tb = __float_as_uint(target);
-        int tex = (int)((tb >> 23) & 0xffu);
-        if (!(target == target) || tex == 255 || tex - ex > 36) {
-            jt = INT64_MAX;  // +inf / NaN / far away
-        } else if (target <= tau) {
-            jt = 1;
-        } else {
-            int64_t Tt = (int64_t)((tb & 0x7fffffu) | (tex ? 0x800000u : 0u)) << (tex - ex);
-            jt = (Tt - T + Dk - 1) / Dk;
+        int32_t jt = INT32_MAX;  // +inf / NaN / far away
+        if (!never) {
+            if (target <= tau) {
+                jt = 1;
+            } else {
+                // a target in a higher binade is at least 2^24 ulps, what the run reaches at most
+                const int up = tex - ex;
+                const uint32_t mt = (tb & 0x7fffffu) | (tex ? 0x800000u : 0u);
+                const uint32_t Tt = up <= 0 ? mt : (up > 1 ? (1u << 26) : mt << 1);
+                jt = (int32_t)((Tt - (uint32_t)T + (uint32_t)Dk - 1u) / (uint32_t)Dk);
+            }
         }
-        int64_t jmax = J < nmax - m ? J : nmax - m;
-        if (jt <= jmax) {
-            tau = (float)ldexp((double)(T + jt * Dk), ex - 150);
-            return m + jt;
-        }
-        tau = (float)ldexp((double)(T + jmax * Dk), ex - 150);
+        const int32_t jmax = (int64_t)J < nmax - m ? J : (int32_t)(nmax - m);
+        const int32_t run = jt <= jmax ? jt : jmax;
+        // (T + run D) 2^(ex - 150): at most 2^24, exact in float32, scaled by its exponent field
+        tau = __uint_as_float(__float_as_uint(__int2float_rn(T + run * Dk)) + ((uint32_t)(ex - 150) << 23));
+        if (jt <= jmax) return m + jt;
         m += jmax;
     }
     return 0;
@@ -412,7 +436,15 @@ ALB_DEVICE double interp_theta(const SceneDev& sc, int layer, double u, int& int
     if (u < cdf[0]) return th[0];
     interval = n - 1;
     if (u >= cdf[n - 1]) return th[n - 1];
-    int lo = 0, hi = n - 1;  // invariant cdf[lo] <= u < cdf[hi]
+    // the guide holds the interval of floor(u 2^16) / 2^16; the wanted one is usually that or the
+    // next (a 14-step search of dependent loads otherwise)
+    int lo = sc.layer_guide[layer][(int)(u * (double)kInvCdf)];
+    int near = 0;
+    while (near < 8 && cdf[lo + 1] <= u) {
+        ++lo;
+        ++near;
+    }
+    int hi = near < 8 ? lo + 1 : n - 1;  // invariant cdf[lo] <= u < cdf[hi]
     while (hi - lo > 1) {
         int mid = (lo + hi) >> 1;
         if (cdf[mid] <= u) lo = mid; else hi = mid;
@@ -427,7 +459,8 @@ ALB_DEVICE double interp_theta(const SceneDev& sc, int layer, double u, int& int
 ALB_DEVICE void rotate_from_z(double dx, double dy, double dz, double l0, double l1, double l2,
                               double& ox, double& oy, double& oz) {
     double n = norm3(dx, dy, dz);
-    double vx = dx / n, vy = dy / n, vz = dz / n;
+    const double ninv = __drcp_rn(n);
+    double vx = div64_by(dx, n, ninv), vy = div64_by(dy, n, ninv), vz = div64_by(dz, n, ninv);
     double c = vz;
     double R[9];
     if (fabs(c - 1.0) <= 1.0010000000000001e-05) {
@@ -741,55 +774,97 @@ ALB_DEVICE void emit_photon(const SceneDev& sc, Ph& ph, Src& src) {
 // Full photon
 // ----------------------------------------------------------------------------------------
 
+// What a lane's photon does next. Lanes with the same kind of event wait for one another
+// (trace_warp), so the surface and seafloor handlers, a twentieth of the events and most of the
+// code, run with several lanes instead of one or two.
+constexpr int kLaneRun = 0, kLaneAir = 1, kLaneExit = 2, kLaneFloor = 3, kLaneDone = 4;
+
+template <class P>
+ALB_DEVICE void write_exit_state(const TraceOut& out, const P& ph, uint64_t i) {
+    if (!out.ex_pos) return;
+    out.ex_pos[3 * i] = ph.px; out.ex_pos[3 * i + 1] = ph.py; out.ex_pos[3 * i + 2] = ph.pz;
+    out.ex_dir[3 * i] = ph.dx; out.ex_dir[3 * i + 1] = ph.dy; out.ex_dir[3 * i + 2] = ph.dz;
+    float* f = out.ex_f + 10 * i;
+    f[0] = ph.E; f[1] = ph.tau; f[2] = ph.taut; f[3] = ph.t0;
+    f[4] = ph.fwi[0]; f[5] = ph.fwi[1]; f[6] = ph.fwi[2];
+    f[7] = ph.sfi[0]; f[8] = ph.sfi[1]; f[9] = ph.sfi[2];
+}
+
+// Variates of photon i of the launch (global number gid).
+ALB_DEVICE void seek(PhiloxSrc& src, uint64_t gid, uint64_t, const int64_t*) {
+    src.plo = (uint32_t)gid;
+    src.phi = (uint32_t)(gid >> 32);
+    src.ctr = 0u;
+}
+ALB_DEVICE void seek(ReplaySrc& src, uint64_t, uint64_t i, const int64_t* offs) {
+    src.pos = offs[i];
+    src.end = offs[i + 1];
+}
+
+// One lane's photon of the float64-geometry tracer.
 template <int PASS, class Src>
-ALB_DEVICE void trace_photon(const SceneDev& sc, const TraceOut& out, Ph& ph, Src& src, uint32_t pid,
-                             unsigned long long& events) {
-    const int64_t S = sc.stop_step[PASS];
-    int guard = 0;
-    while (ph.s < S) {
+struct PreciseLane {
+    const SceneDev& sc;
+    const TraceOut& out;
+    uint64_t first;
+    const int64_t* offs;
+    Src src;
+    Ph ph;
+    uint32_t pid;
+    int guard;
+    double cross_v;  // speed of the segment that ends at a plane
+    unsigned long long events, done;
+
+    ALB_DEVICE int mode() const {
+        return !(ph.s < sc.stop_step[PASS]) ? kLaneDone : (ph.py > sc.ys ? kLaneAir : kLaneRun);
+    }
+    ALB_DEVICE int start(uint64_t i) {
+        pid = (uint32_t)(first + i);
+        seek(src, first + i, i, offs);
+        guard = 0;
+        emit_photon<PASS>(sc, ph, src);
+        return mode();
+    }
+
+    // In air: nothing happens until the step that crosses the surface.
+    ALB_DEVICE int air() {
+        ++guard;
+        const int64_t left = sc.stop_step[PASS] - ph.s;
+        const double v = sc.v_air;
+        const double svx = (ph.dx * v) * sc.dt, svy = (ph.dy * v) * sc.dt, svz = (ph.dz * v) * sc.dt;
+        const int64_t n = (svy < 0.0) ? first_at_or_below(ph.py, svy, sc.ys, left) : left + 1;
+        if (n - 1 >= left) {
+            const double k = (double)left;
+            ph.px = fma(k, svx, ph.px); ph.py = fma(k, svy, ph.py); ph.pz = fma(k, svz, ph.pz);
+            ph.s = sc.stop_step[PASS];
+            return kLaneDone;
+        }
+        const double k = (double)(n - 1);
+        ph.px = fma(k, svx, ph.px); ph.py = fma(k, svy, ph.py); ph.pz = fma(k, svz, ph.pz);
+        ph.s += n - 1;
+        handle_enter<PASS>(sc, out, ph, src, svx, svy, svz, pid);
+        ph.s += 1;
+        ++events;
+        return mode();
+    }
+
+    // In water: to the next scatter, layer change or plane, or one step of a depth-profiled layer.
+    ALB_DEVICE int run() {
         if (++guard > kMaxEventsPerPhoton) {
             set_err(out.err, ALB_ERR_ITER_CAP);
-            break;
+            return kLaneDone;
         }
-        const int64_t left = S - ph.s;
-        if (ph.py > sc.ys) {
-            // in air: nothing happens until the step that crosses the surface
-            double v = sc.v_air;
-            double svx = (ph.dx * v) * sc.dt, svy = (ph.dy * v) * sc.dt, svz = (ph.dz * v) * sc.dt;
-            int64_t n = (svy < 0.0) ? first_at_or_below(ph.py, svy, sc.ys, left) : left + 1;
-            if (n - 1 >= left) {
-                double k = (double)left;
-                ph.px = fma(k, svx, ph.px); ph.py = fma(k, svy, ph.py); ph.pz = fma(k, svz, ph.pz);
-                ph.s = S;
-                break;
-            }
-            double k = (double)(n - 1);
-            ph.px = fma(k, svx, ph.px); ph.py = fma(k, svy, ph.py); ph.pz = fma(k, svz, ph.pz);
-            ph.s += n - 1;
-            handle_enter<PASS>(sc, out, ph, src, svx, svy, svz, pid);
-            ph.s += 1;
-            ++events;
-        } else if (sc.layer_prof[layer_of(sc, ph.py)]) {
+        const int64_t S = sc.stop_step[PASS], left = S - ph.s;
+        const int L = layer_of(sc, ph.py);
+        if (sc.layer_prof[L]) {
             // depth-profiled layer: one integration step, speed and attenuation at its start
             --guard;  // bounded by the step count, not an event
-            const int L = layer_of(sc, ph.py);
             const double v = water_speed(sc, L, ph.py);
             const double svx = (ph.dx * v) * sc.dt, svy = (ph.dy * v) * sc.dt, svz = (ph.dz * v) * sc.dt;
             const double ny = ph.py + svy;
-            if (ny > sc.ys) {
-                handle_exit<PASS>(sc, out, ph, src, svx, svy, svz, pid);
-                ph.s += 1;
-                ++events;
-                ++guard;
-                continue;
-            }
-            if (ny <= sc.yf) {
-                handle_floor<PASS>(sc, out, ph, src, svx, svy, svz, pid);
-                ph.s += 1;
-                ++events;
-                ++guard;
-                continue;
-            }
+            cross_v = v;
+            if (ny > sc.ys) return kLaneExit;
+            if (ny <= sc.yf) return kLaneFloor;
             const double len = norm3(svx, svy, svz);
             const float a = __double2float_rn(profile_alpha64(sc, L, local_depth(sc, L, ph.py)));
             ph.tau = __double2float_rn(__dadd_rn((double)ph.tau, (double)a * len));
@@ -803,42 +878,73 @@ ALB_DEVICE void trace_photon(const SceneDev& sc, const TraceOut& out, Ph& ph, Sr
                 ++events;
                 ++guard;
             }
-        } else {
-            int L = layer_of(sc, ph.py);
-            double v = sc.layer_speed[L];
-            double svx = (ph.dx * v) * sc.dt, svy = (ph.dy * v) * sc.dt, svz = (ph.dz * v) * sc.dt;
-            double len = norm3(svx, svy, svz);
-            int64_t n_plane = left + 1;
-            if (svy > 0.0) n_plane = first_above(ph.py, svy, sc.ys, left) - 1;
-            else if (svy < 0.0) n_plane = first_at_or_below(ph.py, svy, sc.yf, left) - 1;
-            int64_t n_layer = first_layer_change(sc, L, ph.py, svy, left);
-            int64_t nseg = n_plane < n_layer ? n_plane : n_layer;
-            if (nseg > left) nseg = left;
-            double inc = (double)sc.layer_alpha[L] * len;
-            int64_t m = (nseg > 0) ? tau_run(ph.tau, inc, ph.taut, nseg) : 0;
-            // optical depth of the run: m steps to the scatter, else the whole segment
-            if (sc.adjoint) score_tau(sc, ph.sc, L, (float)((double)(m > 0 ? m : nseg) * inc));
-            if (m > 0) {
-                double k = (double)m;
-                ph.px = fma(k, svx, ph.px); ph.py = fma(k, svy, ph.py); ph.pz = fma(k, svz, ph.pz);
-                int64_t step = ph.s + m - 1;
-                handle_scatter<PASS>(sc, out, ph, src, step, pid);
-                ph.s = step + 1;
-                ++events;
-                continue;
-            }
-            double k = (double)nseg;
-            ph.px = fma(k, svx, ph.px); ph.py = fma(k, svy, ph.py); ph.pz = fma(k, svz, ph.pz);
-            ph.s += nseg;
-            if (ph.s >= S) break;
-            if (nseg == n_plane) {
-                if (svy > 0.0) handle_exit<PASS>(sc, out, ph, src, svx, svy, svz, pid);
-                else handle_floor<PASS>(sc, out, ph, src, svx, svy, svz, pid);
-                ph.s += 1;
-                ++events;
+            return mode();
+        }
+        const double v = sc.layer_speed[L];
+        const double svx = (ph.dx * v) * sc.dt, svy = (ph.dy * v) * sc.dt, svz = (ph.dz * v) * sc.dt;
+        const double len = norm3(svx, svy, svz);
+        int64_t n_plane = left + 1;
+        if (svy > 0.0) n_plane = first_above(ph.py, svy, sc.ys, left) - 1;
+        else if (svy < 0.0) n_plane = first_at_or_below(ph.py, svy, sc.yf, left) - 1;
+        const int64_t n_layer = first_layer_change(sc, L, ph.py, svy, left);
+        int64_t nseg = n_plane < n_layer ? n_plane : n_layer;
+        if (nseg > left) nseg = left;
+        const double inc = (double)sc.layer_alpha[L] * len;
+        const int64_t m = (nseg > 0) ? tau_run(ph.tau, inc, ph.taut, nseg) : 0;
+        // optical depth of the run: m steps to the scatter, else the whole segment
+        if (sc.adjoint) score_tau(sc, ph.sc, L, (float)((double)(m > 0 ? m : nseg) * inc));
+        const double k = (double)(m > 0 ? m : nseg);
+        ph.px = fma(k, svx, ph.px); ph.py = fma(k, svy, ph.py); ph.pz = fma(k, svz, ph.pz);
+        if (m > 0) {
+            const int64_t step = ph.s + m - 1;
+            handle_scatter<PASS>(sc, out, ph, src, step, pid);
+            ph.s = step + 1;
+            ++events;
+            return mode();
+        }
+        ph.s += nseg;
+        if (ph.s >= S) return kLaneDone;
+        if (nseg != n_plane) return mode();
+        cross_v = v;
+        return svy > 0.0 ? kLaneExit : kLaneFloor;
+    }
+
+    // The step through the surface from below.
+    ALB_DEVICE int exit() {
+        const double svx = (ph.dx * cross_v) * sc.dt, svy = (ph.dy * cross_v) * sc.dt, svz = (ph.dz * cross_v) * sc.dt;
+        handle_exit<PASS>(sc, out, ph, src, svx, svy, svz, pid);
+        ph.s += 1;
+        ++events;
+        ++guard;
+        const int m = mode();
+        if (m == kLaneAir) {
+            // on its way up it leaves the scene: the rest of its steps at once, as air() takes them
+            const double v = sc.v_air;
+            const double ay = (ph.dy * v) * sc.dt;
+            if (!(ay < 0.0)) {
+                const double k = (double)(sc.stop_step[PASS] - ph.s);
+                ph.px = fma(k, (ph.dx * v) * sc.dt, ph.px); ph.py = fma(k, ay, ph.py); ph.pz = fma(k, (ph.dz * v) * sc.dt, ph.pz);
+                ph.s = sc.stop_step[PASS];
+                return kLaneDone;
             }
         }
+        return m;
     }
-}
+
+    // The step through the seafloor.
+    ALB_DEVICE int floor() {
+        const double svx = (ph.dx * cross_v) * sc.dt, svy = (ph.dy * cross_v) * sc.dt, svz = (ph.dz * cross_v) * sc.dt;
+        handle_floor<PASS>(sc, out, ph, src, svx, svy, svz, pid);
+        ph.s += 1;
+        ++events;
+        ++guard;
+        return mode();
+    }
+
+    ALB_DEVICE void finish(uint64_t i) {
+        write_exit_state(out, ph, i);
+        ++done;
+    }
+};
 
 }  // namespace alb

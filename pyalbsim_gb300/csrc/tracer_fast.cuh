@@ -16,8 +16,6 @@
 
 namespace alb {
 
-constexpr int kInvCdf = 65536;  // inverse-CDF table has kInvCdf + 1 entries per layer
-
 struct FastScene {
     const float* inv_theta[ALB_MAX_LAYERS];  // theta(u) at u = j / kInvCdf
 };
@@ -37,7 +35,7 @@ ALB_DEVICE float uf(uint32_t x) { return ((float)(x >> 9) + 0.5f) * 1.1920928955
 ALB_DEVICE int layer_of_f(const SceneDev& sc, float y) {
     float depth = -(y - (float)sc.ys);
     int i = 0;
-    while (i < sc.n_layers && !((float)sc.layer_bottom[i] > depth)) ++i;
+    while (i < sc.n_layers && !(sc.layer_bottom32[i] > depth)) ++i;
     return i < sc.n_layers ? i : sc.n_layers - 1;
 }
 
@@ -95,12 +93,12 @@ ALB_DEVICE int first_layer_change_f(const SceneDev& sc, int layer, float y0, flo
     float lim;
     if (sy < 0.f) {
         if (layer >= sc.n_layers - 1) return nmax + 1;
-        lim = (float)(sc.ys - sc.layer_bottom[layer]);
+        lim = sc.layer_floor32[layer];
         int n = first_at_or_below_f(y0, sy, lim, nmax);
         return n;
     }
     if (layer == 0) return nmax + 1;
-    lim = (float)(sc.ys - sc.layer_bottom[layer - 1]);
+    lim = sc.layer_floor32[layer - 1];
     return first_above_f(y0, sy, lim, nmax);
 }
 
@@ -125,69 +123,92 @@ ALB_DEVICE void draw_facet_f(const SceneDev& sc, PhiloxSrc& src, float& mx, floa
     mz = -gz * inv;
 }
 
+// One lane's photon of the float32 tracer (the lane modes of tracer.cuh).
 template <int PASS>
-ALB_DEVICE void trace_photon_fast(const SceneDev& sc, const FastScene& fs, const TraceOut& out, PhF& ph,
-                                  PhiloxSrc& src, uint32_t pid, unsigned long long& events) {
-    const int S = (int)sc.stop_step[PASS];
-    const float ys = (float)sc.ys, yf = (float)sc.yf, dt = (float)sc.dt;
-    const float eta = (float)sc.eta, f0 = (float)sc.f0;
-    int guard = 0;
-    while (ph.s < S) {
+struct FastLane {
+    const SceneDev& sc;
+    const FastScene& fs;
+    const TraceOut& out;
+    uint64_t first;
+    PhiloxSrc src;
+    PhF ph;
+    uint32_t pid;
+    int guard;
+    float cross_v;  // metres per step of the segment that ends at a plane
+    unsigned long long events, done;
+
+    ALB_DEVICE int mode() const {
+        return !(ph.s < (int)sc.stop_step[PASS]) ? kLaneDone : (ph.py > (float)sc.ys ? kLaneAir : kLaneRun);
+    }
+    ALB_DEVICE int start(uint64_t i);
+
+    // In air: nothing happens until the step that enters the water.
+    ALB_DEVICE int air() {
+        const int S = (int)sc.stop_step[PASS];
+        const float ys = (float)sc.ys, dt = (float)sc.dt;
+        const float eta = (float)sc.eta, f0 = (float)sc.f0;
+        ++guard;
+        const int left = S - ph.s;
+        float v = (float)sc.v_air * dt;
+        float svx = ph.dx * v, svy = ph.dy * v, svz = ph.dz * v;
+        int n = (svy < 0.f) ? first_at_or_below_f(ph.py, svy, ys, left) : left + 1;
+        if (n - 1 >= left) {
+            float k = (float)left;
+            ph.px = fmaf(k, svx, ph.px); ph.py = fmaf(k, svy, ph.py); ph.pz = fmaf(k, svz, ph.pz);
+            ph.s = S;
+            return kLaneDone;
+        }
+        float k = (float)(n - 1);
+        ph.px = fmaf(k, svx, ph.px); ph.py = fmaf(k, svy, ph.py); ph.pz = fmaf(k, svz, ph.pz);
+        ph.s += n - 1;
+        // entering step (handle_enter)
+        float f = fminf(fmaxf((ys - ph.py) / svy, 0.f), 1.f);
+        float xs = fmaf(f, svx, ph.px), yss = ys, zs = fmaf(f, svz, ph.pz);
+        ph.fwi[0] = xs; ph.fwi[1] = yss; ph.fwi[2] = zs;
+        float F = schlick_f(f0, -ph.dy);
+        emit_event_f<PASS>(out, ALB_SURFACE_REFLECTION, kQuerySurface, ph, xs, yss, zs, ph.s, pid);
+        float mx = 0.f, my = 1.f, mz = 0.f;
+        if (sc.slope_sigma > 0.0) {
+            draw_facet_f(sc, src, mx, my, mz);
+            if (!(-(ph.dx * mx + ph.dy * my + ph.dz * mz) > 0.f)) { mx = 0.f; my = 1.f; mz = 0.f; }
+        }
+        float ci = fminf(fmaxf(-(ph.dx * mx + ph.dy * my + ph.dz * mz), -1.f), 1.f);
+        float ct = sqrtf(fmaxf(0.f, 1.f - eta * eta * (1.f - ci * ci)));
+        float kt = eta * ci - ct;
+        float tx = fmaf(kt, mx, eta * ph.dx), ty = fmaf(kt, my, eta * ph.dy), tz = fmaf(kt, mz, eta * ph.dz);
+        if (!(ty < 0.f)) {  // a steep facet would send the photon up: the mean surface instead
+            ci = fminf(fmaxf(-ph.dy, -1.f), 1.f);
+            ct = sqrtf(fmaxf(0.f, 1.f - eta * eta * (1.f - ci * ci)));
+            tx = eta * ph.dx; ty = eta * ph.dy + (eta * ci - ct); tz = eta * ph.dz;
+        }
+        F = schlick_f(f0, ci);
+        float tn = rsqrtf(fmaf(tx, tx, fmaf(ty, ty, tz * tz)));
+        ph.dx = tx * tn; ph.dy = ty * tn; ph.dz = tz * tn;
+        ph.E *= (1.f - F);
+        float rem = (1.f - f) * sqrtf(fmaf(svx, svx, fmaf(svy, svy, svz * svz)));
+        ph.px = fmaf(ph.dx, rem, xs); ph.py = fmaf(ph.dy, rem, yss); ph.pz = fmaf(ph.dz, rem, zs);
+        ph.taut = -__logf(uf(src.block().x));
+        ph.s += 1;
+        ++events;
+        return mode();
+
+    }
+
+    // In water: to the next scatter, layer change or plane (or one step of a profiled layer).
+    ALB_DEVICE int run() {
+        const int S = (int)sc.stop_step[PASS];
+        const float ys = (float)sc.ys, yf = (float)sc.yf, dt = (float)sc.dt;
         if (++guard > kMaxEventsPerPhoton) {
             set_err(out.err, ALB_ERR_ITER_CAP);
-            break;
+            return kLaneDone;
         }
         const int left = S - ph.s;
-        if (ph.py > ys) {
-            float v = (float)sc.v_air * dt;
-            float svx = ph.dx * v, svy = ph.dy * v, svz = ph.dz * v;
-            int n = (svy < 0.f) ? first_at_or_below_f(ph.py, svy, ys, left) : left + 1;
-            if (n - 1 >= left) {
-                float k = (float)left;
-                ph.px = fmaf(k, svx, ph.px); ph.py = fmaf(k, svy, ph.py); ph.pz = fmaf(k, svz, ph.pz);
-                ph.s = S;
-                break;
-            }
-            float k = (float)(n - 1);
-            ph.px = fmaf(k, svx, ph.px); ph.py = fmaf(k, svy, ph.py); ph.pz = fmaf(k, svz, ph.pz);
-            ph.s += n - 1;
-            // entering step (handle_enter)
-            float f = fminf(fmaxf((ys - ph.py) / svy, 0.f), 1.f);
-            float xs = fmaf(f, svx, ph.px), yss = ys, zs = fmaf(f, svz, ph.pz);
-            ph.fwi[0] = xs; ph.fwi[1] = yss; ph.fwi[2] = zs;
-            float F = schlick_f(f0, -ph.dy);
-            emit_event_f<PASS>(out, ALB_SURFACE_REFLECTION, kQuerySurface, ph, xs, yss, zs, ph.s, pid);
-            float mx = 0.f, my = 1.f, mz = 0.f;
-            if (sc.slope_sigma > 0.0) {
-                draw_facet_f(sc, src, mx, my, mz);
-                if (!(-(ph.dx * mx + ph.dy * my + ph.dz * mz) > 0.f)) { mx = 0.f; my = 1.f; mz = 0.f; }
-            }
-            float ci = fminf(fmaxf(-(ph.dx * mx + ph.dy * my + ph.dz * mz), -1.f), 1.f);
-            float ct = sqrtf(fmaxf(0.f, 1.f - eta * eta * (1.f - ci * ci)));
-            float kt = eta * ci - ct;
-            float tx = fmaf(kt, mx, eta * ph.dx), ty = fmaf(kt, my, eta * ph.dy), tz = fmaf(kt, mz, eta * ph.dz);
-            if (!(ty < 0.f)) {  // a steep facet would send the photon up: the mean surface instead
-                ci = fminf(fmaxf(-ph.dy, -1.f), 1.f);
-                ct = sqrtf(fmaxf(0.f, 1.f - eta * eta * (1.f - ci * ci)));
-                tx = eta * ph.dx; ty = eta * ph.dy + (eta * ci - ct); tz = eta * ph.dz;
-            }
-            F = schlick_f(f0, ci);
-            float tn = rsqrtf(fmaf(tx, tx, fmaf(ty, ty, tz * tz)));
-            ph.dx = tx * tn; ph.dy = ty * tn; ph.dz = tz * tn;
-            ph.E *= (1.f - F);
-            float rem = (1.f - f) * sqrtf(fmaf(svx, svx, fmaf(svy, svy, svz * svz)));
-            ph.px = fmaf(ph.dx, rem, xs); ph.py = fmaf(ph.dy, rem, yss); ph.pz = fmaf(ph.dz, rem, zs);
-            ph.taut = -__logf(uf(src.block().x));
-            ph.s += 1;
-            ++events;
-            continue;
-        }
         int L = layer_of_f(sc, ph.py);
         // a depth-profiled layer is crossed one integration step at a time (speed and
         // attenuation at the step's start depth); those steps are not events for the cap
         const bool prof = sc.layer_prof[L] != 0;
         if (prof) --guard;
-        float v = (prof ? (float)water_speed(sc, L, (double)ph.py) : (float)sc.layer_speed[L]) * dt;
+        float v = (prof ? (float)water_speed(sc, L, (double)ph.py) : sc.layer_speed32[L]) * dt;
         float svx = ph.dx * v, svy = ph.dy * v, svz = ph.dz * v;
         float len = sqrtf(fmaf(svx, svx, fmaf(svy, svy, svz * svz)));
         int n_plane = left + 1;
@@ -239,99 +260,136 @@ ALB_DEVICE void trace_photon_fast(const SceneDev& sc, const FastScene& fs, const
             ph.s = step + 1;
             ++events;
             if (prof) ++guard;
-            continue;
+            return mode();
         }
         float k = (float)nseg;
         ph.px = fmaf(k, svx, ph.px); ph.py = fmaf(k, svy, ph.py); ph.pz = fmaf(k, svz, ph.pz);
         ph.tau = fmaf(k, inc, ph.tau);
         if (sc.adjoint && nseg > 0) score_tau(sc, ph.sc, L, k * inc);
         ph.s += nseg;
-        if (ph.s >= S) break;
-        if (nseg != n_plane) continue;  // layer change (or one profiled step) only
+        if (ph.s >= S) return kLaneDone;
+        if (nseg != n_plane) return mode();  // layer change (or one profiled step) only
         if (prof) ++guard;
-        if (svy > 0.f) {
-            // handle_exit
-            float f = fminf(fmaxf((ys - ph.py) / svy, 0.f), 1.f);
-            float xs = fmaf(f, svx, ph.px), yss = ys, zs = fmaf(f, svz, ph.pz);
-            float mx = 0.f, my = 1.f, mz = 0.f;
-            if (sc.slope_sigma > 0.0) {
-                draw_facet_f(sc, src, mx, my, mz);
-                if (!(ph.dx * mx + ph.dy * my + ph.dz * mz > 0.f)) { mx = 0.f; my = 1.f; mz = 0.f; }
-            }
-            const float cf = fminf(ph.dx * mx + ph.dy * my + ph.dz * mz, 1.f);
-            float F = schlick_f(f0, cf);
-            bool reflect = uf(src.block().x) < F;
-            if (PASS == ALB_FORWARD && !reflect)
-                emit_event_f<PASS>(out, ALB_SURFACE_TRANSMISSION_UP, 0, ph, xs, yss, zs, ph.s, pid);
-            if (reflect) {
-                const float rx = ph.dx - 2.f * cf * mx, ry = ph.dy - 2.f * cf * my, rz = ph.dz - 2.f * cf * mz;
-                if (ry < 0.f) { ph.dx = rx; ph.dy = ry; ph.dz = rz; }
-                else ph.dy = -ph.dy;
-            } else {
-                float ci = fmaxf(cf, -1.f);
-                float ct = sqrtf(fmaxf(0.f, 1.f - eta * eta * (1.f - ci * ci)));
-                float k = eta * ci - ct;
-                float tx = fmaf(-k, mx, eta * ph.dx), ty = fmaf(-k, my, eta * ph.dy), tz = fmaf(-k, mz, eta * ph.dz);
-                if (!(ty > 0.f)) {
-                    ci = fminf(fmaxf(ph.dy, -1.f), 1.f);
-                    ct = sqrtf(fmaxf(0.f, 1.f - eta * eta * (1.f - ci * ci)));
-                    tx = eta * ph.dx; ty = eta * ph.dy - (eta * ci - ct); tz = eta * ph.dz;
-                }
-                float tn = rsqrtf(fmaf(tx, tx, fmaf(ty, ty, tz * tz)));
-                ph.dx = tx * tn; ph.dy = ty * tn; ph.dz = tz * tn;
-            }
-            float rem = (1.f - f) * len;
-            ph.px = fmaf(ph.dx, rem, xs); ph.py = fmaf(ph.dy, rem, yss); ph.pz = fmaf(ph.dz, rem, zs);
-            if (reflect) {
-                const float a = water_alpha_f(sc, ph.py);
-                if (sc.adjoint) score_tau(sc, ph.sc, layer_of_f(sc, ph.py), a * len);
-                ph.tau = fmaf(a, len, ph.tau);
-            } else if (!(ph.py > ys)) {
-                // A transmitted photon is in the air. Near the surface a float32 height is
-                // quantised to ulp(ys) (3e-5 m at 400 m), as coarse as a grazing photon's
-                // vertical step, so the crossing fraction can round to 1 and leave no
-                // remaining step: the photon would sit on the surface, count as in water and
-                // exit a second time (a second transmission record, 1.5% of the photons at
-                // 400 m with 0.05 ns bins). Place it just above the surface instead.
-                ph.py = nextafterf(ys, 1.0e30f);
-            }
+        cross_v = v;
+        return svy > 0.f ? kLaneExit : kLaneFloor;
+
+    }
+
+    // The step through the surface from below (handle_exit).
+    ALB_DEVICE int exit() {
+        const int S = (int)sc.stop_step[PASS];
+        const float ys = (float)sc.ys, dt = (float)sc.dt;
+        const float eta = (float)sc.eta, f0 = (float)sc.f0;
+        const float svx = ph.dx * cross_v, svy = ph.dy * cross_v, svz = ph.dz * cross_v;
+        const float len = sqrtf(fmaf(svx, svx, fmaf(svy, svy, svz * svz)));
+        float f = fminf(fmaxf((ys - ph.py) / svy, 0.f), 1.f);
+        float xs = fmaf(f, svx, ph.px), yss = ys, zs = fmaf(f, svz, ph.pz);
+        float mx = 0.f, my = 1.f, mz = 0.f;
+        if (sc.slope_sigma > 0.0) {
+            draw_facet_f(sc, src, mx, my, mz);
+            if (!(ph.dx * mx + ph.dy * my + ph.dz * mz > 0.f)) { mx = 0.f; my = 1.f; mz = 0.f; }
+        }
+        const float cf = fminf(ph.dx * mx + ph.dy * my + ph.dz * mz, 1.f);
+        float F = schlick_f(f0, cf);
+        bool reflect = uf(src.block().x) < F;
+        if (PASS == ALB_FORWARD && !reflect)
+            emit_event_f<PASS>(out, ALB_SURFACE_TRANSMISSION_UP, 0, ph, xs, yss, zs, ph.s, pid);
+        if (reflect) {
+            const float rx = ph.dx - 2.f * cf * mx, ry = ph.dy - 2.f * cf * my, rz = ph.dz - 2.f * cf * mz;
+            if (ry < 0.f) { ph.dx = rx; ph.dy = ry; ph.dz = rz; }
+            else ph.dy = -ph.dy;
         } else {
-            // handle_seafloor
-            float f = fminf(fmaxf((yf - ph.py) / svy, 0.f), 1.f);
-            float xb = fmaf(f, svx, ph.px), yb = yf, zb = fmaf(f, svz, ph.pz);
-            ph.sfi[0] = xb; ph.sfi[1] = yb; ph.sfi[2] = zb;
-            if (PASS == ALB_FORWARD && out.hm_radius && ph.fwi[0] == ph.fwi[0]) {
-                float ax = ph.fwi[0] - (float)sc.wc[0], az = ph.fwi[2] - (float)sc.wc[2];
-                float bx = xb - (float)sc.fc[0], bz = zb - (float)sc.fc[2];
-                int xi = (int)((sqrtf(ax * ax + az * az) / (float)sc.hm_wext) * sc.hm_bins);
-                int yi = (int)((sqrtf(bx * bx + bz * bz) / (float)sc.hm_fext) * sc.hm_bins);
-                if (xi >= 0 && xi < sc.hm_bins && yi >= 0 && yi < sc.hm_bins)
-                    atomicAdd(out.hm_radius + xi * sc.hm_bins + yi, 1u);
+            float ci = fmaxf(cf, -1.f);
+            float ct = sqrtf(fmaxf(0.f, 1.f - eta * eta * (1.f - ci * ci)));
+            float k = eta * ci - ct;
+            float tx = fmaf(-k, mx, eta * ph.dx), ty = fmaf(-k, my, eta * ph.dy), tz = fmaf(-k, mz, eta * ph.dz);
+            if (!(ty > 0.f)) {
+                ci = fminf(fmaxf(ph.dy, -1.f), 1.f);
+                ct = sqrtf(fmaxf(0.f, 1.f - eta * eta * (1.f - ci * ci)));
+                tx = eta * ph.dx; ty = eta * ph.dy - (eta * ci - ct); tz = eta * ph.dz;
             }
-            emit_event_f<PASS>(out, ALB_BOTTOM_REFLECTION, kQueryBottom, ph, xb, yb, zb, ph.s, pid);
-            // normalize(+y + isotropic unit vector): a cosine lobe about +y
-            U4 b = src.block();
-            float z = fmaf(-2.f, uf(b.x), 1.f);
-            float r = sqrtf(fmaxf(0.f, 1.f - z * z));
-            float sp, cp;
-            __sincosf(6.283185307179586f * uf(b.y), &sp, &cp);
-            float hx = r * cp, hy = 1.f + z, hz = r * sp;
-            float hn = rsqrtf(fmaf(hx, hx, fmaf(hy, hy, hz * hz)));
-            ph.dx = hx * hn; ph.dy = hy * hn; ph.dz = hz * hn;
-            float rem = (1.f - f) * len;
-            ph.px = fmaf(ph.dx, rem, xb); ph.py = fmaf(ph.dy, rem, yb); ph.pz = fmaf(ph.dz, rem, zb);
+            float tn = rsqrtf(fmaf(tx, tx, fmaf(ty, ty, tz * tz)));
+            ph.dx = tx * tn; ph.dy = ty * tn; ph.dz = tz * tn;
+        }
+        float rem = (1.f - f) * len;
+        ph.px = fmaf(ph.dx, rem, xs); ph.py = fmaf(ph.dy, rem, yss); ph.pz = fmaf(ph.dz, rem, zs);
+        if (reflect) {
             const float a = water_alpha_f(sc, ph.py);
-            if (sc.adjoint) {
-                score_tau(sc, ph.sc, layer_of_f(sc, ph.py), a * len);
-                ph.sc.l += sc.inv_albedo;
-            }
+            if (sc.adjoint) score_tau(sc, ph.sc, layer_of_f(sc, ph.py), a * len);
             ph.tau = fmaf(a, len, ph.tau);
-            ph.E *= sc.floor_albedo32;
+        } else if (!(ph.py > ys)) {
+            // A transmitted photon is in the air. Near the surface a float32 height is
+            // quantised to ulp(ys) (3e-5 m at 400 m), as coarse as a grazing photon's
+            // vertical step, so the crossing fraction can round to 1 and leave no
+            // remaining step: the photon would sit on the surface, count as in water and
+            // exit a second time (a second transmission record, 1.5% of the photons at
+            // 400 m with 0.05 ns bins). Place it just above the surface instead.
+            ph.py = nextafterf(ys, 1.0e30f);
         }
         ph.s += 1;
         ++events;
+        const int m = mode();
+        if (m == kLaneAir) {
+            // on its way up it leaves the scene: the rest of its steps at once, as air() takes them
+            const float v = (float)sc.v_air * dt;
+            const float ay = ph.dy * v;
+            if (!(ay < 0.f)) {
+                const float k = (float)(S - ph.s);
+                ph.px = fmaf(k, ph.dx * v, ph.px); ph.py = fmaf(k, ay, ph.py); ph.pz = fmaf(k, ph.dz * v, ph.pz);
+                ph.s = S;
+                return kLaneDone;
+            }
+        }
+        return m;
+
     }
-}
+
+    // The step through the seafloor (handle_seafloor).
+    ALB_DEVICE int floor() {
+        const float yf = (float)sc.yf;
+        const float svx = ph.dx * cross_v, svy = ph.dy * cross_v, svz = ph.dz * cross_v;
+        const float len = sqrtf(fmaf(svx, svx, fmaf(svy, svy, svz * svz)));
+        float f = fminf(fmaxf((yf - ph.py) / svy, 0.f), 1.f);
+        float xb = fmaf(f, svx, ph.px), yb = yf, zb = fmaf(f, svz, ph.pz);
+        ph.sfi[0] = xb; ph.sfi[1] = yb; ph.sfi[2] = zb;
+        if (PASS == ALB_FORWARD && out.hm_radius && ph.fwi[0] == ph.fwi[0]) {
+            float ax = ph.fwi[0] - (float)sc.wc[0], az = ph.fwi[2] - (float)sc.wc[2];
+            float bx = xb - (float)sc.fc[0], bz = zb - (float)sc.fc[2];
+            int xi = (int)((sqrtf(ax * ax + az * az) / (float)sc.hm_wext) * sc.hm_bins);
+            int yi = (int)((sqrtf(bx * bx + bz * bz) / (float)sc.hm_fext) * sc.hm_bins);
+            if (xi >= 0 && xi < sc.hm_bins && yi >= 0 && yi < sc.hm_bins)
+                atomicAdd(out.hm_radius + xi * sc.hm_bins + yi, 1u);
+        }
+        emit_event_f<PASS>(out, ALB_BOTTOM_REFLECTION, kQueryBottom, ph, xb, yb, zb, ph.s, pid);
+        // normalize(+y + isotropic unit vector): a cosine lobe about +y
+        U4 b = src.block();
+        float z = fmaf(-2.f, uf(b.x), 1.f);
+        float r = sqrtf(fmaxf(0.f, 1.f - z * z));
+        float sp, cp;
+        __sincosf(6.283185307179586f * uf(b.y), &sp, &cp);
+        float hx = r * cp, hy = 1.f + z, hz = r * sp;
+        float hn = rsqrtf(fmaf(hx, hx, fmaf(hy, hy, hz * hz)));
+        ph.dx = hx * hn; ph.dy = hy * hn; ph.dz = hz * hn;
+        float rem = (1.f - f) * len;
+        ph.px = fmaf(ph.dx, rem, xb); ph.py = fmaf(ph.dy, rem, yb); ph.pz = fmaf(ph.dz, rem, zb);
+        const float a = water_alpha_f(sc, ph.py);
+        if (sc.adjoint) {
+            score_tau(sc, ph.sc, layer_of_f(sc, ph.py), a * len);
+            ph.sc.l += sc.inv_albedo;
+        }
+        ph.tau = fmaf(a, len, ph.tau);
+        ph.E *= sc.floor_albedo32;
+        ph.s += 1;
+        ++events;
+        return mode();
+
+    }
+
+    ALB_DEVICE void finish(uint64_t i) {
+        write_exit_state(out, ph, i);
+        ++done;
+    }
+};
 
 template <int PASS>
 ALB_DEVICE void emit_photon_fast(const SceneDev& sc, PhF& ph, PhiloxSrc& src) {
@@ -374,6 +432,15 @@ ALB_DEVICE void emit_photon_fast(const SceneDev& sc, PhF& ph, PhiloxSrc& src) {
         ph.dz = (d0 * R[6] + d1 * R[7]) + (l0 * R[6] + l1 * R[7] + z * R[8]);
         ph.t0 = 0.f;
     }
+}
+
+template <int PASS>
+ALB_DEVICE int FastLane<PASS>::start(uint64_t i) {
+    pid = (uint32_t)(first + i);
+    seek(src, first + i, i, nullptr);
+    guard = 0;
+    emit_photon_fast<PASS>(sc, ph, src);
+    return mode();
 }
 
 }  // namespace alb
