@@ -171,6 +171,9 @@ typedef struct AlbCtx AlbCtx;
 /* Simulation(config, rng): validate the scene, upload tables, allocate the context. */
 int alb_create(const AlbSceneParams* scene, int device, AlbCtx** out);
 void alb_destroy(AlbCtx* ctx);
+/* Device memory that contexts have released stays with the process for the next one, at most an
+ * eighth of the device: this gives what is idle of it back. */
+int alb_trim_memory(int device);
 const char* alb_last_error(const AlbCtx* ctx);
 int alb_set_option(AlbCtx* ctx, int key, int64_t value);
 

@@ -145,6 +145,7 @@ EXPORTED = [
     "alb_get_jacobian",
     "alb_create",
     "alb_destroy",
+    "alb_trim_memory",
     "alb_last_error",
     "alb_set_option",
     "alb_trace",
@@ -186,6 +187,7 @@ def load_library(path: str = LIB_PATH):
     lib.alb_create.argtypes = [C.POINTER(AlbSceneParams), C.c_int, C.POINTER(_P)]
     lib.alb_destroy.argtypes = [_P]
     lib.alb_destroy.restype = None
+    lib.alb_trim_memory.argtypes = [C.c_int]
     lib.alb_last_error.argtypes = [_P]
     lib.alb_last_error.restype = C.c_char_p
     lib.alb_set_option.argtypes = [_P, C.c_int, C.c_int64]

@@ -7,6 +7,7 @@
 #include <mutex>
 #include <string>
 #include <thread>
+#include <unordered_set>
 #include <vector>
 
 #include "albgpu.h"
@@ -18,6 +19,7 @@ using namespace alb;
 #include <atomic>
 static std::atomic<long long> g_launches{0};
 namespace alb {
+void set_global_error(const std::string& msg);
 void note_launch() { g_launches.fetch_add(1, std::memory_order_relaxed); }
 long long launches_total() { return g_launches.load(); }
 }  // namespace alb
@@ -26,17 +28,130 @@ long long launches_total() { return g_launches.load(); }
 // Workspace
 // ------------------------------------------------------------------------------------------
 
+// Device memory of every context comes from one pool per device, stream ordered, so that a context
+// made for one run and destroyed after it (run_linear, the batch's workers) does not map and unmap
+// its gigabytes each time and never stalls the device for another worker's stream. The pool
+// keeps at most an eighth of the device that nobody holds; what is over goes back to the driver at
+// the next synchronisation, alb_trim_memory gives back the rest, and so does a cudaMalloc that would
+// fail otherwise (measured: 160 GB beside 160 GB idle in the pool). Blocks over kDirect are cudaMalloc's: a pool
+// maps 16 GB in 13 ms, cudaMalloc in 1 ms, and so large a block would not be kept anyway.
+constexpr uint64_t kDirect = 16ull << 30;
+
+static std::mutex g_direct_mu;
+static std::unordered_set<void*> g_direct;
+
+static cudaMemPool_t device_pool() {
+    static std::mutex mu;
+    static cudaMemPool_t pools[64] = {};
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return nullptr;
+    std::lock_guard<std::mutex> g(mu);
+    if (!pools[dev]) {
+        cudaMemPoolProps props{};
+        props.allocType = cudaMemAllocationTypePinned;
+        props.location.type = cudaMemLocationTypeDevice;
+        props.location.id = dev;
+        cudaMemPool_t pool;
+        if (cudaMemPoolCreate(&pool, &props) != cudaSuccess) {
+            cudaGetLastError();
+            return nullptr;
+        }
+        size_t idle = 0, all = 0;
+        cudaMemGetInfo(&idle, &all);
+        uint64_t keep = all / 8;
+        cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep);
+        pools[dev] = pool;
+    }
+    return pools[dev];
+}
+
+// Bytes the device's pool holds that nobody uses.
+static uint64_t pool_idle() {
+    uint64_t reserved = 0, used = 0;
+    const cudaMemPool_t pool = device_pool();
+    if (!pool || cudaMemPoolGetAttribute(pool, cudaMemPoolAttrReservedMemCurrent, &reserved) != cudaSuccess ||
+        cudaMemPoolGetAttribute(pool, cudaMemPoolAttrUsedMemCurrent, &used) != cudaSuccess) {
+        cudaGetLastError();
+        return 0;
+    }
+    return reserved - used;
+}
+
+extern "C" int alb_trim_memory(int device) {
+    int before = 0;
+    if (cudaGetDevice(&before) != cudaSuccess || cudaSetDevice(device) != cudaSuccess) {
+        cudaGetLastError();
+        set_global_error("alb_trim_memory: no such device");
+        return ALB_ERR_INVALID;
+    }
+    const cudaMemPool_t pool = device_pool();
+    const bool ok = pool && cudaMemPoolTrimTo(pool, 0) == cudaSuccess;
+    cudaSetDevice(before);
+    if (ok) return ALB_OK;
+    cudaGetLastError();
+    set_global_error("alb_trim_memory: the pool could not be trimmed");
+    return ALB_ERR_CUDA;
+}
+
+namespace alb {
+void* dev_alloc(uint64_t bytes, cudaStream_t st) {
+    const cudaMemPool_t pool = device_pool();
+    if (!pool) return nullptr;
+    if (bytes == 0) bytes = 16;
+    for (int attempt = 0; attempt < 2; ++attempt) {
+        void* p = nullptr;
+        if (bytes > kDirect) {
+            if (cudaMalloc(&p, bytes) == cudaSuccess) {
+                std::lock_guard<std::mutex> g(g_direct_mu);
+                g_direct.insert(p);
+                return p;
+            }
+        } else if (cudaMallocFromPoolAsync(&p, bytes, pool, st) == cudaSuccess) return p;
+        cudaGetLastError();
+        if (attempt == 0) {  // once more with every idle block given back to the driver
+            cudaStreamSynchronize(st);
+            cudaMemPoolTrimTo(pool, 0);
+        }
+    }
+    return nullptr;
+}
+
+void dev_free(void* p, cudaStream_t st) {
+    if (!p) return;
+    {
+        std::unique_lock<std::mutex> g(g_direct_mu);
+        if (g_direct.erase(p)) {
+            g.unlock();
+            cudaStreamSynchronize(st);
+            cudaFree(p);
+            return;
+        }
+    }
+    cudaFreeAsync(p, st);
+}
+}  // namespace alb
+
+template <class T>
+static bool take(T*& p, uint64_t bytes, cudaStream_t st) {
+    p = (T*)dev_alloc(bytes, st);
+    return p != nullptr;
+}
+
+template <class T>
+static void drop(T*& p, cudaStream_t st) {
+    dev_free(p, st);
+    p = nullptr;
+}
+
 Workspace::~Workspace() {
-    for (void* p : temps_) cudaFree(p);
-    if (box_) cudaFree(box_);
+    for (void* p : temps_) dev_free(p, st_);
+    dev_free(box_, st_);
 }
 
 void* Workspace::take_bytes(uint64_t bytes) {
-    void* p = nullptr;
-    if (bytes == 0) bytes = 16;
-    if (cudaMallocAsync(&p, bytes, st_) != cudaSuccess) {
+    void* p = dev_alloc(bytes, st_);
+    if (!p) {
         failed_ = true;
-        cudaGetLastError();
         return nullptr;
     }
     temps_.push_back(p);
@@ -45,31 +160,22 @@ void* Workspace::take_bytes(uint64_t bytes) {
 
 void Workspace::release(size_t m) {
     while (temps_.size() > m) {
-        cudaFreeAsync(temps_.back(), st_);
+        dev_free(temps_.back(), st_);
         temps_.pop_back();
     }
 }
 
 unsigned* Workspace::scratch_box() {
-    if (!box_) {
-        if (cudaMalloc(&box_, 64 * sizeof(unsigned)) != cudaSuccess) {
-            failed_ = true;
-            cudaGetLastError();
-        }
-    }
+    if (!box_ && !(box_ = (unsigned*)dev_alloc(64 * sizeof(unsigned), st_))) failed_ = true;
     return box_;
 }
 
-static void* grow(void* old, uint64_t& cap, uint64_t n, size_t elem, bool& failed) {
+static void* grow(void* old, uint64_t& cap, uint64_t n, size_t elem, bool& failed, cudaStream_t st) {
     if (cap >= n && old) return old;
-    if (old) {
-        cudaDeviceSynchronize();
-        cudaFree(old);
-    }
+    dev_free(old, st);
     uint64_t want = std::max<uint64_t>(n + n / 32, 256);
-    void* p = nullptr;
-    if (cudaMalloc(&p, want * elem) != cudaSuccess) {
-        cudaGetLastError();
+    void* p = dev_alloc(want * elem, st);
+    if (!p) {
         failed = true;
         cap = 0;
         return nullptr;
@@ -78,8 +184,8 @@ static void* grow(void* old, uint64_t& cap, uint64_t n, size_t elem, bool& faile
     return p;
 }
 
-void* Workspace::alloc_persistent(void* old, uint64_t& cap, uint64_t n) { return grow(old, cap, n, 16, failed_); }
-void* Workspace::alloc_persistent_u32(void* old, uint64_t& cap, uint64_t n) { return grow(old, cap, n, 4, failed_); }
+void* Workspace::alloc_persistent(void* old, uint64_t& cap, uint64_t n) { return grow(old, cap, n, 16, failed_, st_); }
+void* Workspace::alloc_persistent_u32(void* old, uint64_t& cap, uint64_t n) { return grow(old, cap, n, 4, failed_, st_); }
 
 // ------------------------------------------------------------------------------------------
 // Context
@@ -88,6 +194,7 @@ void* Workspace::alloc_persistent_u32(void* old, uint64_t& cap, uint64_t n) { re
 struct AlbCtx {
     int device = 0;
     cudaStream_t st = 0;
+    bool callers_stream = false;  // st came with ALB_OPT_STREAM
     SceneDev sc{};
     FastScene fast{};
     std::vector<void*> tables;
@@ -96,6 +203,9 @@ struct AlbCtx {
     RecordStore rec[ALB_CHANNELS];
     uint64_t rec_id_cap[ALB_CHANNELS] = {0};
     uint64_t fwi_cap[ALB_CHANNELS] = {0}, sfi_cap[ALB_CHANNELS] = {0}, b_cap[ALB_CHANNELS] = {0};
+    // one control block: record counts [0, 4), query counts [4, 7), error word [7], counters [8, 40),
+    // the scatter gather's work counter [40], counters kept across a retried trace [41, 43)
+    unsigned long long* ctl = nullptr;
     unsigned long long* d_rec_count = nullptr;
     uint64_t h_rec_count[ALB_CHANNELS] = {0};
     double rec_rate[ALB_CHANNELS] = {2.0, 8.0, 1.05, 1.05};
@@ -117,10 +227,11 @@ struct AlbCtx {
     unsigned long long* d_q_count = nullptr;
     uint64_t h_q_count[3] = {0, 0, 0};
     double q_rate[3] = {2.0, 8.0, 1.05};
+    bool rec_rate_known = false, q_rate_known = false;  // measured by a trace of this scene's context
     // accumulators
     unsigned long long* wf = nullptr;  // lo words then hi words, [2][channels][nbins]
     unsigned long long* hm = nullptr;  // sampled heatmaps, [2 maps][2 words][bins*bins]
-    unsigned* hm_radius = nullptr;
+    unsigned *hm_radius = nullptr, *hm_radius_bak = nullptr;
     // adjoint Jacobian: lo words then hi words, [2][kJacParams][channels][nbins]
     unsigned long long* jac = nullptr;
     // sums of one gather by exponent class (every gather leaves them zero)
@@ -140,7 +251,7 @@ struct AlbCtx {
     uint64_t ex_cap = 0, ex_n = 0;
     // misc
     int* d_err = nullptr;
-    unsigned long long* d_stats = nullptr;  // 32 counters, then the scatter gather's work counter
+    unsigned long long* d_stats = nullptr;
     int keep_exit = 0, keep_ids = 0, precise = 1, sort_q = 1;
     int64_t map_cap_hint = 0;
     int launches = 0;
@@ -149,30 +260,56 @@ struct AlbCtx {
     double phase_ms[ALB_PHASES] = {0};
     int64_t phase_calls[ALB_PHASES] = {0};
     int64_t gathered[ALB_CHANNELS] = {0};
-    cudaEvent_t ev[2 * ALB_PHASES] = {};
-    bool ev_ready = false;
+    // recorded phases whose times are read at the next synchronisation, and idle events
+    struct Phase {
+        int phase;
+        cudaEvent_t e0, e1;
+    };
+    std::vector<Phase> pending;
+    std::vector<cudaEvent_t> events;
+    // streams of the small gathers, forked from and joined to st
+    cudaStream_t side[3] = {};
+    cudaEvent_t fork = nullptr, join[3] = {};
 };
 
-// Time one phase: record a start event, run `body`, record a stop event, and fold the
-// elapsed time into the accumulator once the stream has drained (the caller syncs).
+static cudaEvent_t take_event(AlbCtx* c) {
+    cudaEvent_t e = nullptr;
+    if (!c->events.empty()) {
+        e = c->events.back();
+        c->events.pop_back();
+    } else {
+        cudaEventCreate(&e);
+    }
+    return e;
+}
+
+// Time one phase between two events on its stream; the times are folded into the accumulators
+// once the stream has drained (fold_phases).
 struct PhaseTimer {
     AlbCtx* c;
-    int phase;
-    PhaseTimer(AlbCtx* ctx, int p) : c(ctx), phase(p) {
-        if (!c->ev_ready) {
-            for (auto& e : c->ev) cudaEventCreate(&e);
-            c->ev_ready = true;
-        }
-        cudaEventRecord(c->ev[2 * phase], c->st);
+    AlbCtx::Phase p;
+    PhaseTimer(AlbCtx* ctx, int phase, cudaStream_t st) : c(ctx), p{phase, take_event(ctx), take_event(ctx)} {
+        cudaEventRecord(p.e0, st);
     }
-    void stop() {
-        cudaEventRecord(c->ev[2 * phase + 1], c->st);
-        cudaEventSynchronize(c->ev[2 * phase + 1]);
-        float ms = 0.f;
-        if (cudaEventElapsedTime(&ms, c->ev[2 * phase], c->ev[2 * phase + 1]) == cudaSuccess) c->phase_ms[phase] += ms;
-        c->phase_calls[phase] += 1;
+    PhaseTimer(AlbCtx* ctx, int phase) : PhaseTimer(ctx, phase, ctx->st) {}
+    void stop(cudaStream_t st) {
+        cudaEventRecord(p.e1, st);
+        c->phase_calls[p.phase] += 1;
+        c->pending.push_back(p);
     }
+    void stop() { stop(c->st); }
 };
+
+static void fold_phases(AlbCtx* c) {
+    for (const auto& p : c->pending) {
+        float ms = 0.f;
+        if (cudaEventSynchronize(p.e1) == cudaSuccess && cudaEventElapsedTime(&ms, p.e0, p.e1) == cudaSuccess)
+            c->phase_ms[p.phase] += ms;
+        c->events.push_back(p.e0);
+        c->events.push_back(p.e1);
+    }
+    c->pending.clear();
+}
 
 static int fail(AlbCtx* c, int code, const std::string& msg) {
     if (c) c->err = msg;
@@ -185,17 +322,21 @@ static int fail(AlbCtx* c, int code, const std::string& msg) {
         if (e_ != cudaSuccess) return fail(ctx, ALB_ERR_CUDA, std::string(#call ": ") + cudaGetErrorString(e_)); \
     } while (0)
 
-static int check_device(AlbCtx* ctx, const char* where) {
-    cudaError_t e = cudaStreamSynchronize(ctx->st);
+// Waits for the context's stream and reports what failed on it; counts (nullable) receives the
+// record and query counts.
+static int check_device(AlbCtx* ctx, const char* where, unsigned long long* counts = nullptr) {
+    unsigned long long ctl[8] = {0};
+    cudaError_t e = cudaMemcpyAsync(ctl, ctx->ctl, sizeof ctl, cudaMemcpyDeviceToHost, ctx->st);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->st);
     if (e == cudaSuccess) e = cudaGetLastError();
+    fold_phases(ctx);
     if (e != cudaSuccess) return fail(ctx, ALB_ERR_CUDA, std::string(where) + ": " + cudaGetErrorString(e));
     if (ctx->ws.failed()) {
         ctx->ws.clear_failed();
         return fail(ctx, ALB_ERR_CUDA, std::string(where) + ": device allocation failed");
     }
-    int h = 0;
-    CK(cudaMemcpyAsync(&h, ctx->d_err, sizeof(int), cudaMemcpyDeviceToHost, ctx->st));
-    CK(cudaStreamSynchronize(ctx->st));
+    if (counts) std::memcpy(counts, ctl, 7 * 8);
+    const int h = (int)(uint32_t)ctl[7];
     if (h != 0) {
         CK(cudaMemsetAsync(ctx->d_err, 0, sizeof(int), ctx->st));
         CK(cudaStreamSynchronize(ctx->st));
@@ -220,11 +361,8 @@ void set_global_error(const std::string& msg) { g_create_error = msg; }
 
 extern "C" const char* alb_last_error(const AlbCtx* ctx) { return ctx ? ctx->err.c_str() : g_create_error.c_str(); }
 
-static void* table_buf(void*& slot, size_t bytes) {
-    if (!slot && cudaMalloc(&slot, bytes) != cudaSuccess) {
-        cudaGetLastError();
-        slot = nullptr;
-    }
+static void* table_buf(void*& slot, size_t bytes, cudaStream_t st) {
+    if (!slot) slot = dev_alloc(bytes, st);
     return slot;
 }
 
@@ -342,7 +480,7 @@ static std::string set_scene(AlbCtx* ctx, const AlbSceneParams* p) {
         if (L.dlog_weight_g) {
             std::vector<float> d(N);
             for (int i = 0; i < N; ++i) d[i] = (float)L.dlog_weight_g[i];
-            float* dd = (float*)table_buf(ctx->lt[l].dlw, N * sizeof(float));
+            float* dd = (float*)table_buf(ctx->lt[l].dlw, N * sizeof(float), ctx->st);
             if (!dd) return std::string("table allocation failed");
             cudaMemcpyAsync(dd, d.data(), N * sizeof(float), cudaMemcpyHostToDevice, ctx->st);
             cudaStreamSynchronize(ctx->st);
@@ -352,7 +490,7 @@ static std::string set_scene(AlbCtx* ctx, const AlbSceneParams* p) {
         if (L.dlog_sample_g) {
             std::vector<float> d(N);
             for (int i = 0; i < N; ++i) d[i] = (float)L.dlog_sample_g[i];
-            float* dd = (float*)table_buf(ctx->lt[l].dsg, N * sizeof(float));
+            float* dd = (float*)table_buf(ctx->lt[l].dsg, N * sizeof(float), ctx->st);
             if (!dd) return std::string("table allocation failed");
             cudaMemcpyAsync(dd, d.data(), N * sizeof(float), cudaMemcpyHostToDevice, ctx->st);
             cudaStreamSynchronize(ctx->st);
@@ -383,9 +521,9 @@ static std::string set_scene(AlbCtx* ctx, const AlbSceneParams* p) {
             if (L.n_kind < 0 || L.n_kind > 2 || L.a_kind < 0 || L.a_kind > 2) return std::string("unknown profile kind");
             float* lz;
             double* la;  // values, then slopes
-            if (cudaMalloc(&lz, L.lut_n * sizeof(float)) != cudaSuccess) return std::string("table allocation failed");
+            if (!take(lz, L.lut_n * sizeof(float), ctx->st)) return std::string("table allocation failed");
             ctx->tables.push_back(lz);
-            if (cudaMalloc(&la, 2 * L.lut_n * sizeof(double)) != cudaSuccess) return std::string("table allocation failed");
+            if (!take(la, 2 * L.lut_n * sizeof(double), ctx->st)) return std::string("table allocation failed");
             ctx->tables.push_back(la);
             std::vector<double> slopes(L.lut_n, 0.0);
             for (int i = 0; i + 1 < L.lut_n; ++i)
@@ -407,10 +545,10 @@ static std::string set_scene(AlbCtx* ctx, const AlbSceneParams* p) {
             s.layer_a0[l] = L.a_start;
             s.layer_a1[l] = L.a_end;
         }
-        double* th = (double*)table_buf(ctx->lt[l].th, N * sizeof(double));
-        double* cdf = (double*)table_buf(ctx->lt[l].cdf, N * sizeof(double));
-        double* sl = (double*)table_buf(ctx->lt[l].sl, N * sizeof(double));
-        float* w = (float*)table_buf(ctx->lt[l].w, N * sizeof(float));
+        double* th = (double*)table_buf(ctx->lt[l].th, N * sizeof(double), ctx->st);
+        double* cdf = (double*)table_buf(ctx->lt[l].cdf, N * sizeof(double), ctx->st);
+        double* sl = (double*)table_buf(ctx->lt[l].sl, N * sizeof(double), ctx->st);
+        float* w = (float*)table_buf(ctx->lt[l].w, N * sizeof(float), ctx->st);
         if (!th || !cdf || !sl || !w) return std::string("table allocation failed");
         std::vector<double> slope(N, 0.0);
         std::memcpy(slope.data(), L.phase_slope, (N - 1) * sizeof(double));
@@ -424,8 +562,8 @@ static std::string set_scene(AlbCtx* ctx, const AlbSceneParams* p) {
         s.layer_cdf[l] = cdf;
         s.layer_slope[l] = sl;
         s.layer_weight[l] = w;
-        float* dinv = (float*)table_buf(ctx->lt[l].inv, (kInvCdf + 1) * sizeof(float));
-        uint16_t* guide = (uint16_t*)table_buf(ctx->lt[l].guide, (kInvCdf + 1) * sizeof(uint16_t));
+        float* dinv = (float*)table_buf(ctx->lt[l].inv, (kInvCdf + 1) * sizeof(float), ctx->st);
+        uint16_t* guide = (uint16_t*)table_buf(ctx->lt[l].guide, (kInvCdf + 1) * sizeof(uint16_t), ctx->st);
         if (!dinv || !guide) return std::string("table allocation failed");
         launch_phase_tables(cdf, th, sl, dinv, guide, ctx->st);
         s.layer_guide[l] = guide;
@@ -440,11 +578,11 @@ static std::string set_scene(AlbCtx* ctx, const AlbSceneParams* p) {
     if (logs) {
         double* d = nullptr;
         double h[4 * ALB_MAX_LAYERS];
-        if (cudaMalloc(&d, sizeof h) != cudaSuccess) return std::string("table allocation failed");
+        if (!take(d, sizeof h, ctx->st)) return std::string("table allocation failed");
         launch_profile_logs(s, d, ctx->st);
         const cudaError_t e = cudaMemcpyAsync(h, d, sizeof h, cudaMemcpyDeviceToHost, ctx->st);
         cudaStreamSynchronize(ctx->st);
-        cudaFree(d);
+        drop(d, ctx->st);
         if (e != cudaSuccess) return std::string("profile tables failed");
         for (int l = 0; l < s.n_layers; ++l) {
             s.layer_nl0[l] = h[4 * l];
@@ -462,14 +600,8 @@ static std::string ensure_accumulators(AlbCtx* ctx) {
     const SceneDev& s = ctx->sc;
     auto regrow = [&](unsigned long long*& buf, int64_t& have, int64_t need, size_t words_per) -> bool {
         if (buf && have >= need) return true;
-        if (buf) {
-            cudaStreamSynchronize(ctx->st);
-            cudaFree(buf);
-            buf = nullptr;
-        }
-        if (cudaMalloc(&buf, (size_t)need * words_per * 8) != cudaSuccess) {
-            cudaGetLastError();
-            buf = nullptr;
+        drop(buf, ctx->st);
+        if (!take(buf, (size_t)need * words_per * 8, ctx->st)) {
             have = 0;
             return false;
         }
@@ -489,14 +621,11 @@ static std::string ensure_accumulators(AlbCtx* ctx) {
         // two maps of class words: 10 MB at the default 200 bins; larger maps add directly
         if (s.hm_bins <= 512 && !regrow(ctx->heat_cls, ctx->heat_cls_cells, hb, 32)) return "heatmap allocation failed";
         if (!ctx->hm_radius || ctx->hm_radius_cells < hb) {
-            if (ctx->hm_radius) {
-                cudaStreamSynchronize(ctx->st);
-                cudaFree(ctx->hm_radius);
-            }
-            if (cudaMalloc(&ctx->hm_radius, hb * 4) != cudaSuccess) {
-                ctx->hm_radius = nullptr;
+            drop(ctx->hm_radius, ctx->st);
+            drop(ctx->hm_radius_bak, ctx->st);
+            ctx->hm_radius_cells = 0;
+            if (!take(ctx->hm_radius, hb * 4, ctx->st) || !take(ctx->hm_radius_bak, hb * 4, ctx->st))
                 return "heatmap allocation failed";
-            }
             cudaMemsetAsync(ctx->hm_radius, 0, hb * 4, ctx->st);
             ctx->hm_radius_cells = hb;
         }
@@ -504,7 +633,11 @@ static std::string ensure_accumulators(AlbCtx* ctx) {
     return std::string();
 }
 
-extern "C" int alb_create(const AlbSceneParams* p, int device, AlbCtx** out) {
+static int create_on(const AlbSceneParams* p, int device, cudaStream_t st, AlbCtx** out);
+
+extern "C" int alb_create(const AlbSceneParams* p, int device, AlbCtx** out) { return create_on(p, device, nullptr, out); }
+
+static int create_on(const AlbSceneParams* p, int device, cudaStream_t st, AlbCtx** out) {
     if (!p || !out) return ALB_ERR_INVALID;
     *out = nullptr;
     AlbCtx* ctx = new AlbCtx();
@@ -515,22 +648,18 @@ extern "C" int alb_create(const AlbSceneParams* p, int device, AlbCtx** out) {
     };
     ctx->device = device;
     if (cudaSetDevice(device) != cudaSuccess) return bad("cudaSetDevice failed");
-    cudaMemPool_t pool;
-    if (cudaDeviceGetDefaultMemPool(&pool, device) == cudaSuccess) {
-        uint64_t thr = UINT64_MAX;
-        cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &thr);
-    }
+    ctx->st = st;
+    ctx->ws.set_stream(st);
     std::string e = set_scene(ctx, p);
     if (e.empty()) e = ensure_accumulators(ctx);
     if (!e.empty()) return bad(e);
-    if (cudaMalloc(&ctx->d_rec_count, ALB_CHANNELS * 8) != cudaSuccess || cudaMalloc(&ctx->d_q_count, 3 * 8) != cudaSuccess ||
-        cudaMalloc(&ctx->d_err, sizeof(int)) != cudaSuccess || cudaMalloc(&ctx->d_stats, 33 * 8) != cudaSuccess)
-        return bad("counter allocation failed");
-    cudaMemset(ctx->d_rec_count, 0, ALB_CHANNELS * 8);
-    cudaMemset(ctx->d_q_count, 0, 3 * 8);
-    cudaMemset(ctx->d_err, 0, sizeof(int));
-    cudaMemset(ctx->d_stats, 0, 32 * 8);
-    if (cudaDeviceSynchronize() != cudaSuccess) return bad("device initialisation failed");
+    if (!take(ctx->ctl, 64 * 8, st)) return bad("counter allocation failed");
+    ctx->d_rec_count = ctx->ctl;
+    ctx->d_q_count = ctx->ctl + 4;
+    ctx->d_err = (int*)(ctx->ctl + 7);
+    ctx->d_stats = ctx->ctl + 8;
+    cudaMemsetAsync(ctx->ctl, 0, 64 * 8, st);
+    if (cudaStreamSynchronize(st) != cudaSuccess) return bad("device initialisation failed");
     *out = ctx;
     return ALB_OK;
 }
@@ -538,28 +667,44 @@ extern "C" int alb_create(const AlbSceneParams* p, int device, AlbCtx** out) {
 extern "C" void alb_destroy(AlbCtx* ctx) {
     if (!ctx) return;
     cudaSetDevice(ctx->device);
-    cudaDeviceSynchronize();
-    for (void* p : ctx->tables) cudaFree(p);
+    // a caller's stream may be gone by now: wait for the device and free in the default stream
+    if (ctx->callers_stream) {
+        cudaDeviceSynchronize();
+        ctx->st = nullptr;
+        ctx->ws.set_stream(nullptr);
+    }
+    const cudaStream_t st = ctx->st;
+    cudaStreamSynchronize(st);
+    for (void* p : ctx->tables) dev_free(p, st);
     for (int c = 0; c < ALB_CHANNELS; ++c) {
-        cudaFree(ctx->rec[c].a); cudaFree(ctx->rec[c].fwi); cudaFree(ctx->rec[c].sfi);
-        cudaFree(ctx->rec[c].id); cudaFree(ctx->rec[c].sco);
-        MapIndex& m = ctx->map[c];
-        cudaFree(m.a); cudaFree(m.b); cudaFree(m.fwi); cudaFree(m.sfi); cudaFree(m.id); cudaFree(m.sco);
-        cudaFree(m.box_lo); cudaFree(m.box_hi);
+        RecordStore& r = ctx->rec[c];
+        for (void* p : {(void*)r.a, (void*)r.fwi, (void*)r.sfi, (void*)r.id, (void*)r.sco}) dev_free(p, st);
+        release_map_index(ctx->map[c], st);
+        dev_free(ctx->map[c].box_lo, st);
+        dev_free(ctx->map[c].box_hi, st);
     }
-    for (int k = 0; k < 3; ++k) {
-        cudaFree(ctx->qa[k]); cudaFree(ctx->qb[k]); cudaFree(ctx->qc[k]); cudaFree(ctx->qid[k]); cudaFree(ctx->qperm[k]);
-        cudaFree(ctx->qrk[k][0]); cudaFree(ctx->qrk[k][1]); cudaFree(ctx->qs[k]);
+    for (int k = 0; k < 3; ++k)
+        for (void* p : {(void*)ctx->qa[k], (void*)ctx->qb[k], (void*)ctx->qc[k], (void*)ctx->qid[k], (void*)ctx->qperm[k],
+                        (void*)ctx->qrk[k][0], (void*)ctx->qrk[k][1], (void*)ctx->qs[k]})
+            dev_free(p, st);
+    for (void* p : {(void*)ctx->wf, (void*)ctx->cls, (void*)ctx->jac_cls, (void*)ctx->heat_cls, (void*)ctx->hm,
+                    (void*)ctx->hm_radius, (void*)ctx->hm_radius_bak, (void*)ctx->jac, (void*)ctx->ex_pos,
+                    (void*)ctx->ex_dir, (void*)ctx->ex_f, (void*)ctx->ctl})
+        dev_free(p, st);
+    for (auto& t : ctx->lt)
+        for (void* p : {t.th, t.cdf, t.sl, t.w, t.dlw, t.dsg, t.inv, t.guide}) dev_free(p, st);
+    for (const auto& p : ctx->pending) {
+        cudaEventDestroy(p.e0);
+        cudaEventDestroy(p.e1);
     }
-    cudaFree(ctx->wf); cudaFree(ctx->cls); cudaFree(ctx->jac_cls); cudaFree(ctx->heat_cls); cudaFree(ctx->hm); cudaFree(ctx->hm_radius); cudaFree(ctx->jac);
-    for (auto& t : ctx->lt) {
-        cudaFree(t.th); cudaFree(t.cdf); cudaFree(t.sl); cudaFree(t.w); cudaFree(t.dlw); cudaFree(t.dsg); cudaFree(t.inv); cudaFree(t.guide);
-    }
-    cudaFree(ctx->ex_pos); cudaFree(ctx->ex_dir); cudaFree(ctx->ex_f);
-    cudaFree(ctx->d_rec_count); cudaFree(ctx->d_q_count); cudaFree(ctx->d_err); cudaFree(ctx->d_stats);
-    if (ctx->ev_ready)
-        for (auto& e : ctx->ev) cudaEventDestroy(e);
+    for (cudaEvent_t e : ctx->events) cudaEventDestroy(e);
+    if (ctx->fork) cudaEventDestroy(ctx->fork);
+    for (cudaEvent_t e : ctx->join)
+        if (e) cudaEventDestroy(e);
+    for (cudaStream_t x : ctx->side)
+        if (x) cudaStreamDestroy(x);
     delete ctx;
+    cudaStreamSynchronize(st);  // what the pool does not keep goes back to the driver here
 }
 
 extern "C" int alb_set_option(AlbCtx* ctx, int key, int64_t v) {
@@ -571,7 +716,9 @@ extern "C" int alb_set_option(AlbCtx* ctx, int key, int64_t v) {
         case ALB_OPT_MAP_CAPACITY: ctx->map_cap_hint = v; break;
         case ALB_OPT_SORT_QUERIES: ctx->sort_q = (int)v; break;
         case ALB_OPT_STREAM:
+            // every call has waited for its stream, so nothing is pending on the old one
             ctx->st = (cudaStream_t)(intptr_t)v;
+            ctx->callers_stream = true;
             ctx->ws.set_stream(ctx->st);
             break;
         case ALB_OPT_ADJOINT: {
@@ -594,33 +741,38 @@ extern "C" int alb_set_option(AlbCtx* ctx, int key, int64_t v) {
     return ALB_OK;
 }
 
-// grow a record store to hold `need` records, preserving the first `keep`
 // backward photons traced and gathered per chunk when no per-photon state is exported
 constexpr uint64_t kBackwardChunk = 1ull << 22;
+// photons that measure the records (or queries) per photon of a scene not traced before: a large
+// trace into buffers sized by the defaults runs twice
+constexpr uint64_t kPilot = 1ull << 14;
 
+static void release_records(AlbCtx* ctx, int c) {
+    RecordStore& r = ctx->rec[c];
+    for (void* p : {(void*)r.a, (void*)r.fwi, (void*)r.sfi, (void*)r.id, (void*)r.sco}) dev_free(p, ctx->st);
+    r = RecordStore{};
+}
+
+// grow a record store to hold `need` records, preserving the first `keep`
 static int ensure_records(AlbCtx* ctx, int c, uint64_t need, uint64_t keep) {
     RecordStore& r = ctx->rec[c];
     bool want_hm = ctx->sc.heatmap != 0;
     bool want_id = ctx->keep_ids != 0;
     bool want_sco = ctx->sc.adjoint != 0;
     if (r.cap >= need && (!want_id || r.id) && (!want_hm || r.fwi) && (!want_sco || r.sco)) return ALB_OK;
-    uint64_t cap = std::max<uint64_t>(need + need / 16, 1024);
-    if (!keep) {  // nothing to copy: release the old store first, so the peak is one store
-        CK(cudaStreamSynchronize(ctx->st));
-        cudaFree(r.a); cudaFree(r.fwi); cudaFree(r.sfi); cudaFree(r.id); cudaFree(r.sco);
-        r = RecordStore{};
-    }
+    // small stores double, so that a pass of many batches does not copy its records for each
+    uint64_t cap = std::max<uint64_t>(need + (keep ? std::max<uint64_t>(need / 16, std::min<uint64_t>(need, 1ull << 24)) : need / 16), 1024);
+    if (!keep) release_records(ctx, c);  // nothing to copy: the peak is one store
     float4 *a = nullptr, *fwi = nullptr, *sfi = nullptr, *sco = nullptr;
     uint32_t* id = nullptr;
     // every allocation is checked, and a failure frees what this call had taken; the two
     // record halves are interleaved in one allocation (RecordStore)
-    bool ok = cudaMalloc(&a, cap * 32) == cudaSuccess;
-    if (ok && want_hm) ok = cudaMalloc(&fwi, cap * 16) == cudaSuccess && cudaMalloc(&sfi, cap * 16) == cudaSuccess;
-    if (ok && want_id) ok = cudaMalloc(&id, cap * 4) == cudaSuccess;
-    if (ok && want_sco) ok = cudaMalloc(&sco, cap * 16) == cudaSuccess;
+    bool ok = take(a, cap * 32, ctx->st);
+    if (ok && want_hm) ok = take(fwi, cap * 16, ctx->st) && take(sfi, cap * 16, ctx->st);
+    if (ok && want_id) ok = take(id, cap * 4, ctx->st);
+    if (ok && want_sco) ok = take(sco, cap * 16, ctx->st);
     if (!ok) {
-        cudaGetLastError();
-        cudaFree(a); cudaFree(fwi); cudaFree(sfi); cudaFree(id); cudaFree(sco);
+        drop(a, ctx->st); drop(fwi, ctx->st); drop(sfi, ctx->st); drop(id, ctx->st); drop(sco, ctx->st);
         return fail(ctx, ALB_ERR_CUDA, "photon-map store: out of device memory");
     }
     if (keep) {
@@ -632,16 +784,9 @@ static int ensure_records(AlbCtx* ctx, int c, uint64_t need, uint64_t keep) {
         if (want_id && r.id) CK(cudaMemcpyAsync(id, r.id, keep * 4, cudaMemcpyDeviceToDevice, ctx->st));
         if (want_sco && r.sco) CK(cudaMemcpyAsync(sco, r.sco, keep * 16, cudaMemcpyDeviceToDevice, ctx->st));
     }
-    CK(cudaStreamSynchronize(ctx->st));
-    cudaFree(r.a); cudaFree(r.fwi); cudaFree(r.sfi); cudaFree(r.id); cudaFree(r.sco);
+    release_records(ctx, c);
     r.a = a; r.b = a + 1; r.fwi = fwi; r.sfi = sfi; r.id = id; r.sco = sco; r.cap = cap;
     return ALB_OK;
-}
-
-static void release_records(AlbCtx* ctx, int c) {
-    RecordStore& r = ctx->rec[c];
-    cudaFree(r.a); cudaFree(r.fwi); cudaFree(r.sfi); cudaFree(r.id); cudaFree(r.sco);
-    r = RecordStore{};
 }
 
 // Bring a channel's records back into an append store (from its index) before appending.
@@ -671,22 +816,16 @@ static int restore_records(AlbCtx* ctx, int c, uint64_t need) {
 static int ensure_queries(AlbCtx* ctx, int k, uint64_t need) {
     if (ctx->qcap[k] >= need && (!ctx->keep_ids || ctx->qid[k]) && (!ctx->sc.adjoint || ctx->qs[k])) return ALB_OK;
     uint64_t cap = std::max<uint64_t>(need + need / 4, 1024);
-    CK(cudaStreamSynchronize(ctx->st));
-    cudaFree(ctx->qa[k]); cudaFree(ctx->qb[k]); cudaFree(ctx->qc[k]); cudaFree(ctx->qid[k]); cudaFree(ctx->qperm[k]);
-    cudaFree(ctx->qrk[k][0]); cudaFree(ctx->qrk[k][1]); cudaFree(ctx->qs[k]);
-    ctx->qa[k] = ctx->qb[k] = ctx->qc[k] = nullptr; ctx->qperm[k] = nullptr;
-    ctx->qid[k] = nullptr; ctx->qrk[k][0] = ctx->qrk[k][1] = nullptr; ctx->qs[k] = nullptr;
+    const cudaStream_t st = ctx->st;
+    drop(ctx->qa[k], st); drop(ctx->qb[k], st); drop(ctx->qc[k], st); drop(ctx->qid[k], st); drop(ctx->qperm[k], st);
+    drop(ctx->qrk[k][0], st); drop(ctx->qrk[k][1], st); drop(ctx->qs[k], st);
     ctx->qcap[k] = 0;
-    CK(cudaMalloc(&ctx->qa[k], cap * 16));
-    CK(cudaMalloc(&ctx->qb[k], cap * 16));
-    CK(cudaMalloc(&ctx->qc[k], cap * 16));
-    CK(cudaMalloc(&ctx->qperm[k], cap * 4));
-    if (ctx->keep_ids) {
-        CK(cudaMalloc(&ctx->qid[k], cap * 4));
-        CK(cudaMalloc(&ctx->qrk[k][0], cap * 8));
-        CK(cudaMalloc(&ctx->qrk[k][1], cap * 8));
-    }
-    if (ctx->sc.adjoint) CK(cudaMalloc(&ctx->qs[k], cap * 16));
+    bool ok = take(ctx->qa[k], cap * 16, st) && take(ctx->qb[k], cap * 16, st) && take(ctx->qc[k], cap * 16, st) &&
+              take(ctx->qperm[k], cap * 4, st);
+    if (ok && ctx->keep_ids)
+        ok = take(ctx->qid[k], cap * 4, st) && take(ctx->qrk[k][0], cap * 8, st) && take(ctx->qrk[k][1], cap * 8, st);
+    if (ok && ctx->sc.adjoint) ok = take(ctx->qs[k], cap * 16, st);
+    if (!ok) return fail(ctx, ALB_ERR_CUDA, "gather queries: out of device memory");
     ctx->qcap[k] = cap;
     return ALB_OK;
 }
@@ -742,6 +881,75 @@ static int check_map_sizes(AlbCtx* ctx) {
     return ALB_OK;
 }
 
+// Sorts the queries of the last backward trace and gathers them from their maps, queued on the
+// context's stream.
+static int gather_all(AlbCtx* ctx, const Accum& acc, bool lo_zero) {
+    static const int kinds[4] = {kQueryBottom, kQueryScatter, kQuerySurface, kQuerySurface};
+    static const int chans[4] = {ALB_BOTTOM_REFLECTION, ALB_SCATTER, ALB_SURFACE_REFLECTION, ALB_SURFACE_TRANSMISSION_UP};
+    uint64_t total = 0;
+    for (int k = 0; k < 3; ++k) {
+        const uint64_t nq = ctx->h_q_count[k];
+        total += nq;
+        if (nq == 0 || !ctx->sort_q) continue;
+        PhaseTimer ps(ctx, 3);
+        const int rc = sort_queries(ctx->ws, ctx->qa[k], nq, ctx->qperm[k], ctx->st);
+        ps.stop();
+        if (rc != 0) return fail(ctx, ALB_ERR_CUDA, "query sort: device memory allocation failed");
+    }
+    // Few queries leave most of the chip idle in one gather: the planar ones run beside one another on
+    // streams forked here and joined below (the Jacobian and the heatmaps sum through words
+    // that the channels share, so those runs stay in series). A backward call on the
+    // 5 m water scene's maps of 1e5 photons: 1.2 -> 0.9 ms with 5000 photons, 2.0 -> 1.6 ms with 25,000.
+    const bool fork = total < (1ull << 20) && !acc.jac_lo && !acc.hw_lo;
+    if (fork) {
+        if (!ctx->fork) {
+            CK(cudaEventCreateWithFlags(&ctx->fork, cudaEventDisableTiming));
+            for (int i = 0; i < 3; ++i) {
+                CK(cudaEventCreateWithFlags(&ctx->join[i], cudaEventDisableTiming));
+                CK(cudaStreamCreateWithFlags(&ctx->side[i], cudaStreamNonBlocking));
+            }
+        }
+        CK(cudaEventRecord(ctx->fork, ctx->st));
+    }
+    int side = 0, rc = ALB_OK;
+    static const int sequence[4] = {0, 2, 3, 1};  // the scatter gather's CTAs fill whole SMs: last
+    for (int s = 0; s < 4; ++s) {
+        const int g = sequence[s], k = kinds[g], c = chans[g];
+        const uint64_t nq = ctx->h_q_count[k];
+        if (nq == 0) continue;
+        QueryDev q{};
+        q.a = ctx->qa[k];
+        q.b = ctx->qb[k];
+        q.c = ctx->qc[k];
+        q.lo_zero = lo_zero;
+        q.s = ctx->sc.adjoint ? ctx->qs[k] : nullptr;
+        q.perm = ctx->sort_q ? ctx->qperm[k] : nullptr;
+        q.n = nq;
+        q.rk_out = ctx->keep_ids ? ctx->qrk[k][g == 3 ? 1 : 0] : nullptr;
+        q.stats = ctx->d_stats + 4 + 4 * c;  // per channel: leaves, nodes, selects, queries
+        q.inexact = ctx->d_stats + 24 + c;
+        q.retries = ctx->d_stats + 30;
+        q.ticket = (uint32_t*)(ctx->ctl + 40);
+        const bool aside = fork && c != ALB_SCATTER;
+        cudaStream_t st = ctx->st;
+        if (aside) {
+            st = ctx->side[side];
+            CK(cudaStreamWaitEvent(st, ctx->fork, 0));
+        }
+        PhaseTimer pg(ctx, 4 + c, st);
+        launch_gather(ctx->sc, map_dev(ctx->map[c]), q, c, acc, ctx->d_err, &ctx->launches, st);
+        pg.stop(st);
+        if (aside) {
+            const cudaError_t e = cudaEventRecord(ctx->join[side], st);
+            if (e != cudaSuccess) rc = fail(ctx, ALB_ERR_CUDA, cudaGetErrorString(e));
+            ++side;
+        }
+        ctx->gathered[c] += (int64_t)nq;
+    }
+    for (int i = 0; i < side; ++i) CK(cudaStreamWaitEvent(ctx->st, ctx->join[i], 0));
+    return rc;
+}
+
 extern "C" int alb_trace(AlbCtx* ctx, int pass, uint64_t n, uint64_t seed, uint64_t first, const AlbReplay* rp) {
     if (!ctx) return ALB_ERR_INVALID;
     if (pass != ALB_FORWARD && pass != ALB_BACKWARD) return fail(ctx, ALB_ERR_INVALID, "pass must be 0 or 1");
@@ -770,10 +978,12 @@ extern "C" int alb_trace(AlbCtx* ctx, int pass, uint64_t n, uint64_t seed, uint6
     }
     if (ctx->keep_exit) {
         if (ctx->ex_cap < n) {
-            cudaFree(ctx->ex_pos); cudaFree(ctx->ex_dir); cudaFree(ctx->ex_f);
-            CK(cudaMalloc(&ctx->ex_pos, n * 24));
-            CK(cudaMalloc(&ctx->ex_dir, n * 24));
-            CK(cudaMalloc(&ctx->ex_f, n * 40));
+            drop(ctx->ex_pos, ctx->st); drop(ctx->ex_dir, ctx->st); drop(ctx->ex_f, ctx->st);
+            ctx->ex_cap = 0;
+            if (!take(ctx->ex_pos, n * 24, ctx->st) || !take(ctx->ex_dir, n * 24, ctx->st) || !take(ctx->ex_f, n * 40, ctx->st)) {
+                ctx->ws.release(mark);
+                return fail(ctx, ALB_ERR_CUDA, "exit states: out of device memory");
+            }
             ctx->ex_cap = n;
         }
         ctx->ex_n = n;
@@ -781,54 +991,58 @@ extern "C" int alb_trace(AlbCtx* ctx, int pass, uint64_t n, uint64_t seed, uint6
     // slots 28/29 keep the last forward trace's events and photons across the backward trace
     CK(cudaMemsetAsync(ctx->d_stats, 0, 28 * 8, ctx->st));
     CK(cudaMemsetAsync(ctx->d_stats + 30, 0, 8, ctx->st));
+    unsigned long long* const stats_bak = ctx->ctl + 41;
     if (pass == ALB_FORWARD) {
         ctx->maps_built = false;
-        uint64_t before[ALB_CHANNELS];
-        std::memcpy(before, ctx->h_rec_count, sizeof before);
-        std::vector<unsigned> radius_backup;
-        size_t hb = ctx->sc.heatmap ? (size_t)ctx->sc.hm_bins * ctx->sc.hm_bins : 0;
-        for (int attempt = 0; attempt < 3; ++attempt) {
-            for (int c = 0; c < ALB_CHANNELS; ++c) {
-                uint64_t est = (uint64_t)(ctx->rec_rate[c] * (double)n * 1.03) + 4096;
-                if (ctx->map_cap_hint > 0) est = std::max<uint64_t>(est, (uint64_t)ctx->map_cap_hint);
-                int rc = ctx->rec_released[c] ? restore_records(ctx, c, before[c] + est)
-                                               : ensure_records(ctx, c, before[c] + est, before[c]);
-                if (rc) return rc;
-            }
-            if (hb && attempt == 0) {
-                radius_backup.resize(hb);
-                CK(cudaMemcpyAsync(radius_backup.data(), ctx->hm_radius, hb * 4, cudaMemcpyDeviceToHost, ctx->st));
-            }
-            TraceOut o = make_out(ctx);
-            PhaseTimer pt(ctx, 0);
-            launch_trace(ctx->sc, o, ALB_FORWARD, n, first, seed, rp ? &drp : nullptr, &ctx->launches, ctx->st,
-                         ctx->precise ? nullptr : &ctx->fast);
-            pt.stop();
-            int rc = check_device(ctx, "forward trace");
-            if (rc) return rc;
-            unsigned long long cnt[ALB_CHANNELS];
-            CK(cudaMemcpyAsync(cnt, ctx->d_rec_count, sizeof cnt, cudaMemcpyDeviceToHost, ctx->st));
-            CK(cudaStreamSynchronize(ctx->st));
-            bool overflow = false;
-            for (int c = 0; c < ALB_CHANNELS; ++c) {
-                uint64_t added = cnt[c] - before[c];
-                if (n > 0) ctx->rec_rate[c] = std::max(ctx->rec_rate[c] * 0.5, (double)added / (double)n);
-                if (cnt[c] > ctx->rec[c].cap) overflow = true;
-            }
-            if (!overflow) {
-                for (int c = 0; c < ALB_CHANNELS; ++c) ctx->h_rec_count[c] = cnt[c];
+        const size_t hb = ctx->sc.heatmap ? (size_t)ctx->sc.hm_bins * ctx->sc.hm_bins : 0;
+        // photons [p0, p0 + pn) of the call
+        auto part = [&](uint64_t p0, uint64_t pn) -> int {
+            uint64_t before[ALB_CHANNELS];
+            std::memcpy(before, ctx->h_rec_count, sizeof before);
+            CK(cudaMemcpyAsync(stats_bak, ctx->d_stats, 2 * 8, cudaMemcpyDeviceToDevice, ctx->st));
+            if (hb) CK(cudaMemcpyAsync(ctx->hm_radius_bak, ctx->hm_radius, hb * 4, cudaMemcpyDeviceToDevice, ctx->st));
+            for (int attempt = 0; attempt < 3; ++attempt) {
+                for (int c = 0; c < ALB_CHANNELS; ++c) {
+                    uint64_t est = (uint64_t)(ctx->rec_rate[c] * (double)pn * 1.03) + 4096;
+                    if (ctx->map_cap_hint > 0) est = std::max<uint64_t>(est, (uint64_t)ctx->map_cap_hint);
+                    int rc = ctx->rec_released[c] ? restore_records(ctx, c, before[c] + est)
+                                                   : ensure_records(ctx, c, before[c] + est, before[c]);
+                    if (rc) return rc;
+                }
+                TraceOut o = make_out(ctx);
+                PhaseTimer pt(ctx, 0);
+                launch_trace(ctx->sc, o, ALB_FORWARD, pn, first + p0, seed, rp ? &drp : nullptr, &ctx->launches, ctx->st,
+                             ctx->precise ? nullptr : &ctx->fast);
+                pt.stop();
                 CK(cudaMemcpyAsync(ctx->d_stats + 28, ctx->d_stats, 2 * 8, cudaMemcpyDeviceToDevice, ctx->st));
-                ctx->ws.release(mark);
-                return ALB_OK;
+                unsigned long long cnt[7];
+                int rc = check_device(ctx, "forward trace", cnt);
+                if (rc) return rc;
+                bool overflow = false;
+                for (int c = 0; c < ALB_CHANNELS; ++c) {
+                    uint64_t added = cnt[c] - before[c];
+                    if (pn > 0) ctx->rec_rate[c] = std::max(ctx->rec_rate[c] * 0.5, (double)added / (double)pn);
+                    if (cnt[c] > ctx->rec[c].cap) overflow = true;
+                }
+                if (!overflow) {
+                    for (int c = 0; c < ALB_CHANNELS; ++c) ctx->h_rec_count[c] = cnt[c];
+                    if (pn > 0) ctx->rec_rate_known = true;
+                    return ALB_OK;
+                }
+                // undo and retry with the measured sizes
+                CK(cudaMemcpyAsync(ctx->d_stats, stats_bak, 2 * 8, cudaMemcpyDeviceToDevice, ctx->st));
+                CK(cudaMemcpyAsync(ctx->d_rec_count, before, sizeof before, cudaMemcpyHostToDevice, ctx->st));
+                if (hb) CK(cudaMemcpyAsync(ctx->hm_radius, ctx->hm_radius_bak, hb * 4, cudaMemcpyDeviceToDevice, ctx->st));
+                CK(cudaStreamSynchronize(ctx->st));
+                for (int c = 0; c < ALB_CHANNELS; ++c) ctx->rec_rate[c] = (double)(cnt[c] - before[c]) / (double)pn;
             }
-            // undo and retry with the measured sizes
-            CK(cudaMemsetAsync(ctx->d_stats, 0, 2 * 8, ctx->st));
-            CK(cudaMemcpyAsync(ctx->d_rec_count, before, sizeof before, cudaMemcpyHostToDevice, ctx->st));
-            if (hb) CK(cudaMemcpyAsync(ctx->hm_radius, radius_backup.data(), hb * 4, cudaMemcpyHostToDevice, ctx->st));
-            CK(cudaStreamSynchronize(ctx->st));
-            for (int c = 0; c < ALB_CHANNELS; ++c) ctx->rec_rate[c] = (double)(cnt[c] - before[c]) / (double)n;
-        }
-        return fail(ctx, ALB_ERR_CAPACITY, "photon-map capacity could not be established");
+            return fail(ctx, ALB_ERR_CAPACITY, "photon-map capacity could not be established");
+        };
+        const uint64_t pilot = !ctx->rec_rate_known && n > 4 * kPilot && !rp && !ctx->keep_exit ? kPilot : 0;
+        int rc = pilot ? part(0, pilot) : ALB_OK;
+        if (!rc) rc = part(pilot, n - pilot);
+        ctx->ws.release(mark);
+        return rc;
     }
     // backward: trace -> queries -> gathers. Without per-photon exports the photons go in
     // chunks, so that query buffers stay bounded whatever n is (the waveform sums are
@@ -853,69 +1067,59 @@ extern "C" int alb_trace(AlbCtx* ctx, int pass, uint64_t n, uint64_t seed, uint6
     }
     const bool chunked = !ctx->keep_exit && !ctx->keep_ids && !rp;
     const uint64_t chunk = chunked ? kBackwardChunk : std::max<uint64_t>(n, 1);
+    // traces photons [c0, c0 + nc) into the query buffers, which may turn out too small
+    auto trace = [&](uint64_t c0, uint64_t nc, bool& overflow) -> int {
+        for (int k = 0; k < 3; ++k) {
+            uint64_t est = (uint64_t)(ctx->q_rate[k] * (double)nc * 1.1) + 4096;
+            int rc = ensure_queries(ctx, k, est);
+            if (rc) return rc;
+        }
+        CK(cudaMemsetAsync(ctx->d_q_count, 0, 3 * 8, ctx->st));
+        CK(cudaMemcpyAsync(stats_bak, ctx->d_stats, 2 * 8, cudaMemcpyDeviceToDevice, ctx->st));
+        TraceOut o = make_out(ctx);
+        PhaseTimer pt(ctx, 2);
+        launch_trace(ctx->sc, o, ALB_BACKWARD, nc, first + c0, seed, rp ? &drp : nullptr, &ctx->launches, ctx->st,
+                     ctx->precise ? nullptr : &ctx->fast);
+        pt.stop();
+        unsigned long long cnt[7];
+        int rc = check_device(ctx, "backward trace", cnt);
+        if (rc) return rc;
+        overflow = false;
+        for (int k = 0; k < 3; ++k) {
+            ctx->h_q_count[k] = cnt[4 + k];
+            if (nc > 0) ctx->q_rate[k] = std::max(ctx->q_rate[k] * 0.5, (double)cnt[4 + k] / (double)nc);
+            if (cnt[4 + k] > ctx->qcap[k]) overflow = true;
+        }
+        if (overflow)
+            for (int k = 0; k < 3; ++k) ctx->q_rate[k] = (double)cnt[4 + k] / (double)nc;
+        ctx->q_rate_known = ctx->q_rate_known || nc > 0;
+        return ALB_OK;
+    };
+    auto untrace = [&]() -> int {  // the counters as before the trace
+        CK(cudaMemcpyAsync(ctx->d_stats, stats_bak, 2 * 8, cudaMemcpyDeviceToDevice, ctx->st));
+        return ALB_OK;
+    };
     for (uint64_t c0 = 0; c0 == 0 || c0 < n; c0 += chunk) {
         const uint64_t nc = std::min<uint64_t>(chunk, n - c0);
-        for (int attempt = 0; attempt < 3; ++attempt) {
-            for (int k = 0; k < 3; ++k) {
-                uint64_t est = (uint64_t)(ctx->q_rate[k] * (double)nc * 1.1) + 4096;
-                int rc = ensure_queries(ctx, k, est);
-                if (rc) return rc;
-            }
-            CK(cudaMemsetAsync(ctx->d_q_count, 0, 3 * 8, ctx->st));
-            TraceOut o = make_out(ctx);
-            PhaseTimer pt(ctx, 2);
-            launch_trace(ctx->sc, o, ALB_BACKWARD, nc, first + c0, seed, rp ? &drp : nullptr, &ctx->launches,
-                         ctx->st, ctx->precise ? nullptr : &ctx->fast);
-            pt.stop();
-            int rc = check_device(ctx, "backward trace");
+        bool overflow = false;
+        int rc = ALB_OK;
+        if (!ctx->q_rate_known && nc > 4 * kPilot && chunked) {
+            rc = trace(c0, kPilot, overflow);
+            if (!rc) rc = untrace();
             if (rc) return rc;
-            unsigned long long cnt[3];
-            CK(cudaMemcpyAsync(cnt, ctx->d_q_count, sizeof cnt, cudaMemcpyDeviceToHost, ctx->st));
-            CK(cudaStreamSynchronize(ctx->st));
-            bool overflow = false;
-            for (int k = 0; k < 3; ++k) {
-                if (nc > 0) ctx->q_rate[k] = std::max(ctx->q_rate[k] * 0.5, (double)cnt[k] / (double)nc);
-                if (cnt[k] > ctx->qcap[k]) overflow = true;
-                ctx->h_q_count[k] = cnt[k];
-            }
+        }
+        for (int attempt = 0; attempt < 3; ++attempt) {
+            rc = trace(c0, nc, overflow);
+            if (rc) return rc;
             if (!overflow) break;
-            for (int k = 0; k < 3; ++k) ctx->q_rate[k] = (double)cnt[k] / (double)nc;
+            rc = untrace();
+            if (rc) return rc;
             if (attempt == 2) return fail(ctx, ALB_ERR_CAPACITY, "query capacity could not be established");
         }
-        int rc = ctx->sc.radius > 0.0 ? ALB_OK : check_map_sizes(ctx);  // k-NN needs k records
+        rc = ctx->sc.radius > 0.0 ? ALB_OK : check_map_sizes(ctx);  // k-NN needs k records
         if (rc) return rc;
-        static const int kinds[4] = {kQueryBottom, kQueryScatter, kQuerySurface, kQuerySurface};
-        static const int chans[4] = {ALB_BOTTOM_REFLECTION, ALB_SCATTER, ALB_SURFACE_REFLECTION,
-                                     ALB_SURFACE_TRANSMISSION_UP};
-        for (int g = 0; g < 4; ++g) {
-            int k = kinds[g], c = chans[g];
-            uint64_t nq = ctx->h_q_count[k];
-            if (nq == 0) continue;
-            QueryDev q{};
-            q.a = ctx->qa[k];
-            q.b = ctx->qb[k];
-            q.c = ctx->qc[k];
-            q.lo_zero = !ctx->precise && !rp;
-            q.s = ctx->sc.adjoint ? ctx->qs[k] : nullptr;
-            q.n = nq;
-            q.rk_out = ctx->keep_ids ? ctx->qrk[k][g == 3 ? 1 : 0] : nullptr;
-            q.stats = ctx->d_stats + 4 + 4 * c;  // per channel: leaves, nodes, selects, queries
-            q.inexact = ctx->d_stats + 24 + c;
-            q.retries = ctx->d_stats + 30;
-            q.ticket = (uint32_t*)(ctx->d_stats + 32);
-            if (ctx->sort_q) {
-                PhaseTimer ps(ctx, 3);
-                const int src = sort_queries(ctx->ws, ctx->qa[k], nq, ctx->qperm[k], ctx->st);
-                ps.stop();
-                if (src != 0) return fail(ctx, ALB_ERR_CUDA, "query sort: device memory allocation failed");
-                q.perm = ctx->qperm[k];
-            }
-            PhaseTimer pg(ctx, 4 + c);
-            launch_gather(ctx->sc, map_dev(ctx->map[c]), q, c, acc, ctx->d_err, &ctx->launches, ctx->st);
-            pg.stop();
-            ctx->gathered[c] += (int64_t)nq;
-        }
-        rc = check_device(ctx, "gather");
+        rc = gather_all(ctx, acc, !ctx->precise && !rp);
+        if (!rc) rc = check_device(ctx, "gather");
         if (rc) return rc;
         if (n == 0) break;
     }
@@ -927,13 +1131,30 @@ extern "C" int alb_build_maps(AlbCtx* ctx) {
     if (!ctx) return ALB_ERR_INVALID;
     CK(cudaSetDevice(ctx->device));
     PhaseTimer pt(ctx, 1);
+    static const char* const failed = "photon-map index build failed (device memory or partition)";
+    // every channel's build is queued before the first is waited for
+    RecordStore rec[ALB_CHANNELS];
+    bool todo[ALB_CHANNELS];
     for (int c = 0; c < ALB_CHANNELS; ++c) {
-        if (ctx->rec_released[c]) continue;  // already indexed, nothing appended since
-        RecordStore r = ctx->rec[c];
-        if (!ctx->sc.adjoint) r.sco = nullptr;  // a store kept from an adjoint run: no scores now
-        if (build_map_index(ctx->ws, r, ctx->h_rec_count[c], ctx->map[c], ctx->st) != 0)
-            return fail(ctx, ALB_ERR_CAPACITY, "photon-map index build failed (device memory or partition)");
-        CK(cudaStreamSynchronize(ctx->st));
+        todo[c] = !ctx->rec_released[c];  // else indexed already, nothing appended since
+        if (!todo[c]) continue;
+        rec[c] = ctx->rec[c];
+        if (!ctx->sc.adjoint) rec[c].sco = nullptr;  // a store kept from an adjoint run: no scores now
+        if (start_map_index(ctx->ws, rec[c], ctx->h_rec_count[c], ctx->map[c], c, ctx->st) != 0)
+            return fail(ctx, ALB_ERR_CAPACITY, failed);
+        // a large store is released before the next channel's index is allocated
+        if (ctx->h_rec_count[c] > (1ull << 26)) {
+            if (finish_map_index(ctx->ws, rec[c], ctx->map[c], c, ctx->st) != 0) return fail(ctx, ALB_ERR_CAPACITY, failed);
+            todo[c] = false;
+            if (!ctx->keep_records) {
+                release_records(ctx, c);
+                ctx->rec_released[c] = true;
+            }
+        }
+    }
+    for (int c = 0; c < ALB_CHANNELS; ++c) {
+        if (!todo[c]) continue;
+        if (finish_map_index(ctx->ws, rec[c], ctx->map[c], c, ctx->st) != 0) return fail(ctx, ALB_ERR_CAPACITY, failed);
         if (ctx->keep_records) continue;  // the store stays for the next simulation
         release_records(ctx, c);
         ctx->rec_released[c] = true;
@@ -1024,36 +1245,36 @@ extern "C" int alb_get_heatmaps(AlbCtx* ctx, double* water, double* seafloor, fl
     return ALB_OK;
 }
 
-static int read_wf(AlbCtx* ctx, int c, std::vector<double>& out) {
-    int64_t nb = ctx->sc.nbins;
-    std::vector<unsigned long long> lo(nb), hi(nb);
-    CK(cudaMemcpyAsync(lo.data(), ctx->wf + (size_t)c * nb, nb * 8, cudaMemcpyDeviceToHost, ctx->st));
-    CK(cudaMemcpyAsync(hi.data(), ctx->wf + (size_t)ALB_CHANNELS * nb + (size_t)c * nb, nb * 8, cudaMemcpyDeviceToHost,
-                       ctx->st));
+// n 128-bit words of an accumulator to the host as float64 or float32, converted on the device.
+template <class T>
+static int read_fixed(AlbCtx* ctx, const unsigned long long* lo, const unsigned long long* hi, int64_t n, T* out) {
+    const size_t mark = ctx->ws.mark();
+    T* d = (T*)ctx->ws.take_bytes((size_t)n * sizeof(T));
+    if (!d) return fail(ctx, ALB_ERR_CUDA, "read-back buffer: out of device memory");
+    launch_fix_to_float(lo, hi, n, d, ctx->st);
+    const cudaError_t e = cudaMemcpyAsync(out, d, (size_t)n * sizeof(T), cudaMemcpyDeviceToHost, ctx->st);
+    ctx->ws.release(mark);
+    CK(e);
     CK(cudaStreamSynchronize(ctx->st));
-    out.resize(nb);
-    for (int64_t i = 0; i < nb; ++i) out[i] = fix_to_double(lo[i], (long long)hi[i]);
     return ALB_OK;
+}
+
+template <class T>
+static int read_wf(AlbCtx* ctx, int c, T* out) {
+    const int64_t nb = ctx->sc.nbins;
+    return read_fixed(ctx, ctx->wf + (size_t)c * nb, ctx->wf + (size_t)(ALB_CHANNELS + c) * nb, nb, out);
 }
 
 extern "C" int alb_get_waveform(AlbCtx* ctx, int c, float* out, size_t nbins) {
     if (!ctx || !out || c < 0 || c >= ALB_CHANNELS) return ALB_ERR_INVALID;
     if (nbins < (size_t)ctx->sc.nbins) return fail(ctx, ALB_ERR_INVALID, "waveform buffer too small");
-    std::vector<double> w;
-    int rc = read_wf(ctx, c, w);
-    if (rc) return rc;
-    for (size_t i = 0; i < w.size(); ++i) out[i] = (float)w[i];
-    return ALB_OK;
+    return read_wf(ctx, c, out);
 }
 
 extern "C" int alb_get_waveform_f64(AlbCtx* ctx, int c, double* out, size_t nbins) {
     if (!ctx || !out || c < 0 || c >= ALB_CHANNELS) return ALB_ERR_INVALID;
     if (nbins < (size_t)ctx->sc.nbins) return fail(ctx, ALB_ERR_INVALID, "waveform buffer too small");
-    std::vector<double> w;
-    int rc = read_wf(ctx, c, w);
-    if (rc) return rc;
-    std::memcpy(out, w.data(), w.size() * 8);
-    return ALB_OK;
+    return read_wf(ctx, c, out);
 }
 
 extern "C" int alb_get_jacobian(AlbCtx* ctx, int param, int c, double* out, size_t nbins) {
@@ -1066,12 +1287,7 @@ extern "C" int alb_get_jacobian(AlbCtx* ctx, int param, int c, double* out, size
     if (nbins < (size_t)nb) return fail(ctx, ALB_ERR_INVALID, "jacobian buffer too small");
     const size_t off = ((size_t)(param - 1) * ALB_CHANNELS + c) * nb;
     const size_t half = (size_t)kJacParams * ALB_CHANNELS * nb;
-    std::vector<unsigned long long> lo(nb), hi(nb);
-    CK(cudaMemcpyAsync(lo.data(), ctx->jac + off, nb * 8, cudaMemcpyDeviceToHost, ctx->st));
-    CK(cudaMemcpyAsync(hi.data(), ctx->jac + half + off, nb * 8, cudaMemcpyDeviceToHost, ctx->st));
-    CK(cudaStreamSynchronize(ctx->st));
-    for (int64_t i = 0; i < nb; ++i) out[i] = fix_to_double(lo[i], (long long)hi[i]);
-    return ALB_OK;
+    return read_fixed(ctx, ctx->jac + off, ctx->jac + half + off, nb, out);
 }
 
 extern "C" int alb_adjoint(AlbCtx* ctx, const double* dL_dw, size_t nbins, double* grad) {
@@ -1124,7 +1340,7 @@ extern "C" int alb_reset(AlbCtx* ctx) {
     CK(cudaStreamSynchronize(ctx->st));
     for (int c = 0; c < ALB_CHANNELS; ++c) {
         ctx->h_rec_count[c] = 0;
-        release_map_index(ctx->map[c]);  // an empty simulation holds no index memory
+        release_map_index(ctx->map[c], ctx->st);  // an empty simulation holds no index memory
         ctx->map[c].n = 0;
         ctx->map[c].n_real = 0;
         ctx->rec_released[c] = false;
@@ -1214,7 +1430,9 @@ extern "C" int alb_knn(AlbCtx* ctx, const float* pts, uint64_t m, const double* 
     double* dd = (double*)ctx->ws.take_bytes(nq * k * 8);
     MapIndex mi;
     auto done = [&](int rc) {
-        cudaFree(mi.a); cudaFree(mi.b); cudaFree(mi.box_lo); cudaFree(mi.box_hi);
+        release_map_index(mi, ctx->st);
+        dev_free(mi.box_lo, ctx->st);
+        dev_free(mi.box_hi, ctx->st);
         ctx->ws.release(mark);
         return rc;
     };
@@ -1224,7 +1442,7 @@ extern "C" int alb_knn(AlbCtx* ctx, const float* pts, uint64_t m, const double* 
         !ok(cudaMemcpyAsync(dq, qs, nq * 24, cudaMemcpyHostToDevice, ctx->st)))
         return done(fail(ctx, ALB_ERR_CUDA, "knn upload failed"));
     pack_knn_points(dp, m, r.a, ctx->st);
-    if (build_map_index(ctx->ws, r, m, mi, ctx->st) != 0)
+    if (start_map_index(ctx->ws, r, m, mi, 0, ctx->st) != 0 || finish_map_index(ctx->ws, r, mi, 0, ctx->st) != 0)
         return done(fail(ctx, ALB_ERR_CAPACITY, "knn index build failed"));
     if (nq) pack_knn_queries(dq, nq, qa, ctx->st);
     if (sort_queries(ctx->ws, qa, nq, perm, ctx->st) != 0) return done(fail(ctx, ALB_ERR_CUDA, "knn query sort failed"));
@@ -1301,11 +1519,8 @@ static int run_instance(AlbCtx* ctx, AlbBatchInstance& I, int adjoint) {
     if (!rc) rc = alb_trace(ctx, ALB_BACKWARD, I.n_backward, I.seed, 0, nullptr);
     if (rc) return rc;
     const int64_t nb = ctx->sc.nbins;
-    std::vector<double> w;
-    for (int c = 0; c < ALB_CHANNELS && !rc; ++c) {
-        rc = read_wf(ctx, c, w);
-        if (!rc && I.waveform) std::memcpy(I.waveform + (size_t)c * nb, w.data(), nb * 8);
-    }
+    for (int c = 0; c < ALB_CHANNELS && !rc; ++c)
+        if (I.waveform) rc = read_wf(ctx, c, I.waveform + (size_t)c * nb);
     if (!rc && adjoint && I.jacobian)
         for (int p = 1; p < ALB_ADJ_PARAMS && !rc; ++p)
             for (int c = 0; c < ALB_CHANNELS && !rc; ++c)
@@ -1348,7 +1563,7 @@ extern "C" int alb_batch_run(AlbBatchInstance* inst, uint64_t n, const AlbBatchO
     cudaSetDevice(opt->device);
     size_t free_b = 0, total_b = 0;
     cudaMemGetInfo(&free_b, &total_b);
-    const double budget = 0.8 * (double)free_b;
+    const double budget = 0.8 * ((double)free_b + (double)pool_idle());
     const double bytes_per_record = opt->adjoint ? 162.0 : 130.0;
     std::mutex mem_mu;
     std::condition_variable mem_cv;
@@ -1413,12 +1628,11 @@ extern "C" int alb_batch_run(AlbBatchInstance* inst, uint64_t n, const AlbBatchO
                 }
             }
             if (!ctx) {
-                rc = alb_create(I.scene, opt->device, &ctx);
+                rc = create_on(I.scene, opt->device, st, &ctx);
                 if (rc) {
                     msg = g_create_error;
                     ctx = nullptr;
                 } else {
-                    alb_set_option(ctx, ALB_OPT_STREAM, (int64_t)(intptr_t)st);
                     alb_set_option(ctx, ALB_OPT_PRECISE, opt->precise ? 1 : 0);
                     ctx->keep_records = true;
                     if (opt->adjoint) rc = alb_set_option(ctx, ALB_OPT_ADJOINT, 1);

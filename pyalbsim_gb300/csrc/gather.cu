@@ -1767,4 +1767,20 @@ void launch_knn_brute(const float* pts, uint32_t m, const double* queries, uint6
     note_launch();
 }
 
+// 128-bit fixed-point words as floating point numbers (fix_to_double).
+template <class T>
+__global__ void k_fix_to_float(const unsigned long long* __restrict__ lo, const unsigned long long* __restrict__ hi, int64_t n,
+                               T* out) {
+    const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    if (i < n) out[i] = (T)fix_to_double(lo[i], (long long)hi[i]);
+}
+void launch_fix_to_float(const unsigned long long* lo, const unsigned long long* hi, int64_t n, float* out, cudaStream_t st) {
+    k_fix_to_float<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(lo, hi, n, out);
+    note_launch();
+}
+void launch_fix_to_float(const unsigned long long* lo, const unsigned long long* hi, int64_t n, double* out, cudaStream_t st) {
+    k_fix_to_float<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(lo, hi, n, out);
+    note_launch();
+}
+
 }  // namespace alb

@@ -104,8 +104,11 @@ struct Accum {
     unsigned long long* jac_hi;
 };
 
-// Stream-ordered device memory: temporaries come from cudaMallocAsync and are released in
-// stack order; persistent buffers grow on demand.
+// Stream-ordered device memory from the device's pool (albgpu.cu).
+void* dev_alloc(uint64_t bytes, cudaStream_t st);
+void dev_free(void* p, cudaStream_t st);
+
+// Temporaries are released in stack order; persistent buffers grow on demand.
 class Workspace {
   public:
     explicit Workspace(cudaStream_t st = 0) : st_(st) {}
@@ -129,8 +132,11 @@ class Workspace {
 };
 
 // ---- map build (mapbuild.cu)
-int build_map_index(Workspace& ws, const RecordStore& rec, uint64_t n, MapIndex& m, cudaStream_t st);
-void release_map_index(MapIndex& m);
+// Queues the build of one channel's index; finish waits for it and, where the records' keys turn out
+// crowded, rebuilds. slot (0..3): the build's words in the workspace's scratch.
+int start_map_index(Workspace& ws, const RecordStore& rec, uint64_t n, MapIndex& m, int slot, cudaStream_t st);
+int finish_map_index(Workspace& ws, const RecordStore& rec, MapIndex& m, int slot, cudaStream_t st);
+void release_map_index(MapIndex& m, cudaStream_t st);
 int sort_queries(Workspace& ws, const float4* qa, uint64_t n, uint32_t* perm, cudaStream_t st);
 
 // ---- tracer (tracer.cu)
@@ -146,6 +152,8 @@ void launch_profile_logs(const SceneDev& sc, double* out, cudaStream_t st);
 // ---- gather (gather.cu)
 void launch_gather(const SceneDev& sc, const MapDev& map, const QueryDev& q, int channel, const Accum& acc,
                    int* err, int* launches, cudaStream_t st);
+void launch_fix_to_float(const unsigned long long* lo, const unsigned long long* hi, int64_t n, float* out, cudaStream_t st);
+void launch_fix_to_float(const unsigned long long* lo, const unsigned long long* hi, int64_t n, double* out, cudaStream_t st);
 void launch_knn(const MapDev& map, const double* queries, const uint32_t* perm, uint64_t nq, int k, int32_t* out_idx,
                 double* out_dist, int* err, cudaStream_t st);
 void launch_knn_brute(const float* pts, uint32_t m, const double* queries, uint64_t nq, int k, int32_t* out_idx,

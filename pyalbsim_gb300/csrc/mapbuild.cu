@@ -1730,11 +1730,12 @@ static void parent_boxes(MapIndex& m, cudaStream_t st) {
     }
 }
 
-// Bounding box of a[0], a[stride], ... into the workspace's scratch words (ordered ints,
+// Bounding box of a[0], a[stride], ... into the workspace's scratch words from `word` on (ordered ints,
 // min then max), left on the device; nullptr when the scratch could not be allocated.
-static unsigned* bbox_device(Workspace& ws, const float4* a, uint64_t n, cudaStream_t st, uint64_t stride) {
+static unsigned* bbox_device(Workspace& ws, const float4* a, uint64_t n, cudaStream_t st, uint64_t stride, int word = 0) {
     unsigned* box = ws.scratch_box();
     if (!box) return nullptr;
+    box += word;
     cudaMemsetAsync(box, 0xff, 12, st);
     cudaMemsetAsync(box + 3, 0, 12, st);
     int dev = 0, sms = 148;
@@ -1764,8 +1765,8 @@ __global__ void k_finalize(float4* a, float4* __restrict__ b, float4* __restrict
     }
 }
 
-void release_map_index(MapIndex& m) {
-    cudaFree(m.a); cudaFree(m.b); cudaFree(m.fwi); cudaFree(m.sfi); cudaFree(m.id); cudaFree(m.sco);
+void release_map_index(MapIndex& m, cudaStream_t st) {
+    for (void* p : {(void*)m.a, (void*)m.b, (void*)m.fwi, (void*)m.sfi, (void*)m.id, (void*)m.sco}) dev_free(p, st);
     m.a = m.b = m.fwi = m.sfi = m.sco = nullptr;
     m.id = nullptr;
     m.a_cap = m.b_cap = m.fwi_cap = m.sfi_cap = m.id_cap = m.sco_cap = 0;
@@ -1985,7 +1986,9 @@ __global__ void k_crowded(const K* __restrict__ keys, uint64_t n, unsigned* coun
 // 256 others (a box far larger than what its records fill), into exact left-balanced k-d order; and
 // the box tree over leaves of 32. The index's own position array holds the sort's scratch, so the
 // peak is the record store, the index and four bytes per record.
-int build_map_index(Workspace& ws, const RecordStore& rec, uint64_t n, MapIndex& m, cudaStream_t st) {
+static int build_word(int slot) { return 16 + 8 * slot; }  // box in six words, crowded runs in the next
+
+int start_map_index(Workspace& ws, const RecordStore& rec, uint64_t n, MapIndex& m, int slot, cudaStream_t st) {
     m.n = n;
     m.n_real = n;
     if (n == 0) {
@@ -1993,14 +1996,14 @@ int build_map_index(Workspace& ws, const RecordStore& rec, uint64_t n, MapIndex&
         return 0;
     }
     if (n >= (1ull << 32)) return -1;  // record ids are 32-bit
-    if (n + 64 > m.a_cap) release_map_index(m);  // else every array is reused in place
-    const unsigned* box = bbox_device(ws, rec.a, n, st, 2);
+    if (n + 64 > m.a_cap) release_map_index(m, st);  // else every array is reused in place
+    const unsigned* box = bbox_device(ws, rec.a, n, st, 2, build_word(slot));
     m.a = (float4*)ws.alloc_persistent(m.a, m.a_cap, n + 64);
     if (!box || !m.a) return -1;
     const size_t mark = ws.mark();
     uint32_t* order = ws.take_u32(n);
     uint32_t* other = ws.take_u32(n);
-    unsigned* crowded = ws.scratch_box() + 16;
+    unsigned* crowded = ws.scratch_box() + build_word(slot) + 6;
     cudaMemsetAsync(crowded, 0, 4, st);
     // two 16-byte aligned key buffers in the position array (n + 64 float4). Key bits: 24 tell 2^16 records
     // apart even where they fill a thousandth of their box, 32 do for 2^26 (the large scene at 1e6
@@ -2042,21 +2045,28 @@ int build_map_index(Workspace& ws, const RecordStore& rec, uint64_t n, MapIndex&
     k_hilbert_finish<<<(unsigned)((warps + kFinishWarps - 1) / kFinishWarps), kFinishWarps * 32, 0, st>>>(order, rec, n, out);
     note_launch();
     parent_boxes(m, st);
-    unsigned h[7];
-    cudaMemcpyAsync(h, crowded, 4, cudaMemcpyDeviceToHost, st);
-    cudaMemcpyAsync(h + 1, box, 24, cudaMemcpyDeviceToHost, st);
-    cudaStreamSynchronize(st);
     ws.release(mark);
-    if ((uint64_t)h[0] * kRun * 2 <= n) return 0;
+    return 0;
+}
+
+int finish_map_index(Workspace& ws, const RecordStore& rec, MapIndex& m, int slot, cudaStream_t st) {
+    const uint64_t n = m.n;
+    if (n == 0) return 0;
+    unsigned h[7];
+    if (cudaMemcpyAsync(h, ws.scratch_box() + build_word(slot), sizeof h, cudaMemcpyDeviceToHost, st) != cudaSuccess ||
+        cudaStreamSynchronize(st) != cudaSuccess)
+        return -1;
+    if ((uint64_t)h[6] * kRun * 2 <= n) return 0;
     float lo[3], hi[3];
     for (int k = 0; k < 3; ++k) {
-        lo[k] = ord2f(h[1 + k]);
-        hi[k] = ord2f(h[4 + k]);
+        lo[k] = ord2f(h[k]);
+        hi[k] = ord2f(h[3 + k]);
     }
     if (kd_order_fast(ws, rec.a, n, lo, hi, m.a, st) != 0) return -1;
     // one record per thread: the gathers are random, so many loads in flight matter
     const unsigned blocks = (unsigned)((n + 255) / 256);
-    k_finalize<<<blocks, 256, 0, st>>>(m.a, m.b, out.fwi, out.sfi, out.id, out.sco, rec, n);
+    k_finalize<<<blocks, 256, 0, st>>>(m.a, m.b, rec.fwi ? m.fwi : nullptr, rec.fwi ? m.sfi : nullptr,
+                                       rec.id ? m.id : nullptr, rec.sco ? m.sco : nullptr, rec, n);
     note_launch();
     k_leaf_boxes<<<(unsigned)((m.lvl_cnt[0] * 32 + 255) / 256), 256, 0, st>>>(m.a, n, m.box_lo, m.box_hi, m.lvl_cnt[0]);
     note_launch();
