@@ -204,7 +204,7 @@ struct AlbCtx {
     uint64_t rec_id_cap[ALB_CHANNELS] = {0};
     uint64_t fwi_cap[ALB_CHANNELS] = {0}, sfi_cap[ALB_CHANNELS] = {0}, b_cap[ALB_CHANNELS] = {0};
     // one control block: record counts [0, 4), query counts [4, 7), error word [7], counters [8, 40),
-    // the scatter gather's work counter [40], counters kept across a retried trace [41, 43)
+    // counters kept across a retried trace [41, 43), the gathers' work counters [43, 47)
     unsigned long long* ctl = nullptr;
     unsigned long long* d_rec_count = nullptr;
     uint64_t h_rec_count[ALB_CHANNELS] = {0};
@@ -610,7 +610,7 @@ static std::string ensure_accumulators(AlbCtx* ctx) {
         return true;
     };
     if (!regrow(ctx->wf, ctx->wf_bins, s.nbins, (size_t)2 * ALB_CHANNELS) ||
-        !regrow(ctx->cls, ctx->cls_bins, s.nbins, 16))
+        !regrow(ctx->cls, ctx->cls_bins, s.nbins, (size_t)16 * ALB_CHANNELS))
         return "waveform allocation failed";
     if (s.adjoint && (!regrow(ctx->jac, ctx->jac_bins, s.nbins, (size_t)2 * kJacParams * ALB_CHANNELS) ||
                       !regrow(ctx->jac_cls, ctx->jac_cls_bins, s.nbins, (size_t)16 * kJacParams)))
@@ -929,7 +929,7 @@ static int gather_all(AlbCtx* ctx, const Accum& acc, bool lo_zero) {
         q.stats = ctx->d_stats + 4 + 4 * c;  // per channel: leaves, nodes, selects, queries
         q.inexact = ctx->d_stats + 24 + c;
         q.retries = ctx->d_stats + 30;
-        q.ticket = (uint32_t*)(ctx->ctl + 40);
+        q.ticket = (uint32_t*)(ctx->ctl + 43 + c);
         const bool aside = fork && c != ALB_SCATTER;
         cudaStream_t st = ctx->st;
         if (aside) {

@@ -1,4 +1,4 @@
-// Grouped k-NN search of the scatter map (included by gather.cu).
+// Grouped k-NN search of the scatter map and of large planar gathers (included by gather.cu).
 //
 // A warp takes a run of consecutive sorted queries whose common box is small against their k-th
 // distance, walks the box tree once for all of them, and keeps the leaves it meets with their
@@ -21,15 +21,34 @@
 
 namespace alb {
 
-// Squared widening of the previous query's k-th distance: what a query first admits within
-// (kGroupGuess2), and what the run's leaf list covers (kGroupList2, the second attempt).
-constexpr float kGroupGuess2 = 1.21f;
-constexpr float kGroupList2 = 1.5625f;
 constexpr int kGroupLeaves = 128;  // capacity of the leaf list
 // Leaves a run is sized for (estimated from its box): longer runs share one walk among more
 // queries, but every query tests the whole list (large scene, 1e6 photons: 36 -> 31.7 ms, 48 ->
 // 29.2, 64 -> 27.9, 80 -> 27.6).
 constexpr float kGroupTarget = 80.f;
+
+// What depends on how records fill space. kGuess2, kList2: squared widening of the previous query's k-th
+// distance, what a query first admits within and what the run's leaf list covers (the second
+// attempt). side: edge of a leaf over the k-th distance, 32 records against k in the ball.
+// est: leaves that a ball of radius T around a box of the given extents meets, the ball as the
+// cube (square) of its volume. kGrow: count ~ (squared distance)^kGrow.
+struct VolumeRuns {
+    static constexpr float kGuess2 = 1.21f, kList2 = 1.5625f, kGrow = 1.5f;
+    static ALB_DEVICE float side(float k) { return cbrtf(134.04f / k); }
+    static ALB_DEVICE float est(float dx, float dy, float dz, float side, float T) {
+        const float w = side + 1.61f * T;
+        return (dx + w) * (dy + w) * (dz + w) / (side * side * side);
+    }
+};
+// A horizontal plane. (Guesses of 1.15 and 1.3 measured the same to 4%.)
+struct PlaneRuns {
+    static constexpr float kGuess2 = 1.21f, kList2 = 1.5625f, kGrow = 1.f;
+    static ALB_DEVICE float side(float k) { return sqrtf(100.53f / k); }
+    static ALB_DEVICE float est(float dx, float, float dz, float side, float T) {
+        const float w = side + 1.77f * T;
+        return (dx + w) * (dz + w) / (side * side);
+    }
+};
 constexpr int kGroupStack = 192;  // 31 open boxes per level below the root level's 32, 6 levels
 
 template <int CAP>
@@ -55,6 +74,7 @@ struct GroupSmem {
         };
     };
     unsigned long long st[5];
+    int alone, streak;  // queries still to be searched alone, and the next such stretch
     // scratch words of the boundary band, once the one-query search has left its stack
     ALB_DEVICE uint32_t& tmp(int i) {
         if (i < kGroupStack) return stk[i];
@@ -79,7 +99,7 @@ ALB_DEVICE float run_gap(float lo, float hi, float qlo, float qhi, float ql) {
 // Builds the run starting at the first of `avail` queries whose positions the lanes hold (lane i
 // the i-th; la = the largest low part of its coordinates). Every float operation of run_gap is
 // monotone in the query, so a listed leaf's lower bound is never above any covered query's own.
-template <class S>
+template <class G, class S>
 ALB_DEVICE bool build_run(const MapDev& m, S& s, int avail, float x, float y, float z, float la, float r2, float side,
                           QueryRun& run) {
     const int l = lane_id();
@@ -99,12 +119,9 @@ ALB_DEVICE bool build_run(const MapDev& m, S& s, int avail, float x, float y, fl
             la = fmaxf(la, lb);
         }
     }
-    run.T2 = r2 * kGroupList2;
-    // leaves that a ball of radius T around the run's box meets, for cubic leaves of edge side
-    // (the ball as the cube of its volume)
-    const float w = side + 1.61f * sqrtf(run.T2);
-    const float est = (x1 - x0 + w) * (y1 - y0 + w) * (z1 - z0 + w);
-    run.take = max(__popc(__ballot_sync(0xffffffffu, have && est <= kGroupTarget * side * side * side)), 1);
+    run.T2 = r2 * G::kList2;
+    const float est = G::est(x1 - x0, y1 - y0, z1 - z0, side, sqrtf(run.T2));
+    run.take = max(__popc(__ballot_sync(0xffffffffu, have && est <= kGroupTarget)), 1);
     uint32_t* stk = reinterpret_cast<uint32_t*>(s.cd);  // the candidates are free here
     static_assert(S::kCap >= kGroupStack, "the walk's stack lies in the candidate buffer");
     while (true) {
@@ -177,7 +194,7 @@ ALB_DEVICE int count_le(const float (&v)[R], float x) {
     for (int j = 0; j < R; ++j) c += v[j] <= x ? 1 : 0;
     return __reduce_add_sync(0xffffffffu, c);
 }
-template <int R>
+template <class G, int R>
 ALB_DEVICE bool find_cut(const float (&v)[R], int cnt, int k, float hi, float& x) {
     if (cnt == k) {
         x = hi;
@@ -185,7 +202,7 @@ ALB_DEVICE bool find_cut(const float (&v)[R], int cnt, int k, float hi, float& x
     }
     float a = 0.f, b = hi;  // count(a) < k (count(0) = k is the degenerate case below), count(b) > k
     int ca = 0, cb = cnt;
-    x = hi * __powf((float)k / (float)cnt, 2.f / 3.f);
+    x = hi * __powf((float)k / (float)cnt, 1.f / G::kGrow);
 #pragma unroll 1
     for (int it = 0; it < 20; ++it) {
         if (!(x > a && x < b)) x = 0.5f * (a + b);
@@ -208,7 +225,7 @@ ALB_DEVICE bool find_cut(const float (&v)[R], int cnt, int k, float hi, float& x
 // 1: s.ci / s.ce [0 .. k) hold the k nearest, kth their largest float32 distance, kid its map
 // position; 0: the threshold does not prove an answer; -1: a near tie at the k-th place (kth is
 // then a proven bound when > 0), or too many candidates at one distance.
-template <class S>
+template <class G, class S>
 ALB_DEVICE int run_search(const MapDev& m, S& s, int k, int nlist, float fx, float fy, float fz, float lx, float ly,
                           float lz, float thr, float& kth, uint32_t& kid, int& leaves) {
     constexpr int R = S::kCap / 32;
@@ -260,7 +277,7 @@ ALB_DEVICE int run_search(const MapDev& m, S& s, int k, int nlist, float fx, flo
                 float v[R], x;
 #pragma unroll
                 for (int j = 0; j < R; ++j) v[j] = j * 32 + l < cnt ? s.cd[j * 32 + l] : FLT_MAX;
-                if (!find_cut(v, cnt, k, thr, x)) return -1;
+                if (!find_cut<G>(v, cnt, k, thr, x)) return -1;
                 thr = fminf(thr, x * (1.0f + 2.0f * kRelMargin));
                 int out = 0;
 #pragma unroll
@@ -289,7 +306,7 @@ ALB_DEVICE int run_search(const MapDev& m, S& s, int k, int nlist, float fx, flo
     float v[R], x;
 #pragma unroll
     for (int j = 0; j < R; ++j) v[j] = j * 32 + l < cnt ? s.cd[j * 32 + l] : FLT_MAX;
-    if (!find_cut(v, cnt, k, thr, x)) return -1;
+    if (!find_cut<G>(v, cnt, k, thr, x)) return -1;
     // the k-th, and whether another candidate lies within the screening margin of it
     unsigned mx = 0u;
 #pragma unroll

@@ -139,3 +139,27 @@ def test_index_of_crowded_keys_answers_like_kdtree(gpu_available, m):
     pts[: m // 3] = np.round(pts[: m // 3] * 20.0) / 20.0
     pts[0] = [1.0e6, 0.0, 0.0]
     _check_knn(pts.astype(np.float32), rng.uniform(-0.5, 0.5, size=(100, 3)), 33)
+
+
+@pytest.mark.parametrize("adjoint", [False, True])
+@pytest.mark.parametrize("k", [1, 100, 128, 129])
+def test_planar_searches_by_runs_equal_single_ones(gpu_available, k, adjoint):
+    """Planar gathers of 2^16 queries and more search by runs where k <= 128, smaller ones one query at a
+    time, and queries far from the spot leave the runs: the same photons in one backward call and
+    in calls below the limit, bit for bit (the Jacobian too)."""
+    cfg = dataclasses.replace(workloads.small(0.9), photon_mapping_k=k)
+
+    def run(cuts):
+        with GpuEngine(cfg, GpuRunOptions(adjoint=adjoint)) as eng:
+            eng.forward(20_000, 5)
+            eng.build_maps()
+            for a, b in zip(cuts, cuts[1:]):
+                eng.backward(b - a, 5)
+            return eng.waveform_array(f64=True), eng.jacobian() if adjoint else None
+
+    (wa, ja), (wb, jb) = run([0, 66_000]), run([0, 20_000, 40_000, 66_000])
+    assert np.abs(wa).sum() > 0
+    np.testing.assert_array_equal(wa, wb)
+    if adjoint:
+        assert np.abs(ja).sum() > 0
+        np.testing.assert_array_equal(ja, jb)
