@@ -810,18 +810,72 @@ ALB_DEVICE int class_of(float c, long long& v) {
     if (c < 0.f) v = -v;
     return sh >> 2;
 }
-ALB_DEVICE void class_add(unsigned long long* cls, uint32_t n, uint32_t i, float c, unsigned long long* lo,
-                          unsigned long long* hi) {
+// Per-CTA cache of class words for gathers whose neighbours share a few of them: adds to the same sector
+// of L2 come one per cycle, and one slice took 1.4 a nanosecond of the scatter gather of the default
+// scene, whose first-water cells lie in one narrow beam. With heatmaps, 6.2e5 queries: 4.4 -> 3.9 ms; a
+// waveform of 126 bins, 3.1e5 queries: 4.7 -> 2.7; the Jacobian of the gradient's surface gather, 2.5e5
+// queries: 7.9 -> 3.5. Direct-mapped, a slot claimed once by CAS on its
+// tag; a word is held as two 32-bit ones, which shared memory adds natively. Key: the word's number in
+// its array, plus `base` for the second of the two arrays that cache_flush writes.
+template <int N>
+struct WordCache {
+    static constexpr int kSlots = N;
+    uint32_t tag[N], lo[N], hi[N];
+};
+struct NoCache {};
+ALB_DEVICE void word_add(NoCache&, bool, unsigned long long* words, uint64_t i, uint32_t, uint32_t, long long v) {
+    atomicAdd(words + i, (unsigned long long)v);
+}
+template <int N>
+ALB_DEVICE void word_add(WordCache<N>& wc, bool on, unsigned long long* words, uint64_t i, uint32_t base, uint32_t hash,
+                         long long v) {
+    const uint32_t slot = hash % N, key = base + (uint32_t)i;
+    uint32_t t = on ? wc.tag[slot] : ~key;
+    if (t == 0xffffffffu) {
+        t = atomicCAS(&wc.tag[slot], 0xffffffffu, key);
+        if (t == 0xffffffffu) t = key;
+    }
+    if (t == key) {
+        const uint32_t lo = (uint32_t)v, old = atomicAdd(&wc.lo[slot], lo);
+        const uint32_t up = (uint32_t)((unsigned long long)v >> 32) + (old + lo < old ? 1u : 0u);
+        if (up) atomicAdd(&wc.hi[slot], up);
+    } else {
+        atomicAdd(words + i, (unsigned long long)v);
+    }
+}
+ALB_DEVICE void cache_clear(NoCache&) {}
+template <int N>
+ALB_DEVICE void cache_clear(WordCache<N>& wc) {
+    for (int i = threadIdx.x; i < N; i += blockDim.x) {
+        wc.tag[i] = 0xffffffffu;
+        wc.lo[i] = wc.hi[i] = 0u;
+    }
+}
+// (after a block barrier)
+ALB_DEVICE void cache_flush(const NoCache&, unsigned long long*, uint32_t, unsigned long long*) {}
+template <int N>
+ALB_DEVICE void cache_flush(const WordCache<N>& wc, unsigned long long* first, uint32_t n, unsigned long long* second) {
+    for (int i = threadIdx.x; i < N; i += blockDim.x) {
+        const uint32_t t = wc.tag[i];
+        if (t != 0xffffffffu)
+            atomicAdd(t < n ? first + t : second + (t - n), (unsigned long long)wc.hi[i] << 32 | wc.lo[i]);
+    }
+}
+
+template <class C>
+ALB_DEVICE void class_add(C& cache, bool on, uint32_t base, unsigned long long* cls, uint32_t n, uint32_t i, float c,
+                          unsigned long long* lo, unsigned long long* hi) {
     long long v;
     const int k = class_of(c, v);
-    if (k >= 0) atomicAdd(cls + ((uint64_t)(uint32_t)k * n + i), (unsigned long long)v);
+    if (k >= 0) word_add(cache, on, cls, (uint64_t)(uint32_t)k * n + i, base, i + 37u * (uint32_t)k, v);
     else if (k == -2) fix_atomic_add(lo + i, hi + i, f32_to_fix(c));
 }
 
 // The same where the accumulator may have no class words (cls null: direct).
-ALB_DEVICE void cell_add(unsigned long long* cls, uint32_t n, uint32_t i, float c, unsigned long long* lo,
-                         unsigned long long* hi) {
-    if (cls) class_add(cls, n, i, c, lo, hi);
+template <class C>
+ALB_DEVICE void cell_add(C& cache, bool on, uint32_t base, unsigned long long* cls, uint32_t n, uint32_t i, float c,
+                         unsigned long long* lo, unsigned long long* hi) {
+    if (cls) class_add(cache, on, base, cls, n, i, c, lo, hi);
     else fix_atomic_add(lo + i, hi + i, f32_to_fix(c));
 }
 
@@ -972,49 +1026,14 @@ ALB_DEVICE void warp_radius_visit(const MapDev& m, WarpSmem& s, double qx, doubl
     }
 }
 
-// Per-CTA cache of the Jacobian's class words for a planar gather: its neighbours share a few bins, and
-// five parameters at a few hundred words are as many adds to the same words of L2 (surface gather of the
-// gradient's scene, 1e6 photons: 7.9 -> 3.5 ms). Direct-mapped; a word is held as two 32-bit ones.
-constexpr int kJacCache = 512;
-struct JacCache {
-    uint32_t tag[kJacCache], lo[kJacCache], hi[kJacCache];
-};
-struct NoCache {};
-ALB_DEVICE void cache_clear(NoCache&) {}
-ALB_DEVICE void cache_flush(const NoCache&, unsigned long long*) {}
-ALB_DEVICE void cache_add(NoCache&, unsigned long long* words, uint32_t key, uint32_t, long long v) {
-    atomicAdd(words + key, (unsigned long long)v);
-}
-ALB_DEVICE void cache_clear(JacCache& jc) {
-    for (int i = threadIdx.x; i < kJacCache; i += blockDim.x) {
-        jc.tag[i] = 0xffffffffu;
-        jc.lo[i] = jc.hi[i] = 0u;
-    }
-}
-ALB_DEVICE void cache_flush(const JacCache& jc, unsigned long long* words) {
-    for (int i = threadIdx.x; i < kJacCache; i += blockDim.x)
-        if (jc.tag[i] != 0xffffffffu) atomicAdd(words + jc.tag[i], (unsigned long long)jc.hi[i] << 32 | jc.lo[i]);
-}
-ALB_DEVICE void cache_add(JacCache& jc, unsigned long long* words, uint32_t key, uint32_t hash, long long v) {
-    const uint32_t slot = hash % kJacCache;
-    uint32_t t = jc.tag[slot];
-    if (t == 0xffffffffu) {
-        t = atomicCAS(&jc.tag[slot], 0xffffffffu, key);
-        if (t == 0xffffffffu) t = key;
-    }
-    if (t == key) {
-        const uint32_t lo = (uint32_t)v, old = atomicAdd(&jc.lo[slot], lo);
-        const uint32_t up = (uint32_t)((unsigned long long)v >> 32) + (old + lo < old ? 1u : 0u);
-        if (up) atomicAdd(&jc.hi[slot], up);
-    } else {
-        atomicAdd(words + key, (unsigned long long)v);
-    }
-}
-
 // Adjoint (extension): one neighbour's c (s_query + s_record + d ln w / d theta) into the
 // Jacobian for theta = a, b, g, albedo, roughness (128-bit fixed point by class words).
+// Bins below which the number of every class word (the waveform's, then the Jacobian's or two heatmaps')
+// fits 32 bits; a longer waveform's words are not cached.
+constexpr int64_t kCachedBins = 1 << 25;
+
 template <int CHANNEL, class C>
-ALB_DEVICE void jac_add(const SceneDev& sc, const MapDev& m, const Accum& acc, C& cache, int layer, int bin, uint32_t idx,
+ALB_DEVICE void jac_add(const SceneDev& sc, const MapDev& m, const Accum& acc, C& cache, bool on, uint32_t base, int layer, int bin, uint32_t idx,
                         float c, float4 sq, float4 pb, float vx, float vy, float vz) {
     const float4 sp = m.sco ? m.sco[idx] : make_float4(0.f, 0.f, 0.f, 0.f);
     float d[kJacParams];
@@ -1027,7 +1046,6 @@ ALB_DEVICE void jac_add(const SceneDev& sc, const MapDev& m, const Accum& acc, C
         d[2] += __ldg(sc.layer_dlw_g[layer] + scatter_bin(sc, layer, pb.x, pb.y, pb.z, vx, vy, vz));
     if (CHANNEL == ALB_BOTTOM_REFLECTION) d[3] += sc.inv_albedo;
     if (CHANNEL == ALB_SURFACE_REFLECTION) d[4] = sc.dla2_drough * ggx_dlog_da2(sc.ggx_a2, -pb.x, -pb.y, -pb.z, vx, vy, vz);
-    const uint32_t nb = (uint32_t)acc.nbins;
 #pragma unroll
     for (int p = 0; p < kJacParams; ++p) {
         const uint64_t o = ((uint64_t)p * ALB_CHANNELS + CHANNEL) * acc.nbins + bin;
@@ -1035,9 +1053,9 @@ ALB_DEVICE void jac_add(const SceneDev& sc, const MapDev& m, const Accum& acc, C
         int k = -2;
         if (acc.jac_cls) k = class_of(c * d[p], v);
         if (k >= 0) {
-            // (the launch leaves jac_cls out where a word's number would not fit 32 bits)
             const uint32_t plane = (uint32_t)(p * kClasses + k);
-            cache_add(cache, acc.jac_cls, plane * nb + (uint32_t)bin, (uint32_t)bin + 37u * plane, v);
+            word_add(cache, on, acc.jac_cls, (uint64_t)plane * (uint32_t)acc.nbins + (uint32_t)bin, base,
+                     (uint32_t)bin + 37u * plane + 13u, v);
         } else if (k == -2) {
             fix_atomic_add(acc.jac_lo + o, acc.jac_hi + o, f32_to_fix(c * d[p]));
         }
@@ -1059,20 +1077,22 @@ ALB_DEVICE int heat_cell(float x, double c, double ext, double bin, float2 cf, f
 }
 
 // accumulate_to_heatmap (alb_sim/math/accumulate_heatmap.py:6-61) for one neighbour
-ALB_DEVICE void heat_add(const SceneDev& sc, const MapDev& m, const Accum& acc, uint32_t idx, float c) {
+template <class C>
+ALB_DEVICE void heat_add(const SceneDev& sc, const MapDev& m, const Accum& acc, C& cache, bool on, uint32_t base, uint32_t idx,
+                         float c) {
     const float4 fw = m.fwi[idx], sf = m.sfi[idx];
     const uint32_t cells = (uint32_t)(sc.hm_bins * sc.hm_bins);
     if (fw.x == fw.x) {
         const int xi = heat_cell(fw.x, sc.wc[0], sc.hm_wext, sc.hm_wbin, sc.hm_wc32[0], sc.hm_wext32, sc.hm_winv, sc.hm_bins);
         const int zi = heat_cell(fw.z, sc.wc[2], sc.hm_wext, sc.hm_wbin, sc.hm_wc32[1], sc.hm_wext32, sc.hm_winv, sc.hm_bins);
-        if (xi >= 0 && zi >= 0) cell_add(acc.heat_cls, cells, (uint32_t)(xi * sc.hm_bins + zi), c, acc.hw_lo, acc.hw_hi);
+        if (xi >= 0 && zi >= 0) cell_add(cache, on, base, acc.heat_cls, cells, (uint32_t)(xi * sc.hm_bins + zi), c, acc.hw_lo, acc.hw_hi);
     }
     if (sf.x == sf.x) {
         const int xi = heat_cell(sf.x, sc.fc[0], sc.hm_fext, sc.hm_fbin, sc.hm_fc32[0], sc.hm_fext32, sc.hm_finv, sc.hm_bins);
         const int zi = heat_cell(sf.z, sc.fc[2], sc.hm_fext, sc.hm_fbin, sc.hm_fc32[1], sc.hm_fext32, sc.hm_finv, sc.hm_bins);
         if (xi >= 0 && zi >= 0)
-            cell_add(acc.heat_cls ? acc.heat_cls + (uint64_t)kClasses * cells : nullptr, cells,
-                          (uint32_t)(xi * sc.hm_bins + zi), c, acc.hf_lo, acc.hf_hi);
+            cell_add(cache, on, base + kClasses * cells, acc.heat_cls ? acc.heat_cls + (uint64_t)kClasses * cells : nullptr,
+                     cells, (uint32_t)(xi * sc.hm_bins + zi), c, acc.hf_lo, acc.hf_hi);
     }
 }
 
@@ -1100,6 +1120,7 @@ ALB_DEVICE void accumulate(const SceneDev& sc, const MapDev& m, const QueryDev& 
     if (CHANNEL == ALB_SURFACE_TRANSMISSION_UP) wconst = sc.surface_lambert;
     float4 sq = make_float4(0.f, 0.f, 0.f, 0.f);
     if (MODE == kModeKnnAdjoint && q.s) sq = q.s[src];
+    const bool jac_on = acc.nbins < kCachedBins;
     // the next neighbour's record is loaded while this one is weighted
     uint32_t idx_n = l < k ? s.ci[l] : 0u;
     float4 pb_n = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -1126,7 +1147,7 @@ ALB_DEVICE void accumulate(const SceneDev& sc, const MapDev& m, const QueryDev& 
         if (bin >= 0 && bin < acc.nbins) {
             bin_add(bc, acc, CHANNEL, bin, c);
             if (MODE == kModeKnnAdjoint && acc.jac_lo)
-                jac_add<CHANNEL>(sc, m, acc, jc, 0, bin, idx, c, sq, pb, vx, vy, vz);
+                jac_add<CHANNEL>(sc, m, acc, jc, jac_on, 0u, 0, bin, idx, c, sq, pb, vx, vy, vz);
         } else if (!sc.gated) {
             atomicCAS(err, 0, ALB_ERR_CAPACITY);
         }
@@ -1141,7 +1162,10 @@ ALB_DEVICE void accumulate(const SceneDev& sc, const MapDev& m, const QueryDev& 
             float w;
             if (CHANNEL == ALB_BOTTOM_REFLECTION || CHANNEL == ALB_SURFACE_TRANSMISSION_UP) w = wconst;
                         else w = ggx_weight(sc.ggx_a2, (float)sc.f0, -pb.x, -pb.y, -pb.z, vx, vy, vz);
-            heat_add(sc, m, acc, idx, ((Es * m.a[idx].w) * norm) * w);
+            {
+                NoCache none;
+                heat_add(sc, m, acc, none, false, 0u, idx, ((Es * m.a[idx].w) * norm) * w);
+            }
         }
     }
 }
@@ -1151,7 +1175,7 @@ __global__ void __launch_bounds__(kGatherWarps * 32, kGatherBlocksPerSM) k_gathe
                                                               int* err, uint32_t kChunk) {
     __shared__ WarpSmem smem[kGatherWarps];
     __shared__ BinCache bc;
-    __shared__ std::conditional_t<MODE == kModeKnnAdjoint, JacCache, NoCache> jc;
+    __shared__ std::conditional_t<MODE == kModeKnnAdjoint, WordCache<512>, NoCache> jc;  // of acc.jac_cls
     cache_clear(jc);
     for (int i = threadIdx.x; i < kBinCache; i += blockDim.x) {
         bc.tag[i] = -1;
@@ -1201,11 +1225,11 @@ __global__ void __launch_bounds__(kGatherWarps * 32, kGatherBlocksPerSM) k_gathe
                         const int bin = (int)((ts + pb.w) / (float)sc.mult) - (int)sc.gate_lo;
                         if (bin >= 0 && bin < acc.nbins) {
                             bin_add(bc, acc, CHANNEL, bin, c);
-                            if (acc.jac_lo) jac_add<CHANNEL>(sc, m, acc, jc, layer, bin, idx, c, sq, pb, vx, vy, vz);
+                            if (acc.jac_lo) jac_add<CHANNEL>(sc, m, acc, jc, false, 0u, layer, bin, idx, c, sq, pb, vx, vy, vz);
                         } else if (!sc.gated) {
                             atomicCAS(err, 0, ALB_ERR_CAPACITY);
                         }
-                        if (acc.hw_lo && m.fwi) heat_add(sc, m, acc, idx, c);
+                        if (acc.hw_lo && m.fwi) heat_add(sc, m, acc, jc, false, 0u, idx, c);
                     },
                     r);
                 if (r.fail) {
@@ -1276,7 +1300,7 @@ __global__ void __launch_bounds__(kGatherWarps * 32, kGatherBlocksPerSM) k_gathe
     }
     __syncthreads();
     bin_flush<CHANNEL>(bc, acc);
-    cache_flush(jc, acc.jac_cls);
+    cache_flush(jc, nullptr, 0u, acc.jac_cls);
 }
 
 // x / b from r = the float32 nearest 1 / b: the quotient estimate corrected by its exact residual
@@ -1287,10 +1311,10 @@ ALB_DEVICE float div_by(float x, float b, float r) {
     return fmaf(fmaf(-q, b, x), r, q);
 }
 
-// One query's k neighbours s.ci / s.ce [0 .. k) into the waveform's class words (and Jacobian, heatmaps);
+// One query's k neighbours s.cp[0 .. k) into the waveform's class words (and Jacobian, heatmaps);
 // qy the query's float64 depth, rk the k-th distance.
 template <int CHANNEL, int MODE, class S, class J>
-ALB_DEVICE void accumulate_run(const SceneDev& sc, const MapDev& m, const QueryDev& q, const Accum& acc, J& jc,
+ALB_DEVICE void accumulate_run(const SceneDev& sc, const MapDev& m, const QueryDev& q, const Accum& acc, J& cache, bool on,
                                int* err, const S& s, int k, uint32_t src, float Es, float4 qb,
                                double qy, float rk) {
     constexpr bool volume = CHANNEL == ALB_SCATTER;
@@ -1315,11 +1339,12 @@ ALB_DEVICE void accumulate_run(const SceneDev& sc, const MapDev& m, const QueryD
     if (MODE == kModeKnnAdjoint && q.s) sq = q.s[src];
     // the next neighbour's record is loaded while this one is weighted
     float4 pb_n = make_float4(0.f, 0.f, 0.f, 0.f);
-    if (l < k) pb_n = m.b[s.ci[l]];
+    if (l < k) pb_n = m.b[s.cp[l].x];
 #pragma unroll 1
     for (int j = l; j < k; j += 32) {
         const float4 pb = pb_n;
-        if (j + 32 < k) pb_n = m.b[s.ci[j + 32]];
+        const uint2 cp = s.cp[j];
+        if (j + 32 < k) pb_n = m.b[s.cp[j + 32].x];
         if (volume) {
             // scatter_bin with its division by a constant
             const float n = rsqrtf(fmaf(pb.x, pb.x, fmaf(pb.y, pb.y, pb.z * pb.z)));
@@ -1328,22 +1353,30 @@ ALB_DEVICE void accumulate_run(const SceneDev& sc, const MapDev& m, const QueryD
             w = __ldg(wtab + a);
         }
         if (CHANNEL == ALB_SURFACE_REFLECTION) w = ggx_weight(sc.ggx_a2, (float)sc.f0, -pb.x, -pb.y, -pb.z, vx, vy, vz);
-        const float c = ((Es * s.ce[j]) * norm) * w;
+        const float c = ((Es * __uint_as_float(cp.y)) * norm) * w;
         const int bin = (int)div_by(qb.w + pb.w, sc.mult32, sc.mult32_inv) - gate;
         if ((uint32_t)bin < nbins) {
-            class_add(cls, nbins, (uint32_t)bin, c, wf_lo, wf_hi);
+            class_add(cache, on, 0u, cls, nbins, (uint32_t)bin, c, wf_lo, wf_hi);
             if (MODE == kModeKnnAdjoint && acc.jac_lo)
-                jac_add<CHANNEL>(sc, m, acc, jc, layer, bin, s.ci[j], c, sq, pb, vx, vy, vz);
+                jac_add<CHANNEL>(sc, m, acc, cache, on, kClasses * nbins, layer, bin, cp.x, c, sq, pb, vx, vy, vz);
         } else if (!sc.gated) {
             atomicCAS(err, 0, ALB_ERR_CAPACITY);
         }
-        if (MODE != kModeKnn && acc.hw_lo && m.fwi) heat_add(sc, m, acc, s.ci[j], c);
+        if (MODE != kModeKnn && acc.hw_lo && m.fwi) {
+            if constexpr (MODE == kModeKnnHeat) {
+                heat_add(sc, m, acc, cache, on, kClasses * nbins, cp.x, c);
+            } else {
+                NoCache none;
+                heat_add(sc, m, acc, none, false, 0u, cp.x, c);
+            }
+        }
     }
 }
 
 // The search of one query alone, out of line: the grouped kernel takes it for the first query of
 // a CTA, runs whose list does not fit, guesses that fail and near ties, 1-3% of the queries,
-// and its code and registers stay out of the hot loop. bound < 0: s.ci holds k points to take one from.
+// and its code and registers stay out of the hot loop. The k neighbours are left
+// in s.cp. bound < 0: it holds k points to take one from.
 template <class S>
 __device__ __noinline__ bool cold_knn(const MapDev& m, S& s, int k, float fx, float fy, float fz, float lx, float ly,
                                       float lz, float bound, KnnResult& res) {
@@ -1353,14 +1386,23 @@ __device__ __noinline__ bool cold_knn(const MapDev& m, S& s, int k, float fx, fl
         unsigned mx = 0u;
 #pragma unroll 1
         for (int j = lane_id(); j < k; j += 32)
-            mx = max(mx, __float_as_uint(point_dist2(fx, fy, fz, lx, ly, lz, m.a[s.ci[j]])));
+            mx = max(mx, __float_as_uint(point_dist2(fx, fy, fz, lx, ly, lz, m.a[s.cp[j].x])));
         const float t = __uint_as_float(__reduce_max_sync(0xffffffffu, mx)) * (1.f + 1.f / 16384.f);
         bound = t < 1.0e37f ? t : FLT_MAX;
     }
     if (!warp_knn<false, true>(m, s, k, 0.0, 0.0, 0.0, fx, fy, fz, lx, ly, lz, bound, m.b, res)) return false;
     if (!res.fail) {
-        for (int j = lane_id(); j < k; j += 32) s.ce[j] = m.a[s.ci[j]].w;
-        __syncwarp();
+        // s.ci to s.cp, which overlay each other: the last 32 first
+        for (int j = (k - 1) / 32 * 32 + lane_id(); j >= 0; j -= 32) {
+            uint2 c = make_uint2(0u, 0u);
+            if (j < k) {
+                c.x = s.ci[j];
+                c.y = __float_as_uint(m.a[c.x].w);
+            }
+            __syncwarp();
+            if (j < k) s.cp[j] = c;
+            __syncwarp();
+        }
     }
     return true;
 }
@@ -1382,6 +1424,7 @@ struct ScatterPlan {
     uint64_t first, n;  // the launch's range of the sorted queries
     uint32_t pieces;    // segments per level
     int levels;         // level L holds half of what the levels before it left, the last one the rest
+    bool cached;        // class words go through the CTA's cache, where it has one
     uint32_t* ticket;   // segments taken, zero at the launch
 };
 constexpr int kSegChunks = 64;
@@ -1396,7 +1439,8 @@ ALB_DEVICE void segment_range(const ScatterPlan& p, uint32_t g, uint64_t& s0, ui
     s1 = base + m * (j + 1) / p.pieces;
 }
 
-template <int CHANNEL, int MODE, int CAP, int WARPS>
+// SLOTS: slots of the cache of class words, 0: none. LOW: queries have low parts (else lo_zero).
+template <int CHANNEL, int MODE, int CAP, int WARPS, int SLOTS, bool LOW>
 __global__ void __launch_bounds__(WARPS * 32, 1)
     k_gather_runs(const __grid_constant__ SceneDev sc, const __grid_constant__ MapDev m,
                      const __grid_constant__ QueryDev q, const __grid_constant__ Accum acc, int k, int* err,
@@ -1410,8 +1454,10 @@ __global__ void __launch_bounds__(WARPS * 32, 1)
     // (the CTA's segment number << 32) | its global number; a segment's number is fetched by the
     // warp that takes the first chunk of the one before it
     __shared__ unsigned long long ring[kSegRing];
-    __shared__ std::conditional_t<MODE == kModeKnnAdjoint && CHANNEL != ALB_SCATTER, JacCache, NoCache> jc;
-    cache_clear(jc);
+    // class words: the waveform's, then the Jacobian's or the heatmaps'
+    using Cache = std::conditional_t<SLOTS != 0, WordCache<SLOTS>, NoCache>;
+    __shared__ Cache cache;
+    cache_clear(cache);
     if (threadIdx.x < kSegRing) ring[threadIdx.x] = ~0ull;
     __syncthreads();
     if (threadIdx.x == 0) {
@@ -1475,7 +1521,7 @@ __global__ void __launch_bounds__(WARPS * 32, 1)
                         gsrc = q.perm ? q.perm[qi + l] : (uint32_t)(qi + l);
                         const float4 a = q.a[gsrc];
                         gx = a.x; gy = a.y; gz = a.z;
-                        if (!q.lo_zero) {
+                        if (LOW && !q.lo_zero) {
                             const float4 c = q.c[gsrc];
                             la = fmaxf(fabsf(c.x), fmaxf(fabsf(c.y), fabsf(c.z)));
                         }
@@ -1500,7 +1546,7 @@ __global__ void __launch_bounds__(WARPS * 32, 1)
                 fx = __shfl_sync(0xffffffffu, gx, at);
                 fy = __shfl_sync(0xffffffffu, gy, at);
                 fz = __shfl_sync(0xffffffffu, gz, at);
-                if (!q.lo_zero) {
+                if (LOW && !q.lo_zero) {
                     const float4 c = q.c[src];
                     lx = c.x; ly = c.y; lz = c.z;
                 }
@@ -1523,7 +1569,7 @@ __global__ void __launch_bounds__(WARPS * 32, 1)
                     s.st[3] += 1;
                 }
             } else {
-                // a proven k-th distance bounds the search, or, while s.ci still holds them, the previous
+                // a proven k-th distance bounds the search, or, while s.cp still holds them, the previous
                 // query's neighbours; the run's boxes share its scratch
                 const float bound = got < 0 && kth > 0.f ? kth * (1.f + 1.f / 16384.f)
                                     : leaves == 0 && s.st[3] ? -1.f : FLT_MAX;
@@ -1548,7 +1594,7 @@ __global__ void __launch_bounds__(WARPS * 32, 1)
             }
             prev2 = d2;
             const float4 qb = q.b[src];
-            accumulate_run<CHANNEL, MODE>(sc, m, q, acc, jc, err, s, k, src, q.a[src].w, qb, (double)fy + (double)ly, rk);
+            accumulate_run<CHANNEL, MODE>(sc, m, q, acc, cache, plan.cached, err, s, k, src, q.a[src].w, qb, (double)fy + (double)ly, rk);
             __syncwarp();
         }
         if (l == 0) last2 = prev2;
@@ -1562,9 +1608,10 @@ __global__ void __launch_bounds__(WARPS * 32, 1)
         }
         if (q.inexact && s.st[4]) atomicAdd(q.inexact, s.st[4]);
     }
-    if constexpr (!std::is_same_v<decltype(jc), NoCache>) {
+    if constexpr (SLOTS != 0) {
         __syncthreads();
-        cache_flush(jc, acc.jac_cls);
+        cache_flush(cache, acc.cls + (uint64_t)CHANNEL * kClasses * acc.nbins, kClasses * (uint32_t)acc.nbins,
+                    MODE == kModeKnnAdjoint ? acc.jac_cls : acc.heat_cls);
     }
 }
 
@@ -1798,12 +1845,12 @@ static void merge_classes(const SceneDev& sc, const Accum& acc, int channel, boo
     }
 }
 
-template <int CHANNEL, int MODE, int CAP, int WARPS>
+template <int CHANNEL, int MODE, int CAP, int WARPS, int SLOTS, bool LOW = true>
 static void launch_runs(const SceneDev& sc, const MapDev& map, const QueryDev& q, const Accum& acc, int k, int* err,
                            cudaStream_t st) {
     constexpr int bytes = WARPS * (int)sizeof(GroupSmem<CAP>);
-    static_assert(bytes <= 232448, "one CTA's shared memory");
-    auto kernel = k_gather_runs<CHANNEL, MODE, CAP, WARPS>;
+    static_assert(bytes + 12 * SLOTS + 8 * kSegRing + 32 <= 232448, "one CTA's shared memory");
+    auto kernel = k_gather_runs<CHANNEL, MODE, CAP, WARPS, SLOTS, LOW>;
     static std::atomic<bool> attr_set[64];  // per device; batched runs launch from several host threads
     int dev = 0;
     cudaGetDevice(&dev);
@@ -1814,11 +1861,14 @@ static void launch_runs(const SceneDev& sc, const MapDev& map, const QueryDev& q
     // a class word holds kClassMost contributions: more queries go in slices
     const uint64_t most = kClassMost / (uint64_t)k;
     for (uint64_t first = 0; first < q.n; first += most) {
-        ScatterPlan plan{first, std::min<uint64_t>(most, q.n - first), 0u, 1, q.ticket};
+        ScatterPlan plan{first, std::min<uint64_t>(most, q.n - first), 0u, 1, acc.nbins < kCachedBins, q.ticket};
         const uint64_t blocks = std::min<uint64_t>(sm_count(), plan.n);
-        plan.pieces = (uint32_t)(4 * blocks);
-        // levels until a segment's chunks hold eight queries
-        while (plan.levels < 16 && (plan.n >> plan.levels) >= (uint64_t)plan.pieces * kSegChunks * 8) ++plan.levels;
+        using G = std::conditional_t<CHANNEL == ALB_SCATTER, VolumeRuns, PlaneRuns>;
+        uint64_t per = 4;
+        while (per > 1 && plan.n < per * blocks * kSegChunks * G::kChunk) --per;
+        plan.pieces = (uint32_t)(per * blocks);
+        // levels until a segment's chunks hold kChunk queries
+        while (plan.levels < 16 && (plan.n >> plan.levels) >= (uint64_t)plan.pieces * kSegChunks * G::kChunk) ++plan.levels;
         cudaMemsetAsync(q.ticket, 0, sizeof(uint32_t), st);
         kernel<<<(unsigned)blocks, WARPS * 32, bytes, st>>>(sc, map, q, acc, k, err, plan);
         note_launch();
@@ -1839,14 +1889,32 @@ static bool planar_runs(int channel, uint64_t nq, int k) {
     return runs_channel(channel) && nq >= kPlanarRunsMin && k <= 128;
 }
 
+// Bins up to which the scatter gather caches the waveform's class words: 126 bins (a 40 ns record at
+// 3 GHz, 3.1e5 queries) 4.7 -> 2.7 ms; 2858 bins are the same either way, 84,056 bins 22.7 -> 23.7.
+constexpr int64_t kFewBins = 1024;
 template <int CHANNEL, int MODE>
 static void launch_channel(const MapDev& map, const QueryDev& q, const SceneDev& sc, const Accum& acc, int* err,
                            uint64_t nq, int k, cudaStream_t st) {
     if constexpr (MODE != kModeRadius && runs_channel(CHANNEL)) {
         if (CHANNEL == ALB_SCATTER || planar_runs(CHANNEL, nq, k)) {
             // candidates of a first guess: 1.33 k, twice that where the map thickens
-            if (k <= 128) launch_runs<CHANNEL, MODE, 224, 32>(sc, map, q, acc, k, err, st);
-            else if constexpr (CHANNEL == ALB_SCATTER) launch_runs<CHANNEL, MODE, 448, 22>(sc, map, q, acc, k, err, st);
+            constexpr int slots = MODE == kModeKnnHeat || CHANNEL != ALB_SCATTER ? 1024 : 0;
+            if constexpr (CHANNEL == ALB_SCATTER) {
+                if (k > 128) {
+                    launch_runs<CHANNEL, MODE, 448, 22, slots>(sc, map, q, acc, k, err, st);
+                    return;
+                }
+                if constexpr (MODE == kModeKnn) {
+                    if (acc.nbins <= kFewBins) {
+                        launch_runs<CHANNEL, MODE, 224, 32, 1024>(sc, map, q, acc, k, err, st);
+                        return;
+                    }
+                }
+                if (q.lo_zero) launch_runs<CHANNEL, MODE, 224, 32, slots, false>(sc, map, q, acc, k, err, st);
+                else launch_runs<CHANNEL, MODE, 224, 32, slots>(sc, map, q, acc, k, err, st);
+            } else {
+                launch_runs<CHANNEL, MODE, 224, 32, slots>(sc, map, q, acc, k, err, st);
+            }
             return;
         }
     }
@@ -1879,7 +1947,6 @@ void launch_gather(const SceneDev& sc, const MapDev& map, const QueryDev& q, int
     // the gathers by runs keep below kClassMost by slices
     const uint64_t per = sc.radius > 0.0 ? std::max<uint64_t>(map.n, 1) : (uint64_t)k;
     if (q.n > kClassMost / per && (sc.radius > 0.0 || (channel != ALB_SCATTER && !planar_runs(channel, q.n, k)))) acc.jac_cls = acc.heat_cls = nullptr;
-    if ((uint64_t)kJacParams * kClasses * (uint64_t)acc.nbins > 0xffffffffull) acc.jac_cls = nullptr;  // JacCache
     if (sc.radius > 0.0) launch_gather_mode<kModeRadius>(map, q, channel, sc, acc, err, q.n, k, st);
     else if (acc.jac_lo) launch_gather_mode<kModeKnnAdjoint>(map, q, channel, sc, acc, err, q.n, k, st);
     else if (acc.hw_lo && map.fwi) launch_gather_mode<kModeKnnHeat>(map, q, channel, sc, acc, err, q.n, k, st);

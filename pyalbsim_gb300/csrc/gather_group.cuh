@@ -16,7 +16,10 @@
 // What bounds it: instruction issue and L2 latency. One-query search in the same query order, per
 // query of the large scene at 1e6 photons (8.7e6 queries): 7.8 tree nodes walked, 4600 warp
 // instructions, 51.0 ms; in runs: 0.07 nodes, 2650 warp instructions, 31.7 ms (1e7 photons:
-// 492 -> 318 ms).
+// 492 -> 318 ms). With the accumulation by class words and the map in Hilbert order 23.0 ms (231);
+// leaves padded to 32 records, position and energy of a candidate in one access, boxes by centre and half
+// width, and no low parts where the queries have none: 22.2 ms (225), of which the search is three
+// quarters.
 #pragma once
 
 namespace alb {
@@ -31,9 +34,12 @@ constexpr float kGroupTarget = 80.f;
 // distance, what a query first admits within and what the run's leaf list covers (the second
 // attempt). side: edge of a leaf over the k-th distance, 32 records against k in the ball.
 // est: leaves that a ball of radius T around a box of the given extents meets, the ball as the
-// cube (square) of its volume. kGrow: count ~ (squared distance)^kGrow.
+// cube (square) of its volume. kGrow: count ~ (squared distance)^kGrow. kChunk: queries that a chunk of
+// the last level holds at least (planar gathers of 3e5 and 2.5e5 queries: 8 -> 16 0.95 -> 0.78 and 0.65 ->
+// 0.53 ms; the scatter gather of 4e6 adjoint queries 14.1 -> 14.6).
 struct VolumeRuns {
     static constexpr float kGuess2 = 1.21f, kList2 = 1.5625f, kGrow = 1.5f;
+    static constexpr uint64_t kChunk = 8;
     static ALB_DEVICE float side(float k) { return cbrtf(134.04f / k); }
     static ALB_DEVICE float est(float dx, float dy, float dz, float side, float T) {
         const float w = side + 1.61f * T;
@@ -43,6 +49,7 @@ struct VolumeRuns {
 // A horizontal plane. (Guesses of 1.15 and 1.3 measured the same to 4%.)
 struct PlaneRuns {
     static constexpr float kGuess2 = 1.21f, kList2 = 1.5625f, kGrow = 1.f;
+    static constexpr uint64_t kChunk = 16;
     static ALB_DEVICE float side(float k) { return sqrtf(100.53f / k); }
     static ALB_DEVICE float est(float dx, float, float dz, float side, float T) {
         const float w = side + 1.77f * T;
@@ -55,15 +62,17 @@ template <int CAP>
 struct GroupSmem {
     static constexpr int kCap = CAP, kSelectAt = CAP - 32, kTmp = 2 * kGroupStack + 128;
     float cd[CAP];     // candidates: squared float32 distance
-    uint32_t ci[CAP];  // map position
     union {
-        float ce[CAP];    // energy (grouped search)
-        int16_t cl[CAP];  // distance fraction (one-query search)
+        uint2 cp[CAP];  // map position and energy (grouped search: one access for both)
+        struct {
+            uint32_t ci[CAP];  // map position
+            int16_t cl[CAP];   // distance fraction (one-query search)
+        };
     };
     uint32_t leaf[kGroupLeaves];  // the run's leaves
     uint32_t hit[kGroupLeaves];   // those the current query's ball meets
     union {
-        float box[6][kGroupLeaves];  // the run's leaf boxes: lo x, y, z, hi x, y, z
+        float box[6][kGroupLeaves];  // the run's leaf boxes: centre x, y, z, half width x, y, z
         struct {                     // scratch of the one-query search
             uint32_t stk[kGroupStack];
             float stk_d[kGroupStack];
@@ -94,6 +103,18 @@ struct QueryRun {
 ALB_DEVICE float run_gap(float lo, float hi, float qlo, float qhi, float ql) {
     float g = fmaxf(fmaxf(lo - qhi, qlo - hi), 0.f);
     return fmaxf(g * (1.f - 2.384185791015625e-07f) - ql, 0.f);
+}
+
+// Half width of a box around its centre as a float, rounded up, with the largest low part of the run's
+// queries; and a query's gap to the box from both, three operations, never above the true one: |q - c|
+// is off by 2^-24 of itself and the last rounding by 2^-24 of the gap, both below the 2^-22 taken off.
+// (NaN, where a box reaches infinity, counts as no gap.)
+ALB_DEVICE float half_width(float lo, float hi, float low) {
+    const float c = 0.5f * (lo + hi);
+    return __fadd_ru(fmaxf(__fsub_ru(hi, c), __fsub_ru(c, lo)), low);
+}
+ALB_DEVICE float centre_gap(float q, float c, float h) {
+    return fmaxf(fmaf(fabsf(q - c), 1.f - 2.384185791015625e-07f, -h), 0.f);
 }
 
 // Builds the run starting at the first of `avail` queries whose positions the lanes hold (lane i
@@ -158,8 +179,12 @@ ALB_DEVICE bool build_run(const MapDev& m, S& s, int avail, float x, float y, fl
                 if (in) {
                     const int e = n + pos;
                     s.leaf[e] = c;
-                    s.box[0][e] = lo.x; s.box[1][e] = lo.y; s.box[2][e] = lo.z;
-                    s.box[3][e] = hi.x; s.box[4][e] = hi.y; s.box[5][e] = hi.z;
+                    s.box[0][e] = 0.5f * (lo.x + hi.x);
+                    s.box[1][e] = 0.5f * (lo.y + hi.y);
+                    s.box[2][e] = 0.5f * (lo.z + hi.z);
+                    s.box[3][e] = half_width(lo.x, hi.x, bl);
+                    s.box[4][e] = half_width(lo.y, hi.y, bl);
+                    s.box[5][e] = half_width(lo.z, hi.z, bl);
                 }
                 n += __popc(b);
             } else {
@@ -222,7 +247,7 @@ ALB_DEVICE bool find_cut(const float (&v)[R], int cnt, int k, float hi, float& x
 }
 
 // One query against the run's list under the threshold thr (squared, with the band margin).
-// 1: s.ci / s.ce [0 .. k) hold the k nearest, kth their largest float32 distance, kid its map
+// 1: s.cp[0 .. k) holds the k nearest, kth their largest float32 distance, kid its map
 // position; 0: the threshold does not prove an answer; -1: a near tie at the k-th place (kth is
 // then a proven bound when > 0), or too many candidates at one distance.
 template <class G, class S>
@@ -236,21 +261,19 @@ ALB_DEVICE int run_search(const MapDev& m, S& s, int k, int nlist, float fx, flo
     for (int e0 = 0; e0 < nlist; e0 += 32) {
         const int e = e0 + l;
         bool in = false;
-        if (e < nlist)
-            in = box_dist2(fx, fy, fz, lx, ly, lz, make_float4(s.box[0][e], s.box[1][e], s.box[2][e], 0.f),
-                           make_float4(s.box[3][e], s.box[4][e], s.box[5][e], 0.f)) <= thr;
+        if (e < nlist) {
+            const float dx = centre_gap(fx, s.box[0][e], s.box[3][e]), dy = centre_gap(fy, s.box[1][e], s.box[4][e]),
+                        dz = centre_gap(fz, s.box[2][e], s.box[5][e]);
+            in = fmaf(dx, dx, fmaf(dy, dy, dz * dz)) * (1.f - 4.76837158203125e-07f) <= thr;
+        }
         const unsigned b = __ballot_sync(0xffffffffu, in);
         if (in) s.hit[nh + __popc(b & lanemask_lt())] = s.leaf[e];
         nh += __popc(b);
     }
     __syncwarp();
     leaves += nh;
-    const uint32_t n32 = (uint32_t)m.n;
     int cnt = 0;
     kth = 0.f;
-    auto load = [&](uint32_t r) {
-        return r < n32 ? m.a[r] : make_float4(FLT_MAX, FLT_MAX, FLT_MAX, 0.f);  // the last leaf may be partial
-    };
     auto admit = [&](uint32_t r, float4 p, bool on) {
         const float d = point_dist2(fx, fy, fz, lx, ly, lz, p);
         const bool in = on && d <= thr;
@@ -258,8 +281,7 @@ ALB_DEVICE int run_search(const MapDev& m, S& s, int k, int nlist, float fx, flo
         if (in) {
             const int pos = cnt + __popc(b & lanemask_lt());
             s.cd[pos] = d;
-            s.ci[pos] = r;
-            s.ce[pos] = p.w;
+            s.cp[pos] = make_uint2(r, __float_as_uint(p.w));
         }
         cnt += __popc(b);
     };
@@ -267,7 +289,7 @@ ALB_DEVICE int run_search(const MapDev& m, S& s, int k, int nlist, float fx, flo
     for (int i = 0; i < nh; i += 2) {
         // two leaves' records in flight at a time
         const uint32_t r0 = s.hit[i] * 32u + l, r1 = s.hit[min(i + 1, nh - 1)] * 32u + l;
-        const float4 p0 = load(r0), p1 = load(r1);
+        const float4 p0 = m.a[r0], p1 = m.a[r1];  // a partial leaf is padded with far points
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
             admit(h ? r1 : r0, h ? p1 : p0, h == 0 || i + 1 < nh);
@@ -284,14 +306,12 @@ ALB_DEVICE int run_search(const MapDev& m, S& s, int k, int nlist, float fx, flo
                 for (int j = 0; j < R; ++j) {
                     const bool keep = v[j] <= thr;
                     const unsigned b = __ballot_sync(0xffffffffu, keep);
-                    const uint32_t id = s.ci[j * 32 + l];
-                    const float en = s.ce[j * 32 + l];
+                    const uint2 c = s.cp[j * 32 + l];
                     __syncwarp();
                     if (keep) {
                         const int pos = out + __popc(b & lanemask_lt());
                         s.cd[pos] = v[j];
-                        s.ci[pos] = id;
-                        s.ce[pos] = en;
+                        s.cp[pos] = c;
                     }
                     out += __popc(b);
                     __syncwarp();
@@ -326,18 +346,13 @@ ALB_DEVICE int run_search(const MapDev& m, S& s, int k, int nlist, float fx, flo
         if (j * 32 < cnt) {
             const bool keep = v[j] <= x;
             const unsigned b = __ballot_sync(0xffffffffu, keep);
-            const uint32_t id = s.ci[j * 32 + l];
-            const float en = s.ce[j * 32 + l];
+            const uint2 c = s.cp[j * 32 + l];
             if (v[j] == kth) {
-                own = id;
+                own = c.x;
                 mine = true;
             }
             __syncwarp();
-            if (keep) {
-                const int pos = out + __popc(b & lanemask_lt());
-                s.ci[pos] = id;
-                s.ce[pos] = en;
-            }
+            if (keep) s.cp[out + __popc(b & lanemask_lt())] = c;
             out += __popc(b);
             __syncwarp();
         }

@@ -1986,6 +1986,13 @@ __global__ void k_crowded(const K* __restrict__ keys, uint64_t n, unsigned* coun
 // 256 others (a box far larger than what its records fill), into exact left-balanced k-d order; and
 // the box tree over leaves of 32. The index's own position array holds the sort's scratch, so the
 // peak is the record store, the index and four bytes per record.
+// The last leaf's places beyond the records hold points too far for any search to admit (3.4e38 per axis):
+// a search by leaves needs no test of its record numbers.
+static void pad_leaf(const MapIndex& m, cudaStream_t st) {
+    const uint64_t to = (m.n + 31) / 32 * 32;
+    if (to > m.n) cudaMemsetAsync(m.a + m.n, 0x7f, (to - m.n) * sizeof(float4), st);
+}
+
 static int build_word(int slot) { return 16 + 8 * slot; }  // box in six words, crowded runs in the next
 
 int start_map_index(Workspace& ws, const RecordStore& rec, uint64_t n, MapIndex& m, int slot, cudaStream_t st) {
@@ -2045,6 +2052,7 @@ int start_map_index(Workspace& ws, const RecordStore& rec, uint64_t n, MapIndex&
     k_hilbert_finish<<<(unsigned)((warps + kFinishWarps - 1) / kFinishWarps), kFinishWarps * 32, 0, st>>>(order, rec, n, out);
     note_launch();
     parent_boxes(m, st);
+    pad_leaf(m, st);
     ws.release(mark);
     return 0;
 }
@@ -2071,6 +2079,7 @@ int finish_map_index(Workspace& ws, const RecordStore& rec, MapIndex& m, int slo
     k_leaf_boxes<<<(unsigned)((m.lvl_cnt[0] * 32 + 255) / 256), 256, 0, st>>>(m.a, n, m.box_lo, m.box_hi, m.lvl_cnt[0]);
     note_launch();
     parent_boxes(m, st);
+    pad_leaf(m, st);
     return 0;
 }
 
