@@ -743,9 +743,13 @@ extern "C" int alb_set_option(AlbCtx* ctx, int key, int64_t v) {
 
 // backward photons traced and gathered per chunk when no per-photon state is exported
 constexpr uint64_t kBackwardChunk = 1ull << 22;
-// photons that measure the records (or queries) per photon of a scene not traced before: a large
-// trace into buffers sized by the defaults runs twice
+// A trace into buffers that turn out too small runs twice. In a scene not traced before, a small forward call
+// therefore gets room for kManyRecords scatter records per photon (3 KB per photon, given back when the
+// maps are built), and a large one traces its first kPilot photons into as much and measures: those few
+// leave most of the chip idle, 2.7 ms of the float64 tracer's 16.5 for 200 000 photons twice over.
 constexpr uint64_t kPilot = 1ull << 14;
+constexpr uint64_t kSmallCall = 1ull << 18;
+constexpr double kManyRecords = 96.0;
 
 static void release_records(AlbCtx* ctx, int c) {
     RecordStore& r = ctx->rec[c];
@@ -1021,12 +1025,14 @@ extern "C" int alb_trace(AlbCtx* ctx, int pass, uint64_t n, uint64_t seed, uint6
                 bool overflow = false;
                 for (int c = 0; c < ALB_CHANNELS; ++c) {
                     uint64_t added = cnt[c] - before[c];
-                    if (pn > 0) ctx->rec_rate[c] = std::max(ctx->rec_rate[c] * 0.5, (double)added / (double)pn);
+                    const double rate = (double)added / (double)std::max<uint64_t>(pn, 1);
+                    if (ctx->rec_rate_known) ctx->rec_rate[c] = pn ? std::max(ctx->rec_rate[c] * 0.5, rate) : ctx->rec_rate[c];
+                    else if (pn >= 1024) ctx->rec_rate[c] = rate;  // fewer photons measure too little
                     if (cnt[c] > ctx->rec[c].cap) overflow = true;
                 }
                 if (!overflow) {
                     for (int c = 0; c < ALB_CHANNELS; ++c) ctx->h_rec_count[c] = cnt[c];
-                    if (pn > 0) ctx->rec_rate_known = true;
+                    if (pn >= 1024) ctx->rec_rate_known = true;
                     return ALB_OK;
                 }
                 // undo and retry with the measured sizes
@@ -1038,7 +1044,11 @@ extern "C" int alb_trace(AlbCtx* ctx, int pass, uint64_t n, uint64_t seed, uint6
             }
             return fail(ctx, ALB_ERR_CAPACITY, "photon-map capacity could not be established");
         };
-        const uint64_t pilot = !ctx->rec_rate_known && n > 4 * kPilot && !rp && !ctx->keep_exit ? kPilot : 0;
+        const uint64_t pilot = !ctx->rec_rate_known && n > kSmallCall && !rp && !ctx->keep_exit ? kPilot : 0;
+        if (!ctx->rec_rate_known && (pilot || n <= kSmallCall)) {
+            ctx->rec_rate[ALB_BOTTOM_REFLECTION] = 4.0;
+            ctx->rec_rate[ALB_SCATTER] = kManyRecords;
+        }
         int rc = pilot ? part(0, pilot) : ALB_OK;
         if (!rc) rc = part(pilot, n - pilot);
         ctx->ws.release(mark);
@@ -1099,6 +1109,14 @@ extern "C" int alb_trace(AlbCtx* ctx, int pass, uint64_t n, uint64_t seed, uint6
         CK(cudaMemcpyAsync(ctx->d_stats, stats_bak, 2 * 8, cudaMemcpyDeviceToDevice, ctx->st));
         return ALB_OK;
     };
+    // a scene's backward photons make queries as its forward photons make records (within 2% in every
+    // workload here), so the forward rates size the first buffers; a trace into too small ones runs twice
+    if (!ctx->q_rate_known && ctx->rec_rate_known) {
+        ctx->q_rate[kQueryBottom] = ctx->rec_rate[ALB_BOTTOM_REFLECTION];
+        ctx->q_rate[kQueryScatter] = ctx->rec_rate[ALB_SCATTER];
+        ctx->q_rate[kQuerySurface] = std::max(ctx->rec_rate[ALB_SURFACE_REFLECTION], 1.0);
+        ctx->q_rate_known = true;
+    }
     for (uint64_t c0 = 0; c0 == 0 || c0 < n; c0 += chunk) {
         const uint64_t nc = std::min<uint64_t>(chunk, n - c0);
         bool overflow = false;
