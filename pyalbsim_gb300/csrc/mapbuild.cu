@@ -90,40 +90,94 @@ struct KeyGrid {
     int naxes, m, hi;
 };
 
-// Hilbert index of 2 or 3 coordinates of `bits` bits, one level at a time from the top: the octant is
+// Hilbert index of 2 or 3 coordinates of `bits` bits, from the top level down: the octant is
 // mapped through the curve's entry corner e and axis d of the current cube, its Gray rank is the
 // key's next digit, and e and d follow the curve into that octant (Hamilton, "Compact Hilbert
-// indices", Dalhousie CS-2006-07). The small tables are packed in words.
+// indices", Dalhousie CS-2006-07). The curve's state is e + 8 d (e + 4 d in the plane); step3 and step2 take
+// octant o and leave the digit and the next state. The keys take two levels (three in the plane) at a
+// time from a table in shared memory: 1.12e8 keys of 48 bits level by level 3.2 ms, by table 1.1.
+ALB_HOST_DEVICE constexpr uint32_t step3(uint32_t& state, uint32_t o) {
+    uint32_t e = state & 7u, d = state >> 3;
+    o ^= e;
+    const uint32_t r = d == 2u ? 0u : d + 1u;
+    o = ((o * 9u) >> r) & 7u;                            // rotated right by d + 1 of 3 bits
+    const uint32_t w = (0x54672310u >> (4u * o)) & 7u;   // inverse Gray code: 0 1 3 2 7 6 4 5
+    const uint32_t en = (0x56633000u >> (4u * w)) & 7u;  // entry corners: 0 0 0 3 3 6 6 5
+    e ^= (((en * 9u) << r) >> 3) & 7u;                   // rotated left by d + 1
+    d += ((0x01122110u >> (4u * w)) & 3u) + 1u;          // directions: 0 1 1 2 2 1 1 0
+    state = e | (d >= 3u ? d - 3u : d) << 3;
+    return w;
+}
+ALB_HOST_DEVICE constexpr uint32_t step2(uint32_t& state, uint32_t o) {
+    uint32_t e = state & 3u, d = state >> 2;
+    o ^= e;
+    o = d ? o : (((o << 1) | (o >> 1)) & 3u);  // rotated by d + 1 of 2 bits
+    const uint32_t w = o ^ (o >> 1);           // inverse Gray code: 0 1 3 2
+    e ^= w == 3u ? 3u : 0u;                    // entry corners: 0 0 0 3
+    d ^= (w == 0u || w == 3u) ? 1u : 0u;       // directions 0 1 1 0, plus 1, of 2
+    state = e | d << 2;
+    return w;
+}
+
+// [state][coordinate bits, the first coordinate's lowest] -> next state << 6 | six bits of key
+struct HilbertTables {
+    uint16_t t3[24 * 64];  // two bits of each of three coordinates
+    uint16_t t2[8 * 64];   // three bits of each of two
+};
+constexpr HilbertTables hilbert_tables() {
+    HilbertTables t{};
+    for (uint32_t s = 0; s < 24; ++s)
+        for (uint32_t i = 0; i < 64; ++i) {
+            const uint32_t x = i & 3u, y = i >> 2 & 3u, z = i >> 4;
+            uint32_t state = s;
+            const uint32_t a = step3(state, x >> 1 | (y >> 1) << 1 | (z >> 1) << 2);
+            const uint32_t b = step3(state, (x & 1u) | (y & 1u) << 1 | (z & 1u) << 2);
+            t.t3[s * 64 + i] = (uint16_t)(state << 6 | a << 3 | b);
+        }
+    for (uint32_t s = 0; s < 8; ++s)
+        for (uint32_t i = 0; i < 64; ++i) {
+            const uint32_t x = i & 7u, y = i >> 3;
+            uint32_t state = s, key = 0;
+            for (int b = 2; b >= 0; --b) key = key << 2 | step2(state, (x >> b & 1u) | (y >> b & 1u) << 1);
+            t.t2[s * 64 + i] = (uint16_t)(state << 6 | key);
+        }
+    return t;
+}
+__device__ const HilbertTables kHilbertTables = hilbert_tables();
+
 template <class K>
-ALB_DEVICE K hilbert_key3(uint32_t x, uint32_t y, uint32_t z, int bits) {
+ALB_DEVICE K hilbert_key3(const HilbertTables& t, uint32_t x, uint32_t y, uint32_t z, int bits) {
     K key = 0;
-    uint32_t e = 0u, d = 0u;
+    uint32_t s = 0u;
+    int b = bits;
+    if (b & 1) {
+        --b;
+        key = step3(s, (x >> b & 1u) | (y >> b & 1u) << 1 | (z >> b & 1u) << 2);
+    }
 #pragma unroll 2
-    for (int b = bits - 1; b >= 0; --b) {
-        uint32_t o = (((x >> b) & 1u) | (((y >> b) & 1u) << 1) | (((z >> b) & 1u) << 2)) ^ e;
-        const uint32_t r = d == 2u ? 0u : d + 1u;
-        o = ((o * 9u) >> r) & 7u;                           // rotated right by d + 1 of 3 bits
-        const uint32_t w = (0x54672310u >> (4u * o)) & 7u;  // inverse Gray code: 0 1 3 2 7 6 4 5
-        key = (key << 3) | w;
-        const uint32_t en = (0x56633000u >> (4u * w)) & 7u;  // entry corners: 0 0 0 3 3 6 6 5
-        e ^= (((en * 9u) << r) >> 3) & 7u;                   // rotated left by d + 1
-        d += ((0x01122110u >> (4u * w)) & 3u) + 1u;          // directions: 0 1 1 2 2 1 1 0
-        d = d >= 3u ? d - 3u : d;
+    while (b > 0) {
+        b -= 2;
+        const uint32_t v = t.t3[s * 64u + ((x >> b & 3u) | (y >> b & 3u) << 2 | (z >> b & 3u) << 4)];
+        key = (key << 6) | (v & 63u);
+        s = v >> 6;
     }
     return key;
 }
 template <class K>
-ALB_DEVICE K hilbert_key2(uint32_t x, uint32_t y, int bits) {
+ALB_DEVICE K hilbert_key2(const HilbertTables& t, uint32_t x, uint32_t y, int bits) {
     K key = 0;
-    uint32_t e = 0u, d = 0u;
+    uint32_t s = 0u;
+    int b = bits;
+    for (int odd = bits % 3; odd > 0; --odd) {
+        --b;
+        key = (key << 2) | step2(s, (x >> b & 1u) | (y >> b & 1u) << 1);
+    }
 #pragma unroll 2
-    for (int b = bits - 1; b >= 0; --b) {
-        uint32_t o = (((x >> b) & 1u) | (((y >> b) & 1u) << 1)) ^ e;
-        o = d ? o : (((o << 1) | (o >> 1)) & 3u);  // rotated by d + 1 of 2 bits
-        const uint32_t w = o ^ (o >> 1);           // inverse Gray code: 0 1 3 2
-        key = (key << 2) | w;
-        e ^= w == 3u ? 3u : 0u;                    // entry corners: 0 0 0 3
-        d ^= (w == 0u || w == 3u) ? 1u : 0u;       // directions 0 1 1 0, plus 1, of 2
+    while (b > 0) {
+        b -= 3;
+        const uint32_t v = t.t2[s * 64u + ((x >> b & 7u) | (y >> b & 7u) << 3)];
+        key = (key << 6) | (v & 63u);
+        s = v >> 6;
     }
     return key;
 }
@@ -165,7 +219,7 @@ ALB_DEVICE KeyGrid make_key_grid(const unsigned* box, int total) {
 }
 
 template <class K>
-ALB_DEVICE K cell_key(const KeyGrid& g, float x, float y, float z) {
+ALB_DEVICE K cell_key(const KeyGrid& g, const HilbertTables& t, float x, float y, float z) {
     const float v[3] = {x, y, z};
     const float top = (float)((1u << (g.m + g.hi)) - 1u);
     uint32_t c[3];
@@ -177,12 +231,12 @@ ALB_DEVICE K cell_key(const KeyGrid& g, float x, float y, float z) {
     }
     if (g.naxes == 1) return c[0];
     if (g.naxes == 2) {
-        return hilbert_key2<K>(c[0], c[1], g.hi);
+        return hilbert_key2<K>(t, c[0], c[1], g.hi);
     }
     if (g.naxes == 0) return 0u;
     const uint32_t mask = (1u << g.m) - 1u;
-    const K hi = hilbert_key2<K>(c[0] >> g.m, c[1] >> g.m, g.hi);
-    return (hi << (3 * g.m)) | hilbert_key3<K>(c[0] & mask, c[1] & mask, min(c[2], mask), g.m);
+    const K hi = hilbert_key2<K>(t, c[0] >> g.m, c[1] >> g.m, g.hi);
+    return (hi << (3 * g.m)) | hilbert_key3<K>(t, c[0] & mask, c[1] & mask, min(c[2], mask), g.m);
 }
 
 // ------------------------------------------------------------------------------------------
@@ -192,13 +246,15 @@ ALB_DEVICE K cell_key(const KeyGrid& g, float x, float y, float z) {
 // which a block keeps one running offset per digit. A tile is ranked by warps in order, rounds in
 // order and lanes in order, put in digit order in shared memory and written out from there, so
 // that a digit's records leave in runs (16 on average) instead of one by one.
-// Bound by the ranking's latency (a warp match and a shared counter per round) beside its DRAM
-// traffic, 20 B per record and pass (key read for the histogram; key and value read and written):
-// 9.5e7 queries of the large scene at 1e7 photons sort in 5.3 ms with their box and keys (12.3 ms
-// with one tile per block, 32-record ranges scattered straight from registers and
-// a device-wide scan); 8 rounds and 3 blocks per SM against 16 and 2: 5.8 ms, 12 and 2: 5.5 ms.
+// Bound by latency beside its DRAM traffic, 20 B per record and pass (key read for the histogram; key
+// and value read and written): a tile waits for its loads, its ranking (votes and a shared counter per
+// round) and six barriers. The next tile is therefore loaded while a ranked one is written out, in the
+// registers that the ranking has left, which wants the 64 of two blocks per SM: map build of the large scene
+// at 1e7 photons (2.8e8 records of 48 bits) 45.2 ms with three blocks and no loads ahead, 43.9 with them in
+// 42 registers, 40.0 with two blocks; 9, 10 and 12 rounds 40.7, 41.5 and 41.4, 32 warps of 8 in one block
+// 41.0, 8 warps of 16 in three 44.1.
 // ------------------------------------------------------------------------------------------
-constexpr int kRsBlocksPerSM = 3;
+constexpr int kRsBlocksPerSM = 2;
 constexpr int kRsWarps = 16, kRsItems = 8, kRsThreads = kRsWarps * 32;
 constexpr int kRsTile = kRsThreads * kRsItems;
 
@@ -216,15 +272,16 @@ static SortPlan sort_plan(uint64_t n) {
     return SortPlan{(uint32_t)((tiles + each - 1) / each), each * kRsTile};
 }
 
+constexpr int kRsHistThreads = 1024;
 template <class K>
-__global__ void __launch_bounds__(kRsThreads) k_rs_hist(const K* __restrict__ keys, uint64_t n, int shift,
+__global__ void __launch_bounds__(kRsHistThreads) k_rs_hist(const K* __restrict__ keys, uint64_t n, int shift,
                                                          uint64_t per, uint32_t* hist) {
     __shared__ uint32_t h[256];
     if (threadIdx.x < 256) h[threadIdx.x] = 0;
     __syncthreads();
     const uint64_t r0 = blockIdx.x * per, r1 = min(r0 + per, n);
     constexpr int V = 16 / sizeof(K);  // keys of one 16-byte load; r0 is a multiple of the tile: aligned
-    for (uint64_t i = r0 + V * threadIdx.x; i < r1; i += V * kRsThreads) {
+    for (uint64_t i = r0 + V * threadIdx.x; i < r1; i += V * kRsHistThreads) {
         if (i + V <= r1) {
             K v[V];
             *reinterpret_cast<uint4*>(v) = *reinterpret_cast<const uint4*>(keys + i);
@@ -264,6 +321,18 @@ __global__ void __launch_bounds__(256) k_rs_scan(uint32_t* hist, uint32_t blocks
         __syncthreads();
     }
     if (threadIdx.x == 0) total[blockIdx.x] = carry;
+}
+
+// Lanes whose d (9 bits) is this lane's, by a vote per bit (Ashkiani et al., "GPU Multisplit", PPoPP 2016).
+ALB_DEVICE unsigned same_digit(uint32_t d) {
+    unsigned peers = 0xffffffffu;
+#pragma unroll
+    for (int b = 0; b < 9; ++b) {
+        const bool on = d >> b & 1u;
+        const unsigned v = __ballot_sync(0xffffffffu, on);
+        peers &= on ? v : ~v;
+    }
+    return peers;
 }
 
 template <class K>
@@ -310,25 +379,28 @@ __global__ void __launch_bounds__(kRsThreads, kRsBlocksPerSM) k_rs_scatter(const
         if (t < 256) s.goff[t] = base + offs[(uint64_t)t * gridDim.x + blockIdx.x];
     }
     const uint64_t r0 = blockIdx.x * per, r1 = min(r0 + per, n);
+    const uint32_t w0 = w * (kRsItems * 32) + l;
+    K key[kRsItems];
+    uint32_t val[kRsItems], rank[kRsItems];
+    auto load = [&](uint64_t t0) {
+#pragma unroll
+        for (int j = 0; j < kRsItems; ++j) {
+            const uint64_t i = t0 + w0 + j * 32;
+            key[j] = i < r1 ? kin[i] : (K)0;
+            if (!FIRST) val[j] = i < r1 ? vin[i] : 0u;
+        }
+    };
+    load(r0);
     for (uint64_t t0 = r0; t0 < r1; t0 += kRsTile) {
         const uint32_t have = (uint32_t)min((uint64_t)kRsTile, r1 - t0);
         for (int i = t; i < kRsWarps * 256; i += kRsThreads) (&s.wcnt[0][0])[i] = 0u;
-        K key[kRsItems];
-        uint32_t val[kRsItems], rank[kRsItems];
-        const uint32_t w0 = w * (kRsItems * 32) + l;
-#pragma unroll
-        for (int j = 0; j < kRsItems; ++j) {
-            const uint32_t i = w0 + j * 32;
-            key[j] = i < have ? kin[t0 + i] : (K)0;
-            if (!FIRST) val[j] = i < have ? vin[t0 + i] : 0u;
-        }
         __syncthreads();
 #pragma unroll
         for (int j = 0; j < kRsItems; ++j) {
             const uint32_t i = w0 + j * 32;
             const bool valid = i < have;
             const uint32_t d = valid ? (uint32_t)(key[j] >> shift) & 255u : 256u;  // lanes past the end match one another
-            const unsigned peers = __match_any_sync(0xffffffffu, d);
+            const unsigned peers = same_digit(d);
             const uint32_t cur = valid ? s.wcnt[w][d] : 0u;
             __syncwarp();
             rank[j] = cur + __popc(peers & lt);
@@ -363,6 +435,7 @@ __global__ void __launch_bounds__(kRsThreads, kRsBlocksPerSM) k_rs_scatter(const
             }
         }
         __syncthreads();
+        load(t0 + kRsTile);  // the next tile comes in while this one is written out
 #pragma unroll 4
         for (uint32_t i = t; i < have; i += kRsThreads) {
             const K k = s.key[i];
@@ -380,7 +453,10 @@ __global__ void __launch_bounds__(kRsThreads) k_keys(const float4* __restrict__ 
                                                       uint64_t per, const unsigned* __restrict__ box, int total,
                                                       K* keys, uint32_t* hist) {
     __shared__ uint32_t h[256];
+    __shared__ HilbertTables tables;
     if (threadIdx.x < 256) h[threadIdx.x] = 0;
+    for (uint32_t i = threadIdx.x; i < 24 * 64; i += kRsThreads) tables.t3[i] = kHilbertTables.t3[i];
+    for (uint32_t i = threadIdx.x; i < 8 * 64; i += kRsThreads) tables.t2[i] = kHilbertTables.t2[i];
     __syncthreads();
     const KeyGrid g = make_key_grid(box, total);
     const uint64_t r0 = blockIdx.x * per, r1 = min(r0 + per, n);
@@ -392,7 +468,7 @@ __global__ void __launch_bounds__(kRsThreads) k_keys(const float4* __restrict__ 
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
             if (i0 + j * kRsThreads < r1) {
-                const K key = cell_key<K>(g, p[j].x, p[j].y, p[j].z);
+                const K key = cell_key<K>(g, tables, p[j].x, p[j].y, p[j].z);
                 keys[i0 + j * kRsThreads] = key;
                 atomicAdd(&h[(uint32_t)key & 255u], 1u);
             }
@@ -426,7 +502,7 @@ static K* hilbert_sort(Workspace& ws, const float4* a, uint64_t stride, uint64_t
     uint32_t* vout = passes % 2 ? order : other;
     for (int i = 0; i < passes; ++i) {
         if (i == 0) k_keys<K><<<p.blocks, kRsThreads, 0, st>>>(a, stride, n, p.per, box, bits, k0, hist);
-        else k_rs_hist<K><<<p.blocks, kRsThreads, 0, st>>>(k0, n, 8 * i, p.per, hist);
+        else k_rs_hist<K><<<p.blocks, kRsHistThreads, 0, st>>>(k0, n, 8 * i, p.per, hist);
         k_rs_scan<<<256, 256, 0, st>>>(hist, p.blocks, total);
         if (i == 0)
             k_rs_scatter<K, true><<<p.blocks, kRsThreads, sizeof(SortSmem<K>), st>>>(k0, vin, k1, vout, n, 0, p.per, hist, total);
