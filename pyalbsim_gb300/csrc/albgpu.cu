@@ -900,6 +900,11 @@ static int gather_all(AlbCtx* ctx, const Accum& acc, bool lo_zero) {
         ps.stop();
         if (rc != 0) return fail(ctx, ALB_ERR_CUDA, "query sort: device memory allocation failed");
     }
+    // each channel's work items of a fixed-radius gather (8 MB each; without them a query is one warp's)
+    uint32_t* work = nullptr;
+    const size_t mark = ctx->ws.mark();
+    const uint64_t words = 2 + 2 * (uint64_t)kRadiusItems;
+    if (ctx->sc.radius > 0.0 && !(work = ctx->ws.take_u32(4 * words))) ctx->ws.clear_failed();
     // Few queries leave most of the chip idle in one gather: the planar ones run beside one another on
     // streams forked here and joined below (the Jacobian and the heatmaps sum through words
     // that the channels share, so those runs stay in series). A backward call on the
@@ -934,6 +939,7 @@ static int gather_all(AlbCtx* ctx, const Accum& acc, bool lo_zero) {
         q.inexact = ctx->d_stats + 24 + c;
         q.retries = ctx->d_stats + 30;
         q.ticket = (uint32_t*)(ctx->ctl + 43 + c);
+        q.work = work ? work + c * words : nullptr;
         const bool aside = fork && c != ALB_SCATTER;
         cudaStream_t st = ctx->st;
         if (aside) {
@@ -951,6 +957,7 @@ static int gather_all(AlbCtx* ctx, const Accum& acc, bool lo_zero) {
         ctx->gathered[c] += (int64_t)nq;
     }
     for (int i = 0; i < side; ++i) CK(cudaStreamWaitEvent(ctx->st, ctx->join[i], 0));
+    ctx->ws.release(mark);
     return rc;
 }
 

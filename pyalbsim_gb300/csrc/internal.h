@@ -72,6 +72,7 @@ struct MapDev {
 };
 
 // Device view of one kind of gather queries.
+constexpr uint32_t kRadiusItems = 1u << 20;
 struct QueryDev {
     const float4* a;   // x_hi, y_hi, z_hi, energy
     const float4* b;   // dx, dy, dz, time
@@ -85,6 +86,7 @@ struct QueryDev {
     unsigned long long* inexact;  // optional count of answers a buffer bound made inexact (mass ties)
     uint32_t* ticket;  // work counter of the scatter gather
     unsigned long long* retries;  // optional count of searches redone because a first guess did not hold
+    uint32_t* work;  // fixed radius: a counter and room for kRadiusItems work items from word 2 (nullable)
 };
 
 // Waveform / heatmap accumulators (128-bit fixed point, lo and hi words).

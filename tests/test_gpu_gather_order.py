@@ -163,3 +163,23 @@ def test_planar_searches_by_runs_equal_single_ones(gpu_available, k, adjoint):
     if adjoint:
         assert np.abs(ja).sum() > 0
         np.testing.assert_array_equal(ja, jb)
+
+
+def test_radius_work_items_on_both_sides_of_their_room(gpu_available):
+    """A radius that holds the whole map: 700 photons want more work items (a query's boxes of 32 leaves)
+    than the 2^20 there is room for, and the rest is searched in place; half of the photons at a
+    time want fewer. The same photons, bit for bit."""
+    cfg = workloads.small(0.9, radius=2_000.0)
+
+    def run(cuts):
+        with GpuEngine(cfg, GpuRunOptions()) as eng:
+            eng.forward(100_000, 5)
+            eng.build_maps()
+            assert eng.ctx.map_size(1) > 380 * 1024
+            for a, b in zip(cuts, cuts[1:]):
+                eng.backward(b - a, 5)
+            return eng.waveform_array(f64=True)
+
+    a, b = run([0, 700]), run([0, 350, 700])
+    assert np.abs(a).sum() > 0
+    np.testing.assert_array_equal(a, b)
