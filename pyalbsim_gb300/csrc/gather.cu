@@ -1444,21 +1444,24 @@ __device__ __noinline__ bool cold_knn(const MapDev& m, S& s, int k, float fx, fl
 // not fit, up to this many.
 constexpr int kAlone = 64;
 
-// Scatter-map gather, k nearest, by runs of neighbouring queries (gather_group.cuh). One CTA per SM.
+// Gather of the k nearest by runs of neighbouring queries (gather_group.cuh). One CTA per SM.
 // The sorted queries are cut into segments that CTAs take in turn: the first half of them in
-// four per CTA, half of the rest in four per CTA, and so on (ScatterPlan), since the work of a
+// a few per CTA, half of the rest in as many, and so on (ScatterPlan), since the work of a
 // range varies with the density of the map around it: with one range per SM the slowest of 152 SMs
-// issued 19% more than the mean, 27.5 against 22.9 ms at 1e6 photons of the large scene. (Two
-// segments per CTA and level: 22.9 ms, 237 at 1e7 photons; four: 23.1, 234; eight: 23.5, 230.)
-// A segment is 64 chunks; the CTA's warps fetch chunks in turn.
+// issued 19% more than the mean, 27.5 against 22.9 ms at 1e6 photons of the large scene. A segment is
+// 16 to 64 chunks; the CTA's warps fetch chunks in turn. Two segments per CTA and level below 2^24 queries,
+// four above: scatter gather of 6.2e5 queries (default scene) 3.7 and 3.9 ms, 1.7e6 (a scene of the
+// sweep) 5.0 and 5.3, 8.7e6 22.1 and 22.3, 8.7e7 229 and 225.
 struct ScatterPlan {
     uint64_t first, n;  // the launch's range of the sorted queries
     uint32_t pieces;    // segments per level
     int levels;         // level L holds half of what the levels before it left, the last one the rest
+    int chunk_bits;     // a segment is 2^chunk_bits chunks
     bool cached;        // class words go through the CTA's cache, where it has one
     uint32_t* ticket;   // segments taken, zero at the launch
 };
-constexpr int kSegChunks = 64;
+constexpr uint64_t kManyQueries = 1ull << 24;
+constexpr int kSegBits = 6;  // 64 chunks in a segment, fewer for few queries
 constexpr int kSegRing = 64;  // segments of a CTA whose numbers are kept
 
 ALB_DEVICE void segment_range(const ScatterPlan& p, uint32_t g, uint64_t& s0, uint64_t& s1) {
@@ -1499,7 +1502,7 @@ __global__ void __launch_bounds__(WARPS * 32, 1)
     __syncthreads();
     const int w = threadIdx.x >> 5, l = lane_id();
     S& s = smem[w];
-    const uint32_t segments = plan.pieces * (uint32_t)plan.levels;
+    const uint32_t segments = plan.pieces * (uint32_t)plan.levels, chunks = 1u << plan.chunk_bits;
     const float side_rk = G::side((float)k);
     bool failed = false;
     if (l < 5) s.st[l] = 0ull;
@@ -1512,21 +1515,21 @@ __global__ void __launch_bounds__(WARPS * 32, 1)
         uint32_t t = 0u, g = 0u;
         if (l == 0) {
             t = atomicAdd(&next, 1u);
-            const uint32_t seg = t / kSegChunks;
+            const uint32_t seg = t >> plan.chunk_bits;
             volatile unsigned long long* v = ring;
-            if (t % kSegChunks == 0) v[(seg + 1) % kSegRing] = (unsigned long long)(seg + 1) << 32 | atomicAdd(plan.ticket, 1u);
+            if ((t & (chunks - 1u)) == 0u) v[(seg + 1) % kSegRing] = (unsigned long long)(seg + 1) << 32 | atomicAdd(plan.ticket, 1u);
             // published 64 chunks ago; the bound only guards against a lost slot
             unsigned long long e = v[seg % kSegRing];
             for (int wait = 0; (uint32_t)(e >> 32) != seg && wait < (1 << 20); ++wait) e = v[seg % kSegRing];
             if ((uint32_t)(e >> 32) != seg) atomicCAS(err, 0, ALB_ERR_ITER_CAP);
             g = (uint32_t)(e >> 32) == seg ? (uint32_t)e : 0xffffffffu;
         }
-        t = __shfl_sync(0xffffffffu, t, 0) % kSegChunks;
+        t = __shfl_sync(0xffffffffu, t, 0) & (chunks - 1u);
         g = __shfl_sync(0xffffffffu, g, 0);
         if (g >= segments) break;
         uint64_t s0, s1;
         segment_range(plan, g, s0, s1);
-        const uint64_t c0 = s0 + (s1 - s0) * t / kSegChunks, q_end = s0 + (s1 - s0) * (t + 1) / kSegChunks;
+        const uint64_t c0 = s0 + ((s1 - s0) * t >> plan.chunk_bits), q_end = s0 + ((s1 - s0) * (t + 1) >> plan.chunk_bits);
         if (c0 == q_end) continue;
         QueryRun run{0, 0, 0, 0.f};
         uint64_t r_base = 0;  // first query of the run the lanes hold
@@ -1892,14 +1895,13 @@ static void launch_runs(const SceneDev& sc, const MapDev& map, const QueryDev& q
     // a class word holds kClassMost contributions: more queries go in slices
     const uint64_t most = kClassMost / (uint64_t)k;
     for (uint64_t first = 0; first < q.n; first += most) {
-        ScatterPlan plan{first, std::min<uint64_t>(most, q.n - first), 0u, 1, acc.nbins < kCachedBins, q.ticket};
+        ScatterPlan plan{first, std::min<uint64_t>(most, q.n - first), 0u, 1, kSegBits, acc.nbins < kCachedBins, q.ticket};
         const uint64_t blocks = std::min<uint64_t>(sm_count(), plan.n);
         using G = std::conditional_t<CHANNEL == ALB_SCATTER, VolumeRuns, PlaneRuns>;
-        uint64_t per = 4;
-        while (per > 1 && plan.n < per * blocks * kSegChunks * G::kChunk) --per;
-        plan.pieces = (uint32_t)(per * blocks);
-        // levels until a segment's chunks hold kChunk queries
-        while (plan.levels < 16 && (plan.n >> plan.levels) >= (uint64_t)plan.pieces * kSegChunks * G::kChunk) ++plan.levels;
+        plan.pieces = (uint32_t)((plan.n < kManyQueries ? 2 : 4) * blocks);
+        // fewer chunks, or more levels, until a segment's chunks hold kChunk queries
+        while (plan.chunk_bits > 4 && plan.n < (uint64_t)plan.pieces * G::kChunk << plan.chunk_bits) --plan.chunk_bits;
+        while (plan.levels < 16 && (plan.n >> plan.levels) >= (uint64_t)plan.pieces * G::kChunk << plan.chunk_bits) ++plan.levels;
         cudaMemsetAsync(q.ticket, 0, sizeof(uint32_t), st);
         kernel<<<(unsigned)blocks, WARPS * 32, bytes, st>>>(sc, map, q, acc, k, err, plan);
         note_launch();
