@@ -98,7 +98,7 @@ void* dev_alloc(uint64_t bytes, cudaStream_t st) {
     const cudaMemPool_t pool = device_pool();
     if (!pool) return nullptr;
     if (bytes == 0) bytes = 16;
-    for (int attempt = 0; attempt < 2; ++attempt) {
+    for (int attempt = 0; attempt < 3; ++attempt) {
         void* p = nullptr;
         if (bytes > kDirect) {
             if (cudaMalloc(&p, bytes) == cudaSuccess) {
@@ -108,10 +108,10 @@ void* dev_alloc(uint64_t bytes, cudaStream_t st) {
             }
         } else if (cudaMallocFromPoolAsync(&p, bytes, pool, st) == cudaSuccess) return p;
         cudaGetLastError();
-        if (attempt == 0) {  // once more with every idle block given back to the driver
-            cudaStreamSynchronize(st);
-            cudaMemPoolTrimTo(pool, 0);
-        }
+        // again with every idle block given back to the driver: this stream's, then every stream's
+        if (attempt == 0) cudaStreamSynchronize(st);
+        else if (attempt == 1) cudaDeviceSynchronize();
+        if (attempt < 2) cudaMemPoolTrimTo(pool, 0);
     }
     return nullptr;
 }
@@ -764,8 +764,8 @@ static int ensure_records(AlbCtx* ctx, int c, uint64_t need, uint64_t keep) {
     bool want_id = ctx->keep_ids != 0;
     bool want_sco = ctx->sc.adjoint != 0;
     if (r.cap >= need && (!want_id || r.id) && (!want_hm || r.fwi) && (!want_sco || r.sco)) return ALB_OK;
-    // small stores double, so that a pass of many batches does not copy its records for each
-    uint64_t cap = std::max<uint64_t>(need + (keep ? std::max<uint64_t>(need / 16, std::min<uint64_t>(need, 1ull << 24)) : need / 16), 1024);
+    // small stores double (up to 32 MB), so that a pass of many batches does not copy its records for each
+    uint64_t cap = std::max<uint64_t>(need + (keep ? std::max<uint64_t>(need / 16, std::min<uint64_t>(need, 1ull << 20)) : need / 16), 1024);
     if (!keep) release_records(ctx, c);  // nothing to copy: the peak is one store
     float4 *a = nullptr, *fwi = nullptr, *sfi = nullptr, *sco = nullptr;
     uint32_t* id = nullptr;
