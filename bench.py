@@ -33,12 +33,12 @@ METRIC = "photons/s & waveform-grads/s on 1 GB300: batched+adjoint vs plain @≤
 UNIT = "photons/s"
 ALG_BYTES_PER_GATHER = 16 + 100 * 32  # query record + k neighbour records (pos 12, dir 12, E 4, t 4)
 # DRAM bytes per scatter-map query measured by ncu on the same kernel (dram__bytes_read.sum +
-# dram__bytes_write.sum of one k_gather<1, 0> launch / its queries; 1e6-photon case of this scene)
-DRAM_BYTES_PER_SCATTER_QUERY = 893
+# dram__bytes_write.sum of one k_gather_runs<1, 0> launch / its queries; 1e6-photon case of this scene)
+DRAM_BYTES_PER_SCATTER_QUERY = 1015
 # Warp instructions per scatter-map query of the same capture (smsp__inst_executed.sum of one
-# k_gather<1, 0> launch / its queries): the kernel is bound by instruction issue, so its issue
+# k_gather_runs<1, 0> launch / its queries): the kernel is bound by instruction issue, so its issue
 # rate is reported beside the HBM convention
-INST_PER_SCATTER_QUERY = 4615
+INST_PER_SCATTER_QUERY = 2312
 
 
 def workload_config(name: str):
@@ -369,7 +369,7 @@ def main():
     ms_step = ms / args.steps
     value = aggregate_rate(nf + nb, world, ms_step)
 
-    # roofline of the dominant kernel, the scatter-map gather k_gather<1, 0>: HBM-bound by the
+    # roofline of the dominant kernel, the scatter-map gather k_gather_runs<1, 0>: HBM-bound by the
     # algorithmic convention (3216 B per query), timed with CUDA events around its launches
     n_gathers = int(gathers.sum())
     sc_ms, sc_calls = phases["gather_scatter"]
@@ -388,7 +388,7 @@ def main():
         "gathers_per_step": int(n_gathers / args.steps),
         "gathers_per_s": world * (n_gathers / args.steps) / (ms_step / 1e3),
         "dominant_phase": top,
-        "roofline": {"bound": "hbm", "kernel": "k_gather<1, 0> (scatter map, k-NN)", "achieved": achieved, "peak": peak,
+        "roofline": {"bound": "hbm", "kernel": "k_gather_runs<1, 0> (scatter map, k-NN)", "achieved": achieved, "peak": peak,
                      "unit": "GB/s", "frac": achieved / peak if peak else None,
                      "traffic": DRAM_BYTES_PER_SCATTER_QUERY * q_per_launch,
                      "algorithmic_bytes_per_launch": ALG_BYTES_PER_GATHER * q_per_launch,
@@ -448,7 +448,7 @@ def gather_issue_roofline(queries, ms, sms_mhz=None):
     sms, mhz = sms_mhz if sms_mhz is not None else sm_count_and_clock()
     peak = sms * 4 * mhz * 1e6
     achieved = INST_PER_SCATTER_QUERY * queries / (ms / 1e3) if ms > 0 else 0.0
-    return {"bound": "issue", "kernel": "k_gather<1, 0> (scatter map, k-NN)", "achieved": achieved, "peak": peak,
+    return {"bound": "issue", "kernel": "k_gather_runs<1, 0> (scatter map, k-NN)", "achieved": achieved, "peak": peak,
             "unit": "warp instructions/s", "frac": achieved / peak if peak else None,
             "instructions_per_query": INST_PER_SCATTER_QUERY,
             "source": "instructions per query from the ncu capture of a 1e6-photon launch; peak derived: "
