@@ -594,6 +594,10 @@ static std::string set_scene(AlbCtx* ctx, const AlbSceneParams* p) {
     return std::string();
 }
 
+// Sets of class words for the waveform: one per channel, so that gathers may run side by side, or one for
+// all of them where a set is large (128 B per bin).
+static int64_t class_sets(int64_t nbins) { return nbins <= (1 << 20) ? ALB_CHANNELS : 1; }
+
 // Waveform, Jacobian and heatmap accumulators sized for the current scene (grown, never
 // shrunk; a grown buffer is zeroed by the next reset).
 static std::string ensure_accumulators(AlbCtx* ctx) {
@@ -610,7 +614,7 @@ static std::string ensure_accumulators(AlbCtx* ctx) {
         return true;
     };
     if (!regrow(ctx->wf, ctx->wf_bins, s.nbins, (size_t)2 * ALB_CHANNELS) ||
-        !regrow(ctx->cls, ctx->cls_bins, s.nbins, (size_t)16 * ALB_CHANNELS))
+        !regrow(ctx->cls, ctx->cls_bins, s.nbins * class_sets(s.nbins), 16))
         return "waveform allocation failed";
     if (s.adjoint && (!regrow(ctx->jac, ctx->jac_bins, s.nbins, (size_t)2 * kJacParams * ALB_CHANNELS) ||
                       !regrow(ctx->jac_cls, ctx->jac_cls_bins, s.nbins, (size_t)16 * kJacParams)))
@@ -909,7 +913,7 @@ static int gather_all(AlbCtx* ctx, const Accum& acc, bool lo_zero) {
     // streams forked here and joined below (the Jacobian and the heatmaps sum through words
     // that the channels share, so those runs stay in series). A backward call on the
     // 5 m water scene's maps of 1e5 photons: 1.2 -> 0.9 ms with 5000 photons, 2.0 -> 1.6 ms with 25,000.
-    const bool fork = total < (1ull << 20) && !acc.jac_lo && !acc.hw_lo;
+    const bool fork = total < (1ull << 20) && !acc.jac_lo && !acc.hw_lo && acc.cls_step;
     if (fork) {
         if (!ctx->fork) {
             CK(cudaEventCreateWithFlags(&ctx->fork, cudaEventDisableTiming));
@@ -1018,6 +1022,14 @@ extern "C" int alb_trace(AlbCtx* ctx, int pass, uint64_t n, uint64_t seed, uint6
                     if (ctx->map_cap_hint > 0) est = std::max<uint64_t>(est, (uint64_t)ctx->map_cap_hint);
                     int rc = ctx->rec_released[c] ? restore_records(ctx, c, before[c] + est)
                                                    : ensure_records(ctx, c, before[c] + est, before[c]);
+                    if (rc && !ctx->rec_rate_known && attempt == 0 && ctx->rec_rate[ALB_SCATTER] == kManyRecords) {
+                        // no room for so many: as few as a retry can correct
+                        ctx->rec_rate[ALB_BOTTOM_REFLECTION] = 2.0;
+                        ctx->rec_rate[ALB_SCATTER] = 8.0;
+                        ctx->err.clear();
+                        c = -1;
+                        continue;
+                    }
                     if (rc) return rc;
                 }
                 TraceOut o = make_out(ctx);
@@ -1068,6 +1080,7 @@ extern "C" int alb_trace(AlbCtx* ctx, int pass, uint64_t n, uint64_t seed, uint6
     acc.wf_lo = ctx->wf;
     acc.wf_hi = ctx->wf + (size_t)ALB_CHANNELS * ctx->sc.nbins;
     acc.cls = ctx->cls;
+    acc.cls_step = class_sets(ctx->sc.nbins) > 1 ? (uint64_t)16 * ctx->sc.nbins : 0;
     acc.nbins = ctx->sc.nbins;
     if (ctx->sc.adjoint) {
         acc.jac_lo = ctx->jac;

@@ -1363,7 +1363,7 @@ ALB_DEVICE void accumulate_run(const SceneDev& sc, const MapDev& m, const QueryD
     if (CHANNEL == ALB_SURFACE_TRANSMISSION_UP) w = sc.surface_lambert;
     const int gate = (int)sc.gate_lo;
     const uint32_t nbins = (uint32_t)acc.nbins;
-    unsigned long long* cls = acc.cls + (uint64_t)CHANNEL * kClasses * nbins;
+    unsigned long long* cls = acc.cls;
     unsigned long long* wf_lo = acc.wf_lo + (uint64_t)CHANNEL * acc.nbins;
     unsigned long long* wf_hi = acc.wf_hi + (uint64_t)CHANNEL * acc.nbins;
     float4 sq = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -1644,7 +1644,7 @@ __global__ void __launch_bounds__(WARPS * 32, 1)
     }
     if constexpr (SLOTS != 0) {
         __syncthreads();
-        cache_flush(cache, acc.cls + (uint64_t)CHANNEL * kClasses * acc.nbins, kClasses * (uint32_t)acc.nbins,
+        cache_flush(cache, acc.cls, kClasses * (uint32_t)acc.nbins,
                     MODE == kModeKnnAdjoint ? acc.jac_cls : acc.heat_cls);
     }
 }
@@ -1860,7 +1860,7 @@ static void merge_classes(const SceneDev& sc, const Accum& acc, int channel, boo
     const uint32_t nb = (uint32_t)acc.nbins;
     const unsigned blocks = (nb + 255u) / 256u;
     if (waveform) {
-        k_merge_classes<<<blocks, 256, 0, st>>>(acc.cls + (uint64_t)channel * kClasses * nb, nb, acc.wf_lo + (uint64_t)channel * nb,
+        k_merge_classes<<<blocks, 256, 0, st>>>(acc.cls, nb, acc.wf_lo + (uint64_t)channel * nb,
                                                 acc.wf_hi + (uint64_t)channel * nb, 0, 0);
         note_launch();
     }
@@ -1986,6 +1986,7 @@ void launch_gather(const SceneDev& sc, const MapDev& map, const QueryDev& q, int
     if (q.n == 0) return;
     int k = sc.k;
     Accum acc = accum;
+    acc.cls += (uint64_t)channel * acc.cls_step;
     // contributions of the launch at most (a fixed radius admits any number of the map's records);
     // the gathers by runs keep below kClassMost by slices
     const uint64_t per = sc.radius > 0.0 ? std::max<uint64_t>(map.n, 1) : (uint64_t)k;

@@ -99,7 +99,8 @@ struct Accum {
     unsigned long long* hf_hi;
     int64_t nbins;
     // sums of one gather by exponent class, [16][cells], all zero between gathers (gather.cu, class_add)
-    unsigned long long* cls;       // waveform
+    unsigned long long* cls;       // waveform: the gather's channel, or the first of them
+    uint64_t cls_step;             // from one channel's words to the next one's, 0: the channels share them
     unsigned long long* jac_cls;   // Jacobian, one set per parameter (nullable)
     unsigned long long* heat_cls;  // water, then seafloor heatmap (nullable)
     unsigned long long* jac_lo;  // adjoint [5 params][channels][nbins] (nullable)

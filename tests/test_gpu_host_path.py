@@ -2,6 +2,8 @@
 another, and device memory kept between contexts change no value. A waveform is a sum of integers, so
 the same photons give the same bits however the calls divide them."""
 
+import dataclasses
+
 import numpy as np
 import pytest
 
@@ -44,3 +46,25 @@ def test_trim_refuses_an_unknown_device(gpu_available):
     with GpuEngine(workloads.small(), GpuRunOptions()) as eng:
         assert eng.ctx.lib.alb_trim_memory(4096) != 0
         eng.forward(100, 1)  # the device in use is unchanged
+
+
+def test_shared_class_words_of_a_long_timeline(gpu_available):
+    """More than 2^20 bins: the channels share one set of class words and gather in series. A window of the
+    timeline has few bins, one set per channel and gathers side by side: the same bits in it."""
+    cfg = workloads.small()
+    cfg = dataclasses.replace(cfg, sensor=dataclasses.replace(cfg.sensor, sample_rate=32 * cfg.sensor.sample_rate))
+
+    def run(c):
+        with GpuEngine(c, GpuRunOptions()) as eng:
+            eng.forward(5_000, 5)
+            eng.build_maps()
+            eng.backward(1_500, 5)
+            return eng.waveform_array(f64=True)
+
+    full = run(cfg)
+    assert full.shape[-1] > 1 << 20
+    hit = np.flatnonzero(full.any(axis=0))
+    start, bins = int(hit[0]), int(min(hit[-1] - hit[0] + 1, 1 << 19))
+    part = run(dataclasses.replace(cfg, waveform_gate=(start, bins)))
+    assert part.shape[-1] == bins and np.abs(part).sum() > 0
+    np.testing.assert_array_equal(part, full[:, start:start + bins])
