@@ -8,9 +8,11 @@ import numpy as np
 import pytest
 
 from pyalbsim_gb300 import workloads
+from pyalbsim_gb300.batch import surface_gate
 from pyalbsim_gb300.config import SimulationConfig
 from pyalbsim_gb300.config.gpu import GpuRunOptions
 from pyalbsim_gb300.engine import GpuEngine
+from pyalbsim_gb300.scene import build_scene
 
 pytestmark = pytest.mark.gpu
 
@@ -63,8 +65,7 @@ def test_shared_class_words_of_a_long_timeline(gpu_available):
 
     full = run(cfg)
     assert full.shape[-1] > 1 << 20
-    hit = np.flatnonzero(full.any(axis=0))
-    start, bins = int(hit[0]), int(min(hit[-1] - hit[0] + 1, 1 << 19))
-    part = run(dataclasses.replace(cfg, waveform_gate=(start, bins)))
-    assert part.shape[-1] == bins and np.abs(part).sum() > 0
-    np.testing.assert_array_equal(part, full[:, start:start + bins])
+    gated = dataclasses.replace(cfg, waveform_gate=surface_gate(cfg, length=100e-9))
+    part, first = run(gated), build_scene(gated).gate_start
+    assert part.shape[-1] < 1 << 20 and np.abs(part).sum() > 0
+    np.testing.assert_array_equal(part, full[:, first:first + part.shape[-1]])
