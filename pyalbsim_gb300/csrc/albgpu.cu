@@ -36,6 +36,10 @@ long long launches_total() { return g_launches.load(); }
 // fail otherwise (measured: 160 GB beside 160 GB idle in the pool). Blocks over kDirect are cudaMalloc's: a pool
 // maps 16 GB in 13 ms, cudaMalloc in 1 ms, and so large a block would not be kept anyway.
 constexpr uint64_t kDirect = 16ull << 30;
+// In a batch's worker threads: blocks over 1 GB. Workers fill the device with instances of many sizes, and
+// a pool's blocks of one size do not serve the next (2 of 128 instances of the sweep ran out of memory).
+constexpr uint64_t kDirectBatch = 1ull << 30;
+static thread_local uint64_t t_direct = kDirect;
 
 static std::mutex g_direct_mu;
 static std::unordered_set<void*> g_direct;
@@ -100,7 +104,7 @@ void* dev_alloc(uint64_t bytes, cudaStream_t st) {
     if (bytes == 0) bytes = 16;
     for (int attempt = 0; attempt < 3; ++attempt) {
         void* p = nullptr;
-        if (bytes > kDirect) {
+        if (bytes > t_direct) {
             if (cudaMalloc(&p, bytes) == cudaSuccess) {
                 std::lock_guard<std::mutex> g(g_direct_mu);
                 g_direct.insert(p);
@@ -1614,6 +1618,7 @@ extern "C" int alb_batch_run(AlbBatchInstance* inst, uint64_t n, const AlbBatchO
     };
     auto worker = [&]() {
         cudaSetDevice(opt->device);
+        t_direct = kDirectBatch;
         double held = 0.0;
         cudaStream_t st = nullptr;
         if (cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking) != cudaSuccess) st = nullptr;
