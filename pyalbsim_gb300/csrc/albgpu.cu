@@ -717,6 +717,7 @@ extern "C" void alb_destroy(AlbCtx* ctx) {
 
 extern "C" int alb_set_option(AlbCtx* ctx, int key, int64_t v) {
     if (!ctx) return ALB_ERR_INVALID;
+    CK(cudaSetDevice(ctx->device));
     switch (key) {
         case ALB_OPT_KEEP_EXIT_STATES: ctx->keep_exit = (int)v; break;
         case ALB_OPT_KEEP_RECORD_IDS: ctx->keep_ids = (int)v; break;
@@ -1290,6 +1291,7 @@ extern "C" int alb_get_heatmaps(AlbCtx* ctx, double* water, double* seafloor, fl
 // n 128-bit words of an accumulator to the host as float64 or float32, converted on the device.
 template <class T>
 static int read_fixed(AlbCtx* ctx, const unsigned long long* lo, const unsigned long long* hi, int64_t n, T* out) {
+    CK(cudaSetDevice(ctx->device));
     const size_t mark = ctx->ws.mark();
     T* d = (T*)ctx->ws.take_bytes((size_t)n * sizeof(T));
     if (!d) return fail(ctx, ALB_ERR_CUDA, "read-back buffer: out of device memory");
@@ -1364,6 +1366,7 @@ extern "C" int alb_export_map_scores(AlbCtx* ctx, int c, float* scores, size_t n
 
 extern "C" int alb_reset_waveform(AlbCtx* ctx) {
     if (!ctx) return ALB_ERR_INVALID;
+    CK(cudaSetDevice(ctx->device));
     CK(cudaMemsetAsync(ctx->wf, 0, (size_t)2 * ALB_CHANNELS * ctx->sc.nbins * 8, ctx->st));
     if (ctx->hm) CK(cudaMemsetAsync(ctx->hm, 0, (size_t)4 * ctx->sc.hm_bins * ctx->sc.hm_bins * 8, ctx->st));
     if (ctx->jac)
