@@ -235,7 +235,7 @@ struct AlbCtx {
     // accumulators
     unsigned long long* wf = nullptr;  // lo words then hi words, [2][channels][nbins]
     unsigned long long* hm = nullptr;  // sampled heatmaps, [2 maps][2 words][bins*bins]
-    unsigned *hm_radius = nullptr, *hm_radius_bak = nullptr;
+    unsigned *hm_radius = nullptr, *hm_radius_bak = nullptr;  // the copies: before the call, before its second part
     // adjoint Jacobian: lo words then hi words, [2][kJacParams][channels][nbins]
     unsigned long long* jac = nullptr;
     // sums of one gather by exponent class (every gather leaves them zero)
@@ -632,7 +632,7 @@ static std::string ensure_accumulators(AlbCtx* ctx) {
             drop(ctx->hm_radius, ctx->st);
             drop(ctx->hm_radius_bak, ctx->st);
             ctx->hm_radius_cells = 0;
-            if (!take(ctx->hm_radius, hb * 4, ctx->st) || !take(ctx->hm_radius_bak, hb * 4, ctx->st))
+            if (!take(ctx->hm_radius, hb * 4, ctx->st) || !take(ctx->hm_radius_bak, 2 * hb * 4, ctx->st))
                 return "heatmap allocation failed";
             cudaMemsetAsync(ctx->hm_radius, 0, hb * 4, ctx->st);
             ctx->hm_radius_cells = hb;
@@ -1015,12 +1015,15 @@ extern "C" int alb_trace(AlbCtx* ctx, int pass, uint64_t n, uint64_t seed, uint6
     if (pass == ALB_FORWARD) {
         ctx->maps_built = false;
         const size_t hb = ctx->sc.heatmap ? (size_t)ctx->sc.hm_bins * ctx->sc.hm_bins : 0;
+        uint64_t before_call[ALB_CHANNELS];
+        std::memcpy(before_call, ctx->h_rec_count, sizeof before_call);
         // photons [p0, p0 + pn) of the call
         auto part = [&](uint64_t p0, uint64_t pn) -> int {
+            unsigned* const radius_bak = ctx->hm_radius_bak + (p0 ? hb : 0);
             uint64_t before[ALB_CHANNELS];
             std::memcpy(before, ctx->h_rec_count, sizeof before);
             CK(cudaMemcpyAsync(stats_bak, ctx->d_stats, 2 * 8, cudaMemcpyDeviceToDevice, ctx->st));
-            if (hb) CK(cudaMemcpyAsync(ctx->hm_radius_bak, ctx->hm_radius, hb * 4, cudaMemcpyDeviceToDevice, ctx->st));
+            if (hb) CK(cudaMemcpyAsync(radius_bak, ctx->hm_radius, hb * 4, cudaMemcpyDeviceToDevice, ctx->st));
             for (int attempt = 0; attempt < 3; ++attempt) {
                 for (int c = 0; c < ALB_CHANNELS; ++c) {
                     uint64_t est = (uint64_t)(ctx->rec_rate[c] * (double)pn * 1.03) + 4096;
@@ -1062,7 +1065,7 @@ extern "C" int alb_trace(AlbCtx* ctx, int pass, uint64_t n, uint64_t seed, uint6
                 // undo and retry with the measured sizes
                 CK(cudaMemcpyAsync(ctx->d_stats, stats_bak, 2 * 8, cudaMemcpyDeviceToDevice, ctx->st));
                 CK(cudaMemcpyAsync(ctx->d_rec_count, before, sizeof before, cudaMemcpyHostToDevice, ctx->st));
-                if (hb) CK(cudaMemcpyAsync(ctx->hm_radius, ctx->hm_radius_bak, hb * 4, cudaMemcpyDeviceToDevice, ctx->st));
+                if (hb) CK(cudaMemcpyAsync(ctx->hm_radius, radius_bak, hb * 4, cudaMemcpyDeviceToDevice, ctx->st));
                 CK(cudaStreamSynchronize(ctx->st));
                 for (int c = 0; c < ALB_CHANNELS; ++c) ctx->rec_rate[c] = (double)(cnt[c] - before[c]) / (double)pn;
             }
@@ -1074,7 +1077,16 @@ extern "C" int alb_trace(AlbCtx* ctx, int pass, uint64_t n, uint64_t seed, uint6
             ctx->rec_rate[ALB_SCATTER] = kManyRecords;
         }
         int rc = pilot ? part(0, pilot) : ALB_OK;
-        if (!rc) rc = part(pilot, n - pilot);
+        if (!rc) {
+            rc = part(pilot, n - pilot);
+            if (rc && pilot) {
+                // the call as a whole leaves nothing: the pilot's records and crossings go too
+                std::memcpy(ctx->h_rec_count, before_call, sizeof before_call);
+                cudaMemcpyAsync(ctx->d_rec_count, before_call, sizeof before_call, cudaMemcpyHostToDevice, ctx->st);
+                if (hb) cudaMemcpyAsync(ctx->hm_radius, ctx->hm_radius_bak, hb * 4, cudaMemcpyDeviceToDevice, ctx->st);
+                cudaStreamSynchronize(ctx->st);
+            }
+        }
         ctx->ws.release(mark);
         return rc;
     }

@@ -8,6 +8,7 @@ import pytest
 
 import fake_cuda
 from pyalbsim_gb300 import workloads
+from pyalbsim_gb300.config import SimulationConfig
 from pyalbsim_gb300._native import ALB_OPT_ADJOINT, NativeContext, scene_struct
 from pyalbsim_gb300.scene import build_scene
 
@@ -56,3 +57,33 @@ def test_calls_use_the_context_s_device_whatever_is_current(lib):
             call(ctx[d])
             assert not fake_cuda.violations(lib)
     assert lib.fake_used(0) == 0 and lib.fake_used(1) == 0
+
+
+def _rates(lib, records, queries=(1.0, 8.0, 1.0)):
+    lib.fake_rates(np.array(records, np.float64).ctypes.data, np.array(queries, np.float64).ctypes.data)
+
+
+@pytest.mark.parametrize("first", [False, True])
+def test_a_forward_call_out_of_memory_leaves_the_simulation_as_it_was(lib, first):
+    """A large first call measures its record rates on its first photons, then has no room for the rest: the
+    records and the radius heatmap are those from before the call, so that it can be made again."""
+    _rates(lib, [1.0, 90.0, 1.0, 1.0])
+    ctx = Context(lib, build_scene(SimulationConfig()))
+    if first:  # records of an earlier call (too few photons to measure rates)
+        ctx.trace(True, 500)
+    sizes = [ctx.map_size(c) for c in range(4)]
+    radius = ctx.heatmaps()[2]
+    n = 400_000
+    lib.fake_limit(0, lib.fake_used(0) + (1 << 30))  # the pilot's records take 0.1 GB, the rest 2.4
+    with pytest.raises(RuntimeError, match="out of device memory"):
+        ctx.trace(True, n)
+    traced = lib.fake_traced()
+    assert 0 < traced < n  # the pilot ran
+    assert [ctx.map_size(c) for c in range(4)] == sizes
+    np.testing.assert_array_equal(ctx.heatmaps()[2], radius)
+    lib.fake_limit(0, 1 << 40)
+    ctx.trace(True, n)
+    assert [ctx.map_size(c) - s for c, s in enumerate(sizes)] == [n, 90 * n, n, n]
+    assert ctx.heatmaps()[2][0] - radius[0] == n
+    ctx.close()
+    assert not fake_cuda.violations(lib)
