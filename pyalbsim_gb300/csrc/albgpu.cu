@@ -895,8 +895,9 @@ static int check_map_sizes(AlbCtx* ctx) {
 }
 
 // Sorts the queries of the last backward trace and gathers them from their maps, queued on the
-// context's stream.
-static int gather_all(AlbCtx* ctx, const Accum& acc, bool lo_zero) {
+// context's stream. side: how many of the context's side streams were given work; they are joined
+// to its stream on success only.
+static int queue_gathers(AlbCtx* ctx, const Accum& acc, bool lo_zero, int& side) {
     static const int kinds[4] = {kQueryBottom, kQueryScatter, kQuerySurface, kQuerySurface};
     static const int chans[4] = {ALB_BOTTOM_REFLECTION, ALB_SCATTER, ALB_SURFACE_REFLECTION, ALB_SURFACE_TRANSMISSION_UP};
     uint64_t total = 0;
@@ -911,7 +912,6 @@ static int gather_all(AlbCtx* ctx, const Accum& acc, bool lo_zero) {
     }
     // each channel's work items of a fixed-radius gather (8 MB each; without them a query is one warp's)
     uint32_t* work = nullptr;
-    const size_t mark = ctx->ws.mark();
     const uint64_t words = 2 + 2 * (uint64_t)kRadiusItems;
     if (ctx->sc.radius > 0.0 && !(work = ctx->ws.take_u32(4 * words))) ctx->ws.clear_failed();
     // Few queries leave most of the chip idle in one gather: the planar ones run beside one another on
@@ -929,7 +929,6 @@ static int gather_all(AlbCtx* ctx, const Accum& acc, bool lo_zero) {
         }
         CK(cudaEventRecord(ctx->fork, ctx->st));
     }
-    int side = 0, rc = ALB_OK;
     static const int sequence[4] = {0, 2, 3, 1};  // the scatter gather's CTAs fill whole SMs: last
     for (int s = 0; s < 4; ++s) {
         const int g = sequence[s], k = kinds[g], c = chans[g];
@@ -952,23 +951,32 @@ static int gather_all(AlbCtx* ctx, const Accum& acc, bool lo_zero) {
         const bool aside = fork && c != ALB_SCATTER;
         cudaStream_t st = ctx->st;
         if (aside) {
-            st = ctx->side[side];
+            st = ctx->side[side++];
             CK(cudaStreamWaitEvent(st, ctx->fork, 0));
         }
         PhaseTimer pg(ctx, 4 + c, st);
         launch_gather(ctx->sc, map_dev(ctx->map[c]), q, c, acc, ctx->d_err, &ctx->launches, st);
         pg.stop(st);
-        if (aside) {
-            const cudaError_t e = cudaEventRecord(ctx->join[side], st);
-            if (e != cudaSuccess) rc = fail(ctx, ALB_ERR_CUDA, cudaGetErrorString(e));
-            ++side;
-        }
+        if (aside) CK(cudaEventRecord(ctx->join[side - 1], st));
         ctx->gathered[c] += (int64_t)nq;
     }
     for (int i = 0; i < side; ++i) CK(cudaStreamWaitEvent(ctx->st, ctx->join[i], 0));
+    return ALB_OK;
+}
+
+static int gather_all(AlbCtx* ctx, const Accum& acc, bool lo_zero) {
+    const size_t mark = ctx->ws.mark();
+    int side = 0;
+    const int rc = queue_gathers(ctx, acc, lo_zero, side);
+    if (rc) {
+        // what is queued still uses the query buffers and the scratch
+        for (int i = 0; i < side; ++i) cudaStreamSynchronize(ctx->side[i]);
+        cudaStreamSynchronize(ctx->st);
+    }
     ctx->ws.release(mark);
     return rc;
 }
+
 
 extern "C" int alb_trace(AlbCtx* ctx, int pass, uint64_t n, uint64_t seed, uint64_t first, const AlbReplay* rp) {
     if (!ctx) return ALB_ERR_INVALID;

@@ -87,3 +87,27 @@ def test_a_forward_call_out_of_memory_leaves_the_simulation_as_it_was(lib, first
     assert ctx.heatmaps()[2][0] - radius[0] == n
     ctx.close()
     assert not fake_cuda.violations(lib)
+
+
+@pytest.mark.parametrize("radius", [None, 0.5])
+def test_gathers_that_cannot_be_joined_are_waited_for(lib, radius):
+    """The gathers of a small call run on streams of their own. Whichever event of the call cannot be
+    recorded, no stream works on after it, nothing was freed under one, and no scratch stays taken."""
+    ctx = Context(lib, build_scene(workloads.small(0.9, radius=radius)))
+    ctx.trace(True, 3000)
+    ctx.build_maps()
+    ctx.trace(False, 800)
+    used, failed = lib.fake_used(0), 0
+    for n in range(1, 30):
+        lib.fake_fail_record(n)
+        try:
+            ctx.trace(False, 800)
+        except RuntimeError:
+            failed += 1
+        assert lib.fake_busy() == 0, n
+        assert lib.fake_used(0) == used, n
+        assert not fake_cuda.violations(lib), n
+    assert failed == 4  # the fork and the three joins; the others are times of phases
+    lib.fake_fail_record(0)
+    ctx.close()
+    assert lib.fake_used(0) == 0
