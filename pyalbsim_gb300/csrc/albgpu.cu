@@ -292,14 +292,20 @@ static cudaEvent_t take_event(AlbCtx* c) {
 struct PhaseTimer {
     AlbCtx* c;
     AlbCtx::Phase p;
+    bool stopped = false;
     PhaseTimer(AlbCtx* ctx, int phase, cudaStream_t st) : c(ctx), p{phase, take_event(ctx), take_event(ctx)} {
         cudaEventRecord(p.e0, st);
     }
     PhaseTimer(AlbCtx* ctx, int phase) : PhaseTimer(ctx, phase, ctx->st) {}
+    PhaseTimer(const PhaseTimer&) = delete;
+    ~PhaseTimer() {  // a phase left on an error counts for nothing
+        if (!stopped) c->events.insert(c->events.end(), {p.e0, p.e1});
+    }
     void stop(cudaStream_t st) {
         cudaEventRecord(p.e1, st);
         c->phase_calls[p.phase] += 1;
         c->pending.push_back(p);
+        stopped = true;
     }
     void stop() { stop(c->st); }
 };

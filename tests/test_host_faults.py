@@ -111,3 +111,17 @@ def test_gathers_that_cannot_be_joined_are_waited_for(lib, radius):
     lib.fake_fail_record(0)
     ctx.close()
     assert lib.fake_used(0) == 0
+
+
+def test_a_failed_map_build_keeps_no_timing_events(lib):
+    ctx = Context(lib, build_scene(workloads.small()))
+    ctx.trace(True, 100_000)
+    lib.fake_limit(0, lib.fake_used(0))
+    events = []
+    for _ in range(3):
+        with pytest.raises(RuntimeError, match="index build failed"):
+            ctx.build_maps()
+        events.append(lib.fake_events())
+    assert events[2] == events[0]
+    ctx.close()
+    assert lib.fake_events() == 0
