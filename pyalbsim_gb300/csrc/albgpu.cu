@@ -322,7 +322,10 @@ static void fold_phases(AlbCtx* c) {
 }
 
 static int fail(AlbCtx* c, int code, const std::string& msg) {
-    if (c) c->err = msg;
+    if (c) {
+        c->err = msg;
+        c->ws.clear_failed();  // this call has reported it
+    }
     return code;
 }
 

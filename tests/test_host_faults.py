@@ -125,3 +125,22 @@ def test_a_failed_map_build_keeps_no_timing_events(lib):
     assert events[2] == events[0]
     ctx.close()
     assert lib.fake_events() == 0
+
+
+def test_a_call_does_not_report_an_earlier_call_s_allocation_failure(lib):
+    """After a map build or a search that had no memory, the same call with memory succeeds."""
+    ctx = Context(lib, build_scene(workloads.small()))
+    ctx.trace(True, 100_000)
+    pts, qs = np.zeros((5_000, 3), np.float32), np.zeros((100, 3))
+    lib.fake_limit(0, lib.fake_used(0))
+    with pytest.raises(RuntimeError, match="index build failed"):
+        ctx.build_maps()
+    with pytest.raises(RuntimeError, match="knn allocation failed"):
+        ctx.knn(pts, qs, 3)
+    with pytest.raises(RuntimeError, match="read-back buffer"):
+        ctx.waveform(1)
+    lib.fake_limit(0, 1 << 40)
+    ctx.build_maps()
+    ctx.knn(pts, qs, 3)
+    ctx.trace(False, 100)
+    ctx.close()
