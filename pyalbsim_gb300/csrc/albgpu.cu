@@ -611,6 +611,12 @@ static std::string set_scene(AlbCtx* ctx, const AlbSceneParams* p) {
 // all of them where a set is large (128 B per bin).
 static int64_t class_sets(int64_t nbins) { return nbins <= (1 << 20) ? ALB_CHANNELS : 1; }
 
+// Bytes of what ensure_accumulators allocates.
+static double accumulator_bytes(int64_t nbins, bool adjoint, int64_t heat_cells) {
+    const double words = 2.0 * ALB_CHANNELS + 16.0 * class_sets(nbins) + (adjoint ? (2.0 * ALB_CHANNELS + 16.0) * kJacParams : 0.0);
+    return 8.0 * words * nbins + heat_cells * (8.0 * (heat_cells <= 512 * 512 ? 4 + 32 : 4) + 3 * 4.0);
+}
+
 // Waveform, Jacobian and heatmap accumulators sized for the current scene (grown, never
 // shrunk; a grown buffer is zeroed by the next reset).
 static std::string ensure_accumulators(AlbCtx* ctx) {
@@ -763,11 +769,15 @@ extern "C" int alb_set_option(AlbCtx* ctx, int key, int64_t v) {
 constexpr uint64_t kBackwardChunk = 1ull << 22;
 // A trace into buffers that turn out too small runs twice. In a scene not traced before, a small forward call
 // therefore gets room for kManyRecords scatter records per photon (3 KB per photon, given back when the
-// maps are built), and a large one traces its first kPilot photons into as much and measures: those few
+// maps are built, or kept with the record stores by a batch's workers), and a large one traces its first kPilot photons into as much and measures: those few
 // leave most of the chip idle, 2.7 ms of the float64 tracer's 16.5 for 200 000 photons twice over.
 constexpr uint64_t kPilot = 1ull << 14;
 constexpr uint64_t kSmallCall = 1ull << 18;
+constexpr double kFewRecords = 4.0;  // bottom reflections in that room
 constexpr double kManyRecords = 96.0;
+
+// Records per photon that a first small call has room for (alb_trace's and ensure_records' allowances).
+static double first_call_records() { return 1.03 * (1.0 + 1.0 / 16.0) * (kFewRecords + kManyRecords + 2.0 * 1.05); }
 
 static void release_records(AlbCtx* ctx, int c) {
     RecordStore& r = ctx->rec[c];
@@ -986,7 +996,6 @@ static int gather_all(AlbCtx* ctx, const Accum& acc, bool lo_zero) {
     return rc;
 }
 
-
 extern "C" int alb_trace(AlbCtx* ctx, int pass, uint64_t n, uint64_t seed, uint64_t first, const AlbReplay* rp) {
     if (!ctx) return ALB_ERR_INVALID;
     if (pass != ALB_FORWARD && pass != ALB_BACKWARD) return fail(ctx, ALB_ERR_INVALID, "pass must be 0 or 1");
@@ -1090,7 +1099,7 @@ extern "C" int alb_trace(AlbCtx* ctx, int pass, uint64_t n, uint64_t seed, uint6
         };
         const uint64_t pilot = !ctx->rec_rate_known && n > kSmallCall && !rp && !ctx->keep_exit ? kPilot : 0;
         if (!ctx->rec_rate_known && (pilot || n <= kSmallCall)) {
-            ctx->rec_rate[ALB_BOTTOM_REFLECTION] = 4.0;
+            ctx->rec_rate[ALB_BOTTOM_REFLECTION] = kFewRecords;
             ctx->rec_rate[ALB_SCATTER] = kManyRecords;
         }
         int rc = pilot ? part(0, pilot) : ALB_OK;
@@ -1619,10 +1628,11 @@ extern "C" int alb_batch_run(AlbBatchInstance* inst, uint64_t n, const AlbBatchO
     std::stable_sort(order.begin(), order.end(), [&](uint64_t a, uint64_t b) {
         return inst[a].n_forward + inst[a].n_backward > inst[b].n_forward + inst[b].n_backward;
     });
-    int64_t max_bins = 0;
+    int64_t max_bins = 0, max_cells = 0;
     for (uint64_t i = 0; i < n; ++i) {
         const AlbSceneParams* sp = inst[i].scene;
         max_bins = std::max<int64_t>(max_bins, sp->gate_bins > 0 ? sp->gate_bins : 2 * sp->steps);
+        if (sp->heatmap_enabled) max_cells = std::max<int64_t>(max_cells, (int64_t)sp->heatmap_bins * sp->heatmap_bins);
     }
     std::atomic<uint64_t> next{0};
     std::mutex msg_mu;
@@ -1633,7 +1643,9 @@ extern "C" int alb_batch_run(AlbBatchInstance* inst, uint64_t n, const AlbBatchO
     // has room or it is the only one running, and a worker dropping to instances a quarter
     // of its footprint releases its context. Footprint = forward photons x records per
     // photon (the largest seen so far x 1.5, 200 before any instance finished) x bytes per
-    // record (append store, index, build temporaries; scores with the adjoint) + 64 MiB.
+    // record (append store, index, build temporaries; scores with the adjoint), + the room that a
+    // context's first small call takes beyond those records and keeps (kManyRecords), + the sums of
+    // the longest timeline and the largest heatmap (ensure_accumulators), + 64 MiB.
     cudaSetDevice(opt->device);
     size_t free_b = 0, total_b = 0;
     cudaMemGetInfo(&free_b, &total_b);
@@ -1644,9 +1656,12 @@ extern "C" int alb_batch_run(AlbBatchInstance* inst, uint64_t n, const AlbBatchO
     double held_total = 0.0, rpp_seen = 0.0;
     int running = 0;
     int exclusive = 0;  // workers waiting to rerun an instance alone; the others hold no memory then
+    const double sums = accumulator_bytes(max_bins, opt->adjoint != 0, max_cells) + 64.0 * 1048576.0;
     auto need_of = [&](const AlbBatchInstance& I) {
         const double rpp = rpp_seen > 0.0 ? 1.5 * rpp_seen : 200.0;
-        return (double)I.n_forward * rpp * bytes_per_record + 64.0 * 1048576.0;
+        const double spare = I.n_forward <= kSmallCall ? std::max(0.0, first_call_records() - rpp) : 0.0;
+        const double bytes_per_spare = 32.0 + (opt->adjoint ? 16.0 : 0.0) + (max_cells ? 32.0 : 0.0);
+        return (double)I.n_forward * (rpp * bytes_per_record + spare * bytes_per_spare) + sums;
     };
     auto worker = [&]() {
         cudaSetDevice(opt->device);

@@ -3,6 +3,7 @@
 // devices runs without a GPU. Two devices; a device's memory has a limit that a test sets; a traced photon
 // leaves a fixed number of records and queries. Every launch, memset and free is checked: memory on the
 // device that is current, nothing freed while another stream still works.
+#include <chrono>
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
@@ -10,6 +11,7 @@
 #include <mutex>
 #include <set>
 #include <string>
+#include <thread>
 
 #include "fake_cuda.h"
 
@@ -28,6 +30,7 @@ struct State {
     double rec[4] = {1, 8, 1, 1}, query[3] = {1, 8, 1};
     int fail_record = 0;  // the n-th event record from now fails (0: none)
     uint64_t traced = 0;  // photons of every trace
+    int trace_ms = 0;
     int violations = 0;
     std::string what;
 };
@@ -62,6 +65,7 @@ void fake::launched(cudaStream_t st) {
     g->busy.insert(st);
 }
 void fake::traced(uint64_t photons) {
+    std::this_thread::sleep_for(std::chrono::milliseconds(g->trace_ms));
     Lock l(mu);
     g->traced += photons;
 }
@@ -114,6 +118,7 @@ void fake_rates(const double* rec, const double* query) {
     memcpy(g->rec, rec, sizeof g->rec);
     memcpy(g->query, query, sizeof g->query);
 }
+void fake_trace_ms(int ms) { g->trace_ms = ms; }
 void fake_fail_record(int n) { g->fail_record = n; }
 int fake_violations(char* out, int n) {
     snprintf(out, n, "%s", g->what.c_str());

@@ -144,3 +144,36 @@ def test_a_call_does_not_report_an_earlier_call_s_allocation_failure(lib):
     ctx.knn(pts, qs, 3)
     ctx.trace(False, 100)
     ctx.close()
+
+
+def _batch(lib, monkeypatch, scenes, n_forward, n_backward, **options):
+    from pyalbsim_gb300 import _native
+
+    monkeypatch.setattr(_native, "_lib", lib)
+    lib.fake_trace_ms(2)  # the workers run side by side
+    n = len(scenes)
+    return _native.batch_run(scenes, [n_forward] * n, [n_backward] * n, range(n), **options)[2]
+
+
+def test_batch_admits_the_room_that_a_first_call_takes(lib, monkeypatch):
+    """A context's first small call takes room for far more records than most scenes make, and a batch worker
+    keeps it: what the workers hold together stays within 80% of the device, and no instance runs twice."""
+    _rates(lib, [1.0, 6.0, 1.0, 1.0], [1.0, 6.0, 1.0])
+    lib.fake_limit(0, 40 << 30)
+    scene = build_scene(workloads.small())
+    status = _batch(lib, monkeypatch, [scene] * 600, 200_000, 50_000, streams=64)
+    assert not status.any()
+    assert lib.fake_traced() == 600 * 250_000
+    assert lib.fake_peak(0) < 0.8 * (40 << 30)
+
+
+def test_batch_admits_the_sums_of_a_long_timeline(lib, monkeypatch):
+    """Few photons, but 84 000 bins with their Jacobian: 0.13 GB of sums for each worker's context."""
+    _rates(lib, [1.0, 6.0, 1.0, 1.0], [1.0, 6.0, 1.0])
+    lib.fake_limit(0, 2 << 30)
+    scene = build_scene(workloads.large(hg=0.9))
+    assert scene.n_bins > 80_000
+    status = _batch(lib, monkeypatch, [scene] * 60, 2_000, 500, streams=40, adjoint=True)
+    assert not status.any()
+    assert lib.fake_traced() == 60 * 2_500
+    assert lib.fake_peak(0) < 0.8 * (2 << 30)
