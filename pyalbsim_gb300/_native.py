@@ -229,6 +229,13 @@ def raise_for(code: int, message: str):
     raise RuntimeError(f"albgpu error {code}: {message}")
 
 
+def trim_memory(device: int = 0):
+    """Give the device memory back that closed contexts have left with this process for its next ones (at
+    most an eighth of the device)."""
+    lib = load_library()
+    raise_for(lib.alb_trim_memory(int(device)), lib.alb_last_error(None).decode())
+
+
 def scene_struct(scene: SceneModel):
     """Pack a SceneModel into AlbSceneParams; returns (struct, keepalive arrays)."""
     p = AlbSceneParams()

@@ -19,6 +19,7 @@ from pyalbsim_gb300._native import (
     ALB_OPT_PRECISE,
     ALB_OPT_SORT_QUERIES,
     NativeContext,
+    trim_memory,  # noqa: F401  (for callers that share the device)
 )
 from pyalbsim_gb300.config.gpu import GpuRunOptions
 from pyalbsim_gb300.photon_mapping.photon_map_data import PhotonMapData

@@ -31,6 +31,7 @@ struct State {
     int fail_record = 0;  // the n-th event record from now fails (0: none)
     uint64_t traced = 0;  // photons of every trace
     int trace_ms = 0;
+    int trims[kDevices] = {0, 0};
     int violations = 0;
     std::string what;
 };
@@ -124,6 +125,7 @@ int fake_violations(char* out, int n) {
     snprintf(out, n, "%s", g->what.c_str());
     return g->violations;
 }
+int fake_trims(int device) { return g->trims[device]; }
 int fake_events() { return (int)g->events.size(); }
 int fake_busy() { return (int)g->busy.size(); }
 
@@ -171,7 +173,11 @@ cudaError_t cudaMemPoolGetAttribute(cudaMemPool_t, cudaMemPoolAttr, void* v) {
     return cudaSuccess;
 }
 cudaError_t cudaMemPoolSetAttribute(cudaMemPool_t, cudaMemPoolAttr, void*) { return cudaSuccess; }
-cudaError_t cudaMemPoolTrimTo(cudaMemPool_t, size_t) { return cudaSuccess; }
+cudaError_t cudaMemPoolTrimTo(cudaMemPool_t pool, size_t) {
+    Lock l(mu);
+    ++g->trims[(uintptr_t)pool - 1];
+    return cudaSuccess;
+}
 cudaError_t cudaMemcpy(void* d, const void* s, size_t n, cudaMemcpyKind) {
     memmove(d, s, n);
     return cudaSuccess;

@@ -177,3 +177,15 @@ def test_batch_admits_the_sums_of_a_long_timeline(lib, monkeypatch):
     assert not status.any()
     assert lib.fake_traced() == 60 * 2_500
     assert lib.fake_peak(0) < 0.8 * (2 << 30)
+
+
+def test_trim_memory_gives_a_device_s_idle_memory_back(lib, monkeypatch):
+    from pyalbsim_gb300 import _native
+    from pyalbsim_gb300.engine import trim_memory
+
+    monkeypatch.setattr(_native, "_lib", lib)
+    lib.cudaSetDevice(0)
+    trim_memory(1)
+    assert (lib.fake_trims(0), lib.fake_trims(1)) == (0, 1)
+    with pytest.raises(ValueError, match="no such device"):
+        trim_memory(2)
