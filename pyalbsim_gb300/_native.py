@@ -490,8 +490,8 @@ class NativeContext:
     def stats(self):
         """Counters of the last trace (events, photons), of the last forward trace
         (forward_events, forward_photons) and of the gathers (per channel: leaves
-        opened, internal nodes expanded, candidate reductions, queries, and queries whose
-        answer a buffer bound made inexact, which takes mass ties of distances)."""
+        opened, internal nodes expanded, candidate reductions, queries, and inexact answers:
+        always 0, whatever the ties of distances)."""
         out = np.zeros(32, np.int64)
         self._check(self.lib.alb_stats(self.h, _ptr(out), 32))
         st = {"events": int(out[0]), "photons": int(out[1]), "launches": int(out[2]),

@@ -207,7 +207,7 @@ struct AlbCtx {
     RecordStore rec[ALB_CHANNELS];
     uint64_t rec_id_cap[ALB_CHANNELS] = {0};
     uint64_t fwi_cap[ALB_CHANNELS] = {0}, sfi_cap[ALB_CHANNELS] = {0}, b_cap[ALB_CHANNELS] = {0};
-    // one control block: record counts [0, 4), query counts [4, 7), error word [7], counters [8, 40),
+    // one control block: record counts [0, 4), query counts [4, 7), error word and crowded channels [7], counters [8, 40),
     // counters kept across a retried trace [41, 43), the gathers' work counters [43, 47)
     unsigned long long* ctl = nullptr;
     unsigned long long* d_rec_count = nullptr;
@@ -336,8 +336,8 @@ static int fail(AlbCtx* c, int code, const std::string& msg) {
     } while (0)
 
 // Waits for the context's stream and reports what failed on it; counts (nullable) receives the
-// record and query counts.
-static int check_device(AlbCtx* ctx, const char* where, unsigned long long* counts = nullptr) {
+// record and query counts, crowded (nullable) the channels whose searches left queries.
+static int check_device(AlbCtx* ctx, const char* where, unsigned long long* counts = nullptr, uint32_t* crowded = nullptr) {
     unsigned long long ctl[8] = {0};
     cudaError_t e = cudaMemcpyAsync(ctl, ctx->ctl, sizeof ctl, cudaMemcpyDeviceToHost, ctx->st);
     if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->st);
@@ -350,9 +350,12 @@ static int check_device(AlbCtx* ctx, const char* where, unsigned long long* coun
     }
     if (counts) std::memcpy(counts, ctl, 7 * 8);
     const int h = (int)(uint32_t)ctl[7];
-    if (h != 0) {
-        CK(cudaMemsetAsync(ctx->d_err, 0, sizeof(int), ctx->st));
+    if (crowded) *crowded = (uint32_t)(ctl[7] >> 32);
+    if (ctl[7] != 0) {
+        CK(cudaMemsetAsync(ctx->d_err, 0, 8, ctx->st));
         CK(cudaStreamSynchronize(ctx->st));
+    }
+    if (h != 0) {
         const char* what = h == ALB_ERR_ITER_CAP ? "a device loop hit its iteration cap"
                            : h == ALB_ERR_REPLAY ? "a replay stream ran out of variates"
                            : h == ALB_ERR_TOO_FEW ? "a photon map holds fewer records than k"
@@ -913,12 +916,32 @@ static int check_map_sizes(AlbCtx* ctx) {
     return ALB_OK;
 }
 
+static const int kGatherKind[4] = {kQueryBottom, kQueryScatter, kQuerySurface, kQuerySurface};
+static const int kGatherChannel[4] = {ALB_BOTTOM_REFLECTION, ALB_SCATTER, ALB_SURFACE_REFLECTION, ALB_SURFACE_TRANSMISSION_UP};
+
+// The queries of gather g as left by the last backward trace.
+static QueryDev query_dev(AlbCtx* ctx, int g, bool lo_zero) {
+    const int k = kGatherKind[g], c = kGatherChannel[g];
+    QueryDev q{};
+    q.a = ctx->qa[k];
+    q.b = ctx->qb[k];
+    q.c = ctx->qc[k];
+    q.lo_zero = lo_zero;
+    q.s = ctx->sc.adjoint ? ctx->qs[k] : nullptr;
+    q.perm = ctx->sort_q ? ctx->qperm[k] : nullptr;
+    q.n = ctx->h_q_count[k];
+    q.rk_out = ctx->keep_ids ? ctx->qrk[k][g == 3 ? 1 : 0] : nullptr;
+    q.stats = ctx->d_stats + 4 + 4 * c;  // per channel: leaves, nodes, selects, queries
+    q.crowded = (uint32_t*)ctx->d_err + 1;
+    q.retries = ctx->d_stats + 30;
+    q.ticket = (uint32_t*)(ctx->ctl + 43 + c);
+    return q;
+}
+
 // Sorts the queries of the last backward trace and gathers them from their maps, queued on the
 // context's stream. side: how many of the context's side streams were given work; they are joined
 // to its stream on success only.
 static int queue_gathers(AlbCtx* ctx, const Accum& acc, bool lo_zero, int& side) {
-    static const int kinds[4] = {kQueryBottom, kQueryScatter, kQuerySurface, kQuerySurface};
-    static const int chans[4] = {ALB_BOTTOM_REFLECTION, ALB_SCATTER, ALB_SURFACE_REFLECTION, ALB_SURFACE_TRANSMISSION_UP};
     uint64_t total = 0;
     for (int k = 0; k < 3; ++k) {
         const uint64_t nq = ctx->h_q_count[k];
@@ -950,22 +973,9 @@ static int queue_gathers(AlbCtx* ctx, const Accum& acc, bool lo_zero, int& side)
     }
     static const int sequence[4] = {0, 2, 3, 1};  // the scatter gather's CTAs fill whole SMs: last
     for (int s = 0; s < 4; ++s) {
-        const int g = sequence[s], k = kinds[g], c = chans[g];
-        const uint64_t nq = ctx->h_q_count[k];
-        if (nq == 0) continue;
-        QueryDev q{};
-        q.a = ctx->qa[k];
-        q.b = ctx->qb[k];
-        q.c = ctx->qc[k];
-        q.lo_zero = lo_zero;
-        q.s = ctx->sc.adjoint ? ctx->qs[k] : nullptr;
-        q.perm = ctx->sort_q ? ctx->qperm[k] : nullptr;
-        q.n = nq;
-        q.rk_out = ctx->keep_ids ? ctx->qrk[k][g == 3 ? 1 : 0] : nullptr;
-        q.stats = ctx->d_stats + 4 + 4 * c;  // per channel: leaves, nodes, selects, queries
-        q.inexact = ctx->d_stats + 24 + c;
-        q.retries = ctx->d_stats + 30;
-        q.ticket = (uint32_t*)(ctx->ctl + 43 + c);
+        const int g = sequence[s], c = kGatherChannel[g];
+        QueryDev q = query_dev(ctx, g, lo_zero);
+        if (q.n == 0) continue;
         q.work = work ? work + c * words : nullptr;
         const bool aside = fork && c != ALB_SCATTER;
         cudaStream_t st = ctx->st;
@@ -977,7 +987,7 @@ static int queue_gathers(AlbCtx* ctx, const Accum& acc, bool lo_zero, int& side)
         launch_gather(ctx->sc, map_dev(ctx->map[c]), q, c, acc, ctx->d_err, &ctx->launches, st);
         pg.stop(st);
         if (aside) CK(cudaEventRecord(ctx->join[side - 1], st));
-        ctx->gathered[c] += (int64_t)nq;
+        ctx->gathered[c] += (int64_t)q.n;
     }
     for (int i = 0; i < side; ++i) CK(cudaStreamWaitEvent(ctx->st, ctx->join[i], 0));
     return ALB_OK;
@@ -1199,8 +1209,20 @@ extern "C" int alb_trace(AlbCtx* ctx, int pass, uint64_t n, uint64_t seed, uint6
         }
         rc = ctx->sc.radius > 0.0 ? ALB_OK : check_map_sizes(ctx);  // k-NN needs k records
         if (rc) return rc;
-        rc = gather_all(ctx, acc, !ctx->precise && !rp);
-        if (!rc) rc = check_device(ctx, "gather");
+        const bool lo_zero = !ctx->precise && !rp;
+        uint32_t crowded = 0;
+        rc = gather_all(ctx, acc, lo_zero);
+        if (!rc) rc = check_device(ctx, "gather", nullptr, &crowded);
+        if (!rc && crowded) {
+            for (int g = 0; g < 4; ++g) {
+                const int c = kGatherChannel[g];
+                if (!(crowded >> c & 1u)) continue;
+                PhaseTimer pg(ctx, 4 + c);
+                launch_gather_crowded(ctx->sc, map_dev(ctx->map[c]), query_dev(ctx, g, lo_zero), c, acc, ctx->d_err, ctx->st);
+                pg.stop();
+            }
+            rc = check_device(ctx, "gather");
+        }
         if (rc) return rc;
         if (n == 0) break;
     }
@@ -1529,8 +1551,13 @@ extern "C" int alb_knn(AlbCtx* ctx, const float* pts, uint64_t m, const double* 
         return done(fail(ctx, ALB_ERR_CAPACITY, "knn index build failed"));
     if (nq) pack_knn_queries(dq, nq, qa, ctx->st);
     if (sort_queries(ctx->ws, qa, nq, perm, ctx->st) != 0) return done(fail(ctx, ALB_ERR_CUDA, "knn query sort failed"));
-    launch_knn(map_dev(mi), dq, perm, nq, k, di, dd, ctx->d_err, ctx->st);
-    const int rc = check_device(ctx, "knn");
+    launch_knn(map_dev(mi), dq, perm, nq, k, di, dd, ctx->d_err, (uint32_t*)ctx->d_err + 1, ctx->st);
+    uint32_t crowded = 0;
+    int rc = check_device(ctx, "knn", nullptr, &crowded);
+    if (!rc && crowded) {
+        launch_knn_crowded(map_dev(mi), dq, nq, k, di, dd, ctx->d_err, ctx->st);
+        rc = check_device(ctx, "knn");
+    }
     if (rc) return done(rc);
     if (!ok(cudaMemcpyAsync(idx, di, nq * k * 4, cudaMemcpyDeviceToHost, ctx->st)) ||
         !ok(cudaMemcpyAsync(dist, dd, nq * k * 8, cudaMemcpyDeviceToHost, ctx->st)) ||

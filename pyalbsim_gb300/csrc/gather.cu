@@ -56,7 +56,7 @@ struct WarpSmem {
     double bd[kBand];    // near-tie band: float64 distances
     uint32_t bi[kBand];  // map positions
     uint64_t bt[kBand];  // tie keys from the record's content (or 0)
-    unsigned long long st[5];  // the warp's search counters: leaves, nodes, selects, queries, inexact
+    unsigned long long st[4];  // the warp's search counters: leaves, nodes, selects, queries
     // scratch words of the boundary band (the stack is free after the search)
     ALB_DEVICE uint32_t& tmp(int i) { return i < kStack ? stk[i] : reinterpret_cast<uint32_t*>(stk_d)[i - kStack]; }
 };
@@ -363,22 +363,39 @@ struct KnnResult {
     int leaves;    // leaves opened (32 records each)
     int nodes;     // internal nodes expanded
     int selects;   // candidate-buffer reductions
-    int clipped;   // 1 if a buffer bound forced an inexact answer (mass ties)
     int fail;      // 0, or why the search has no answer (s.ci is then not valid):
-                   // ALB_ERR_ITER_CAP (traversal guard) or ALB_ERR_INVALID (fewer than k
-                   // finite points admitted: a NaN or infinite query or map coordinates)
+                   // ALB_ERR_ITER_CAP (traversal guard), ALB_ERR_INVALID (fewer than k
+                   // finite points admitted: a NaN or infinite query or map coordinates) or
+                   // kCrowded (more near ties than its buffers hold)
 };
+// Searches whose near ties fill their buffers (coincident points, or a lattice of them) are left by the kernels
+// below, marked, and answered by a launch of their own (k_gather_crowded, k_knn_crowded), which happens only where
+// some are. Called from the searches' loops, the code that resolves any number of ties cost a whole run of the
+// large scene 13% at 1e6 photons (34.6 -> 39.6 ms) and 16% at 1e7, by the registers that a call takes.
+constexpr int kCrowded = 1;
+ALB_DEVICE void leave_crowded(const QueryDev& q, uint32_t src, int channel) {
+    if (lane_id() == 0) {
+        atomicOr(reinterpret_cast<unsigned*>(&q.c[src].w), 1u << channel);
+        atomicOr(q.crowded, 1u << channel);
+    }
+    __syncwarp();
+}
 
-// Position of a point: a map record's, or one of a packed array.
-ALB_DEVICE float4 point_at(const MapDev& m, uint32_t i) { return m.a[i]; }
-template <class P>
-ALB_DEVICE float4 point_at(const P& p, uint32_t i) { return p.at(i); }
+// Positions of points: a map's records, or a packed array.
+struct MapPoints {
+    const float4* a;
+    ALB_DEVICE float4 at(uint32_t r) const { return a[r]; }
+};
+struct PackedPoints {
+    const float* p;
+    ALB_DEVICE float4 at(uint32_t r) const { return make_float4(p[3 * r], p[3 * r + 1], p[3 * r + 2], 0.f); }
+};
 
 // float64 ranking of the band entries bi[0..nb) by (distance, tie key, map position); the
 // `take` smallest go to ci[dst ..] in rank order. Returns the float64 squared distance of
 // the take-th (0 if the band holds fewer).
-template <class M, class S>
-ALB_DEVICE double rank_band(const M& m, S& s, int dst, int nb, int take, double qx, double qy,
+template <class P, class S>
+ALB_DEVICE double rank_band(P pts, S& s, int dst, int nb, int take, double qx, double qy,
                             double qz, const float4* tie_rec) {
     const int l = lane_id();
     double di = 0.0;
@@ -387,7 +404,7 @@ ALB_DEVICE double rank_band(const M& m, S& s, int dst, int nb, int take, double 
     int rank = 0;
     if (l < nb) {
         ii = s.bi[l];
-        const float4 a = point_at(m, ii);
+        const float4 a = pts.at(ii);
         di = point_dist2_f64(qx, qy, qz, a);
         ti = tie_rec ? record_tie_key(a, tie_rec[ii]) : 0ull;
         s.bd[l] = di;
@@ -410,12 +427,74 @@ ALB_DEVICE double rank_band(const M& m, S& s, int dst, int nb, int take, double 
     return rk2;
 }
 
+// Leaves of the entries [off, off + n) the k nearest by (float64 distance, tie key, map position), whatever
+// their ties, and returns the float64 squared distance of the k-th. Every entry is ranked against every
+// other one in registers: 288 entries take some 15 000 instructions, but only searches with more entries at
+// one distance than their buffers hold come here, which takes coincident points or a lattice of them.
+template <class P, class S>
+__device__ __noinline__ double keep_nearest(P pts, S& s, int off, int n, int k, double qx, double qy, double qz,
+                                            const float4* tie_rec) {
+    constexpr int R = S::kCap / 32;
+    const int l = lane_id();
+    uint64_t d[R], t[R];
+    uint32_t id[R];
+    int rank[R];
+#pragma unroll
+    for (int i = 0; i < R; ++i) {
+        const bool on = i * 32 + l < n;
+        id[i] = on ? s.ci[off + i * 32 + l] : 0u;
+        d[i] = t[i] = ~0ull;  // behind every entry
+        rank[i] = 0;
+        if (on) {
+            const float4 a = pts.at(id[i]);
+            d[i] = (uint64_t)__double_as_longlong(point_dist2_f64(qx, qy, qz, a));  // non-negative: ordered like its bits
+            t[i] = tie_rec ? record_tie_key(a, tie_rec[id[i]]) : 0ull;
+        }
+    }
+#pragma unroll
+    for (int j = 0; j < R; ++j) {
+#pragma unroll 1
+        for (int src = 0; src < min(32, n - j * 32); ++src) {
+            const uint64_t dj = __shfl_sync(0xffffffffu, d[j], src), tj = __shfl_sync(0xffffffffu, t[j], src);
+            const uint32_t ij = __shfl_sync(0xffffffffu, id[j], src);
+#pragma unroll
+            for (int i = 0; i < R; ++i)
+                rank[i] += dj < d[i] || (dj == d[i] && (tj < t[i] || (tj == t[i] && ij < id[i]))) ? 1 : 0;
+        }
+    }
+    int out = 0;
+    uint64_t last = 0ull;
+#pragma unroll
+    for (int i = 0; i < R; ++i) {
+        if (i * 32 >= n) break;
+        const int at = off + i * 32 + l;
+        const bool keep = i * 32 + l < n && rank[i] < k;
+        const float e = keep ? s.cd[at] : 0.f;
+        const int16_t c = keep ? s.cl[at] : (int16_t)0;
+        const unsigned b = __ballot_sync(0xffffffffu, keep);
+        __syncwarp();
+        if (keep) {
+            const int pos = off + out + __popc(b & lanemask_lt());
+            s.cd[pos] = e;
+            s.ci[pos] = id[i];
+            s.cl[pos] = c;
+        }
+        out += __popc(b);
+        const unsigned own = __ballot_sync(0xffffffffu, keep && rank[i] == k - 1);
+        if (own) last = __shfl_sync(0xffffffffu, d[i], __ffs(own) - 1);
+        __syncwarp();
+    }
+    return __longlong_as_double((long long)last);
+}
+
 // The k_sub nearest among the entries [off, off + n) whose cd/cl hold refined keys: keys more
 // than one unit below the k_sub-th are in, keys within one unit of it are ranked in float64.
-// The chosen map positions end up in ci[off .. off + k_sub).
-template <class M, class S>
-ALB_DEVICE double select_refined(const M& m, S& s, int off, int n, int k_sub, double qx, double qy,
-                                 double qz, const float4* tie_rec, int& clipped) {
+// The chosen map positions end up in ci[off .. off + k_sub). A band of more than kBand entries is ranked with
+// TIES (in scratch words: the search is done with its stack), and otherwise left: fail = kCrowded.
+template <bool TIES, class P, class S>
+ALB_DEVICE double select_refined(P pts, S& s, int off, int n, int k_sub, double qx, double qy,
+                                 double qz, const float4* tie_rec, int& fail) {
+    static_assert(S::kCap <= S::kTmp, "the band is a subset of the candidates");
     const int l = lane_id();
     const uint64_t K = warp_kth_key<6>(s, off, n, k_sub);
     int n_in = 0, n_band = 0;
@@ -434,16 +513,22 @@ ALB_DEVICE double select_refined(const M& m, S& s, int off, int n, int k_sub, do
         if (band) {
             const int pos = n_band + __popc(bb & lanemask_lt());
             if (pos < kBand) s.bi[pos] = id;
+            else if (TIES) s.tmp(pos) = id;
         }
         n_in += __popc(bin);
         n_band += __popc(bb);
         __syncwarp();
     }
     if (n_band > kBand) {
-        n_band = kBand;
-        clipped = 1;
+        if (!TIES) {
+            fail = kCrowded;
+            return 0.0;
+        }
+        for (int j = l; j < n_band; j += 32) s.ci[off + n_in + j] = j < kBand ? s.bi[j] : s.tmp(j);
+        __syncwarp();
+        return keep_nearest(pts, s, off + n_in, n_band, k_sub - n_in, qx, qy, qz, tie_rec);
     }
-    return rank_band(m, s, off + n_in, n_band, k_sub - n_in, qx, qy, qz, tie_rec);
+    return rank_band(pts, s, off + n_in, n_band, k_sub - n_in, qx, qy, qz, tie_rec);
 }
 
 // Full k-NN search for one query. Returns false when the map has fewer than k records; the
@@ -460,7 +545,8 @@ ALB_DEVICE double select_refined(const M& m, S& s, int off, int n, int k_sub, do
 // holds entries within one float32 ulp of the k-th: needed where many points sit at nearly
 // the same distance (queries far from a dense planar map). Without it candidates carry the
 // float32 screening distance and only a crowded final band is refined.
-template <bool REFINE, bool QSPLIT = false, class S>
+// TIES: any number of near ties is resolved; without it a search whose buffers they fill ends with kCrowded.
+template <bool REFINE, bool QSPLIT = false, bool TIES = false, class S>
 ALB_DEVICE bool warp_knn(const MapDev& m, S& s, int k, double qx, double qy, double qz, float fx,
                          float fy, float fz, float lx, float ly, float lz, float bound, const float4* tie_rec,
                          KnnResult& res) {
@@ -468,9 +554,9 @@ ALB_DEVICE bool warp_knn(const MapDev& m, S& s, int k, double qx, double qy, dou
     if (m.n_real < (uint64_t)k) return false;
     float thr = bound;  // admission threshold (float32 squared distance, with margin)
     int cnt = 0;
-    res.leaves = res.nodes = res.selects = res.clipped = res.fail = 0;
-    // The carried bound first, then none: a bound can only fail through a degenerate previous
-    // result (a clipped boundary band).
+    res.leaves = res.nodes = res.selects = res.fail = 0;
+    // The carried bound first, then none (a caller's bound is a promise that k points lie within it; one that does
+    // not hold costs a second search).
     float start = bound;
     for (int attempt = 0; attempt < 2; ++attempt) {
         if (attempt == 1) {
@@ -532,11 +618,15 @@ ALB_DEVICE bool warp_knn(const MapDev& m, S& s, int k, double qx, double qy, dou
                 // rank among the k nearest, nothing beyond can; otherwise the float32
                 // screening margin decides
                 cnt = warp_compact(s, cnt, REFINE ? __uint_as_float(__float_as_uint(kth) + 1u) : thr);
-                if (cnt > S::kCap - 32) {  // mass ties
-                    cnt = warp_compact(s, cnt, kth);
-                    res.clipped = 1;
+                if (cnt > S::kCap - 32) {  // more near ties than there is room for: the k best so far are enough
+                    if (TIES) {
+                        keep_nearest(MapPoints{m.a}, s, 0, cnt, k, qx, qy, qz, tie_rec);
+                        cnt = k;
+                    } else {
+                        res.fail = kCrowded;
+                        sp = 0;
+                    }
                 }
-                if (cnt > S::kCap - 32) cnt = S::kCap - 32;  // keeps the buffer in bounds
             }
         };
         auto load_leaf = [&](uint32_t leaf) {
@@ -623,7 +713,7 @@ ALB_DEVICE bool warp_knn(const MapDev& m, S& s, int k, double qx, double qy, dou
     }
     double rk2;
     if (REFINE) {
-        rk2 = select_refined(m, s, 0, cnt, k, qx, qy, qz, tie_rec, res.clipped);
+        rk2 = select_refined<TIES>(MapPoints{m.a}, s, 0, cnt, k, qx, qy, qz, tie_rec, res.fail);
     } else {
         // float32 k-th; entries clearly below it are in, the band within the screening
         // margin around it is resolved exactly (refined keys when it is crowded)
@@ -650,12 +740,11 @@ ALB_DEVICE bool warp_knn(const MapDev& m, S& s, int k, double qx, double qy, dou
             n_band += __popc(bb);
             __syncwarp();
         }
-        static_assert(S::kCap <= S::kTmp, "the band is a subset of the candidates");
         const int take = k - n_in;
         if (n_band <= kBand) {
             if (l < n_band) s.bi[l] = s.tmp(l);
             __syncwarp();
-            rk2 = rank_band(m, s, n_in, n_band, take, qx, qy, qz, tie_rec);
+            rk2 = rank_band(MapPoints{m.a}, s, n_in, n_band, take, qx, qy, qz, tie_rec);
         } else {
 #pragma unroll 1
             for (int j = l; j < n_band; j += 32) {
@@ -667,12 +756,23 @@ ALB_DEVICE bool warp_knn(const MapDev& m, S& s, int k, double qx, double qy, dou
                 s.ci[n_in + j] = id;
             }
             __syncwarp();
-            rk2 = select_refined(m, s, n_in, n_band, take, qx, qy, qz, tie_rec, res.clipped);
+            rk2 = select_refined<TIES>(MapPoints{m.a}, s, n_in, n_band, take, qx, qy, qz, tie_rec, res.fail);
         }
     }
     res.rk2 = rk2;
     res.rkf = sqrt_to_f32(rk2);
     return true;
+}
+
+// The search of a query whose near ties fill a search's buffers (the map holds at least k records).
+template <class S>
+__device__ __noinline__ KnnResult crowded_knn(const MapDev& m, S& s, int k, double qx, double qy, double qz,
+                                              const float4* tie_rec) {
+    const float fx = (float)qx, fy = (float)qy, fz = (float)qz;
+    KnnResult r;
+    warp_knn<true, false, true>(m, s, k, qx, qy, qz, fx, fy, fz, (float)(qx - (double)fx), (float)(qy - (double)fy),
+                                (float)(qz - (double)fz), FLT_MAX, tie_rec, r);
+    return r;
 }
 
 }  // namespace alb
@@ -987,7 +1087,7 @@ ALB_DEVICE void warp_radius_visit(const MapDev& m, WarpSmem& s, const RadiusWork
     const double R2 = R * R;
     const float thr = __double2float_ru(R2) * (1.0f + 2.0f * kRelMargin);
     const float lo_band = __double2float_rd(R2) * (1.0f - 2.0f * kRelMargin);
-    res.leaves = res.nodes = res.selects = res.clipped = res.fail = 0;
+    res.leaves = res.nodes = res.selects = res.fail = 0;
     res.rk2 = R2;
     res.rkf = (float)R;
     if (m.nlevels <= 0) return;  // an empty map contributes nothing
@@ -1219,7 +1319,7 @@ __global__ void __launch_bounds__(kGatherWarps * 32, kGatherBlocksPerSM) k_gathe
     bool failed = false;
     // search counters accumulate in the warp's shared memory, not in registers held through
     // every search
-    if (l < 5) s.st[l] = 0ull;
+    if (l < 4) s.st[l] = 0ull;
     __syncwarp();
     for (uint64_t ch = (uint64_t)blockIdx.x * kGatherWarps + w; ch < chunks && !failed; ch += warps) {
         const uint64_t q_end = min((ch + 1) * kChunk, queries);
@@ -1272,7 +1372,6 @@ __global__ void __launch_bounds__(kGatherWarps * 32, kGatherBlocksPerSM) k_gathe
                     s.st[0] += r.leaves;
                     s.st[1] += r.nodes;
                     s.st[3] += second ? 0 : 1;
-                    s.st[4] += r.clipped;
                 }
                 if (q.rk_out && l == 0) q.rk_out[src] = sc.radius;
                 __syncwarp();
@@ -1300,6 +1399,11 @@ __global__ void __launch_bounds__(kGatherWarps * 32, kGatherBlocksPerSM) k_gathe
                 failed = true;
                 break;
             }
+            if (r.fail == kCrowded) {
+                leave_crowded(q, (uint32_t)src, CHANNEL);
+                have_prev = false;
+                continue;
+            }
             if (r.fail) {  // no valid neighbour set: report it and stop this warp's work
                 if (l == 0) atomicCAS(err, 0, r.fail);
                 failed = true;
@@ -1314,7 +1418,6 @@ __global__ void __launch_bounds__(kGatherWarps * 32, kGatherBlocksPerSM) k_gathe
                 s.st[1] += r.nodes;
                 s.st[2] += r.selects;
                 s.st[3] += 1;
-                s.st[4] += r.clipped;
             }
             accumulate<CHANNEL, MODE>(sc, m, q, acc, bc, jc, err, s, k, src, qa.w, qb, r.rkf);
             __syncwarp();
@@ -1327,7 +1430,6 @@ __global__ void __launch_bounds__(kGatherWarps * 32, kGatherBlocksPerSM) k_gathe
             atomicAdd(q.stats + 2, s.st[2]);
             atomicAdd(q.stats + 3, s.st[3]);
         }
-        if (q.inexact && s.st[4]) atomicAdd(q.inexact, s.st[4]);
     }
     __syncthreads();
     bin_flush<CHANNEL>(bc, acc);
@@ -1404,6 +1506,21 @@ ALB_DEVICE void accumulate_run(const SceneDev& sc, const MapDev& m, const QueryD
     }
 }
 
+// s.ci to s.cp, which overlay each other: the last 32 first.
+template <class S>
+ALB_DEVICE void pack_neighbours(const MapDev& m, S& s, int k) {
+    for (int j = (k - 1) / 32 * 32 + lane_id(); j >= 0; j -= 32) {
+        uint2 c = make_uint2(0u, 0u);
+        if (j < k) {
+            c.x = s.ci[j];
+            c.y = __float_as_uint(m.a[c.x].w);
+        }
+        __syncwarp();
+        if (j < k) s.cp[j] = c;
+        __syncwarp();
+    }
+}
+
 // The search of one query alone, out of line: the grouped kernel takes it for the first query of
 // a CTA, runs whose list does not fit, guesses that fail and near ties, 1-3% of the queries,
 // and its code and registers stay out of the hot loop. The k neighbours are left
@@ -1422,19 +1539,8 @@ __device__ __noinline__ bool cold_knn(const MapDev& m, S& s, int k, float fx, fl
         bound = t < 1.0e37f ? t : FLT_MAX;
     }
     if (!warp_knn<false, true>(m, s, k, 0.0, 0.0, 0.0, fx, fy, fz, lx, ly, lz, bound, m.b, res)) return false;
-    if (!res.fail) {
-        // s.ci to s.cp, which overlay each other: the last 32 first
-        for (int j = (k - 1) / 32 * 32 + lane_id(); j >= 0; j -= 32) {
-            uint2 c = make_uint2(0u, 0u);
-            if (j < k) {
-                c.x = s.ci[j];
-                c.y = __float_as_uint(m.a[c.x].w);
-            }
-            __syncwarp();
-            if (j < k) s.cp[j] = c;
-            __syncwarp();
-        }
-    }
+    // (of a crowded search k of its candidates: records all the same, for the next query's bound)
+    if (!res.fail || res.fail == kCrowded) pack_neighbours(m, s, k);
     return true;
 }
 
@@ -1505,7 +1611,7 @@ __global__ void __launch_bounds__(WARPS * 32, 1)
     const uint32_t segments = plan.pieces * (uint32_t)plan.levels, chunks = 1u << plan.chunk_bits;
     const float side_rk = G::side((float)k);
     bool failed = false;
-    if (l < 5) s.st[l] = 0ull;
+    if (l < 4) s.st[l] = 0ull;
     if (l == 0) {
         s.alone = 0;
         s.streak = 1;
@@ -1610,6 +1716,10 @@ __global__ void __launch_bounds__(WARPS * 32, 1)
                 run.take = 0;
                 KnnResult r;
                 const bool enough = cold_knn(m, s, k, fx, fy, fz, lx, ly, lz, bound, r);
+                if (enough && r.fail == kCrowded) {
+                    leave_crowded(q, src, CHANNEL);
+                    continue;
+                }
                 if (!enough || r.fail) {  // no valid neighbour set: report it and stop this warp's work
                     if (l == 0) atomicCAS(err, 0, enough ? r.fail : ALB_ERR_TOO_FEW);
                     failed = true;
@@ -1623,7 +1733,6 @@ __global__ void __launch_bounds__(WARPS * 32, 1)
                     s.st[1] += r.nodes;
                     s.st[2] += r.selects;
                     s.st[3] += 1;
-                    s.st[4] += r.clipped;
                 }
             }
             prev2 = d2;
@@ -1640,7 +1749,6 @@ __global__ void __launch_bounds__(WARPS * 32, 1)
             atomicAdd(q.stats + 2, s.st[2]);
             atomicAdd(q.stats + 3, s.st[3]);
         }
-        if (q.inexact && s.st[4]) atomicAdd(q.inexact, s.st[4]);
     }
     if constexpr (SLOTS != 0) {
         __syncthreads();
@@ -1649,15 +1757,46 @@ __global__ void __launch_bounds__(WARPS * 32, 1)
     }
 }
 
-// The float64 squared distance from (qx, qy, qz) to point r, for the answers of a search.
-struct MapPoints {
-    const float4* a;
-    ALB_DEVICE float4 at(uint32_t r) const { return a[r]; }
-};
-struct PackedPoints {
-    const float* p;
-    ALB_DEVICE float4 at(uint32_t r) const { return make_float4(p[3 * r], p[3 * r + 1], p[3 * r + 2], 0.f); }
-};
+// The queries that this channel's gather left (kCrowded): the k nearest under any number of ties, and their sums.
+// A warp looks at 32 queries' marks at a time. One mode: what it sums is decided by the accumulators it is given.
+constexpr int kCrowdedWarps = 4;
+template <int CHANNEL>
+__global__ void __launch_bounds__(kCrowdedWarps * 32) k_gather_crowded(const __grid_constant__ SceneDev sc, const __grid_constant__ MapDev m,
+                                                                       const __grid_constant__ QueryDev q,
+                                                                       const __grid_constant__ Accum acc, int k, int* err,
+                                                                       uint64_t first, uint64_t end) {
+    __shared__ GroupSmem<448> smem[kCrowdedWarps];
+    const int w = threadIdx.x >> 5, l = lane_id();
+    GroupSmem<448>& s = smem[w];
+    NoCache none;
+    if (l < 4) s.st[l] = 0ull;
+    __syncwarp();
+    const uint64_t step = 32ull * gridDim.x * kCrowdedWarps;
+    for (uint64_t base = first + 32ull * ((uint64_t)blockIdx.x * kCrowdedWarps + w); base < end; base += step) {
+        const bool left = base + l < end && (__float_as_uint(q.c[base + l].w) >> CHANNEL & 1u);
+        for (unsigned todo = __ballot_sync(0xffffffffu, left); todo; todo &= todo - 1u) {
+            const uint32_t src = (uint32_t)(base + __ffs(todo) - 1);
+            const float4 qa = q.a[src], qc = q.c[src];
+            const double qx = (double)qa.x + (double)qc.x, qy = (double)qa.y + (double)qc.y, qz = (double)qa.z + (double)qc.z;
+            const KnnResult r = crowded_knn(m, s, k, qx, qy, qz, m.b);
+            if (r.fail) {
+                if (l == 0) atomicCAS(err, 0, r.fail);
+                continue;
+            }
+            pack_neighbours(m, s, k);
+            if (q.rk_out && l == 0) q.rk_out[src] = sqrt(r.rk2);
+            if (l == 0) {
+                s.st[0] += r.leaves;
+                s.st[1] += r.nodes;
+                s.st[2] += r.selects;
+                s.st[3] += 1;
+            }
+            accumulate_run<CHANNEL, kModeKnnAdjoint>(sc, m, q, acc, none, false, err, s, k, src, qa.w, q.b[src], qy, r.rkf);
+            __syncwarp();
+        }
+    }
+    if (l < 4 && q.stats && s.st[3]) atomicAdd(q.stats + l, s.st[l]);
+}
 
 // One query's k neighbours s.ci[0 .. k) in order of (float64 distance, index), as out_idx / out_dist
 // rows of k. Every distance is formed once and ranked as its bit pattern against the others in
@@ -1722,12 +1861,14 @@ ALB_DEVICE void write_failed(int k, int32_t* out_idx, double* out_dist) {
     __syncwarp();
 }
 
+constexpr int32_t kLeft = -2;  // a crowded query's first index, until its answer replaces it
+
 // Standalone KDTree.query(x, k): sorted indices (the w lanes of the map's records) and float64
 // distances. Queries go in `perm` order, `chunk` consecutive ones per warp, each bounded by the
 // farthest of its predecessor's neighbours.
 __global__ void __launch_bounds__(kGatherWarps * 32, kGatherBlocksPerSM)
     k_knn(MapDev m, const double* __restrict__ qs, const uint32_t* __restrict__ perm, uint64_t nq, uint32_t chunk, int k,
-          int32_t* out_idx, double* out_dist, int* err) {
+          int32_t* out_idx, double* out_dist, int* err, uint32_t* crowded) {
     __shared__ WarpSmem smem[kGatherWarps];
     const int w = threadIdx.x >> 5, l = lane_id();
     WarpSmem& s = smem[w];
@@ -1754,8 +1895,40 @@ __global__ void __launch_bounds__(kGatherWarps * 32, kGatherBlocksPerSM)
             if (!warp_knn<true>(m, s, k, qx, qy, qz, fx, fy, fz, lx, ly, lz, bound, nullptr, r)) why = ALB_ERR_TOO_FEW;
             else if (r.fail) why = r.fail;
             have_prev = !why;
+            if (why == kCrowded) {
+                if (l == 0) {
+                    out_idx[qi * k] = kLeft;
+                    atomicOr(crowded, 1u);
+                }
+                __syncwarp();
+                continue;
+            }
             if (why) {
                 if (l == 0) atomicCAS(err, 0, why);
+                write_failed(k, out_idx + qi * k, out_dist + qi * k);
+                continue;
+            }
+            write_sorted(MapPoints{m.a}, s, k, qx, qy, qz, m.a, out_idx + qi * k, out_dist + qi * k);
+        }
+    }
+}
+
+// The queries that k_knn left.
+__global__ void __launch_bounds__(kCrowdedWarps * 32) k_knn_crowded(const __grid_constant__ MapDev m, const double* __restrict__ qs,
+                                                                    uint64_t nq, int k, int32_t* out_idx, double* out_dist,
+                                                                    int* err) {
+    __shared__ WarpSmem smem[kCrowdedWarps];
+    const int w = threadIdx.x >> 5, l = lane_id();
+    WarpSmem& s = smem[w];
+    const uint64_t step = 32ull * gridDim.x * kCrowdedWarps;
+    for (uint64_t base = 32ull * ((uint64_t)blockIdx.x * kCrowdedWarps + w); base < nq; base += step) {
+        const bool left = base + l < nq && out_idx[(base + l) * k] == kLeft;
+        for (unsigned todo = __ballot_sync(0xffffffffu, left); todo; todo &= todo - 1u) {
+            const uint64_t qi = base + __ffs(todo) - 1;
+            const double qx = qs[3 * qi], qy = qs[3 * qi + 1], qz = qs[3 * qi + 2];
+            const int fail = crowded_knn(m, s, k, qx, qy, qz, nullptr).fail;
+            if (fail) {
+                if (l == 0) atomicCAS(err, 0, fail);
                 write_failed(k, out_idx + qi * k, out_dist + qi * k);
                 continue;
             }
@@ -1768,63 +1941,92 @@ __global__ void __launch_bounds__(kGatherWarps * 32, kGatherBlocksPerSM)
 // query: no index, no scratch memory, one launch. At 4096 points the 128 screening steps cost what
 // a walk over a tree does, and the tree's one-CTA build cost 0.8 ms on top.
 constexpr int kBruteWarps = 4;
-__global__ void __launch_bounds__(kBruteWarps * 32) k_knn_brute(const float* __restrict__ pts, uint32_t m,
-                                                                const double* __restrict__ qs, uint64_t nq, int k,
-                                                                int32_t* out_idx, double* out_dist) {
+
+// One query (TIES as in warp_knn): 0, or ALB_ERR_INVALID (fewer than k points admitted) or kCrowded.
+template <bool TIES>
+ALB_DEVICE int brute_knn(PackedPoints pp, uint32_t m, WarpSmem& s, int k, double qx, double qy, double qz) {
+    const int l = lane_id();
+    const float fx = (float)qx, fy = (float)qy, fz = (float)qz;
+    const float lx = (float)(qx - (double)fx), ly = (float)(qy - (double)fy), lz = (float)(qz - (double)fz);
+    float thr = FLT_MAX;
+    int cnt = 0;
+    constexpr int kAhead = 4;  // steps whose points are loaded together
+    for (uint32_t r0 = 0; r0 < m; r0 += 32 * kAhead) {
+        float4 p[kAhead];
+#pragma unroll
+        for (int i = 0; i < kAhead; ++i) {
+            const uint32_t r = r0 + i * 32 + l;
+            p[i] = r < m ? pp.at(r) : make_float4(0.f, 0.f, 0.f, 0.f);
+        }
+#pragma unroll
+        for (int i = 0; i < kAhead; ++i) {
+            const uint32_t r = r0 + i * 32 + l;
+            const float d = point_dist2(fx, fy, fz, lx, ly, lz, p[i]);
+            const bool take = r < m && d <= thr;
+            const unsigned b = __ballot_sync(0xffffffffu, take);
+            if (take) {
+                const int pos = cnt + __popc(b & lanemask_lt());
+                float hi, lo;
+                point_dist2_df(fx, fy, fz, lx, ly, lz, p[i], hi, lo);
+                s.ci[pos] = r;
+                s.cd[pos] = hi;
+                s.cl[pos] = frac16(hi, lo);
+            }
+            cnt += __popc(b);
+            __syncwarp();
+            if (cnt >= k && (thr == FLT_MAX || cnt > kCap - 32)) {
+                // refined distances within one float32 ulp of the k-th can still rank
+                const float kth = warp_kth32(s, 0, cnt, k);
+                thr = fminf(thr, kth * (1.0f + 2.0f * kRelMargin));
+                cnt = warp_compact(s, cnt, __uint_as_float(__float_as_uint(kth) + 1u));
+                if (cnt > kCap - 32) {  // more near ties than there is room for: the k best so far are enough
+                    if (!TIES) return kCrowded;
+                    keep_nearest(pp, s, 0, cnt, k, qx, qy, qz, nullptr);
+                    cnt = k;
+                }
+            }
+        }
+    }
+    if (cnt < k) return ALB_ERR_INVALID;
+    // select_refined ranks the near ties on their float64 distances
+    int fail = 0;
+    select_refined<TIES>(pp, s, 0, cnt, k, qx, qy, qz, nullptr, fail);
+    return fail;
+}
+
+__device__ __noinline__ int crowded_brute(PackedPoints pp, uint32_t m, WarpSmem& s, int k, double qx, double qy, double qz) {
+    return brute_knn<true>(pp, m, s, k, qx, qy, qz);
+}
+
+__global__ void __launch_bounds__(kBruteWarps * 32, 8) k_knn_brute(const float* __restrict__ pts, uint32_t m,
+                                                                   const double* __restrict__ qs, uint64_t nq, int k,
+                                                                   int32_t* out_idx, double* out_dist) {
     __shared__ WarpSmem smem[kBruteWarps];
-    const int w = threadIdx.x >> 5, l = lane_id();
-    WarpSmem& s = smem[w];
+    WarpSmem& s = smem[threadIdx.x >> 5];
     const PackedPoints pp{pts};
-    for (uint64_t qi = (uint64_t)blockIdx.x * kBruteWarps + w; qi < nq; qi += (uint64_t)gridDim.x * kBruteWarps) {
+    const uint64_t q0 = (uint64_t)blockIdx.x * kBruteWarps + (threadIdx.x >> 5), step = (uint64_t)gridDim.x * kBruteWarps;
+    bool crowded = false;
+    for (uint64_t qi = q0; qi < nq; qi += step) {
         const double qx = qs[3 * qi], qy = qs[3 * qi + 1], qz = qs[3 * qi + 2];
-        const float fx = (float)qx, fy = (float)qy, fz = (float)qz;
-        const float lx = (float)(qx - (double)fx), ly = (float)(qy - (double)fy), lz = (float)(qz - (double)fz);
-        float thr = FLT_MAX;
-        int cnt = 0, clipped = 0;
-        constexpr int kAhead = 4;  // steps whose points are loaded together
-        for (uint32_t r0 = 0; r0 < m; r0 += 32 * kAhead) {
-            float4 p[kAhead];
-#pragma unroll
-            for (int i = 0; i < kAhead; ++i) {
-                const uint32_t r = r0 + i * 32 + l;
-                p[i] = r < m ? pp.at(r) : make_float4(0.f, 0.f, 0.f, 0.f);
-            }
-#pragma unroll
-            for (int i = 0; i < kAhead; ++i) {
-                const uint32_t r = r0 + i * 32 + l;
-                const float d = point_dist2(fx, fy, fz, lx, ly, lz, p[i]);
-                const bool take = r < m && d <= thr;
-                const unsigned b = __ballot_sync(0xffffffffu, take);
-                if (take) {
-                    const int pos = cnt + __popc(b & lanemask_lt());
-                    float hi, lo;
-                    point_dist2_df(fx, fy, fz, lx, ly, lz, p[i], hi, lo);
-                    s.ci[pos] = r;
-                    s.cd[pos] = hi;
-                    s.cl[pos] = frac16(hi, lo);
-                }
-                cnt += __popc(b);
-                __syncwarp();
-                if (cnt >= k && (thr == FLT_MAX || cnt > kCap - 32)) {
-                    // refined distances within one float32 ulp of the k-th can still rank
-                    const float kth = warp_kth32(s, 0, cnt, k);
-                    thr = fminf(thr, kth * (1.0f + 2.0f * kRelMargin));
-                    cnt = warp_compact(s, cnt, __uint_as_float(__float_as_uint(kth) + 1u));
-                    if (cnt > kCap - 32) {  // mass ties
-                        cnt = warp_compact(s, cnt, kth);
-                        clipped = 1;
-                    }
-                    if (cnt > kCap - 32) cnt = kCap - 32;
-                }
-            }
-        }
-        if (cnt < k) {
+        const int fail = brute_knn<false>(pp, m, s, k, qx, qy, qz);
+        if (!fail) {
+            write_sorted(pp, s, k, qx, qy, qz, nullptr, out_idx + qi * k, out_dist + qi * k);
+        } else {
+            crowded = crowded || fail == kCrowded;
             write_failed(k, out_idx + qi * k, out_dist + qi * k);
-            continue;
+            if (fail == kCrowded && lane_id() == 0) out_idx[qi * k] = kLeft;
+            __syncwarp();
         }
-        // select_refined ranks the near ties on their float64 distances
-        select_refined(pp, s, 0, cnt, k, qx, qy, qz, nullptr, clipped);
-        write_sorted(pp, s, k, qx, qy, qz, nullptr, out_idx + qi * k, out_dist + qi * k);
+    }
+    if (!crowded) return;
+    // the caller's stream may be under capture, so these queries have no launch of their own
+    for (uint64_t qi = q0; qi < nq; qi += step) {
+        int32_t first = 0;
+        if (lane_id() == 0) first = out_idx[qi * k];
+        if (__shfl_sync(0xffffffffu, first, 0) != kLeft) continue;
+        const double qx = qs[3 * qi], qy = qs[3 * qi + 1], qz = qs[3 * qi + 2];
+        if (crowded_brute(pp, m, s, k, qx, qy, qz)) write_failed(k, out_idx + qi * k, out_dist + qi * k);
+        else write_sorted(pp, s, k, qx, qy, qz, nullptr, out_idx + qi * k, out_dist + qi * k);
     }
 }
 
@@ -1998,12 +2200,48 @@ void launch_gather(const SceneDev& sc, const MapDev& map, const QueryDev& q, int
     if (launches) ++*launches;
 }
 
+// Blocks of the launches over marks: 32 queries to a warp's step, one wave at most.
+static unsigned crowded_blocks(uint64_t nq) {
+    const uint64_t want = (nq + 32 * kCrowdedWarps - 1) / (32 * kCrowdedWarps);
+    return (unsigned)std::min<uint64_t>(want, (uint64_t)sm_count() * 4);
+}
+
+template <int CHANNEL>
+static void launch_crowded_channel(const SceneDev& sc, const MapDev& map, const QueryDev& q, const Accum& acc, int* err,
+                                   cudaStream_t st) {
+    const uint64_t most = kClassMost / (uint64_t)sc.k;
+    for (uint64_t first = 0; first < q.n; first += most) {
+        const uint64_t end = std::min<uint64_t>(q.n, first + most);
+        k_gather_crowded<CHANNEL><<<crowded_blocks(end - first), kCrowdedWarps * 32, 0, st>>>(sc, map, q, acc, sc.k, err, first, end);
+        note_launch();
+        merge_classes(sc, acc, CHANNEL, true, st);
+    }
+}
+
+void launch_gather_crowded(const SceneDev& sc, const MapDev& map, const QueryDev& q, int channel, const Accum& accum,
+                           int* err, cudaStream_t st) {
+    Accum acc = accum;
+    acc.cls += (uint64_t)channel * acc.cls_step;
+    switch (channel) {
+        case ALB_BOTTOM_REFLECTION: launch_crowded_channel<ALB_BOTTOM_REFLECTION>(sc, map, q, acc, err, st); break;
+        case ALB_SCATTER: launch_crowded_channel<ALB_SCATTER>(sc, map, q, acc, err, st); break;
+        case ALB_SURFACE_REFLECTION: launch_crowded_channel<ALB_SURFACE_REFLECTION>(sc, map, q, acc, err, st); break;
+        default: launch_crowded_channel<ALB_SURFACE_TRANSMISSION_UP>(sc, map, q, acc, err, st); break;
+    }
+}
+
 void launch_knn(const MapDev& map, const double* queries, const uint32_t* perm, uint64_t nq, int k, int32_t* out_idx,
-                double* out_dist, int* err, cudaStream_t st) {
+                double* out_dist, int* err, uint32_t* crowded, cudaStream_t st) {
     if (nq == 0) return;
     const uint32_t chunk = query_chunk(nq, false);
     k_knn<<<gather_blocks((nq + chunk - 1) / chunk), kGatherWarps * 32, 0, st>>>(map, queries, perm, nq, chunk, k, out_idx,
-                                                                                  out_dist, err);
+                                                                                  out_dist, err, crowded);
+    note_launch();
+}
+
+void launch_knn_crowded(const MapDev& map, const double* queries, uint64_t nq, int k, int32_t* out_idx, double* out_dist,
+                        int* err, cudaStream_t st) {
+    k_knn_crowded<<<crowded_blocks(nq), kCrowdedWarps * 32, 0, st>>>(map, queries, nq, k, out_idx, out_dist, err);
     note_launch();
 }
 

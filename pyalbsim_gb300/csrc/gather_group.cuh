@@ -82,7 +82,7 @@ struct GroupSmem {
             uint64_t bt[kBand];
         };
     };
-    unsigned long long st[5];
+    unsigned long long st[4];
     int alone, streak;  // queries still to be searched alone, and the next such stretch
     // scratch words of the boundary band, once the one-query search has left its stack
     ALB_DEVICE uint32_t& tmp(int i) {

@@ -76,14 +76,14 @@ constexpr uint32_t kRadiusItems = 1u << 20;
 struct QueryDev {
     const float4* a;   // x_hi, y_hi, z_hi, energy
     const float4* b;   // dx, dy, dz, time
-    const float4* c;   // x_lo, y_lo, z_lo
+    float4* c;         // x_lo, y_lo, z_lo, and a bit for each channel whose gather left the query (0 before)
     bool lo_zero;      // every low part is zero (the float32 tracer's queries)
     const float4* s;   // adjoint path scores (a, b, g, albedo), nullable
     const uint32_t* perm;  // optional processing order
     uint64_t n;
     double* rk_out;    // optional per-query k-th neighbour distance
     unsigned long long* stats;    // optional [leaves, nodes, selects, queries] accumulators
-    unsigned long long* inexact;  // optional count of answers a buffer bound made inexact (mass ties)
+    uint32_t* crowded;  // a bit for each channel that has left queries
     uint32_t* ticket;  // work counter of the scatter gather
     unsigned long long* retries;  // optional count of searches redone because a first guess did not hold
     uint32_t* work;  // fixed radius: a counter and room for kRadiusItems work items from word 2 (nullable)
@@ -155,10 +155,15 @@ void launch_profile_logs(const SceneDev& sc, double* out, cudaStream_t st);
 // ---- gather (gather.cu)
 void launch_gather(const SceneDev& sc, const MapDev& map, const QueryDev& q, int channel, const Accum& acc,
                    int* err, int* launches, cudaStream_t st);
+// The queries that a channel's gather left.
+void launch_gather_crowded(const SceneDev& sc, const MapDev& map, const QueryDev& q, int channel, const Accum& acc,
+                           int* err, cudaStream_t st);
 void launch_fix_to_float(const unsigned long long* lo, const unsigned long long* hi, int64_t n, float* out, cudaStream_t st);
 void launch_fix_to_float(const unsigned long long* lo, const unsigned long long* hi, int64_t n, double* out, cudaStream_t st);
 void launch_knn(const MapDev& map, const double* queries, const uint32_t* perm, uint64_t nq, int k, int32_t* out_idx,
-                double* out_dist, int* err, cudaStream_t st);
+                double* out_dist, int* err, uint32_t* crowded, cudaStream_t st);
+void launch_knn_crowded(const MapDev& map, const double* queries, uint64_t nq, int k, int32_t* out_idx, double* out_dist,
+                        int* err, cudaStream_t st);
 void launch_knn_brute(const float* pts, uint32_t m, const double* queries, uint64_t nq, int k, int32_t* out_idx,
                       double* out_dist, cudaStream_t st);
 void pack_knn_points(const float* pts, uint64_t m, float4* rec, cudaStream_t st);

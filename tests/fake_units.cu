@@ -48,7 +48,9 @@ void launch_fix_to_float(const unsigned long long* lo, const unsigned long long*
 void launch_fix_to_float(const unsigned long long* lo, const unsigned long long* hi, int64_t n, double* out, cudaStream_t st) {
     fix_to_float(lo, hi, n, out, st);
 }
-void launch_knn(const MapDev&, const double*, const uint32_t*, uint64_t, int, int32_t*, double*, int*, cudaStream_t) {}
+void launch_knn(const MapDev&, const double*, const uint32_t*, uint64_t, int, int32_t*, double*, int*, uint32_t*, cudaStream_t) {}
+void launch_knn_crowded(const MapDev&, const double*, uint64_t, int, int32_t*, double*, int*, cudaStream_t) {}
+void launch_gather_crowded(const SceneDev&, const MapDev&, const QueryDev&, int, const Accum&, int*, cudaStream_t) {}
 void launch_knn_brute(const float*, uint32_t, const double*, uint64_t, int, int32_t*, double*, cudaStream_t) {}
 void pack_knn_points(const float*, uint64_t, float4*, cudaStream_t) {}
 void pack_knn_queries(const double*, uint64_t, float4*, cudaStream_t) {}
