@@ -298,7 +298,8 @@ int alb_batch_run(AlbBatchInstance* instances, uint64_t n, const AlbBatchOptions
  * by this library, [4 + 4c .. 7 + 4c] gather counters of channel c (leaves, nodes, selects,
  * queries), [24 + c] zero (once counted answers that a buffer made inexact: none is), [28] events and [29] photons of the last
  * forward trace, [30] neighbour searches of the last trace redone because their first,
- * guessed threshold did not hold. n entries are written (at most 32). */
+ * guessed threshold did not hold, [31] its gather queries whose near ties filled a search's buffers and
+ * that a launch of their own answered. n entries are written (at most 32). */
 int alb_stats(AlbCtx* ctx, int64_t* out, int n);
 
 /* Accumulated device time (ms, CUDA events on the context's stream) and call counts per

@@ -934,6 +934,7 @@ static QueryDev query_dev(AlbCtx* ctx, int g, bool lo_zero) {
     q.stats = ctx->d_stats + 4 + 4 * c;  // per channel: leaves, nodes, selects, queries
     q.crowded = (uint32_t*)ctx->d_err + 1;
     q.retries = ctx->d_stats + 30;
+    q.n_crowded = ctx->d_stats + 31;
     q.ticket = (uint32_t*)(ctx->ctl + 43 + c);
     return q;
 }
@@ -1046,7 +1047,7 @@ extern "C" int alb_trace(AlbCtx* ctx, int pass, uint64_t n, uint64_t seed, uint6
     }
     // slots 28/29 keep the last forward trace's events and photons across the backward trace
     CK(cudaMemsetAsync(ctx->d_stats, 0, 28 * 8, ctx->st));
-    CK(cudaMemsetAsync(ctx->d_stats + 30, 0, 8, ctx->st));
+    CK(cudaMemsetAsync(ctx->d_stats + 30, 0, 2 * 8, ctx->st));
     unsigned long long* const stats_bak = ctx->ctl + 41;
     if (pass == ALB_FORWARD) {
         ctx->maps_built = false;

@@ -86,6 +86,7 @@ struct QueryDev {
     uint32_t* crowded;  // a bit for each channel that has left queries
     uint32_t* ticket;  // work counter of the scatter gather
     unsigned long long* retries;  // optional count of searches redone because a first guess did not hold
+    unsigned long long* n_crowded;  // count of the left queries that were answered
     uint32_t* work;  // fixed radius: a counter and room for kRadiusItems work items from word 2 (nullable)
 };
 

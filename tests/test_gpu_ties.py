@@ -102,3 +102,32 @@ def test_gather_of_repeated_photons(gpu_available, copies, k, once, n_backward, 
     a, b = _waveform(k, copies, n_backward, precise), _waveform(once, 1, n_backward, precise)
     assert all(np.abs(w).sum() > 0 for w in b)
     np.testing.assert_allclose(a, b * (k // once), rtol=4 * np.finfo(np.float64).eps, atol=0)
+
+
+@pytest.mark.parametrize("divergence", [1e-12, 3e-8, 1e-6])
+def test_surface_gather_around_a_narrow_beam(gpu_available, divergence):
+    """A beam of hardly any width: every surface query has its neighbours, out of 100 000, within a few
+    units of double-float distance or at one point. The k-th distance is scipy's, and the same photons in one
+    call and in several give the same bits."""
+    from scipy.spatial import cKDTree
+
+    cfg = workloads.small()
+    cfg = dataclasses.replace(cfg, laser=dataclasses.replace(cfg.laser, divergence_angle=divergence))
+
+    def run(cuts):
+        with GpuEngine(cfg) as eng:
+            eng.keep_record_ids()
+            eng.forward(100_000, 5)
+            eng.build_maps()
+            for a, b in zip(cuts, cuts[1:]):
+                eng.backward(b - a, 5)
+            return (eng.waveform_array(f64=True), eng.ctx.stats()["crowded_queries"], eng.ctx.export_queries(2),
+                    eng.ctx.export_map(2)[0])
+
+    a, crowded, q, pts = run([0, 2_000])
+    b = run([0, 700, 2_000])[0]
+    assert (crowded > 1_000) == (divergence < 1e-7)
+    d = cKDTree(pts.astype(np.float64)).query(q["pos"], k=[cfg.photon_mapping_k])[0][:, 0]
+    np.testing.assert_allclose(q["rk"], d, rtol=4 * np.finfo(np.float64).eps, atol=0)
+    assert np.abs(a[2]).sum() > 0
+    np.testing.assert_array_equal(a, b)
