@@ -1559,8 +1559,10 @@ ALB_DEVICE void pack_neighbours(const MapDev& m, S& s, int k) {
 // The search of one query alone, out of line: the grouped kernel takes it for the first query of
 // a CTA, runs whose list does not fit, guesses that fail and near ties, 1-3% of the queries,
 // and its code and registers stay out of the hot loop. The k neighbours are left
-// in s.cp. bound < 0: it holds k points to take one from.
-template <class S>
+// in s.cp. bound < 0: it holds k points to take one from. REFINE for planes, as in k_gather: around a dense spot more
+// records lie within float32's margin of a far query's k-th distance than the buffer holds (the same times with and
+// without it on the large scene).
+template <bool REFINE, class S>
 __device__ __noinline__ bool cold_knn(const MapDev& m, S& s, int k, float fx, float fy, float fz, float lx, float ly,
                                       float lz, float bound, KnnResult& res) {
     if (bound < 0.f) {
@@ -1573,7 +1575,7 @@ __device__ __noinline__ bool cold_knn(const MapDev& m, S& s, int k, float fx, fl
         const float t = __uint_as_float(__reduce_max_sync(0xffffffffu, mx)) * (1.f + 1.f / 16384.f);
         bound = t < 1.0e37f ? t : FLT_MAX;
     }
-    if (!warp_knn<false, true>(m, s, k, 0.0, 0.0, 0.0, fx, fy, fz, lx, ly, lz, bound, m.b, res)) return false;
+    if (!warp_knn<REFINE, true>(m, s, k, 0.0, 0.0, 0.0, fx, fy, fz, lx, ly, lz, bound, m.b, res)) return false;
     // (of a crowded search k of its candidates: records all the same, for the next query's bound)
     if (!res.fail || res.fail == kCrowded) pack_neighbours(m, s, k);
     return true;
@@ -1750,7 +1752,7 @@ __global__ void __launch_bounds__(WARPS * 32, 1)
                                     : leaves == 0 && s.st[3] ? -1.f : FLT_MAX;
                 run.take = 0;
                 KnnResult r;
-                const bool enough = cold_knn(m, s, k, fx, fy, fz, lx, ly, lz, bound, r);
+                const bool enough = cold_knn<CHANNEL != ALB_SCATTER>(m, s, k, fx, fy, fz, lx, ly, lz, bound, r);
                 if (enough && r.fail == kCrowded) {
                     leave_crowded(q, src, CHANNEL);
                     continue;
