@@ -1,0 +1,51 @@
+"""Device functions of the library on arrays of their own (device_checks.cu, compiled here)."""
+
+import ctypes as C
+import os
+import subprocess
+
+import numpy as np
+import pytest
+
+from pyalbsim_gb300.build import ARCH, CSRC, FLAGS, INCLUDE, nvcc_path
+
+pytestmark = pytest.mark.gpu
+HERE = os.path.dirname(os.path.abspath(__file__))
+
+
+@pytest.fixture(scope="module")
+def dev(gpu_available, tmp_path_factory):
+    out = str(tmp_path_factory.mktemp("device") / "checks.so")
+    cmd = [nvcc_path(), *ARCH, *FLAGS, "-shared", "-I", INCLUDE, "-I", CSRC, "-o", out, os.path.join(HERE, "device_checks.cu")]
+    r = subprocess.run(cmd, capture_output=True, text=True)
+    assert r.returncode == 0, r.stderr
+    return C.CDLL(out)
+
+
+def _gpu(a):
+    import torch
+
+    return torch.from_numpy(np.ascontiguousarray(a)).cuda()
+
+
+def _p(t):
+    return C.c_void_p(t.data_ptr())
+
+
+@pytest.mark.parametrize("on", [0, 1])
+def test_word_cache_adds_to_the_words_it_is_given(dev, on):
+    """Cached and direct adds end in the words. Off, a key may wrap to any value (arrays of more than 2^32
+    words): nothing is cached, whatever the key, so nothing is flushed into another array's word."""
+    i = np.array([0, 5, 7, 5, 0, 3], np.uint64)
+    v = np.array([1, -2, 1 << 40, 30, -(1 << 33), 7], np.int64)
+    # off: keys 0 (of word 5 too), and the mark of an empty slot
+    base = np.zeros(6, np.uint32) if on else np.array([0, 2**32 - 5, 0, 2**32 - 5, 0, 2**32 - 4], np.uint32)
+    words, other = _gpu(np.zeros(8, np.int64)), _gpu(np.zeros(8, np.int64))
+    args = [_gpu(i.view(np.int64)), _gpu(base.view(np.int32)), _gpu(v)]
+    first, second = (words, other) if on else (other, other)
+    rc = dev.check_word_cache(_p(words), *[_p(a) for a in args], 6, on, _p(first), C.c_uint32(8 if on else 0), _p(second))
+    assert rc == 0
+    want = np.zeros(8, np.int64)
+    np.add.at(want, i.astype(np.int64), v)
+    np.testing.assert_array_equal(words.cpu().numpy(), want)
+    assert not other.cpu().numpy().any()
