@@ -290,8 +290,10 @@ ALB_DEVICE double norm3(double x, double y, double z) {
     return sqrt(__dadd_rn(__dadd_rn(__dmul_rn(x, x), __dmul_rn(y, y)), __dmul_rn(z, z)));
 }
 
-// Steps of size sy from y0 to lim, to a millionth (the callers correct the count with the exact
-// comparison): a float32 quotient costs two FP64 instructions where the float64 one costs a dozen.
+// Steps of size sy from y0 to lim, to 3.6e-7 of itself (two roundings to float32 and a division good to 2 ulp): a
+// float32 quotient costs two FP64 instructions where the float64 one costs a dozen. The callers correct the
+// count with the exact comparison; the one decision they take on the estimate alone, that it lies beyond the span,
+// has a margin of 2^-20 of the span.
 ALB_DEVICE double steps_to(double y0, double sy, double lim) {
     const float d = (float)(lim - y0), s = (float)sy;
     return fabsf(s) > 1.0e-30f && fabsf(d) > 1.0e-30f ? (double)__fdividef(d, s) : (lim - y0) / sy;
@@ -300,7 +302,7 @@ ALB_DEVICE double steps_to(double y0, double sy, double lim) {
 // Smallest n >= 1 (<= nmax + 1) with y0 + n * sy <= lim, for sy < 0 and y0 > lim.
 ALB_DEVICE int64_t first_at_or_below(double y0, double sy, double lim, int64_t nmax) {
     const double est = steps_to(y0, sy, lim);
-    if (!(est < (double)nmax + 8.0)) return nmax + 1;
+    if (!(est < fma((double)nmax, 1.0 + 9.5367431640625e-07, 8.0))) return nmax + 1;
     int64_t n = (int64_t)ceil(est);
     if (n < 1) n = 1;
     if (n > nmax + 1) n = nmax + 1;
@@ -315,7 +317,7 @@ ALB_DEVICE int64_t first_at_or_below(double y0, double sy, double lim, int64_t n
 // Smallest n >= 1 (<= nmax + 1) with y0 + n * sy > lim, for sy > 0 and y0 <= lim.
 ALB_DEVICE int64_t first_above(double y0, double sy, double lim, int64_t nmax) {
     const double est = steps_to(y0, sy, lim);
-    if (!(est < (double)nmax + 8.0)) return nmax + 1;
+    if (!(est < fma((double)nmax, 1.0 + 9.5367431640625e-07, 8.0))) return nmax + 1;
     int64_t n = (int64_t)floor(est) + 1;
     if (n < 1) n = 1;
     if (n > nmax + 1) n = nmax + 1;

@@ -1,6 +1,7 @@
 // Device functions of the library, called on arrays (test_gpu_device_functions.py).
 #include <cstdint>
 
+#include "tracer.cuh"
 #include "word_cache.cuh"
 
 using namespace alb;
@@ -21,5 +22,25 @@ extern "C" int check_word_cache(void* words, const void* i, const void* base, co
                                 uint32_t n_first, void* second) {
     k_word_cache<<<1, 32>>>((unsigned long long*)words, (const uint64_t*)i, (const uint32_t*)base, (const long long*)v, n, on,
                             (unsigned long long*)first, n_first, (unsigned long long*)second);
+    return (int)cudaDeviceSynchronize();
+}
+
+// Whether the step counts of the float64 tracer are the smallest n with y0 + n sy <= lim (down) or > lim (up), or
+// nmax + 1 where no n <= nmax is: bad[0] counts the others.
+__global__ void k_steps(const double* y0, const double* sy, const double* lim, int64_t n, int64_t nmax, unsigned long long* bad) {
+    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
+        const bool down = sy[i] < 0.0;
+        const int64_t m = down ? first_at_or_below(y0[i], sy[i], lim[i], nmax) : first_above(y0[i], sy[i], lim[i], nmax);
+        auto past = [&](int64_t k) {
+            const double y = fma((double)k, sy[i], y0[i]);
+            return down ? y <= lim[i] : y > lim[i];
+        };
+        const bool ok = m >= 1 && m <= nmax + 1 && (m == nmax + 1 || past(m)) && (m == 1 || !past(m - 1));
+        if (!ok) atomicAdd(bad, 1ull);
+    }
+}
+
+extern "C" int check_steps(const void* y0, const void* sy, const void* lim, int64_t n, int64_t nmax, void* bad) {
+    k_steps<<<512, 256>>>((const double*)y0, (const double*)sy, (const double*)lim, n, nmax, (unsigned long long*)bad);
     return (int)cudaDeviceSynchronize();
 }

@@ -49,3 +49,21 @@ def test_word_cache_adds_to_the_words_it_is_given(dev, on):
     np.add.at(want, i.astype(np.int64), v)
     np.testing.assert_array_equal(words.cpu().numpy(), want)
     assert not other.cpu().numpy().any()
+
+
+@pytest.mark.parametrize("nmax", [1, 7, 4_000, 420_000, 8_000_000, 30_000_000, 300_000_000])
+@pytest.mark.parametrize("down", [True, False])
+def test_steps_to_a_plane_are_the_first_past_it(dev, nmax, down):
+    """Crossings at the last steps of a span, the first after it and anywhere in it, with steps and heights of
+    every size: the count is decided by the exact comparison, however far the estimate is off."""
+    rng = np.random.default_rng(nmax)
+    n = 200_000
+    at = np.where(rng.random(n) < 0.7, nmax + rng.integers(-2, 4, n), np.floor(nmax * rng.random(n))).clip(0)
+    sy = np.exp(rng.uniform(np.log(1e-9), np.log(2.0), n)) * (-1.0 if down else 1.0)
+    y0 = rng.uniform(-40.0, 0.0, n)
+    lim = y0 + (at - rng.uniform(0.2, 0.8, n)) * sy
+    lim = np.where(at > 0, lim, np.nextafter(y0, y0 + sy))  # the start is on the near side of the plane
+    bad = _gpu(np.zeros(1, np.int64))
+    args = [_gpu(a) for a in (y0, sy, lim)]
+    assert dev.check_steps(*[_p(a) for a in args], C.c_int64(n), C.c_int64(nmax), _p(bad)) == 0
+    assert bad.item() == 0
