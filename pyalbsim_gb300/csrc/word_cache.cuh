@@ -24,13 +24,9 @@ ALB_DEVICE void word_add(NoCache&, bool, unsigned long long* words, uint64_t i, 
 template <int N>
 ALB_DEVICE void word_add(WordCache<N>& wc, bool on, unsigned long long* words, uint64_t i, uint32_t base, uint32_t hash,
                          long long v) {
-    if (!on) {
-        atomicAdd(words + i, (unsigned long long)v);
-        return;
-    }
     const uint32_t slot = hash % N, key = base + (uint32_t)i;
-    uint32_t t = wc.tag[slot];
-    if (t == 0xffffffffu) {
+    uint32_t t = on ? wc.tag[slot] : ~key;
+    if (on && t == 0xffffffffu) {
         t = atomicCAS(&wc.tag[slot], 0xffffffffu, key);
         if (t == 0xffffffffu) t = key;
     }
