@@ -189,3 +189,18 @@ def test_trim_memory_gives_a_device_s_idle_memory_back(lib, monkeypatch):
     assert (lib.fake_trims(0), lib.fake_trims(1)) == (0, 1)
     with pytest.raises(ValueError, match="no such device"):
         trim_memory(2)
+
+
+@pytest.mark.parametrize("records", [6.0, 40.0])
+def test_a_first_call_without_its_full_room_takes_less(lib, records):
+    """No memory for 96 scatter records a photon: the call starts with room for 8, and is traced again where the
+    scene makes more."""
+    _rates(lib, [1.0, records, 1.0, 1.0])
+    ctx = Context(lib, build_scene(workloads.small()))
+    n = 200_000
+    lib.fake_limit(0, lib.fake_used(0) + (400 << 20))  # 0.67 GB for 96 records a photon, 0.06 for 8, 0.28 for 40
+    ctx.trace(True, n)
+    assert [ctx.map_size(c) for c in range(4)] == [n, records * n, n, n]
+    assert lib.fake_traced() == (n if records < 8 else 2 * n)
+    ctx.close()
+    assert lib.fake_used(0) == 0 and not fake_cuda.violations(lib)
