@@ -1420,14 +1420,6 @@ __global__ void __launch_bounds__(kGatherWarps * 32, kGatherBlocksPerSM) k_gathe
     cache_flush(jc, nullptr, 0u, acc.jac_cls);
 }
 
-// x / b from r = the float32 nearest 1 / b: the quotient estimate corrected by its exact residual
-// (Markstein, "Computation of elementary functions on the IBM RISC System/6000 processor", IBM J.
-// Res. Dev. 34, 1990), the correctly rounded quotient the division operator gives.
-ALB_DEVICE float div_by(float x, float b, float r) {
-    const float q = x * r;
-    return fmaf(fmaf(-q, b, x), r, q);
-}
-
 // One query's k neighbours s.cp[0 .. k) into the waveform's class words (and Jacobian, heatmaps);
 // qy the query's float64 depth, rk the k-th distance.
 template <int CHANNEL, int MODE, class S, class J>

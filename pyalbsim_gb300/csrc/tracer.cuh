@@ -216,14 +216,6 @@ ALB_DEVICE int layer_of(const SceneDev& sc, double y) {
 // below the layer top (depth - float32 layer offset, water.py:306-308).
 // ----------------------------------------------------------------------------------------
 
-// x / b for float64 from r = the float64 nearest 1 / b: the quotient estimate corrected by its exact
-// residual (Markstein, IBM J. Res. Dev. 34, 1990), the correctly rounded quotient of the division
-// operator at a quarter of its FP64 instructions (two FP64 lanes per SM and cycle here).
-ALB_DEVICE double div64_by(double x, double b, double r) {
-    const double q = x * r;
-    return fma(fma(-q, b, x), r, q);
-}
-
 // Profile value at the fraction q = z / h of a layer: kind 1 is LinearParameter
 // (float32: t = f32(q), f32(start) + t * f32(end - start)), kind 2 ExponentialParameter
 // (float64, from the logarithm l0 of its start and the difference dl to its end's), kind 0 the

@@ -44,3 +44,17 @@ extern "C" int check_steps(const void* y0, const void* sy, const void* lim, int6
     k_steps<<<512, 256>>>((const double*)y0, (const double*)sy, (const double*)lim, n, nmax, (unsigned long long*)bad);
     return (int)cudaDeviceSynchronize();
 }
+
+// Quotients by a constant against the division operator: bad[0] counts float32 ones, bad[1] float64 ones.
+__global__ void k_quotients(const double* x, const double* b, int64_t n, unsigned long long* bad) {
+    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
+        const float xf = (float)x[i], bf = (float)b[i];
+        if (div_by(xf, bf, __fdiv_rn(1.0f, bf)) != __fdiv_rn(xf, bf)) atomicAdd(bad, 1ull);
+        if (div64_by(x[i], b[i], __drcp_rn(b[i])) != __ddiv_rn(x[i], b[i])) atomicAdd(bad + 1, 1ull);
+    }
+}
+
+extern "C" int check_quotients(const void* x, const void* b, int64_t n, void* bad) {
+    k_quotients<<<512, 256>>>((const double*)x, (const double*)b, n, (unsigned long long*)bad);
+    return (int)cudaDeviceSynchronize();
+}

@@ -67,3 +67,27 @@ def test_steps_to_a_plane_are_the_first_past_it(dev, nmax, down):
     args = [_gpu(a) for a in (y0, sy, lim)]
     assert dev.check_steps(*[_p(a) for a in args], C.c_int64(n), C.c_int64(nmax), _p(bad)) == 0
     assert bad.item() == 0
+
+
+@pytest.mark.parametrize("kind", ["random", "mantissas", "times", "angles", "heights"])
+def test_quotients_by_a_constant_are_the_division_operator_s(dev, kind):
+    """Random operands, mantissas next to powers of two (where a quotient's estimate is off the most), and the
+    operands in use: times over the sample step, angles over the bin width, depths over a layer's height."""
+    rng = np.random.default_rng(3)
+    n = 1 << 24
+    if kind == "random":
+        x, b = np.exp(rng.uniform(-30, 30, n)) * rng.choice([-1.0, 1.0], n), np.exp(rng.uniform(-30, 30, n))
+    elif kind == "mantissas":
+        near = lambda: (rng.choice([1.0, 2.0], n) + rng.choice([-1.0, 1.0], n)  # noqa: E731
+                        * rng.integers(0, 40, n) * rng.choice([2.0**-23, 2.0**-52], n)) * 2.0 ** rng.integers(-20, 20, n)
+        x, b = near(), near()
+    elif kind == "times":
+        x, b = rng.uniform(0.0, 1e6, n), rng.integers(1, 200, n).astype(np.float64)
+    elif kind == "angles":
+        x, b = rng.uniform(0.0, np.pi, n), np.full(n, np.pi / rng.integers(100, 20_000))
+    else:
+        x, b = rng.uniform(0.0, 60.0, n), rng.uniform(0.1, 60.0, n)
+    bad = _gpu(np.zeros(2, np.int64))
+    args = [_gpu(x), _gpu(b)]
+    assert dev.check_quotients(*[_p(a) for a in args], C.c_int64(n), _p(bad)) == 0
+    assert bad.tolist() == [0, 0]
