@@ -131,3 +131,29 @@ def test_surface_gather_around_a_narrow_beam(gpu_available, divergence):
     np.testing.assert_allclose(q["rk"], d, rtol=4 * np.finfo(np.float64).eps, atol=0)
     assert np.abs(a[2]).sum() > 0
     np.testing.assert_array_equal(a, b)
+
+
+@pytest.mark.parametrize("k", [1, 2, 4, 5, 8, 9, 16])
+@pytest.mark.parametrize("m", [16, 1_023, 1_024, 1_025, 4_096])
+def test_many_queries_of_few_neighbours(gpu_available, m, k):
+    """From 2^14 queries (k <= 4) or 2^16 (k <= 16) on, a lane answers a query; the same queries in smaller calls
+    are answered by warps. Random points, a lattice with many ties, coincident points, and queries without an
+    answer: the same indices and distances."""
+    rng = np.random.default_rng(m)
+    n = 1 << (14 if k <= 4 else 16)
+    third = m // 3
+    pts = rng.normal(size=(m, 3))
+    pts[:third] = np.round(pts[:third] * 2.0) / 2.0
+    pts[third : third + third // 2] = [1.0, 0.0, 0.0]
+    pts = np.ascontiguousarray(pts.astype(np.float32))
+    qs = rng.normal(size=(n, 3))
+    qs[::3] = np.round(qs[::3] * 4.0) / 4.0
+    qs[5, 1], qs[77, 0] = np.nan, np.inf
+    dist, idx = _noalloc(pts, qs, k)
+    for a in range(0, n, n // 8):
+        d, i = _noalloc(pts, np.ascontiguousarray(qs[a : a + n // 8]), k)
+        np.testing.assert_array_equal(dist[a : a + n // 8], d)
+        np.testing.assert_array_equal(idx[a : a + n // 8], i)
+    assert (idx[[5, 77]] == -1).all() and np.isnan(dist[[5, 77]]).all()
+    ok = np.setdiff1d(np.arange(0, n, 37), [5, 77])
+    _check(lambda p, q, kk: (dist[ok], idx[ok]), pts, qs[ok], k)
