@@ -302,8 +302,8 @@ int alb_batch_run(AlbBatchInstance* instances, uint64_t n, const AlbBatchOptions
  * that a launch of their own answered. n entries are written (at most 32). */
 int alb_stats(AlbCtx* ctx, int64_t* out, int n);
 
-/* Accumulated device time (ms, CUDA events on the context's stream) and call counts per
- * phase since the last reset: 0 forward trace, 1 map build, 2 backward trace,
+/* Accumulated device time (ms, CUDA events on the phase's stream; gathers of a small call run side
+ * by side, so phases can add up to more than the call) and call counts per phase since the last reset: 0 forward trace, 1 map build, 2 backward trace,
  * 3 query sort, 4..7 gather of channel 0..3. out_ms/out_calls hold ALB_PHASES entries;
  * gathers[4] (nullable) receives the number of queries gathered per channel.
  * reset != 0 clears the accumulators after reading. */

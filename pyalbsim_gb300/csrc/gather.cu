@@ -1253,7 +1253,7 @@ ALB_DEVICE void accumulate(const SceneDev& sc, const MapDev& m, const QueryDev& 
         }
         float w;
         if (CHANNEL == ALB_BOTTOM_REFLECTION || CHANNEL == ALB_SURFACE_TRANSMISSION_UP) w = wconst;
-                else w = ggx_weight(sc.ggx_a2, (float)sc.f0, -pb.x, -pb.y, -pb.z, vx, vy, vz);
+        else w = ggx_weight(sc.ggx_a2, (float)sc.f0, -pb.x, -pb.y, -pb.z, vx, vy, vz);
         const float c = ((Es * Ep) * norm) * w;
         const int bin = (int)((ts + pb.w) / (float)sc.mult) - (int)sc.gate_lo;
         if (bin >= 0 && bin < acc.nbins) {
@@ -1273,7 +1273,7 @@ ALB_DEVICE void accumulate(const SceneDev& sc, const MapDev& m, const QueryDev& 
             const float4 pb = m.b[idx];
             float w;
             if (CHANNEL == ALB_BOTTOM_REFLECTION || CHANNEL == ALB_SURFACE_TRANSMISSION_UP) w = wconst;
-                        else w = ggx_weight(sc.ggx_a2, (float)sc.f0, -pb.x, -pb.y, -pb.z, vx, vy, vz);
+            else w = ggx_weight(sc.ggx_a2, (float)sc.f0, -pb.x, -pb.y, -pb.z, vx, vy, vz);
             {
                 NoCache none;
                 heat_add(sc, m, acc, none, false, 0u, idx, ((Es * m.a[idx].w) * norm) * w);
@@ -1602,7 +1602,7 @@ __global__ void __launch_bounds__(WARPS * 32, 1)
             const uint32_t seg = t >> plan.chunk_bits;
             volatile unsigned long long* v = ring;
             if ((t & (chunks - 1u)) == 0u) v[(seg + 1) % kSegRing] = (unsigned long long)(seg + 1) << 32 | atomicAdd(plan.ticket, 1u);
-            // published 64 chunks ago; the bound only guards against a lost slot
+            // published a segment (16 to 64 chunks) ago; the bound only guards against a lost slot
             unsigned long long e = v[seg % kSegRing];
             for (int wait = 0; (uint32_t)(e >> 32) != seg && wait < (1 << 20); ++wait) e = v[seg % kSegRing];
             if ((uint32_t)(e >> 32) != seg) atomicCAS(err, 0, ALB_ERR_ITER_CAP);
@@ -2119,7 +2119,7 @@ static uint32_t query_chunk(uint64_t nq, bool radius) {
     return (uint32_t)std::min<uint64_t>(kQueryChunk, std::max<uint64_t>(fit, kQueryChunkMin));
 }
 
-// The class words that a gather of `channel` filled (waveform: the scatter gather only).
+// The class words that a gather of `channel` filled (waveform: gathers by runs and of crowded queries only).
 static void merge_classes(const SceneDev& sc, const Accum& acc, int channel, bool waveform, cudaStream_t st) {
     const uint32_t nb = (uint32_t)acc.nbins;
     const unsigned blocks = (nb + 255u) / 256u;

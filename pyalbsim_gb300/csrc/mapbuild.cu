@@ -1870,8 +1870,8 @@ struct FinishSmem {
     uint32_t slot[kRun];
 };
 
-// One 32-byte record (both halves) by a single load: two 16-byte loads of one record at different
-// times fetched its DRAM sectors twice (262 B of traffic per record instead of 147).
+// One 32-byte record (both halves) by a single load, half the load instructions of two 16-byte ones. The time is
+// DRAM's either way, 4.8 and 4.9 ms for 1.1e8 records: records are fetched at random, 262 B of traffic each.
 ALB_DEVICE void load_record(const float4* p, float4& a, float4& b) {
     asm volatile("ld.global.nc.v8.f32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
                  : "=f"(a.x), "=f"(a.y), "=f"(a.z), "=f"(a.w), "=f"(b.x), "=f"(b.y), "=f"(b.z), "=f"(b.w)
