@@ -1384,12 +1384,14 @@ __global__ void __launch_bounds__(kGatherWarps * 32, kGatherBlocksPerSM) k_gathe
                 failed = true;
                 break;
             }
-            if (r.fail == kCrowded) {
-                leave_crowded(q, (uint32_t)src, CHANNEL);
-                have_prev = false;
-                continue;
-            }
-            if (r.fail) {  // no valid neighbour set: report it and stop this warp's work
+            if (r.fail) {
+                if (r.fail == kCrowded) {
+                    leave_crowded(q, (uint32_t)src, CHANNEL);
+                    have_prev = false;
+                    if (l == 0) s.st[3] += 1;
+                    continue;
+                }
+                // no valid neighbour set: report it and stop this warp's work
                 if (l == 0) atomicCAS(err, 0, r.fail);
                 failed = true;
                 break;
@@ -1501,12 +1503,14 @@ ALB_DEVICE void pack_neighbours(const MapDev& m, S& s, int k) {
 // The search of one query alone, out of line: the grouped kernel takes it for the first query of
 // a CTA, runs whose list does not fit, guesses that fail and near ties, 1-3% of the queries,
 // and its code and registers stay out of the hot loop. The k neighbours are left
-// in s.cp. bound < 0: it holds k points to take one from. REFINE for planes, as in k_gather: around a dense spot more
-// records lie within float32's margin of a far query's k-th distance than the buffer holds (the same times with and
-// without it on the large scene).
-template <bool REFINE, class S>
+// in s.cp. bound < 0: it holds k points to take one from. For planes with double-float distances, as in k_gather: around a
+// dense spot more records lie within float32's margin of a far query's k-th distance than the buffer holds (the same
+// times with and without on the large scene). A crowded query is left here, with k of its candidates and an infinite
+// k-th distance: what the caller then adds for it is zero. A branch for it in the caller's loop cost the adjoint's
+// scatter gather 6% (12.6 -> 13.4 ms).
+template <int CHANNEL, class S>
 __device__ __noinline__ bool cold_knn(const MapDev& m, S& s, int k, float fx, float fy, float fz, float lx, float ly,
-                                      float lz, float bound, KnnResult& res) {
+                                      float lz, float bound, KnnResult& res, const QueryDev& q, uint32_t src) {
     if (bound < 0.f) {
         // k points lie within the farthest of them; the float32 screening error (below 2^-21) is far
         // inside the 2^-14 inflation
@@ -1517,9 +1521,14 @@ __device__ __noinline__ bool cold_knn(const MapDev& m, S& s, int k, float fx, fl
         const float t = __uint_as_float(__reduce_max_sync(0xffffffffu, mx)) * (1.f + 1.f / 16384.f);
         bound = t < 1.0e37f ? t : FLT_MAX;
     }
-    if (!warp_knn<REFINE, true>(m, s, k, 0.0, 0.0, 0.0, fx, fy, fz, lx, ly, lz, bound, m.b, res)) return false;
-    // (of a crowded search k of its candidates: records all the same, for the next query's bound)
-    if (!res.fail || res.fail == kCrowded) pack_neighbours(m, s, k);
+    if (!warp_knn<CHANNEL != ALB_SCATTER, true>(m, s, k, 0.0, 0.0, 0.0, fx, fy, fz, lx, ly, lz, bound, m.b, res)) return false;
+    if (res.fail == kCrowded) {
+        leave_crowded(q, src, CHANNEL);
+        res.fail = 0;
+        res.rk2 = -1.0;
+        res.rkf = __int_as_float(0x7f800000);
+    }
+    if (!res.fail) pack_neighbours(m, s, k);
     return true;
 }
 
@@ -1694,11 +1703,7 @@ __global__ void __launch_bounds__(WARPS * 32, 1)
                                     : leaves == 0 && s.st[3] ? -1.f : FLT_MAX;
                 run.take = 0;
                 KnnResult r;
-                const bool enough = cold_knn<CHANNEL != ALB_SCATTER>(m, s, k, fx, fy, fz, lx, ly, lz, bound, r);
-                if (enough && r.fail == kCrowded) {
-                    leave_crowded(q, src, CHANNEL);
-                    continue;
-                }
+                const bool enough = cold_knn<CHANNEL>(m, s, k, fx, fy, fz, lx, ly, lz, bound, r, q, src);
                 if (!enough || r.fail) {  // no valid neighbour set: report it and stop this warp's work
                     if (l == 0) atomicCAS(err, 0, enough ? r.fail : ALB_ERR_TOO_FEW);
                     failed = true;
@@ -1774,7 +1779,8 @@ __global__ void __launch_bounds__(kCrowdedWarps * 32) k_gather_crowded(const __g
             __syncwarp();
         }
     }
-    if (l < 4 && q.stats && s.st[3]) atomicAdd(q.stats + l, s.st[l]);
+    // (the gathers counted these queries when they left them)
+    if (l < 3 && q.stats && s.st[3]) atomicAdd(q.stats + l, s.st[l]);
     if (l == 0 && s.st[3]) atomicAdd(q.n_crowded, s.st[3]);
 }
 
