@@ -34,11 +34,11 @@ UNIT = "photons/s"
 ALG_BYTES_PER_GATHER = 16 + 100 * 32  # query record + k neighbour records (pos 12, dir 12, E 4, t 4)
 # DRAM bytes per scatter-map query measured by ncu on the same kernel (dram__bytes_read.sum +
 # dram__bytes_write.sum of one k_gather_runs<1, 0> launch / its queries; 1e6-photon case of this scene)
-DRAM_BYTES_PER_SCATTER_QUERY = 1015
+DRAM_BYTES_PER_SCATTER_QUERY = 999
 # Warp instructions per scatter-map query of the same capture (smsp__inst_executed.sum of one
 # k_gather_runs<1, 0> launch / its queries): the kernel is bound by instruction issue, so its issue
 # rate is reported beside the HBM convention
-INST_PER_SCATTER_QUERY = 2312
+INST_PER_SCATTER_QUERY = 2294
 
 
 def workload_config(name: str):
