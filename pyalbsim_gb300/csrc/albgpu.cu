@@ -1054,6 +1054,7 @@ extern "C" int alb_trace(AlbCtx* ctx, int pass, uint64_t n, uint64_t seed, uint6
         const size_t hb = ctx->sc.heatmap ? (size_t)ctx->sc.hm_bins * ctx->sc.hm_bins : 0;
         uint64_t before_call[ALB_CHANNELS];
         std::memcpy(before_call, ctx->h_rec_count, sizeof before_call);
+        bool saved = false;  // the radius heatmap as it was has been copied
         // photons [p0, p0 + pn) of the call
         auto part = [&](uint64_t p0, uint64_t pn) -> int {
             unsigned* const radius_bak = ctx->hm_radius_bak + (p0 ? hb : 0);
@@ -1061,6 +1062,7 @@ extern "C" int alb_trace(AlbCtx* ctx, int pass, uint64_t n, uint64_t seed, uint6
             std::memcpy(before, ctx->h_rec_count, sizeof before);
             CK(cudaMemcpyAsync(stats_bak, ctx->d_stats, 2 * 8, cudaMemcpyDeviceToDevice, ctx->st));
             if (hb) CK(cudaMemcpyAsync(radius_bak, ctx->hm_radius, hb * 4, cudaMemcpyDeviceToDevice, ctx->st));
+            saved = true;
             for (int attempt = 0; attempt < 3; ++attempt) {
                 for (int c = 0; c < ALB_CHANNELS; ++c) {
                     uint64_t est = (uint64_t)(ctx->rec_rate[c] * (double)pn * 1.03) + 4096;
@@ -1114,15 +1116,13 @@ extern "C" int alb_trace(AlbCtx* ctx, int pass, uint64_t n, uint64_t seed, uint6
             ctx->rec_rate[ALB_SCATTER] = kManyRecords;
         }
         int rc = pilot ? part(0, pilot) : ALB_OK;
-        if (!rc) {
-            rc = part(pilot, n - pilot);
-            if (rc && pilot) {
-                // the call as a whole leaves nothing: the pilot's records and crossings go too
-                std::memcpy(ctx->h_rec_count, before_call, sizeof before_call);
-                cudaMemcpyAsync(ctx->d_rec_count, before_call, sizeof before_call, cudaMemcpyHostToDevice, ctx->st);
-                if (hb) cudaMemcpyAsync(ctx->hm_radius, ctx->hm_radius_bak, hb * 4, cudaMemcpyDeviceToDevice, ctx->st);
-                cudaStreamSynchronize(ctx->st);
-            }
+        if (!rc) rc = part(pilot, n - pilot);
+        if (rc) {
+            // the call as a whole leaves nothing: no records (a pilot's included) and no crossings
+            std::memcpy(ctx->h_rec_count, before_call, sizeof before_call);
+            cudaMemcpyAsync(ctx->d_rec_count, before_call, sizeof before_call, cudaMemcpyHostToDevice, ctx->st);
+            if (hb && saved) cudaMemcpyAsync(ctx->hm_radius, ctx->hm_radius_bak, hb * 4, cudaMemcpyDeviceToDevice, ctx->st);
+            cudaStreamSynchronize(ctx->st);
         }
         ctx->ws.release(mark);
         return rc;

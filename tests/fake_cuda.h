@@ -10,4 +10,5 @@ void launched(cudaStream_t st);
 void traced(uint64_t photons);
 double record_rate(int channel);
 double query_rate(int kind);
+int trace_error();  // the code that the next trace leaves on the device (0: none), once
 }  // namespace fake

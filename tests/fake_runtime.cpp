@@ -30,7 +30,7 @@ struct State {
     double rec[4] = {1, 8, 1, 1}, query[3] = {1, 8, 1};
     int fail_record = 0;  // the n-th event record from now fails (0: none)
     uint64_t traced = 0;  // photons of every trace
-    int trace_ms = 0;
+    int trace_ms = 0, trace_error = 0;
     int trims[kDevices] = {0, 0};
     int violations = 0;
     std::string what;
@@ -72,6 +72,11 @@ void fake::traced(uint64_t photons) {
 }
 double fake::record_rate(int channel) { return g->rec[channel]; }
 double fake::query_rate(int kind) { return g->query[kind]; }
+int fake::trace_error() {
+    const int e = g->trace_error;
+    g->trace_error = 0;
+    return e;
+}
 
 namespace {
 
@@ -120,6 +125,7 @@ void fake_rates(const double* rec, const double* query) {
     memcpy(g->query, query, sizeof g->query);
 }
 void fake_trace_ms(int ms) { g->trace_ms = ms; }
+void fake_fail_trace(int code) { g->trace_error = code; }
 void fake_fail_record(int n) { g->fail_record = n; }
 int fake_violations(char* out, int n) {
     snprintf(out, n, "%s", g->what.c_str());

@@ -11,6 +11,7 @@ void launch_trace(const SceneDev&, const TraceOut& out, int pass, uint64_t n, ui
     fake::on_device(out.rec_count, "trace");
     fake::launched(st);
     fake::traced(n);  // takes the time that a test sets
+    if (const int e = fake::trace_error()) *out.err = e;
     if (pass == ALB_FORWARD && out.hm_radius) out.hm_radius[0] += (unsigned)n;
     if (pass == ALB_FORWARD)
         for (int c = 0; c < 4; ++c) out.rec_count[c] += (unsigned long long)(fake::record_rate(c) * (double)n);

@@ -89,6 +89,22 @@ def test_a_forward_call_out_of_memory_leaves_the_simulation_as_it_was(lib, first
     assert not fake_cuda.violations(lib)
 
 
+def test_a_forward_call_with_a_device_error_leaves_the_simulation_as_it_was(lib):
+    """A trace that hits its iteration cap, or a replay that runs out of variates, has appended records by then."""
+    ctx = Context(lib, build_scene(SimulationConfig()))
+    ctx.trace(True, 2_000)
+    sizes, radius = [ctx.map_size(c) for c in range(4)], ctx.heatmaps()[2]
+    lib.fake_fail_trace(-6)
+    with pytest.raises(RuntimeError, match="iteration cap|replay|device error"):
+        ctx.trace(True, 3_000)
+    assert [ctx.map_size(c) for c in range(4)] == sizes
+    np.testing.assert_array_equal(ctx.heatmaps()[2], radius)
+    ctx.trace(True, 3_000)
+    assert [ctx.map_size(c) - n for c, n in enumerate(sizes)] == [3_000, 24_000, 3_000, 3_000]
+    assert ctx.heatmaps()[2][0] - radius[0] == 3_000
+    ctx.close()
+
+
 @pytest.mark.parametrize("radius", [None, 0.5])
 def test_gathers_that_cannot_be_joined_are_waited_for(lib, radius):
     """The gathers of a small call run on streams of their own. Whichever event of the call cannot be
