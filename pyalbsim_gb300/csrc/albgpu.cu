@@ -1007,6 +1007,15 @@ static int gather_all(AlbCtx* ctx, const Accum& acc, bool lo_zero) {
     return rc;
 }
 
+// What a call takes of the workspace goes back when it returns, on an error too.
+struct ScratchScope {
+    AlbCtx* ctx;
+    size_t mark;
+    explicit ScratchScope(AlbCtx* c) : ctx(c), mark(c->ws.mark()) {}
+    ScratchScope(const ScratchScope&) = delete;
+    ~ScratchScope() { ctx->ws.release(mark); }
+};
+
 extern "C" int alb_trace(AlbCtx* ctx, int pass, uint64_t n, uint64_t seed, uint64_t first, const AlbReplay* rp) {
     if (!ctx) return ALB_ERR_INVALID;
     if (pass != ALB_FORWARD && pass != ALB_BACKWARD) return fail(ctx, ALB_ERR_INVALID, "pass must be 0 or 1");
@@ -1018,7 +1027,7 @@ extern "C" int alb_trace(AlbCtx* ctx, int pass, uint64_t n, uint64_t seed, uint6
     ctx->err.clear();
     // replay streams to the device
     AlbReplay drp{};
-    size_t mark = ctx->ws.mark();
+    const ScratchScope scratch(ctx);
     if (rp) {
         if (!rp->offsets || !rp->values || !rp->tau) return fail(ctx, ALB_ERR_INVALID, "incomplete replay");
         int64_t* o = (int64_t*)ctx->ws.take_bytes((n + 1) * 8);
@@ -1037,10 +1046,8 @@ extern "C" int alb_trace(AlbCtx* ctx, int pass, uint64_t n, uint64_t seed, uint6
         if (ctx->ex_cap < n) {
             drop(ctx->ex_pos, ctx->st); drop(ctx->ex_dir, ctx->st); drop(ctx->ex_f, ctx->st);
             ctx->ex_cap = 0;
-            if (!take(ctx->ex_pos, n * 24, ctx->st) || !take(ctx->ex_dir, n * 24, ctx->st) || !take(ctx->ex_f, n * 40, ctx->st)) {
-                ctx->ws.release(mark);
+            if (!take(ctx->ex_pos, n * 24, ctx->st) || !take(ctx->ex_dir, n * 24, ctx->st) || !take(ctx->ex_f, n * 40, ctx->st))
                 return fail(ctx, ALB_ERR_CUDA, "exit states: out of device memory");
-            }
             ctx->ex_cap = n;
         }
         ctx->ex_n = n;
@@ -1124,7 +1131,6 @@ extern "C" int alb_trace(AlbCtx* ctx, int pass, uint64_t n, uint64_t seed, uint6
             if (hb && saved) cudaMemcpyAsync(ctx->hm_radius, ctx->hm_radius_bak, hb * 4, cudaMemcpyDeviceToDevice, ctx->st);
             cudaStreamSynchronize(ctx->st);
         }
-        ctx->ws.release(mark);
         return rc;
     }
     // backward: trace -> queries -> gathers. Without per-photon exports the photons go in
@@ -1227,7 +1233,6 @@ extern "C" int alb_trace(AlbCtx* ctx, int pass, uint64_t n, uint64_t seed, uint6
         if (rc) return rc;
         if (n == 0) break;
     }
-    ctx->ws.release(mark);
     return ALB_OK;
 }
 

@@ -105,6 +105,26 @@ def test_a_forward_call_with_a_device_error_leaves_the_simulation_as_it_was(lib)
     ctx.close()
 
 
+def test_a_failed_replay_keeps_no_device_memory(lib):
+    """A replayed backward call on maps of too few records (an ordinary error: more photons are traced and the call
+    repeated) gives the uploaded variates back."""
+    _rates(lib, [0.01, 0.01, 0.01, 0.01])
+    ctx = Context(lib, build_scene(workloads.small()))
+    ctx.trace(True, 1_000)
+    ctx.build_maps()
+    replay = (np.zeros(11, np.int64), np.zeros(100_000), np.zeros(100_000, np.float32))
+    used = []
+    for _ in range(3):
+        with pytest.raises(IndexError, match="fewer than k"):
+            ctx.trace(False, 10, replay=replay)
+        used.append(lib.fake_used(0))
+    assert used[2] == used[0] < 1 << 30
+    with pytest.raises(ValueError, match="replay offsets"):
+        ctx.trace(False, 11, replay=replay)
+    ctx.close()
+    assert lib.fake_used(0) == 0
+
+
 @pytest.mark.parametrize("radius", [None, 0.5])
 def test_gathers_that_cannot_be_joined_are_waited_for(lib, radius):
     """The gathers of a small call run on streams of their own. Whichever event of the call cannot be
